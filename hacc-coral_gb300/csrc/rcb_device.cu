@@ -43,7 +43,6 @@ __device__ __forceinline__ int lsb_exp(float t) {
 
 constexpr int kChunk = 4096;        // elements per statistics / partition chunk
 constexpr int kChunkThreads = 256;  // threads per chunk (16 elements each)
-constexpr int kWalkStack = 256;     // DFS stack of the list walk
 constexpr int kNodeMax = 16384;     // largest node the one-block partition takes
 constexpr int kChainSteps = 32;     // chain steps before the one-block partition jumps pointers
 constexpr int kPlainSteps = 4;      // single chain steps before the chunk partition jumps runs
@@ -53,9 +52,9 @@ enum { C_NCHUNK = 0, C_NSPLIT = 1, C_NFALLBACK = 2, C_NLEAF = 3, C_NSEG = 4, C_N
        C_NTIGHT = 12, C_SEGOVF = 13, C_MAXCNT = 14, C_ERR = 15, C_BUCKET = 16, C_FILL = 48,
        C_SUBFB = 80, C_CHAINS = 81, C_COUNT = 82 };
 
-// Segments a leaf's walk can leave in its own region of the one-pass walk;
-// a leaf with more sends the build to the counting walk and a second pass.
-constexpr int kLocalSegs = 64;
+// Segments a leaf's walk can leave in its own region of the one-pass walk (8
+// bytes each); a leaf with more sends the build to a second, placing walk.
+constexpr int kLocalSegs = 256;
 
 __device__ __forceinline__ double warp_sum(double v) {
 #pragma unroll
@@ -2339,146 +2338,203 @@ __global__ void k_leaf_compact(const int64_t *leaf_at, const int64_t *pos_of, in
 }
 
 // ---------------------------------------------------------------------------
-// Interaction lists (calcInternodeForce, RCBForceTree.cxx:923-1144), one
-// thread per processed leaf; a counting pass and a writing pass.
+// Interaction lists (calcInternodeForce, RCBForceTree.cxx:923-1144), a warp
+// per processed leaf.
+//
+// The reference's walk is a depth-first search whose emissions must keep their
+// order.  One lane taking one node at a time is a chain of dependent node
+// loads (116-260 of them a leaf at leaf sizes 128-32), so the warp takes the
+// top 32 stack entries at once: every lane decides its node, and the results
+// go back in stack order -- an interaction in place as a finished entry, two
+// children in place of their parent -- while the finished entries ahead of
+// the first expanded one, whose place in the list is then known, leave the
+// stack for the list.  11-18 steps a leaf instead of 116-260.
 // ---------------------------------------------------------------------------
-// MODE 0: counts (segments and entries per leaf); 1: writes the segments at
-// seg_base / list_base; 2: counts and writes the first kLocalSegs segments
-// of each leaf into its own region (dst relative to the leaf's list),
-// flagging leaves with more in counters[C_SEGOVF].
+constexpr int kWalkWarps = 4;
+constexpr int kWalkCap = 640;      // stack entries a leaf; the window narrows as it
+constexpr int kWalkReserve = 256;  // fills, to one node at a time over the last 256
+
+// MODE 1: writes the segments at seg_base / list_base; 2: counts (segments and
+// entries per leaf) and writes the first kLocalSegs segments (start, count) of
+// each leaf into its own region, flagging leaves with more in
+// counters[C_SEGOVF].
 template <int MODE>
-__global__ void k_walk(const DNode *__restrict__ nodes, int32_t nnodes, const int32_t *leaf_ids,
-                       int64_t nleaves, TreeConfig cfg, int64_t n, int64_t *seg_cnt, int64_t *list_len,
-                       const int64_t *seg_base, const int64_t *list_base, SegDesc *segs,
-                       int32_t *err, int64_t *counters) {
-  constexpr bool WRITE = MODE == 1;
-  const int64_t li = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
-  if (li >= nleaves) return;
+__global__ void __launch_bounds__(32 * kWalkWarps)
+    k_walk(const DNode *__restrict__ nodes, int32_t nnodes, const int32_t *leaf_ids,
+           int64_t nleaves, TreeConfig cfg, int64_t n, int64_t *seg_cnt, int64_t *list_len,
+           const int64_t *seg_base, const int64_t *list_base, SegDesc *segs, int2 *local,
+           int32_t *err, int64_t *counters) {
+  static_assert(MODE == 1 || MODE == 2, "walk mode");
+  // entries: a node still to decide (x = node, y = 0, or -1 for a child of an
+  // ancestor of the leaf, which no distance test drops), or a finished segment
+  // (x = start, y = count > 0)
+  __shared__ int2 stack_[kWalkWarps][kWalkCap];
+  const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const unsigned full = 0xffffffffu, below = (1u << lane) - 1u;
+  const int64_t li = int64_t(blockIdx.x) * kWalkWarps + w;
+  if (li >= nleaves) return;  // whole warps
+  int2 *const st = stack_[w];
   const int32_t tl = leaf_ids[li];
   const DNode T = nodes[tl];
   const float fsr = cfg.fsrrmax;
   const float fsr2 = fmul_(fsr, fsr);
   const float tan_oa = cfg.tan_oa;
   const int k = cfg.tdpts;
-  int32_t stack[kWalkStack];
-  int sp = 0;
   int64_t nseg = 0, len = 0;
-  const int64_t sb = WRITE ? seg_base[li] : 0, lb = WRITE ? list_base[li] : 0;
-  auto emit = [&](int64_t start, int64_t count) {
-    if (count <= 0) return;
-    if (WRITE) segs[sb + nseg] = SegDesc{int32_t(start), int32_t(count), lb + len};
-    if (MODE == 2 && nseg < kLocalSegs)
-      segs[li * kLocalSegs + nseg] = SegDesc{int32_t(start), int32_t(count), len};
-    ++nseg;
-    len += count;
-  };
-  auto push = [&](int32_t v) {
-    if (sp < kWalkStack) stack[sp++] = v;
-    else atomicExch(err, 1);
-  };
-  auto close_to = [&](const DNode &C) {
-    for (int i = 0; i < 3; ++i) {
-      float dist = 0.f;
-      if (T.xmax[i] < C.xmin[i]) dist = fsub_(C.xmin[i], T.xmax[i]);
-      else if (T.xmin[i] > C.xmax[i]) dist = fsub_(T.xmin[i], C.xmax[i]);
-      if (dist > fsr) return false;
-    }
-    return true;
-  };
-  push(0);
-  int64_t pops = 0;
-  while (sp > 0) {
-    if (++pops > int64_t(nnodes) + 1) {  // a tree walk visits each node at most once
-      atomicExch(err, 3);
-      break;
-    }
-    const int32_t t = stack[--sp];
-    if (t < 0 || t >= nnodes) {
-      atomicExch(err, 3);
-      break;
-    }
-    const DNode Q = nodes[t];
-    if (Q.cl >= nnodes || Q.cr >= nnodes) {
-      atomicExch(err, 3);
-      break;
-    }
-    if (t != tl && Q.offset <= T.offset && T.offset + T.count <= Q.offset + Q.count) {
-      if (Q.cl != tl && Q.cl > 0 && nodes[Q.cl].count > 0) push(Q.cl);
-      if (Q.cr != tl && Q.cr > 0 && nodes[Q.cr].count > 0) push(Q.cr);
-      continue;
-    }
-    const float dx = fsub_(Q.xc[0], T.xc[0]), dy = fsub_(Q.xc[1], T.xc[1]),
-                dz = fsub_(Q.xc[2], T.xc[2]);
-    const float dist2 = norm2_(dx, dy, dz);
-    const float sx = fsub_(Q.xmax[0], Q.xmin[0]), sy = fsub_(Q.xmax[1], Q.xmin[1]),
-                sz = fsub_(Q.xmax[2], Q.xmin[2]);
-    const float l2 = smin_(fmul_(sx, sx), smin_(fmul_(sy, sy), fmul_(sz, sz)));
-    const float dtt2 = fmul_(fmul_(dist2, tan_oa), tan_oa);
-    bool big = l2 > dtt2;
-    for (int i = 0; i < 2 && !big; ++i)
-      for (int j = 0; j < 2 && !big; ++j) {
-        const float x1 = fsub_((i == 0 ? Q.xmin : Q.xmax)[0], T.xc[0]);
-        const float y1 = fsub_((j == 0 ? Q.xmin : Q.xmax)[1], T.xc[1]);
-        const float z1 = fsub_(Q.xmin[2], T.xc[2]);
-        const float x2 = fsub_((i == 0 ? Q.xmax : Q.xmin)[0], T.xc[0]);
-        const float y2 = fsub_((j == 0 ? Q.xmax : Q.xmin)[1], T.xc[1]);
-        const float z2 = fsub_(Q.xmax[2], T.xc[2]);
-        big = norm2_(fsub_(x1, x2), fsub_(y1, y2), fsub_(z1, z2)) > dtt2;
+  const int64_t sb = MODE == 1 ? seg_base[li] : 0, lb = MODE == 1 ? list_base[li] : 0;
+  // the lanes' segments (start, count), in lane order, where `on`
+  auto emit = [&](bool on, int32_t start, int32_t count) {
+    const unsigned m = __ballot_sync(full, on);
+    const int64_t q = nseg + __popc(m & below);
+    int incl = on ? count : 0;  // the segments of one step are disjoint: at most n entries
+    if (MODE == 1) {
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const int v = __shfl_up_sync(full, incl, o);
+        if (lane >= o) incl += v;
       }
-    if (!big) {
-      if (dist2 > fsr2) continue;
-      if (Q.count <= k) emit(Q.offset, Q.count);
-      else emit(n + int64_t(t) * k, k);
-      continue;
+      if (on) segs[sb + q] = SegDesc{start, count, lb + len + incl - count};
+      len += __shfl_sync(full, incl, 31);
+    } else {
+      if (on && q < kLocalSegs) local[li * kLocalSegs + q] = make_int2(start, count);
+      len += __reduce_add_sync(full, incl);
     }
-    if (Q.cr == 0 && Q.cl == 0) {
-      emit(Q.offset, Q.count);
-      continue;
+    nseg += __popc(m);
+  };
+  if (lane == 0) st[0] = make_int2(0, -1);
+  __syncwarp();
+  int sp = 1;
+  int64_t visited = 0;
+  while (sp > 0) {
+    const int width = min(min(32, sp), max(1, kWalkCap - kWalkReserve - sp));
+    int nout = 0;
+    int2 o0 = make_int2(0, 0), o1 = o0;  // this lane's results, in list order
+    bool expand = false, fresh = false, bad = false;
+    if (lane < width) {
+      const int2 e = st[sp - 1 - lane];
+      if (e.y > 0) {
+        nout = 1;
+        o0 = e;
+      } else {
+        const int32_t t = e.x;
+        fresh = true;
+        bad = t < 0 || t >= nnodes;
+        DNode Q{};
+        if (!bad) {
+          Q = nodes[t];
+          bad = Q.cl >= nnodes || Q.cr >= nnodes;
+        }
+        bool go = !bad && Q.count > 0;
+        const bool anc =
+            t != tl && Q.offset <= T.offset && T.offset + T.count <= Q.offset + Q.count;
+        if (go && !anc && e.y == 0) {
+          // per-axis gap between the target leaf's box and the node's
+          for (int i = 0; i < 3; ++i) {
+            float dist = 0.f;
+            if (T.xmax[i] < Q.xmin[i]) dist = fsub_(Q.xmin[i], T.xmax[i]);
+            else if (T.xmin[i] > Q.xmax[i]) dist = fsub_(T.xmin[i], Q.xmax[i]);
+            if (dist > fsr) go = false;
+          }
+        }
+        if (go) {
+          bool big = true;
+          float dist2 = 0.f;
+          if (!anc) {
+            const float dx = fsub_(Q.xc[0], T.xc[0]), dy = fsub_(Q.xc[1], T.xc[1]),
+                        dz = fsub_(Q.xc[2], T.xc[2]);
+            dist2 = norm2_(dx, dy, dz);
+            const float sx = fsub_(Q.xmax[0], Q.xmin[0]), sy = fsub_(Q.xmax[1], Q.xmin[1]),
+                        sz = fsub_(Q.xmax[2], Q.xmin[2]);
+            const float l2 = smin_(fmul_(sx, sx), smin_(fmul_(sy, sy), fmul_(sz, sz)));
+            const float dtt2 = fmul_(fmul_(dist2, tan_oa), tan_oa);
+            big = l2 > dtt2;
+            for (int i = 0; i < 2 && !big; ++i)
+              for (int j = 0; j < 2 && !big; ++j) {
+                const float x1 = fsub_((i == 0 ? Q.xmin : Q.xmax)[0], T.xc[0]);
+                const float y1 = fsub_((j == 0 ? Q.xmin : Q.xmax)[1], T.xc[1]);
+                const float z1 = fsub_(Q.xmin[2], T.xc[2]);
+                const float x2 = fsub_((i == 0 ? Q.xmax : Q.xmin)[0], T.xc[0]);
+                const float y2 = fsub_((j == 0 ? Q.xmax : Q.xmin)[1], T.xc[1]);
+                const float z2 = fsub_(Q.xmax[2], T.xc[2]);
+                big = norm2_(fsub_(x1, x2), fsub_(y1, y2), fsub_(z1, z2)) > dtt2;
+              }
+          }
+          if (anc || (big && (Q.cl != 0 || Q.cr != 0))) {
+            // the right child first; the leaf itself comes last of all
+            const int fl = anc ? -1 : 0;
+            if (Q.cr > 0 && !(anc && Q.cr == tl)) {
+              o0 = make_int2(Q.cr, fl);
+              nout = 1;
+            }
+            if (Q.cl > 0 && !(anc && Q.cl == tl)) {
+              (nout ? o1 : o0) = make_int2(Q.cl, fl);
+              ++nout;
+            }
+            expand = nout > 0;
+          } else if (big || dist2 <= fsr2) {
+            nout = 1;
+            o0 = big || Q.count <= k ? make_int2(Q.offset, Q.count)
+                                     : make_int2(int32_t(n + int64_t(t) * k), k);
+          }
+        }
+      }
     }
-    if (Q.cl > 0 && nodes[Q.cl].count > 0 && close_to(nodes[Q.cl])) push(Q.cl);
-    if (Q.cr > 0 && nodes[Q.cr].count > 0 && close_to(nodes[Q.cr])) push(Q.cr);
+    if (__any_sync(full, bad)) {
+      if (bad) atomicExch(err, 3);
+      break;
+    }
+    visited += __popc(__ballot_sync(full, fresh));
+    if (visited > int64_t(nnodes) + 1) {  // a tree walk visits each node at most once
+      if (lane == 0) atomicExch(err, 3);
+      break;
+    }
+    const unsigned ex = __ballot_sync(full, expand);
+    const int lead = ex ? __ffs(int(ex)) - 1 : width;
+    if (lead > 0) emit(lane < lead && nout > 0, o0.x, o0.y);
+    if (lane < lead) nout = 0;
+    const unsigned c1 = __ballot_sync(full, nout >= 1), c2 = __ballot_sync(full, nout == 2);
+    const int total = __popc(c1) + __popc(c2);
+    const int base = sp - width;
+    if (base + total > kWalkCap) {
+      if (lane == 0) atomicExch(err, 1);
+      break;
+    }
+    const int at = base + total - 1 - (__popc(c1 & below) + __popc(c2 & below));
+    __syncwarp();  // every lane has read its entry
+    if (nout >= 1) st[at] = o0;
+    if (nout == 2) st[at - 1] = o1;
+    sp = base + total;
+    __syncwarp();
   }
-  emit(T.offset, T.count);
-  if (!WRITE) {
+  emit(lane == 0, T.offset, T.count);
+  if (MODE == 2 && lane == 0) {
     seg_cnt[li] = nseg;
     list_len[li] = len;
-  }
-  if (MODE == 2 && nseg > kLocalSegs) atomicExch((unsigned long long *)&counters[C_SEGOVF], 1ull);
-}
-
-// The one-pass walk's per-leaf regions packed leaf after leaf, with each
-// segment's destination made absolute.
-__global__ void k_pack_segs(const SegDesc *__restrict__ local, const int64_t *seg_cnt,
-                            const int64_t *seg_base, const int64_t *list_base, int64_t nleaves,
-                            SegDesc *__restrict__ segs) {
-  const int lane = threadIdx.x & 31;
-  const int64_t warps = (int64_t(gridDim.x) * blockDim.x) >> 5;
-  for (int64_t li = (int64_t(blockIdx.x) * blockDim.x + threadIdx.x) >> 5; li < nleaves;
-       li += warps) {
-    const int64_t c = seg_cnt[li], sb = seg_base[li], lb = list_base[li];
-    for (int64_t q = lane; q < c; q += 32) {
-      SegDesc d = local[li * kLocalSegs + q];
-      d.dst += lb;
-      segs[sb + q] = d;
-    }
+    if (nseg > kLocalSegs) atomicExch((unsigned long long *)&counters[C_SEGOVF], 1ull);
   }
 }
 
 // Expands each leaf's segments into the index array at the leaf's list_base,
-// keeping only the entries within sqrt(cull2) of the leaf's box: the others
-// are farther than the cutoff from every particle of the leaf, so the
-// reference's mask gives them exactly 0.  Warp per leaf: the leaf's box as
-// centre and half-width (widened by 4 ulps of
-// the coordinates, as in the batched kernel), then its segments 32 entries at
-// a time, compacting the kept entries by ballot.
-__global__ void k_expand_pruned(const SegDesc *__restrict__ segs,
-                                const int64_t *__restrict__ seg_base,
-                                const int64_t *__restrict__ seg_cnt,
-                                const int64_t *__restrict__ list_base,
-                                const DNode *__restrict__ nodes,
-                                const int32_t *__restrict__ leaf_ids, int64_t nleaves,
-                                const float4 *__restrict__ table, float cull2,
-                                int32_t *__restrict__ idx, int64_t *__restrict__ kept) {
+// keeping only the entries within sqrt(cull2) of the leaf's box (cull2 <= 0:
+// every entry): the others are farther than the cutoff from every particle of
+// the leaf, so the reference's mask gives them exactly 0.  Warp per leaf: the
+// leaf's box as centre and half-width (widened by 4 ulps of the coordinates,
+// as in the batched kernel), then its segments 32 at a time as one run of
+// entries -- the segment of a lane's entry from the segment starts inside the
+// 32-entry window, so short segments leave no lane idle -- kU windows' loads
+// in flight, the kept entries compacted by ballot.  LOCAL: the segments come
+// from the one-pass walk's regions and are also packed leaf after leaf into
+// segs, with their place in the full lists.
+template <bool LOCAL>
+__global__ void __launch_bounds__(256)
+    k_expand_pruned(const int2 *__restrict__ local, SegDesc *__restrict__ segs,
+                    const int64_t *__restrict__ seg_base, const int64_t *__restrict__ seg_cnt,
+                    const int64_t *__restrict__ list_base, const DNode *__restrict__ nodes,
+                    const int32_t *__restrict__ leaf_ids, int64_t nleaves,
+                    const float4 *__restrict__ table, float cull2, int32_t *__restrict__ idx,
+                    int64_t *__restrict__ kept) {
+  constexpr int kU = 4;
+  const unsigned full = 0xffffffffu;
   const int lane = threadIdx.x & 31;
   const unsigned below = (1u << lane) - 1u;
   const int64_t warps = (int64_t(gridDim.x) * blockDim.x) >> 5;
@@ -2491,25 +2547,63 @@ __global__ void k_expand_pruned(const SegDesc *__restrict__ segs,
     const float hy = fmaf(fmaxf(fabsf(loy), fabsf(hiy)), 4.8e-7f, 0.5f * (hiy - loy));
     const float hz = fmaf(fmaxf(fabsf(loz), fabsf(hiz)), 4.8e-7f, 0.5f * (hiz - loz));
     const float cx = 0.5f * (lox + hix), cy = 0.5f * (loy + hiy), cz = 0.5f * (loz + hiz);
-    int32_t *out = idx + list_base[li];
-    int64_t nk = 0;
-    const int64_t s0 = seg_base[li], s1 = s0 + seg_cnt[li];
-    for (int64_t q = s0; q < s1; ++q) {
-      const SegDesc S = segs[q];
-      for (int k0 = 0; k0 < S.count; k0 += 32) {
-        const int k = k0 + lane;
-        bool keep = false;
-        if (k < S.count) {
-          const float4 J = table[S.start + k];
-          const float dx = fmaxf(fabsf(J.x - cx) - hx, 0.f);
-          const float dy = fmaxf(fabsf(J.y - cy) - hy, 0.f);
-          const float dz = fmaxf(fabsf(J.z - cz) - hz, 0.f);
-          keep = fmaf(dx, dx, fmaf(dy, dy, dz * dz)) < cull2;
+    const int64_t lbase = list_base[li], sbase = seg_base[li];
+    int32_t *out = idx + lbase;
+    int64_t nk = 0, done = 0;  // entries kept, entries before this batch of segments
+    const int nsegs = int(seg_cnt[li]);
+    for (int q0 = 0; q0 < nsegs; q0 += 32) {
+      const bool on = q0 + lane < nsegs;
+      int start = 0, count = 0;
+      if (on) {
+        if (LOCAL) {
+          const int2 S = local[li * kLocalSegs + q0 + lane];
+          start = S.x;
+          count = S.y;
+        } else {
+          const SegDesc S = segs[sbase + q0 + lane];
+          start = S.start;
+          count = S.count;
         }
-        const unsigned m = __ballot_sync(0xffffffffu, keep);
-        if (keep) out[nk + __popc(m & below)] = S.start + k;
-        nk += __popc(m);
       }
+      int incl = count;
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const int v = __shfl_up_sync(full, incl, o);
+        if (lane >= o) incl += v;
+      }
+      const int pre = incl - count;
+      const int total = __shfl_sync(full, incl, 31);
+      if (LOCAL && on) segs[sbase + q0 + lane] = SegDesc{start, count, lbase + done + pre};
+      const int shift = start - pre;  // table index of entry e of this segment: shift + e
+      for (int b0 = 0; b0 < total; b0 += 32 * kU) {
+        float4 J[kU];
+        int32_t at[kU];
+#pragma unroll
+        for (int u = 0; u < kU; ++u) {
+          const int b = b0 + 32 * u;
+          // segments starting before the window, and where others start in it
+          const int before = __popc(__ballot_sync(full, on && pre < b));
+          const unsigned bit = on && pre >= b && pre < b + 32 ? 1u << (pre - b) : 0u;
+          const unsigned starts = __reduce_or_sync(full, bit);
+          const int s = before - 1 + __popc(starts & (below | (1u << lane)));
+          at[u] = __shfl_sync(full, shift, max(0, min(31, s))) + b + lane;
+          if (b + lane < total) J[u] = table[at[u]];
+        }
+#pragma unroll
+        for (int u = 0; u < kU; ++u) {
+          bool keep = b0 + 32 * u + lane < total;
+          if (keep && cull2 > 0.f) {
+            const float dx = fmaxf(fabsf(J[u].x - cx) - hx, 0.f);
+            const float dy = fmaxf(fabsf(J[u].y - cy) - hy, 0.f);
+            const float dz = fmaxf(fabsf(J[u].z - cz) - hz, 0.f);
+            keep = fmaf(dx, dx, fmaf(dy, dy, dz * dz)) < cull2;
+          }
+          const unsigned m = __ballot_sync(full, keep);
+          if (keep) out[nk + __popc(m & below)] = at[u];
+          nk += __popc(m);
+        }
+      }
+      done += total;
     }
     if (lane == 0) kept[li] = nk;
   }
@@ -3591,10 +3685,11 @@ cudaError_t DeviceTree::build(const TreeConfig &cfg, int64_t n, const float4 *po
   // build to a second, placing walk)
   DT_CHECK(grow(segs_local_, cap_segl_, nlw * kLocalSegs, s));
   DT_CHECK(cudaMemsetAsync(counters_ + C_SEGOVF, 0, sizeof(int64_t), s));
+  const unsigned gW = unsigned((nleaves + kWalkWarps - 1) / kWalkWarps);
   if (nleaves > 0) {
-    k_walk<2><<<unsigned((nleaves + 127) / 128), 128, 0, s>>>(
-        nodes_, nnodes, leaf_ids_, nleaves, cfg, n, seg_cnt, list_len, nullptr, nullptr,
-        segs_local_, walk_err_, counters_);
+    k_walk<2><<<gW, 32 * kWalkWarps, 0, s>>>(nodes_, nnodes, leaf_ids_, nleaves, cfg, n, seg_cnt,
+                                             list_len, nullptr, nullptr, nullptr, segs_local_,
+                                             walk_err_, counters_);
     ++info_.launches;
     // the groups after the walk's blocks, which then have their SMs first
     DT_CHECK(launch_groups(nleaves, group_, aux_));
@@ -3622,28 +3717,23 @@ cudaError_t DeviceTree::build(const TreeConfig &cfg, int64_t n, const float4 *po
   DT_CHECK(grow(idx_list_, cap_idx_, size_t(std::max<int64_t>(nent, 1)), s));
   DT_CHECK(grow(leafdesc_, cap_ld_, nlw, s));
   if (nleaves > 0) {
+    int64_t *kept = node_tmp_ + 4 * nlw;
+    const unsigned blocks =
+        unsigned(std::min<int64_t>((nleaves + 7) / 8, int64_t(sm_count()) * 64));
     if (h_counters_[C_SEGOVF]) {
-      k_walk<1><<<unsigned((nleaves + 127) / 128), 128, 0, s>>>(
-          nodes_, nnodes, leaf_ids_, nleaves, cfg, n, nullptr, nullptr, seg_base, list_base, segs_,
-          walk_err_, counters_);
+      k_walk<1><<<gW, 32 * kWalkWarps, 0, s>>>(nodes_, nnodes, leaf_ids_, nleaves, cfg, n, nullptr,
+                                               nullptr, seg_base, list_base, segs_, nullptr,
+                                               walk_err_, counters_);
       ++info_.launches;
+      k_expand_pruned<false><<<blocks, 256, 0, s>>>(nullptr, segs_, seg_base, seg_cnt, list_base,
+                                                    nodes_, leaf_ids_, nleaves, table_, cfg.prune2,
+                                                    idx_list_, kept);
     } else {
-      k_pack_segs<<<unsigned(std::min<int64_t>((nleaves + 7) / 8, int64_t(sm_count()) * 64)), 256, 0, s>>>(
-          segs_local_, seg_cnt, seg_base, list_base, nleaves, segs_);
-      ++info_.launches;
+      k_expand_pruned<true><<<blocks, 256, 0, s>>>(segs_local_, segs_, seg_base, seg_cnt, list_base,
+                                                   nodes_, leaf_ids_, nleaves, table_, cfg.prune2,
+                                                   idx_list_, kept);
     }
-    int64_t *kept = nullptr;
-    if (cfg.prune2 > 0.0f) {
-      kept = node_tmp_ + 4 * nlw;
-      int64_t blocks = std::min<int64_t>((nleaves + 7) / 8, int64_t(sm_count()) * 64);
-      k_expand_pruned<<<unsigned(blocks), 256, 0, s>>>(segs_, seg_base, seg_cnt, list_base, nodes_,
-                                                       leaf_ids_, nleaves, table_, cfg.prune2,
-                                                       idx_list_, kept);
-      ++info_.launches;
-    } else {
-      DT_CHECK(launch_expand_segments(segs_, nseg, idx_list_, s));
-      info_.launches += nseg > 0;
-    }
+    ++info_.launches;
     k_leaf_desc<<<unsigned((nleaves + 127) / 128), 128, 0, s>>>(
         nodes_, leaf_ids_, nleaves, list_len, kept, list_base, leafdesc_, counters_);
     ++info_.launches;

@@ -163,7 +163,7 @@ class DeviceTree {
   SegDesc *segs_ = nullptr;
   size_t cap_seg_ = 0;
   bool node_attr_ = false;         // k_part_node's shared-memory limit raised
-  SegDesc *segs_local_ = nullptr;  // the one-pass walk's per-leaf regions
+  int2 *segs_local_ = nullptr;     // the one-pass walk's per-leaf regions (start, count)
   size_t cap_segl_ = 0;
   int32_t *idx_list_ = nullptr;
   size_t cap_idx_ = 0;
