@@ -45,10 +45,6 @@ int blocks_for(int64_t n) {
   return int(b < cap ? (b > 0 ? b : 1) : cap);
 }
 
-template <typename T> struct Cplx;
-template <> struct Cplx<double> { using type = double2; };
-template <> struct Cplx<float> { using type = float2; };
-
 // Alive-block index of local cell c (one axis), or -1 when the reference's
 // deposit would land outside the alive block (dropped by
 // fft_copy_arr_forward).
@@ -137,28 +133,107 @@ __global__ void k_green(int ng, int nh, const double *__restrict__ filter,
   }
 }
 
-// SolverBase::kspace_solve_gradient (src/dfft/solver.hpp:506-547) for the
-// three axes at once: grad_a = I * (-g(k_a)) * green * rho_k, i.e.
-// (t * Im rho, -t * Re rho) with t = g(k_a) * green.
-template <typename T>
+// Double precision: the potential's spectrum, green * rho_k, in place.
 __global__ void __launch_bounds__(kThreads)
-    k_spectra(int ng, int nh, const typename Cplx<T>::type *__restrict__ rho,
-              const T *__restrict__ green, const T *__restrict__ g,
-              typename Cplx<T>::type *__restrict__ out) {
-  using C = typename Cplx<T>::type;
+    k_potential(int64_t m, double2 *__restrict__ rho, const double *__restrict__ green) {
+  for (int64_t i = blockIdx.x * int64_t(blockDim.x) + threadIdx.x; i < m;
+       i += int64_t(gridDim.x) * blockDim.x) {
+    const double G = green[i];
+    double2 r = rho[i];
+    r.x *= G;
+    r.y *= G;
+    rho[i] = r;
+  }
+}
+
+// The solver's gradient factor g(k) = 4/3 sin k - 1/6 sin 2k is the spectrum
+// of the 4th-order central difference, i g(k) <-> D f = 2/3 (f(+1) - f(-1)) -
+// 1/12 (f(+2) - f(-2)) on the periodic grid (0 on the planes k = 0 and ng/2,
+// as the half-spectrum solve has it), so the three gradient fields
+// -D_a potential need one inverse transform, not three.  The double-precision
+// transforms are bound by the FP64 pipe (0.93 of the 1.07 ms of a 128^3 kick
+// were one forward and three inverse transforms; 0.68 ms now); the differences
+// read the potential from L2.  The potential's rounding, about 1e-16 of it, is some
+// ng / 2 pi times larger beside the gradient's than before: below 1e-13 at the
+// largest grid, with the fields rounded to float (6e-8).  Single precision has
+// no such room and keeps the three spectra.
+// A thread per (y, z) column marches kGradSpan cells along x with its five
+// x values in registers; the y and z neighbours come through L1.
+constexpr int kGradSpan = 16;
+constexpr double kD1 = 2.0 / 3.0, kD2 = -1.0 / 12.0;
+
+__device__ __forceinline__ int wrap(int i, int ng) { return i < 0 ? i + ng : (i >= ng ? i - ng : i); }
+
+__global__ void __launch_bounds__(256)
+    k_gradient(int ng, const double *__restrict__ phi, float4 *__restrict__ out) {
+  const int z = int(blockIdx.x) * 32 + int(threadIdx.x), y = int(blockIdx.y) * 8 + int(threadIdx.y);
+  if (z >= ng || y >= ng) return;
+  const int x0 = int(blockIdx.z) * kGradSpan, x1 = min(ng, x0 + kGradSpan);
+  const int64_t plane = int64_t(ng) * ng;
+  const int64_t row = int64_t(y) * ng;
+  const int64_t yp1 = int64_t(wrap(y + 1, ng)) * ng, ym1 = int64_t(wrap(y - 1, ng)) * ng;
+  const int64_t yp2 = int64_t(wrap(y + 2, ng)) * ng, ym2 = int64_t(wrap(y - 2, ng)) * ng;
+  const int zp1 = wrap(z + 1, ng), zm1 = wrap(z - 1, ng), zp2 = wrap(z + 2, ng), zm2 = wrap(z - 2, ng);
+  auto at = [&](int x) { return phi[int64_t(wrap(x, ng)) * plane + row + z]; };
+  double a = at(x0 - 2), b = at(x0 - 1), c = at(x0), d = at(x0 + 1);
+  for (int x = x0; x < x1; ++x) {
+    const double e = at(x + 2);
+    const double *p = phi + int64_t(x) * plane;
+    const double gx = kD1 * (d - b) + kD2 * (e - a);
+    const double gy = kD1 * (p[yp1 + z] - p[ym1 + z]) + kD2 * (p[yp2 + z] - p[ym2 + z]);
+    const double gz = kD1 * (p[row + zp1] - p[row + zm1]) + kD2 * (p[row + zp2] - p[row + zm2]);
+    out[int64_t(x) * plane + row + z] = make_float4(float(-gx), float(-gy), float(-gz), 0.0f);
+    a = b;
+    b = c;
+    c = d;
+    d = e;
+  }
+}
+
+// The transpose for the adjoint: sum_a D_a adj_a of the deposited cotangents
+// (planar), in double: one forward transform instead of three.
+__global__ void __launch_bounds__(kThreads)
+    k_divergence(int ng, const float *__restrict__ adj, double *__restrict__ out) {
+  const int64_t m = int64_t(ng) * ng * ng;
+  const float *const ax = adj, *const ay = adj + m, *const az = adj + 2 * m;
+  for (int64_t i = blockIdx.x * int64_t(blockDim.x) + threadIdx.x; i < m;
+       i += int64_t(gridDim.x) * blockDim.x) {
+    const int z = int(i % ng);
+    const int64_t t = i / ng;
+    const int y = int(t % ng), x = int(t / ng);
+    auto cell = [&](int u, int v, int w) {
+      return (int64_t(wrap(u, ng)) * ng + wrap(v, ng)) * ng + wrap(w, ng);
+    };
+    double s = kD1 * (double(ax[cell(x + 1, y, z)]) - double(ax[cell(x - 1, y, z)])) +
+               kD2 * (double(ax[cell(x + 2, y, z)]) - double(ax[cell(x - 2, y, z)]));
+    s += kD1 * (double(ay[cell(x, y + 1, z)]) - double(ay[cell(x, y - 1, z)])) +
+         kD2 * (double(ay[cell(x, y + 2, z)]) - double(ay[cell(x, y - 2, z)]));
+    s += kD1 * (double(az[cell(x, y, z + 1)]) - double(az[cell(x, y, z - 1)])) +
+         kD2 * (double(az[cell(x, y, z + 2)]) - double(az[cell(x, y, z - 2)]));
+    out[i] = s;
+  }
+}
+
+// Single precision: SolverBase::kspace_solve_gradient
+// (src/dfft/solver.hpp:506-547) for the three axes at once:
+// grad_a = I * (-g(k_a)) * green * rho_k, i.e. (t * Im rho, -t * Re rho) with
+// t = g(k_a) * green.
+__global__ void __launch_bounds__(kThreads)
+    k_spectra(int ng, int nh, const float2 *__restrict__ rho, const float *__restrict__ green,
+              const float *__restrict__ g, float2 *__restrict__ out) {
   const int64_t m = int64_t(ng) * ng * nh;
   for (int64_t i = blockIdx.x * int64_t(blockDim.x) + threadIdx.x; i < m;
        i += int64_t(gridDim.x) * blockDim.x) {
     const int kz = int(i % nh);
     const int64_t t = i / nh;
     const int ky = int(t % ng), kx = int(t / ng);
-    const T G = green[i];
-    const C r = rho[i];
+    const float G = green[i];
+    const float2 r = rho[i];
     const int k[3] = {kx, ky, kz};
 #pragma unroll
     for (int a = 0; a < 3; ++a) {
-      const T s = g[k[a]] * G;
-      C o;
+      const float s = g[k[a]] * G;
+      float2 o;
       o.x = s * r.y;
       o.y = -(s * r.x);
       out[a * m + i] = o;
@@ -167,12 +242,11 @@ __global__ void __launch_bounds__(kThreads)
 }
 
 // fft_copy_arr_backward (src/simulation/mc3.cxx:228-245) of the three
-// components: float(real part) into one float4 per cell.
-template <typename T>
-__global__ void k_pack(int64_t m, const T *__restrict__ g, float4 *__restrict__ out) {
+// components into one float4 per cell.
+__global__ void k_pack(int64_t m, const float *__restrict__ g, float4 *__restrict__ out) {
   for (int64_t i = blockIdx.x * int64_t(blockDim.x) + threadIdx.x; i < m;
        i += int64_t(gridDim.x) * blockDim.x)
-    out[i] = make_float4(float(g[i]), float(g[m + i]), float(g[2 * m + i]), 0.0f);
+    out[i] = make_float4(g[i], g[m + i], g[2 * m + i], 0.0f);
 }
 
 // Particles::inverse_cic (src/cpu/Particles.cxx:647-714) for the three
@@ -248,7 +322,10 @@ __device__ __forceinline__ bool cic_of(float xx, float yy, float zz, int nglt, C
 }
 
 // Transpose of the interpolation for the three cotangent components:
-// adj_a[image(c)] += W(x - c) vbar_a.
+// adj_a[image(c)] += W(x - c) vbar_a.  Planar fields: particles come sorted by
+// cell, so a warp's atomics on one corner fall on consecutive words (one
+// 16-byte vector reduction per corner instead, on float4 cells, was no faster:
+// the bytes that reach L2's atomic units are the bound).
 __global__ void __launch_bounds__(kThreads)
     k_adj_deposit(int64_t n, const float *__restrict__ x, const float *__restrict__ y,
                   const float *__restrict__ z, const float *__restrict__ vbx,
@@ -289,22 +366,12 @@ __global__ void __launch_bounds__(kThreads)
   }
 }
 
-template <typename T>
-__global__ void k_to_real3(int64_t m3, const float *__restrict__ a, T *__restrict__ b) {
-  for (int64_t i = blockIdx.x * int64_t(blockDim.x) + threadIdx.x; i < m3;
-       i += int64_t(gridDim.x) * blockDim.x)
-    b[i] = T(a[i]);
-}
-
-// The transposed solve, summed over the three components:
+// Single precision: the transposed solve, summed over the three components:
 // phibar_k = sum_a conj(S_a) adj_a,k with S_a = -I g(k_a) green, i.e.
 // green * sum_a I g(k_a) adj_a,k.
-template <typename T>
 __global__ void __launch_bounds__(kThreads)
-    k_adj_spectra(int ng, int nh, const typename Cplx<T>::type *__restrict__ a3,
-                  const T *__restrict__ green, const T *__restrict__ g,
-                  typename Cplx<T>::type *__restrict__ out) {
-  using C = typename Cplx<T>::type;
+    k_adj_spectra(int ng, int nh, const float2 *__restrict__ a3, const float *__restrict__ green,
+                  const float *__restrict__ g, float2 *__restrict__ out) {
   const int64_t m = int64_t(ng) * ng * nh;
   for (int64_t i = blockIdx.x * int64_t(blockDim.x) + threadIdx.x; i < m;
        i += int64_t(gridDim.x) * blockDim.x) {
@@ -312,16 +379,16 @@ __global__ void __launch_bounds__(kThreads)
     const int64_t t = i / nh;
     const int ky = int(t % ng), kx = int(t / ng);
     const int k[3] = {kx, ky, kz};
-    T re = T(0), im = T(0);
+    float re = 0.0f, im = 0.0f;
 #pragma unroll
     for (int a = 0; a < 3; ++a) {
-      const C v = a3[a * m + i];
-      const T ga = g[k[a]];
+      const float2 v = a3[a * m + i];
+      const float ga = g[k[a]];
       re -= ga * v.y;
       im += ga * v.x;
     }
-    const T G = green[i];
-    C o;
+    const float G = green[i];
+    float2 o;
     o.x = G * re;
     o.y = G * im;
     out[i] = o;
@@ -436,10 +503,12 @@ bool Solver::prepare(int ng, int prec, cudaStream_t s, std::string *err) {
   if (!cu_ok(cudaMalloc(&rho_, m * sizeof(float)), "pm rho", err)) return release(), false;
   if (prec == PREC_F64 && !cu_ok(cudaMalloc(&real_, m * rs), "pm real", err)) return release(), false;
   if (!cu_ok(cudaMalloc(&spec_, mh * cs), "pm spectrum", err)) return release(), false;
-  if (!cu_ok(cudaMalloc(&gspec_, 3 * mh * cs), "pm gradient spectra", err)) return release(), false;
-  if (!cu_ok(cudaMalloc(&greal_, 3 * m * rs), "pm gradient fields", err)) return release(), false;
+  if (prec == PREC_F32) {
+    if (!cu_ok(cudaMalloc(&gspec_, 3 * mh * cs), "pm gradient spectra", err)) return release(), false;
+    if (!cu_ok(cudaMalloc(&greal_, 3 * m * rs), "pm gradient fields", err)) return release(), false;
+    if (!cu_ok(cudaMalloc(&gtab_, ng * rs), "pm gradient table", err)) return release(), false;
+  }
   if (!cu_ok(cudaMalloc(&green_, mh * rs), "pm green", err)) return release(), false;
-  if (!cu_ok(cudaMalloc(&gtab_, ng * rs), "pm gradient table", err)) return release(), false;
   if (!cu_ok(cudaMalloc(&grad_, m * sizeof(float4)), "pm gradient grid", err)) return release(), false;
 
   // tables (host, double) -> Green's function (device)
@@ -465,23 +534,16 @@ bool Solver::prepare(int ng, int prec, cudaStream_t s, std::string *err) {
                                                          (float *)green_);
     ok = cu_ok(cudaGetLastError(), "pm green kernel", err);
   }
-  if (ok) {
-    if (prec == PREC_F64) {
-      ok = cu_ok(cudaMemcpyAsync(gtab_, gradient.data(), ng * sizeof(double), cudaMemcpyHostToDevice, s),
-                 "pm gradient table copy", err);
-    } else {
-      std::vector<float> gf(gradient.begin(), gradient.end());
-      ok = cu_ok(cudaMemcpyAsync(gtab_, gf.data(), ng * sizeof(float), cudaMemcpyHostToDevice, s),
-                 "pm gradient table copy", err);
-      if (ok) ok = cu_ok(cudaStreamSynchronize(s), "pm tables", err);
-    }
-  }
+  std::vector<float> gf(gradient.begin(), gradient.end());
+  if (ok && prec == PREC_F32)
+    ok = cu_ok(cudaMemcpyAsync(gtab_, gf.data(), ng * sizeof(float), cudaMemcpyHostToDevice, s),
+               "pm gradient table copy", err);
   if (ok) ok = cu_ok(cudaStreamSynchronize(s), "pm tables", err);
   cudaFree(d_tab);
   if (!ok) return release(), false;
 
-  // plans (64-bit sizes): one forward real-to-complex transform, one
-  // batched inverse of the three gradient spectra
+  // plans (64-bit sizes): one forward real-to-complex transform, one inverse
+  // (of the potential; in single precision of the three gradient spectra)
   long long dims[3] = {ng, ng, ng};
   const bool f64 = prec == PREC_F64;
   size_t ws = 0;
@@ -494,7 +556,7 @@ bool Solver::prepare(int ng, int prec, cudaStream_t s, std::string *err) {
   if (!fft_ok(cufftCreate(&inv_), "pm inverse plan", err)) return release(), false;
   have_inv_ = true;
   if (!fft_ok(cufftMakePlanMany64(inv_, 3, dims, nullptr, 1, mh, nullptr, 1, m,
-                                  f64 ? CUFFT_Z2D : CUFFT_C2R, 3, &ws),
+                                  f64 ? CUFFT_Z2D : CUFFT_C2R, f64 ? 1 : 3, &ws),
               "pm inverse plan", err))
     return release(), false;
   ng_ = ng;
@@ -528,28 +590,28 @@ bool Solver::solve(cudaStream_t s, std::string *err) {
     if (!fft_ok(cufftExecD2Z(fwd_, (cufftDoubleReal *)real_, (cufftDoubleComplex *)spec_),
                 "pm forward transform", err))
       return false;
-    k_spectra<double><<<blocks_for(mh), kThreads, 0, s>>>(ng, nh, (const double2 *)spec_,
-                                                          (const double *)green_,
-                                                          (const double *)gtab_, (double2 *)gspec_);
+    k_potential<<<blocks_for(mh), kThreads, 0, s>>>(mh, (double2 *)spec_, (const double *)green_);
     ++launches;
-    if (!cu_ok(cudaGetLastError(), "pm spectra kernel", err)) return false;
-    if (!fft_ok(cufftExecZ2D(inv_, (cufftDoubleComplex *)gspec_, (cufftDoubleReal *)greal_),
+    if (!cu_ok(cudaGetLastError(), "pm potential kernel", err)) return false;
+    if (!fft_ok(cufftExecZ2D(inv_, (cufftDoubleComplex *)spec_, (cufftDoubleReal *)real_),
                 "pm inverse transform", err))
       return false;
-    k_pack<double><<<blocks_for(m), kThreads, 0, s>>>(m, (const double *)greal_, grad_);
+    k_gradient<<<dim3(unsigned((ng + 31) / 32), unsigned((ng + 7) / 8),
+                      unsigned((ng + kGradSpan - 1) / kGradSpan)),
+                 dim3(32, 8), 0, s>>>(ng, (const double *)real_, grad_);
   } else {
     if (!fft_ok(cufftExecR2C(fwd_, (cufftReal *)rho_, (cufftComplex *)spec_), "pm forward transform",
                 err))
       return false;
-    k_spectra<float><<<blocks_for(mh), kThreads, 0, s>>>(ng, nh, (const float2 *)spec_,
-                                                         (const float *)green_,
-                                                         (const float *)gtab_, (float2 *)gspec_);
+    k_spectra<<<blocks_for(mh), kThreads, 0, s>>>(ng, nh, (const float2 *)spec_,
+                                                  (const float *)green_, (const float *)gtab_,
+                                                  (float2 *)gspec_);
     ++launches;
     if (!cu_ok(cudaGetLastError(), "pm spectra kernel", err)) return false;
     if (!fft_ok(cufftExecC2R(inv_, (cufftComplex *)gspec_, (cufftReal *)greal_),
                 "pm inverse transform", err))
       return false;
-    k_pack<float><<<blocks_for(m), kThreads, 0, s>>>(m, (const float *)greal_, grad_);
+    k_pack<<<blocks_for(m), kThreads, 0, s>>>(m, (const float *)greal_, grad_);
   }
   ++launches;
   fft_execs += 2;
@@ -582,27 +644,24 @@ bool Solver::export_fields(float *rho, float *grad, bool to_host, cudaStream_t s
 }
 
 bool Solver::prepare_vjp(std::string *err) {
-  if (have_fwd3_ && have_inv1_ && adj_) return true;
   const int ng = ng_, nh = ng / 2 + 1;
   const int64_t m = int64_t(ng) * ng * ng, mh = int64_t(ng) * ng * nh;
   if (!adj_ && !cu_ok(cudaMalloc(&adj_, 3 * m * sizeof(float)), "pm adjoint fields", err))
     return false;
+  if (prec_ == PREC_F64) return true;  // the forward solve's own plans
   long long dims[3] = {ng, ng, ng};
-  const bool f64 = prec_ == PREC_F64;
   size_t ws = 0;
   if (!have_fwd3_) {
     if (!fft_ok(cufftCreate(&fwd3_), "pm adjoint forward plan", err)) return false;
     have_fwd3_ = true;
-    if (!fft_ok(cufftMakePlanMany64(fwd3_, 3, dims, nullptr, 1, m, nullptr, 1, mh,
-                                    f64 ? CUFFT_D2Z : CUFFT_R2C, 3, &ws),
+    if (!fft_ok(cufftMakePlanMany64(fwd3_, 3, dims, nullptr, 1, m, nullptr, 1, mh, CUFFT_R2C, 3, &ws),
                 "pm adjoint forward plan", err))
       return false;
   }
   if (!have_inv1_) {
     if (!fft_ok(cufftCreate(&inv1_), "pm adjoint inverse plan", err)) return false;
     have_inv1_ = true;
-    if (!fft_ok(cufftMakePlanMany64(inv1_, 3, dims, nullptr, 1, mh, nullptr, 1, m,
-                                    f64 ? CUFFT_Z2D : CUFFT_C2R, 1, &ws),
+    if (!fft_ok(cufftMakePlanMany64(inv1_, 3, dims, nullptr, 1, mh, nullptr, 1, m, CUFFT_C2R, 1, &ws),
                 "pm adjoint inverse plan", err))
       return false;
   }
@@ -623,29 +682,27 @@ bool Solver::vjp(const Params &p, int64_t n, const float *x, const float *y, con
                                                    adj_);
   ++launches;
   if (!cu_ok(cudaGetLastError(), "pm adjoint deposit", err)) return false;
-  if (!fft_ok(cufftSetStream(fwd3_, s), "pm adjoint stream", err)) return false;
-  if (!fft_ok(cufftSetStream(inv1_, s), "pm adjoint stream", err)) return false;
   const float cm = p.gpscal * p.gpscal * p.gpscal;
   const float coef = p.fscal * p.tau;
   if (prec_ == PREC_F64) {
-    k_to_real3<double><<<blocks_for(3 * m), kThreads, 0, s>>>(3 * m, adj_, (double *)greal_);
-    if (!fft_ok(cufftExecD2Z(fwd3_, (cufftDoubleReal *)greal_, (cufftDoubleComplex *)gspec_),
+    k_divergence<<<blocks_for(m), kThreads, 0, s>>>(ng, adj_, (double *)real_);
+    if (!fft_ok(cufftExecD2Z(fwd_, (cufftDoubleReal *)real_, (cufftDoubleComplex *)spec_),
                 "pm adjoint forward transform", err))
       return false;
-    k_adj_spectra<double><<<blocks_for(mh), kThreads, 0, s>>>(
-        ng, nh, (const double2 *)gspec_, (const double *)green_, (const double *)gtab_,
-        (double2 *)spec_);
-    if (!fft_ok(cufftExecZ2D(inv1_, (cufftDoubleComplex *)spec_, (cufftDoubleReal *)real_),
+    k_potential<<<blocks_for(mh), kThreads, 0, s>>>(mh, (double2 *)spec_, (const double *)green_);
+    if (!fft_ok(cufftExecZ2D(inv_, (cufftDoubleComplex *)spec_, (cufftDoubleReal *)real_),
                 "pm adjoint inverse transform", err))
       return false;
     k_vjp_interp<double><<<blocks_for(n), kThreads, 0, s>>>(
         n, x, y, z, vbx, vby, vbz, ng, p.ngo, nglt, grad_, (const double *)real_, cm, coef, xbx,
         xby, xbz);
   } else {
+    if (!fft_ok(cufftSetStream(fwd3_, s), "pm adjoint stream", err)) return false;
+    if (!fft_ok(cufftSetStream(inv1_, s), "pm adjoint stream", err)) return false;
     if (!fft_ok(cufftExecR2C(fwd3_, (cufftReal *)adj_, (cufftComplex *)gspec_),
                 "pm adjoint forward transform", err))
       return false;
-    k_adj_spectra<float><<<blocks_for(mh), kThreads, 0, s>>>(
+    k_adj_spectra<<<blocks_for(mh), kThreads, 0, s>>>(
         ng, nh, (const float2 *)gspec_, (const float *)green_, (const float *)gtab_,
         (float2 *)spec_);
     // the density grid is free once the solve ran: the inverse lands there

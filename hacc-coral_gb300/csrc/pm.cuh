@@ -31,10 +31,14 @@
 //     where both k and -k carry the same factor: there the spectrum is
 //     anti-Hermitian and its real part is zero, so the factor is 0 on those
 //     planes and the half-spectrum inverse gives the reference's real part;
-//   * the three gradient components are solved in one batched inverse
-//     transform and interpolated in one pass over the particles (the
-//     reference's three inverse_cic passes update different components from
-//     the same positions).
+//   * the gradient factor is the spectrum of the 4th-order central difference:
+//     in double precision one inverse transform gives the potential and its
+//     differences the three gradient components (and the adjoint one forward
+//     transform of the cotangents' divergence); single precision solves the
+//     three components in one batched inverse transform;
+//   * the three components are interpolated in one pass over the particles
+//     (the reference's three inverse_cic passes update different components
+//     from the same positions).
 #pragma once
 
 #include <cstdint>
@@ -103,19 +107,19 @@ class Solver {
   int ng_ = 0, prec_ = -1;
   cufftHandle fwd_ = 0, inv_ = 0;
   bool have_fwd_ = false, have_inv_ = false;
-  // adjoint: batched forward of the three deposited cotangent fields, single
-  // inverse of the combined spectrum (made on the first vjp)
+  // single-precision adjoint: batched forward of the three deposited cotangent
+  // fields, single inverse of the combined spectrum (made on the first vjp)
   cufftHandle fwd3_ = 0, inv1_ = 0;
   bool have_fwd3_ = false, have_inv1_ = false;
   float *adj_ = nullptr;     // 3 x ng^3: deposited cotangents (float atomics)
   bool prepare_vjp(std::string *err);
   float *rho_ = nullptr;     // ng^3
-  void *real_ = nullptr;     // ng^3 real (T): transform input (double only)
+  void *real_ = nullptr;     // ng^3 double: transform input, potential (double only)
   void *spec_ = nullptr;     // ng^2 (ng/2+1) complex (T)
-  void *gspec_ = nullptr;    // 3 x ng^2 (ng/2+1) complex (T)
-  void *greal_ = nullptr;    // 3 x ng^3 real (T)
+  void *gspec_ = nullptr;    // 3 x ng^2 (ng/2+1) complex (single only)
+  void *greal_ = nullptr;    // 3 x ng^3 real (single only)
   void *green_ = nullptr;    // ng^2 (ng/2+1) real (T)
-  void *gtab_ = nullptr;     // ng real (T): gradient factor per wave index
+  void *gtab_ = nullptr;     // ng real: gradient factor per wave index (single only)
   float4 *grad_ = nullptr;   // ng^3
 };
 
