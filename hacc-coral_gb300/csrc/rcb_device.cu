@@ -50,7 +50,7 @@ constexpr int kPlainSteps = 4;      // single chain steps before the chunk parti
 enum { C_NCHUNK = 0, C_NSPLIT = 1, C_NFALLBACK = 2, C_NLEAF = 3, C_NSEG = 4, C_NENT = 5,
        C_PAIRS = 6, C_PADDED = 7, C_NITEMS = 8, C_MAXLEN = 9, C_TDONE1 = 10, C_TDONE2 = 11,
        C_NTIGHT = 12, C_SEGOVF = 13, C_MAXCNT = 14, C_ERR = 15, C_BUCKET = 16, C_FILL = 48,
-       C_SUBFB = 80, C_CHAINS = 81, C_COUNT = 82 };
+       C_SUBFB = 80, C_CHAINS = 81, C_TICKET = 82, C_COUNT = 83 };
 
 // Segments a leaf's walk can leave in its own region of the one-pass walk (8
 // bytes each); a leaf with more sends the build to a second, placing walk.
@@ -205,6 +205,36 @@ __device__ __forceinline__ int64_t block_exclusive_scan(const int64_t (&v)[kScan
     run += v[k];
   }
   return wsum[31];
+}
+
+// Exclusive scans of a and b in place, in one block, for n up to a few blocks'
+// worth; the totals into *ta and *tb.  (Two three-kernel scans otherwise.)
+constexpr int64_t kScanPairMax = 4 * kScanBlock;
+__global__ void __launch_bounds__(kScanThreads)
+    k_scan_pair(const int64_t *a, const int64_t *b, int64_t *oa, int64_t *ob, int64_t n,
+                int64_t *ta, int64_t *tb) {
+  int64_t ca = 0, cb = 0;
+  for (int64_t base = 0; base < n; base += kScanBlock) {
+    const int64_t i0 = base + int64_t(threadIdx.x) * kScanPer;
+    int64_t v[kScanPer], o[kScanPer];
+    for (int which = 0; which < 2; ++which) {
+      const int64_t *in = which ? b : a;
+      int64_t *out = which ? ob : oa;
+      int64_t &carry = which ? cb : ca;
+#pragma unroll
+      for (int k = 0; k < kScanPer; ++k) v[k] = i0 + k < n ? in[i0 + k] : 0;
+      const int64_t total = block_exclusive_scan(v, o);
+#pragma unroll
+      for (int k = 0; k < kScanPer; ++k)
+        if (i0 + k < n) out[i0 + k] = carry + o[k];
+      carry += total;
+      __syncthreads();  // the scan's shared sums are reused
+    }
+  }
+  if (threadIdx.x == 0) {
+    *ta = ca;
+    *tb = cb;
+  }
 }
 
 // Levels of at most kScanBlock nodes, in one block: the chunks of every node
@@ -2155,186 +2185,190 @@ __device__ __forceinline__ float pptdr_(const DNode &t) {
                                  smin_(fsub_(t.xc[1], t.xmin[1]), fsub_(t.xc[2], t.xmin[2]))))));
 }
 
-__device__ __forceinline__ void pppts_(int k, float tdr, const float *xc, float *px, float *py,
-                                       float *pz) {
-  for (int i = 0; i < k; ++i) {
-    const float ex = k == 12 ? c_design[i][0] : 0.f, ey = k == 12 ? c_design[i][1] : 0.f,
-                ez = k == 12 ? c_design[i][2] : 0.f;
-    px[i] = fadd_(fmul_(tdr, ex), xc[0]);
-    py[i] = fadd_(fmul_(tdr, ey), xc[1]);
-    pz[i] = fadd_(fmul_(tdr, ez), xc[2]);
-  }
+// Design point j of a node: its centre of mass plus tdr times the unit point
+// (offset 0 for the monopole's one point).
+template <int K>
+__device__ __forceinline__ void pppt_(int j, float tdr, const float *xc, float &x, float &y,
+                                      float &z) {
+  const float ex = K == 12 ? c_design[j][0] : 0.f, ey = K == 12 ? c_design[j][1] : 0.f,
+              ez = K == 12 ? c_design[j][2] : 0.f;
+  x = fadd_(fmul_(tdr, ex), xc[0]);
+  y = fadd_(fmul_(tdr, ey), xc[1]);
+  z = fadd_(fmul_(tdr, ez), xc[2]);
 }
 
-// Adds `count` sources (x, y, z, m from src(i)) to the pseudo-particle masses.
-template <typename Src>
-__device__ void pp_accum_(int k, int32_t count, Src src, const float *xc, const float *px,
-                          const float *py, const float *pz, float *ppm, float tdr) {
-  const float K = float(k);
-  const float odr0 = __fdiv_rn(1.0f, K);
-  for (int32_t i = 0; i < count; ++i) {
-    float sx, sy, sz, sm;
-    src(i, sx, sy, sz, sm);
+// One pseudo-particle's mass over its node's sources, added in source order.
+template <int K>
+struct PointMass {
+  float xj, yj, zj, rj2, rj, m;
+  __device__ __forceinline__ void start(int j, float tdr, const float *xc) {
+    float x, y, z;
+    pppt_<K>(j, tdr, xc, x, y, z);
+    xj = fsub_(x, xc[0]);
+    yj = fsub_(y, xc[1]);
+    zj = fsub_(z, xc[2]);
+    rj2 = norm2_(xj, yj, zj);
+    rj = __fsqrt_rn(rj2);
+    m = 0.f;
+  }
+  __device__ __forceinline__ void add(float sx, float sy, float sz, float sm, float tdr,
+                                      const float *xc) {
     const float xi = fsub_(sx, xc[0]), yi = fsub_(sy, xc[1]), zi = fsub_(sz, xc[2]);
     const float ri = __fsqrt_rn(norm2_(xi, yi, zi));
-    for (int j = 0; j < k; ++j) {
-      const float xj = fsub_(px[j], xc[0]), yj = fsub_(py[j], xc[1]), zj = fsub_(pz[j], xc[2]);
-      const float rj2 = norm2_(xj, yj, zj);
-      float odr1 = 0.f, odr2 = 0.f;
-      if (rj2 != 0.f) {
-        const float rj = __fsqrt_rn(rj2);
-        const float aij = __fdiv_rn(fadd_(fadd_(fmul_(xi, xj), fmul_(yi, yj)), fmul_(zi, zj)),
-                                    fmul_(ri, rj));
-        const float rt = __fdiv_rn(ri, tdr);
-        odr1 = fmul_(fmul_(__fdiv_rn(3.0f, K), rt), aij);
-        const float a = fmul_(fmul_(__fdiv_rn(5.0f, K), rt), rt);
-        const float b = fsub_(fmul_(fmul_(3.0f, aij), aij), 1.0f);
-        odr2 = __double2float_rn(__dmul_rn(__dmul_rn(double(a), 0.5), double(b)));
-      }
-      ppm[j] = fadd_(ppm[j], fmul_(sm, fadd_(fadd_(odr0, odr1), odr2)));
+    float odr1 = 0.f, odr2 = 0.f;
+    if (rj2 != 0.f) {
+      const float aij = __fdiv_rn(fadd_(fadd_(fmul_(xi, xj), fmul_(yi, yj)), fmul_(zi, zj)),
+                                  fmul_(ri, rj));
+      const float rt = __fdiv_rn(ri, tdr);
+      odr1 = fmul_(fmul_(3.0f / K, rt), aij);
+      const float a = fmul_(fmul_(5.0f / K, rt), rt);
+      const float b = fsub_(fmul_(fmul_(3.0f, aij), aij), 1.0f);
+      // the reference multiplies a * 0.5 * b in double and rounds once: a
+      // product of two floats is exact there, and so is half of b here (b is
+      // 0 or far above the subnormals)
+      odr2 = fmul_(a, fmul_(0.5f, b));
     }
+    m = fadd_(m, fmul_(sm, fadd_(fadd_(1.0f / K, odr1), odr2)));
   }
-}
-
-// Node ranges of up to kTopLevels levels: level l is [b[l], b[l + 1]).
-constexpr int kTopLevels = 48;
-struct LevelSpan {
-  int32_t b[kTopLevels + 1];
-  int32_t n;
 };
 
-// Pseudo-particles of node t, its children done first.
-__device__ void pseudo_node(DNode *nodes, int32_t t, const float4 *__restrict__ pos, float *ppm_all,
-                            int k, float ppc, int32_t nd) {
-  DNode &T = nodes[t];
-  T.tdr = fmul_(ppc, pptdr_(T));
-  float ppm[12];
-  for (int j = 0; j < 12; ++j) ppm[j] = 0.f;
-  float px[12], py[12], pz[12];
-  if (T.cl == 0 && T.cr == 0) {
-    // leaf by size: masses from its particles when it has more than k;
-    // a leaf left by a failed split keeps zero masses (its children are empty)
-    if (T.count <= nd && T.count > k) {
-      const float4 *p = pos + T.offset;
-      if (k == 1) {
-        // the monopole's point is the centre of mass: every term's weight is
-        // 1/1 + 0 + 0 (pp_accum_ with rj2 == 0), so the mass is the
-        // sequential float sum of the particle masses
-        float m = 0.f;
-#pragma unroll 8
-        for (int32_t i = 0; i < T.count; ++i) m = fadd_(m, fmul_(p[i].w, 1.0f));
-        ppm[0] = m;
-      } else {
-        pppts_(k, T.tdr, T.xc, px, py, pz);
-        pp_accum_(k, T.count, [&](int32_t i, float &x, float &y, float &z, float &m) {
-          const float4 q = p[i];
-          x = q.x; y = q.y; z = q.z; m = q.w;
-        }, T.xc, px, py, pz, ppm, T.tdr);
-      }
-    }
-  } else {
-    pppts_(k, T.tdr, T.xc, px, py, pz);
-    for (int s = 0; s < 2; ++s) {
-      const DNode &C = nodes[s == 0 ? T.cl : T.cr];
-      if (C.count <= 0) continue;
-      if (C.count <= k) {
-        const float4 *p = pos + C.offset;
-        pp_accum_(k, C.count, [&](int32_t i, float &x, float &y, float &z, float &m) {
-          const float4 q = p[i];
-          x = q.x; y = q.y; z = q.z; m = q.w;
-        }, T.xc, px, py, pz, ppm, T.tdr);
-      } else {
-        float cx[12], cy[12], cz[12];
-        pppts_(k, C.tdr, C.xc, cx, cy, cz);
-        const float *cm = ppm_all + int64_t(s == 0 ? T.cl : T.cr) * k;
-        pp_accum_(k, k, [&](int32_t i, float &x, float &y, float &z, float &m) {
-          x = cx[i]; y = cy[i]; z = cz[i]; m = cm[i];
-        }, T.xc, px, py, pz, ppm, T.tdr);
-      }
-    }
-  }
-  for (int j = 0; j < k; ++j) ppm_all[int64_t(t) * k + j] = ppm[j];
-}
-
-// Pseudo-particles of the nodes [lb, le), a warp per node.  A monopole leaf's
-// mass is the sequential float sum of its particles' masses: the warp loads
-// 32 at a time (coalesced) and every lane adds them in order from shuffles.
-// Other nodes: lane 0.
-__global__ void k_pseudo(DNode *nodes, int32_t lb, int32_t le, const float4 *__restrict__ pos,
-                         float *ppm_all, int k, float ppc, int32_t nd) {
-  const int32_t t = lb + int32_t((int64_t(blockIdx.x) * blockDim.x + threadIdx.x) >> 5);
-  const int lane = threadIdx.x & 31;
-  if (t >= le) return;  // whole warps
-  DNode &T = nodes[t];
-  if (k == 1 && T.cl == 0 && T.cr == 0 && T.count <= nd && T.count > 1) {
-    const float *w = reinterpret_cast<const float *>(pos + T.offset) + 3;
-    const int32_t c = T.count;
-    float m = 0.f;
-    for (int32_t i0 = 0; i0 < c; i0 += 32) {
-      const float v = i0 + lane < c ? w[4 * (i0 + lane)] : 0.f;
-      const int nv = min(32, c - i0);
-      for (int j = 0; j < nv; ++j) m = fadd_(m, fmul_(__shfl_sync(0xffffffffu, v, j), 1.0f));
-    }
-    if (lane == 0) {
-      T.tdr = fmul_(ppc, pptdr_(T));
-      ppm_all[t] = m;
-    }
-    return;
-  }
-  if (lane == 0) pseudo_node(nodes, t, pos, ppm_all, k, ppc, nd);
-}
-
-// The top levels' pseudo-particles in one block, deepest level first, a
-// thread per node (every level here has at most blockDim.x nodes).
-__global__ void __launch_bounds__(1024)
-    k_pseudo_top(DNode *nodes, LevelSpan lv, const float4 *__restrict__ pos, float *ppm_all, int k,
-                 float ppc, int32_t nd) {
-  for (int l = lv.n - 1; l >= 0; --l) {
-    for (int32_t t = lv.b[l] + int32_t(threadIdx.x); t < lv.b[l + 1]; t += int32_t(blockDim.x))
-      pseudo_node(nodes, t, pos, ppm_all, k, ppc, nd);
-    __syncthreads();  // the next level up reads these nodes
-  }
-}
-
-// Position table: particles, then every node's pseudo-particles.
-__global__ void k_table_pseudo(const DNode *nodes, int32_t nnodes, const float *ppm_all, int k,
-                               float4 *table, int64_t n) {
-  const int32_t t = blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= nnodes) return;
-  const DNode &T = nodes[t];
-  float px[12], py[12], pz[12];
-  pppts_(k, T.tdr, T.xc, px, py, pz);
-  for (int j = 0; j < k; ++j)
-    table[n + int64_t(t) * k + j] = make_float4(px[j], py[j], pz[j], ppm_all[int64_t(t) * k + j]);
-}
-
-// ---------------------------------------------------------------------------
-// Processed leaves (calcInternodeForces, RCBForceTree.cxx:1150-1197): leaves
-// inside the force box, in the reference's DFS order, which visits the right
-// child first, i.e. by decreasing particle offset.
-// ---------------------------------------------------------------------------
-__global__ void k_mark_leaves(const DNode *nodes, int32_t nnodes, TreeConfig cfg, int64_t n,
-                              int64_t *leaf_at) {
-  const int32_t t = blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= nnodes) return;
-  const DNode &T = nodes[t];
-  if (T.cl != 0 || T.cr != 0 || T.count <= 0) return;
-  bool inside = true;
+// The leaf test of calcInternodeForces (RCBForceTree.cxx:1150-1197): leaves
+// with a face of their box inside the force box on every axis.
+__device__ __forceinline__ bool leaf_in_force_box(const DNode &T, const TreeConfig &cfg) {
+  bool inside = T.count > 0;
   for (int i = 0; i < 3; ++i)
     inside &= (T.xmax[i] < cfg.max_force[i] && T.xmax[i] > cfg.min_force[i]) ||
               (T.xmin[i] < cfg.max_force[i] && T.xmin[i] > cfg.min_force[i]);
-  if (inside) leaf_at[n - 1 - T.offset] = t;  // reversed: decreasing offset
+  return inside;
 }
 
-__global__ void k_leaf_flags(const int64_t *leaf_at, int64_t n, int64_t *flag) {
-  const int64_t i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
-  if (i < n) flag[i] = leaf_at[i] >= 0;
+// Links upward: up[t] = (parent, 0) of every node; the arrival counter's bit 8
+// marks a left child (its sibling is t + 1: children are made in pairs).
+constexpr int kLeftChild = 0x100;
+__global__ void k_links(const DNode *nodes, int32_t nnodes, int2 *up) {
+  const int32_t t = blockIdx.x * blockDim.x + threadIdx.x;
+  if (t >= nnodes) return;
+  const int32_t cl = nodes[t].cl;
+  if (t == 0) up[0] = make_int2(-1, 0);
+  if (cl > 0) {
+    up[cl] = make_int2(t, kLeftChild);
+    up[cl + 1] = make_int2(t, 0);
+  }
 }
 
-__global__ void k_leaf_compact(const int64_t *leaf_at, const int64_t *pos_of, int64_t n,
-                               int32_t *leaf_ids) {
-  const int64_t i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
-  if (i < n && leaf_at[i] >= 0) leaf_ids[pos_of[i]] = int32_t(leaf_at[i]);
+// Every node's pseudo-particles (masses into ppm, points into the position
+// table), tdr and the number of processed leaves below it, from the leaves up
+// in one launch: a warp per leaf does its leaf, and whichever warp arrives
+// second at a node goes on with it.  Lane j < K holds point j and adds the
+// node's sources in the reference's order (all of a leaf's particles, or each
+// child's particles or points, left child first), so the points of a node run
+// in parallel and no level waits for a launch of its own.  A monopole leaf's
+// mass is the sequential float sum of its particles' masses, loaded 32 at a
+// time and added in order from shuffles.  (With one lane a node and a launch a
+// level, 12-point masses took 3.6 of the 9.8 ms of a clustered 48^3 forward and
+// adjoint, and a 32^3 kick's monopoles 52 us.)
+template <int K>
+__global__ void __launch_bounds__(128)
+    k_pseudo_up(DNode *nodes, int32_t nnodes, int2 *up, const float4 *__restrict__ pos, float *ppm,
+                float4 *table, int64_t n, TreeConfig cfg, int32_t *processed) {
+  const unsigned full = 0xffffffffu;
+  const int lane = threadIdx.x & 31;
+  int32_t t = int32_t((int64_t(blockIdx.x) * blockDim.x + threadIdx.x) >> 5);
+  if (t >= nnodes) return;  // whole warps
+  if (nodes[t].cl != 0) return;
+  for (int climbed = 0; climbed <= nnodes; ++climbed) {
+    const DNode T = nodes[t];
+    const float tdr = fmul_(cfg.ppc, pptdr_(T));
+    const int j = lane < K ? lane : 0;
+    PointMass<K> P;
+    P.start(j, tdr, T.xc);
+    int32_t below = 0;  // processed leaves
+    if (T.cl == 0) {
+      below = leaf_in_force_box(T, cfg) ? 1 : 0;
+      // masses from its particles when it has more than K; a leaf left by a
+      // failed split keeps zero masses (its children are empty)
+      if (T.count <= cfg.nd && T.count > K) {
+        const float4 *p = pos + T.offset;
+        if (K == 1) {
+          // every term's weight is 1/1 + 0 + 0 (PointMass with rj2 == 0)
+          const float *w = reinterpret_cast<const float *>(p) + 3;
+          for (int32_t i0 = 0; i0 < T.count; i0 += 32) {
+            const float v = i0 + lane < T.count ? w[4 * (i0 + lane)] : 0.f;
+            const int nv = min(32, T.count - i0);
+            for (int i = 0; i < nv; ++i) P.m = fadd_(P.m, fmul_(__shfl_sync(full, v, i), 1.0f));
+          }
+        } else {
+#pragma unroll 4
+          for (int32_t i = 0; i < T.count; ++i) {
+            const float4 q = p[i];
+            P.add(q.x, q.y, q.z, q.w, tdr, T.xc);
+          }
+        }
+      }
+    } else {
+      for (int s = 0; s < 2; ++s) {
+        const int32_t c = T.cl + s;
+        const DNode &C = nodes[c];
+        const int32_t cc = C.count;
+        below += __ldcg(processed + c);
+        if (cc <= K) {
+          const float4 *p = pos + C.offset;
+          for (int32_t i = 0; i < cc; ++i) {
+            const float4 q = p[i];
+            P.add(q.x, q.y, q.z, q.w, tdr, T.xc);
+          }
+        } else {
+          const float ctdr = __ldcg(&C.tdr);
+          const float cxc[3] = {C.xc[0], C.xc[1], C.xc[2]};
+#pragma unroll
+          for (int i = 0; i < K; ++i) {
+            float x, y, z;
+            pppt_<K>(i, ctdr, cxc, x, y, z);
+            P.add(x, y, z, __ldcg(ppm + int64_t(c) * K + i), tdr, T.xc);
+          }
+        }
+      }
+    }
+    if (lane < K) {
+      float x, y, z;
+      pppt_<K>(j, tdr, T.xc, x, y, z);
+      ppm[int64_t(t) * K + j] = P.m;
+      table[n + int64_t(t) * K + j] = make_float4(x, y, z, P.m);
+    }
+    if (lane == 0) {
+      nodes[t].tdr = tdr;
+      processed[t] = below;
+    }
+    if (t == 0) return;
+    const int32_t parent = up[t].x;
+    __threadfence();
+    __syncwarp();
+    int arrived = 0;
+    if (lane == 0) arrived = atomicAdd(&up[parent].y, 1) & 0xff;
+    if (__shfl_sync(full, arrived, 0) == 0) return;  // the sibling's warp goes on
+    __threadfence();
+    t = parent;
+  }
+}
+
+// ---------------------------------------------------------------------------
+// Processed leaves, in the reference's DFS order, which visits the right child
+// first: a leaf's rank is the number of processed leaves right of its path,
+// counted on the way up.
+// ---------------------------------------------------------------------------
+__global__ void k_leaf_rank(const DNode *nodes, int32_t nnodes, const int2 *up,
+                            const int32_t *processed, int32_t *leaf_ids, int64_t *counters) {
+  const int32_t t0 = blockIdx.x * blockDim.x + threadIdx.x;
+  if (t0 >= nnodes) return;
+  if (t0 == 0) counters[C_NLEAF] = processed[0];
+  if (nodes[t0].cl != 0 || processed[t0] == 0) return;
+  int32_t rank = 0, t = t0;
+  for (int climbed = 0; t > 0 && climbed <= nnodes; ++climbed) {
+    const int2 u = up[t];
+    if (u.y & kLeftChild) rank += processed[t + 1];
+    t = u.x;
+  }
+  leaf_ids[rank] = t0;
 }
 
 // ---------------------------------------------------------------------------
@@ -2354,6 +2388,8 @@ constexpr int kWalkWarps = 4;
 constexpr int kWalkCap = 640;      // stack entries a leaf; the window narrows as it
 constexpr int kWalkReserve = 256;  // fills, to one node at a time over the last 256
 
+// The leaves are the first counters[C_NLEAF] of leaf_ids (max_leaves bounds
+// them: the host need not wait for their number).
 // MODE 1: writes the segments at seg_base / list_base; 2: counts (segments and
 // entries per leaf) and writes the first kLocalSegs segments (start, count) of
 // each leaf into its own region, flagging leaves with more in
@@ -2361,7 +2397,7 @@ constexpr int kWalkReserve = 256;  // fills, to one node at a time over the last
 template <int MODE>
 __global__ void __launch_bounds__(32 * kWalkWarps)
     k_walk(const DNode *__restrict__ nodes, int32_t nnodes, const int32_t *leaf_ids,
-           int64_t nleaves, TreeConfig cfg, int64_t n, int64_t *seg_cnt, int64_t *list_len,
+           int64_t max_leaves, TreeConfig cfg, int64_t n, int64_t *seg_cnt, int64_t *list_len,
            const int64_t *seg_base, const int64_t *list_base, SegDesc *segs, int2 *local,
            int32_t *err, int64_t *counters) {
   static_assert(MODE == 1 || MODE == 2, "walk mode");
@@ -2372,7 +2408,11 @@ __global__ void __launch_bounds__(32 * kWalkWarps)
   const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const unsigned full = 0xffffffffu, below = (1u << lane) - 1u;
   const int64_t li = int64_t(blockIdx.x) * kWalkWarps + w;
-  if (li >= nleaves) return;  // whole warps
+  if (li >= max_leaves) return;  // whole warps
+  if (li >= counters[C_NLEAF]) {
+    if (MODE == 2 && lane == 0) seg_cnt[li] = list_len[li] = 0;
+    return;
+  }
   int2 *const st = stack_[w];
   const int32_t tl = leaf_ids[li];
   const DNode T = nodes[tl];
@@ -2610,36 +2650,6 @@ __global__ void __launch_bounds__(256)
 }
 
 
-__global__ void k_leaf_desc(const DNode *nodes, const int32_t *leaf_ids, int64_t nleaves,
-                            const int64_t *list_len, const int64_t *kept_len,
-                            const int64_t *list_base, LeafDesc *ld, int64_t *counters) {
-  const int64_t li = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
-  long long pairs = 0, padded = 0, mx = 0;
-  if (li < nleaves) {
-    const DNode &T = nodes[leaf_ids[li]];
-    LeafDesc d{};
-    d.offset = T.offset;
-    d.count = T.count;
-    d.list_len = int32_t(list_len[li]);
-    d.kept_len = int32_t(kept_len ? kept_len[li] : list_len[li]);
-    d.list_begin = list_base[li];
-    ld[li] = d;
-    pairs = (long long)T.count * list_len[li];
-    padded = (long long)((T.count + 31) / 32) * 32 * d.kept_len;
-    mx = d.kept_len;
-  }
-  for (int o = 16; o > 0; o >>= 1) {
-    pairs += __shfl_xor_sync(0xffffffffu, pairs, o);
-    padded += __shfl_xor_sync(0xffffffffu, padded, o);
-    mx = max(mx, __shfl_xor_sync(0xffffffffu, mx, o));
-  }
-  if ((threadIdx.x & 31) == 0) {
-    atomicAdd((unsigned long long *)&counters[C_PAIRS], (unsigned long long)pairs);
-    atomicAdd((unsigned long long *)&counters[C_PADDED], (unsigned long long)padded);
-    atomicMax((long long *)&counters[C_MAXLEN], mx);
-  }
-}
-
 // ---------------------------------------------------------------------------
 // Groups of <= 32 spatially close particles per processed leaf (Morton order
 // inside the leaf's box) and the batched kernel's work items.
@@ -2658,24 +2668,19 @@ __device__ __forceinline__ float o2f(uint32_t o) {
   return __uint_as_float((o & 0x80000000u) ? (o & 0x7fffffffu) : ~o);
 }
 
-// Splits each processed leaf into groups of G particles (the last one
-// shorter) by recursive median splits along the longest axis, left parts a
-// multiple of G: the particles of a group are close, so the batched kernel's box test
-// keeps few list entries.  Every level sorts all segments of the leaf at once
-// by (segment, coordinate along the segment's longest axis).
-__global__ void __launch_bounds__(kGroupThreads)
-    k_groups(const DNode *nodes, const int32_t *leaf_ids, int64_t nleaves,
-             const float4 *__restrict__ pos, int32_t *gidx, int G) {
+// Splits a leaf into groups of G particles (the last one shorter) by recursive
+// median splits along the longest axis, left parts a multiple of G: the
+// particles of a group are close, so the batched kernel's box test keeps few
+// list entries.  Every level sorts all segments of the leaf at once by
+// (segment, coordinate along the segment's longest axis).
+__device__ void group_large_leaf(const DNode &T, const float4 *__restrict__ pos, int32_t *gidx,
+                                 int G) {
   __shared__ uint64_t key[kGroupSort];
   __shared__ int32_t val[kGroupSort];
   __shared__ int32_t seg_a[kGroupSort / 16 + 1], seg_c[kGroupSort / 16 + 1];
   __shared__ uint32_t seg_lo[3][kGroupSort / 16 + 1], seg_hi[3][kGroupSort / 16 + 1];
   __shared__ int nseg_s, more_s;
-  const int64_t li = blockIdx.x;
-  if (li >= nleaves) return;
-  const DNode &T = nodes[leaf_ids[li]];
   const int32_t c = T.count;
-  if (c <= kGW) return;  // k_groups_warp
   if (c > kGroupSort) {
     for (int32_t i = threadIdx.x; i < c; i += blockDim.x) gidx[T.offset + i] = T.offset + i;
     return;
@@ -2782,13 +2787,35 @@ __global__ void __launch_bounds__(kGroupThreads)
   for (int i = threadIdx.x; i < c; i += blockDim.x) gidx[T.offset + i] = val[i];
 }
 
+// The leaves too large for k_groups_warp, block by block: each block looks
+// kGroupThreads leaves over and groups the large ones among them (a block a
+// leaf, most of them returning at once, took 31 us of a 128^3 kick).
+__global__ void __launch_bounds__(kGroupThreads)
+    k_groups(const DNode *nodes, const int32_t *leaf_ids, const int64_t *nleaves,
+             const float4 *__restrict__ pos, int32_t *gidx, int G) {
+  __shared__ int32_t big[kGroupThreads];
+  __shared__ int nbig;
+  if (threadIdx.x == 0) nbig = 0;
+  __syncthreads();
+  const int64_t li = int64_t(blockIdx.x) * kGroupThreads + threadIdx.x;
+  if (li < *nleaves) {
+    const int32_t t = leaf_ids[li];
+    if (nodes[t].count > kGW) big[atomicAdd(&nbig, 1)] = t;
+  }
+  __syncthreads();
+  for (int b = 0; b < nbig; ++b) {
+    group_large_leaf(nodes[big[b]], pos, gidx, G);
+    __syncthreads();  // the next leaf reuses the shared arrays
+  }
+}
+
 // Warp-per-leaf grouping for leaves of at most kGW particles (the usual
 // case; larger leaves take k_groups).  Same median splits as k_groups: per
 // level, every segment above G particles is sorted along its longest axis by
 // ranking (each element counts the keys below its own, ties by position) and
 // split at G * ceil(groups / 2).
 __global__ void __launch_bounds__(32 * kGWarps)
-    k_groups_warp(const DNode *nodes, const int32_t *leaf_ids, int64_t nleaves,
+    k_groups_warp(const DNode *nodes, const int32_t *leaf_ids, const int64_t *nleaves,
                   const float4 *__restrict__ pos, int32_t *gidx, int G) {
   __shared__ float key[kGWarps][kGW];
   __shared__ int32_t val[kGWarps][2][kGW];
@@ -2797,7 +2824,7 @@ __global__ void __launch_bounds__(32 * kGWarps)
   __shared__ int8_t seg_ax[kGWarps][kGW / 16 + 1];
   const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int64_t li = int64_t(blockIdx.x) * kGWarps + w;
-  if (li >= nleaves) return;
+  if (li >= *nleaves) return;
   const DNode &T = nodes[leaf_ids[li]];
   const int c = T.count;
   if (c <= 0 || c > kGW) return;
@@ -2905,39 +2932,101 @@ __device__ __forceinline__ int len_bucket(int64_t len) {
   return 31 - min(31, b);
 }
 
-__global__ void k_item_hist(const LeafDesc *ld, int64_t nleaves, int64_t jsplit, int G,
-                            int64_t *counters) {
+// Work items per length bucket, block sums first; the last block turns them
+// into the buckets' first positions.  DESC: also the leaf descriptors and the
+// list statistics.
+template <bool DESC>
+__global__ void __launch_bounds__(128)
+    k_leaf_items(const DNode *nodes, const int32_t *leaf_ids, int64_t nleaves,
+                 const int64_t *list_len, const int64_t *kept_len, const int64_t *list_base,
+                 LeafDesc *ld, int64_t jsplit, int G, int64_t *counters) {
+  __shared__ unsigned long long hist[32];
+  __shared__ bool last;
+  if (threadIdx.x < 32) hist[threadIdx.x] = 0;
+  __syncthreads();
   const int64_t li = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
-  if (li >= nleaves) return;
-  const LeafDesc &L = ld[li];
-  const int64_t nch = max64(1, (L.kept_len + jsplit - 1) / jsplit);
-  const int64_t items = int64_t((L.count + G - 1) / G) * nch;
-  atomicAdd((unsigned long long *)&counters[C_BUCKET + len_bucket(min64(L.kept_len, jsplit))],
-            (unsigned long long)items);
-}
-
-__global__ void k_item_bases(int64_t *counters) {
-  if (threadIdx.x != 0 || blockIdx.x != 0) return;
-  int64_t run = 0;
-  for (int b = 0; b < 32; ++b) {
-    counters[C_FILL + b] = run;
-    run += counters[C_BUCKET + b];
+  long long pairs = 0, padded = 0, mx = 0;
+  if (li < nleaves) {
+    LeafDesc d{};
+    if (DESC) {
+      const DNode &T = nodes[leaf_ids[li]];
+      d.offset = T.offset;
+      d.count = T.count;
+      d.list_len = int32_t(list_len[li]);
+      d.kept_len = int32_t(kept_len[li]);
+      d.list_begin = list_base[li];
+      ld[li] = d;
+      pairs = (long long)T.count * list_len[li];
+      padded = (long long)((T.count + 31) / 32) * 32 * d.kept_len;
+      mx = d.kept_len;
+    } else {
+      d = ld[li];
+    }
+    const int64_t nch = max64(1, (d.kept_len + jsplit - 1) / jsplit);
+    atomicAdd(&hist[len_bucket(min64(d.kept_len, jsplit))],
+              (unsigned long long)(int64_t((d.count + G - 1) / G) * nch));
   }
-  counters[C_NITEMS] = run;
+  if (DESC) {
+    for (int o = 16; o > 0; o >>= 1) {
+      pairs += __shfl_xor_sync(0xffffffffu, pairs, o);
+      padded += __shfl_xor_sync(0xffffffffu, padded, o);
+      mx = max(mx, __shfl_xor_sync(0xffffffffu, mx, o));
+    }
+    if ((threadIdx.x & 31) == 0) {
+      atomicAdd((unsigned long long *)&counters[C_PAIRS], (unsigned long long)pairs);
+      atomicAdd((unsigned long long *)&counters[C_PADDED], (unsigned long long)padded);
+      atomicMax((long long *)&counters[C_MAXLEN], mx);
+    }
+  }
+  __syncthreads();
+  if (threadIdx.x < 32 && hist[threadIdx.x])
+    atomicAdd((unsigned long long *)&counters[C_BUCKET + threadIdx.x], hist[threadIdx.x]);
+  __threadfence();
+  __syncthreads();
+  if (threadIdx.x == 0)
+    last = atomicAdd((unsigned long long *)&counters[C_TICKET], 1ull) == gridDim.x - 1;
+  __syncthreads();
+  if (!last || threadIdx.x >= 32) return;
+  __threadfence();
+  const int64_t mine = __ldcg(counters + C_BUCKET + threadIdx.x);
+  int64_t run = mine;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const int64_t v = __shfl_up_sync(0xffffffffu, run, o);
+    if (int(threadIdx.x) >= o) run += v;
+  }
+  counters[C_FILL + threadIdx.x] = run - mine;
+  if (threadIdx.x == 31) counters[C_NITEMS] = run;
 }
 
-__global__ void k_item_fill(const LeafDesc *ld, int64_t nleaves, int64_t jsplit, int G,
-                            int64_t *counters, PairItem *items) {
+__global__ void __launch_bounds__(128)
+    k_item_fill(const LeafDesc *ld, int64_t nleaves, int64_t jsplit, int G, int64_t *counters,
+                PairItem *items) {
+  // positions inside the block's share of each bucket, then one global
+  // reservation a bucket
+  __shared__ unsigned long long cnt[32], base[32];
+  if (threadIdx.x < 32) cnt[threadIdx.x] = 0;
+  __syncthreads();
   const int64_t li = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
-  if (li >= nleaves) return;
-  const LeafDesc &L = ld[li];
-  const int64_t nch = max64(1, (L.kept_len + jsplit - 1) / jsplit);
-  const int32_t ng = (L.count + G - 1) / G;
-  const int64_t items_n = int64_t(ng) * nch;
+  LeafDesc L{};
+  int64_t nch = 0, items_n = 0;
+  unsigned long long at = 0;
+  int b = 0;
+  if (li < nleaves) {
+    L = ld[li];
+    nch = max64(1, (L.kept_len + jsplit - 1) / jsplit);
+    items_n = int64_t((L.count + G - 1) / G) * nch;
+    b = len_bucket(min64(L.kept_len, jsplit));
+    at = atomicAdd(&cnt[b], (unsigned long long)items_n);
+  }
+  __syncthreads();
+  if (threadIdx.x < 32 && cnt[threadIdx.x])
+    base[threadIdx.x] =
+        atomicAdd((unsigned long long *)&counters[C_FILL + threadIdx.x], cnt[threadIdx.x]);
+  __syncthreads();
   if (items_n == 0) return;
-  const int b = len_bucket(min64(L.kept_len, jsplit));
-  int64_t at = int64_t(atomicAdd((unsigned long long *)&counters[C_FILL + b],
-                                 (unsigned long long)items_n));
+  PairItem *out = items + base[b] + at;
+  const int32_t ng = (L.count + G - 1) / G;
   for (int32_t g = 0; g < ng; ++g)
     for (int64_t c = 0; c < nch; ++c) {
       PairItem it{};
@@ -2946,7 +3035,7 @@ __global__ void k_item_fill(const LeafDesc *ld, int64_t nleaves, int64_t jsplit,
       it.g_begin = L.offset + G * g;
       it.g_count = min(G, L.count - G * g);
       it.flags = nch > 1 ? 1 : 0;
-      items[at++] = it;
+      *out++ = it;
     }
 }
 
@@ -3269,12 +3358,6 @@ __global__ void k_iota(int32_t *p, int64_t n) {
     p[i] = int32_t(i);
 }
 
-__global__ void k_fill_i64(int64_t *p, int64_t n, int64_t v) {
-  for (int64_t i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x; i < n;
-       i += int64_t(gridDim.x) * blockDim.x)
-    p[i] = v;
-}
-
 __global__ void k_root(DNode *nodes, int64_t n, TreeConfig cfg) {
   DNode &R = nodes[0];
   R.count = int32_t(n);
@@ -3309,7 +3392,7 @@ inline bool wm_level(int64_t L, int64_t n) { return L * 2048 >= n; }
 DeviceTree::~DeviceTree() {
   void *ptrs[] = {epos_, tpos_, oid_, toid_, idx_, nodes_, ppm_, chunk_node_, chunk_base_, part_,
                   left_cnt_, left_base_, scan_tmp_, node_tmp_, fallback_, counters_, leaf_ids_,
-                  leaf_tmp_, leafdesc_, segs_, idx_list_, table_, items_, items_tmp_, gidx_,
+                  up_, processed_, leafdesc_, segs_, idx_list_, table_, items_, items_tmp_, gidx_,
                   tight_chunks_, tight_nodes_, segs_local_, ridx_, sub_nodes_, sub_first_,
                   sub_hist_, sub_pos_, sub_tot_, sub_stats_, wpre_, chains_};
   for (void *p : ptrs)
@@ -3361,7 +3444,6 @@ cudaError_t DeviceTree::build(const TreeConfig &cfg, int64_t n, const float4 *po
   const auto t0 = std::chrono::steady_clock::now();
   const int k = cfg.tdpts;
   const size_t nn = size_t(std::max<int64_t>(n, 1));
-  n_ = n;
   DT_CHECK(grow(tight_chunks_, cap_tc_,
                 (size_t(n) / kTightChunk + kTightNodes + 1) * (sizeof(TightChunk) / sizeof(double)), s));
   DT_CHECK(grow(tight_nodes_, cap_tn_, size_t(kTightNodes) * (sizeof(TightNode) / sizeof(double)), s));
@@ -3607,75 +3689,40 @@ cudaError_t DeviceTree::build(const TreeConfig &cfg, int64_t n, const float4 *po
   build_ms_ = std::chrono::duration<double, std::milli>(t1 - t0).count();
   info_.levels = int64_t(level_begin.size()) - 1;
 
-  // ---- pseudo-particles, deepest level first ----
-  DT_CHECK(grow(ppm_, cap_ppm_, size_t(nnodes) * k + 1, s));
-  {
-    // the top levels of at most 1024 nodes each in one launch, the rest a
-    // launch per level
-    const int64_t nlev = int64_t(level_begin.size()) - 1;
-    int64_t lt = 0;
-    while (lt < nlev && lt < kTopLevels && level_begin[lt + 1] - level_begin[lt] <= 1024) ++lt;
-    for (int64_t l = nlev - 1; l >= lt; --l) {
-      const int32_t lb = level_begin[l], le = level_begin[l + 1];
-      if (le > lb) {
-        k_pseudo<<<unsigned((int64_t(le - lb) * 32 + 255) / 256), 256, 0, s>>>(
-            nodes_, lb, le, epos_, ppm_, k, cfg.ppc, cfg.nd);
-        ++info_.launches;
-      }
-    }
-    if (lt > 0) {
-      LevelSpan lv{};
-      lv.n = int32_t(lt);
-      for (int64_t l = 0; l <= lt; ++l) lv.b[l] = level_begin[l];
-      k_pseudo_top<<<1, 1024, 0, s>>>(nodes_, lv, epos_, ppm_, k, cfg.ppc, cfg.nd);
-      ++info_.launches;
-    }
-  }
+  // ---- pseudo-particles and processed leaves, from the leaves up ----
   const int64_t ntab = n + int64_t(nnodes) * k;
+  // a binary tree's leaves: the processed ones are at most as many
+  const int64_t max_leaves = (int64_t(nnodes) + 1) / 2;
+  DT_CHECK(grow(ppm_, cap_ppm_, size_t(nnodes) * k + 1, s));
   DT_CHECK(grow(table_, cap_tab_, size_t(std::max<int64_t>(ntab, 1)), s));
+  DT_CHECK(grow(up_, cap_up_, size_t(nnodes), s));
+  DT_CHECK(grow(processed_, cap_pr_, size_t(nnodes), s));
+  DT_CHECK(grow(leaf_ids_, cap_leaf_, size_t(max_leaves), s));
   if (n > 0)
     DT_CHECK(cudaMemcpyAsync(table_, epos_, size_t(n) * sizeof(float4), cudaMemcpyDeviceToDevice, s));
-  k_table_pseudo<<<unsigned((nnodes + 127) / 128), 128, 0, s>>>(nodes_, nnodes, ppm_, k, table_, n);
-  ++info_.launches;
+  const unsigned gN = unsigned((nnodes + 127) / 128), gP = unsigned((int64_t(nnodes) * 32 + 127) / 128);
+  k_links<<<gN, 128, 0, s>>>(nodes_, nnodes, up_);
+  if (k == 12)
+    k_pseudo_up<12><<<gP, 128, 0, s>>>(nodes_, nnodes, up_, epos_, ppm_, table_, n, cfg, processed_);
+  else
+    k_pseudo_up<1><<<gP, 128, 0, s>>>(nodes_, nnodes, up_, epos_, ppm_, table_, n, cfg, processed_);
+  k_leaf_rank<<<gN, 128, 0, s>>>(nodes_, nnodes, up_, processed_, leaf_ids_, counters_);
+  info_.launches += 3;
   DT_CHECK(cudaGetLastError());
-
-  // ---- processed leaves in DFS order ----
-  const int64_t nl_cap = std::max<int64_t>(n, 1);
-  DT_CHECK(grow(leaf_tmp_, cap_lt_, size_t(2 * nl_cap), s));
-  DT_CHECK(grow(leaf_ids_, cap_leaf_, size_t(nl_cap), s));
-  DT_CHECK(grow(scan_tmp_, cap_scan_, size_t(scan_tmp_size(nl_cap)), s));
-  int64_t *leaf_at = leaf_tmp_, *lflag = leaf_tmp_ + nl_cap;
-  k_fill_i64<<<grid_for(nl_cap, 256), 256, 0, s>>>(leaf_at, nl_cap, -1);
-  ++info_.launches;
-  k_mark_leaves<<<unsigned((nnodes + 127) / 128), 128, 0, s>>>(nodes_, nnodes, cfg, n, leaf_at);
-  ++info_.launches;
-  k_leaf_flags<<<unsigned((nl_cap + 255) / 256), 256, 0, s>>>(leaf_at, nl_cap, lflag);
-  ++info_.launches;
-  DT_CHECK(scan_counted(lflag, lflag, nl_cap, counters_ + C_NLEAF, scan_tmp_, s));
-  k_leaf_compact<<<unsigned((nl_cap + 255) / 256), 256, 0, s>>>(leaf_at, lflag, nl_cap, leaf_ids_);
-  ++info_.launches;
-  DT_CHECK(cudaGetLastError());
-  DT_CHECK(cudaMemcpyAsync(h_counters_ + C_NLEAF, counters_ + C_NLEAF, sizeof(int64_t),
-                           cudaMemcpyDeviceToHost, s));
-  DT_CHECK(cudaStreamSynchronize(s));
-  const int64_t nleaves = h_counters_[C_NLEAF];
-  info_.processed_leaves = nleaves;
   // the groups need only the leaves: on the second stream, beside the walk
   // (forked here, launched after the walk)
   group_ = cfg.group == 16 ? 16 : 32;
   DT_CHECK(grow(gidx_, cap_gidx_, size_t(std::max<int64_t>(n, 1)), s));
-  if (nleaves > 0) {
-    if (!aux_) {
-      DT_CHECK(cudaStreamCreateWithFlags(&aux_, cudaStreamNonBlocking));
-      DT_CHECK(cudaEventCreateWithFlags(&ev_fork_, cudaEventDisableTiming));
-      DT_CHECK(cudaEventCreateWithFlags(&ev_groups_, cudaEventDisableTiming));
-    }
-    DT_CHECK(cudaEventRecord(ev_fork_, s));
-    DT_CHECK(cudaStreamWaitEvent(aux_, ev_fork_, 0));
+  if (!aux_) {
+    DT_CHECK(cudaStreamCreateWithFlags(&aux_, cudaStreamNonBlocking));
+    DT_CHECK(cudaEventCreateWithFlags(&ev_fork_, cudaEventDisableTiming));
+    DT_CHECK(cudaEventCreateWithFlags(&ev_groups_, cudaEventDisableTiming));
   }
+  DT_CHECK(cudaEventRecord(ev_fork_, s));
+  DT_CHECK(cudaStreamWaitEvent(aux_, ev_fork_, 0));
 
   // ---- lists: count, scan, write ----
-  const size_t nlw = size_t(std::max<int64_t>(nleaves, 1));
+  const size_t nlw = size_t(max_leaves);
   DT_CHECK(grow(node_tmp_, cap_nt_, 5 * nlw + 4, s));
   int64_t *seg_cnt = node_tmp_, *list_len = node_tmp_ + nlw, *seg_base = node_tmp_ + 2 * nlw,
           *list_base = node_tmp_ + 3 * nlw;
@@ -3685,23 +3732,26 @@ cudaError_t DeviceTree::build(const TreeConfig &cfg, int64_t n, const float4 *po
   // build to a second, placing walk)
   DT_CHECK(grow(segs_local_, cap_segl_, nlw * kLocalSegs, s));
   DT_CHECK(cudaMemsetAsync(counters_ + C_SEGOVF, 0, sizeof(int64_t), s));
-  const unsigned gW = unsigned((nleaves + kWalkWarps - 1) / kWalkWarps);
-  if (nleaves > 0) {
-    k_walk<2><<<gW, 32 * kWalkWarps, 0, s>>>(nodes_, nnodes, leaf_ids_, nleaves, cfg, n, seg_cnt,
-                                             list_len, nullptr, nullptr, nullptr, segs_local_,
-                                             walk_err_, counters_);
+  k_walk<2><<<unsigned((max_leaves + kWalkWarps - 1) / kWalkWarps), 32 * kWalkWarps, 0, s>>>(
+      nodes_, nnodes, leaf_ids_, max_leaves, cfg, n, seg_cnt, list_len, nullptr, nullptr, nullptr,
+      segs_local_, walk_err_, counters_);
+  ++info_.launches;
+  // the groups after the walk's blocks, which then have their SMs first
+  DT_CHECK(launch_groups(max_leaves, group_, aux_));
+  DT_CHECK(cudaEventRecord(ev_groups_, aux_));
+  groups_ready_ = group_;
+  if (max_leaves <= kScanPairMax) {
+    k_scan_pair<<<1, kScanThreads, 0, s>>>(seg_cnt, list_len, seg_base, list_base, max_leaves,
+                                           counters_ + C_NSEG, counters_ + C_NENT);
     ++info_.launches;
-    // the groups after the walk's blocks, which then have their SMs first
-    DT_CHECK(launch_groups(nleaves, group_, aux_));
-    DT_CHECK(cudaEventRecord(ev_groups_, aux_));
-    groups_ready_ = group_;
-    DT_CHECK(scan_counted(seg_cnt, seg_base, nleaves, counters_ + C_NSEG, scan_tmp_, s));
-    DT_CHECK(scan_counted(list_len, list_base, nleaves, counters_ + C_NENT, scan_tmp_, s));
+  } else {
+    DT_CHECK(scan_counted(seg_cnt, seg_base, max_leaves, counters_ + C_NSEG, scan_tmp_, s));
+    DT_CHECK(scan_counted(list_len, list_base, max_leaves, counters_ + C_NENT, scan_tmp_, s));
   }
   DT_CHECK(cudaGetLastError());
-  // segments, entries, the overflow flag and the error flag in one copy
-  DT_CHECK(cudaMemcpyAsync(h_counters_ + C_NSEG, counters_ + C_NSEG,
-                           (C_ERR + 1 - C_NSEG) * sizeof(int64_t), cudaMemcpyDeviceToHost, s));
+  // leaves, segments, entries, the overflow flag and the error flag in one copy
+  DT_CHECK(cudaMemcpyAsync(h_counters_ + C_NLEAF, counters_ + C_NLEAF,
+                           (C_ERR + 1 - C_NLEAF) * sizeof(int64_t), cudaMemcpyDeviceToHost, s));
   DT_CHECK(cudaStreamSynchronize(s));
   const int32_t h_err = *reinterpret_cast<const int32_t *>(h_counters_ + C_ERR);
   if (h_err) {
@@ -3709,18 +3759,23 @@ cudaError_t DeviceTree::build(const TreeConfig &cfg, int64_t n, const float4 *po
                       : "interaction-list walk visited more nodes than the tree has";
     return cudaErrorUnknown;
   }
-  const int64_t nseg = nleaves > 0 ? h_counters_[C_NSEG] : 0;
-  const int64_t nent = nleaves > 0 ? h_counters_[C_NENT] : 0;
+  const int64_t nleaves = h_counters_[C_NLEAF];
+  info_.processed_leaves = nleaves;
+  const int64_t nseg = h_counters_[C_NSEG];
+  const int64_t nent = h_counters_[C_NENT];
   info_.segments = nseg;
   info_.list_entries = nent;
   DT_CHECK(grow(segs_, cap_seg_, size_t(std::max<int64_t>(nseg, 1)), s));
   DT_CHECK(grow(idx_list_, cap_idx_, size_t(std::max<int64_t>(nent, 1)), s));
   DT_CHECK(grow(leafdesc_, cap_ld_, nlw, s));
+  DT_CHECK(cudaMemsetAsync(counters_ + C_BUCKET, 0, 32 * sizeof(int64_t), s));
+  DT_CHECK(cudaMemsetAsync(counters_ + C_TICKET, 0, sizeof(int64_t), s));
   if (nleaves > 0) {
     int64_t *kept = node_tmp_ + 4 * nlw;
     const unsigned blocks =
         unsigned(std::min<int64_t>((nleaves + 7) / 8, int64_t(sm_count()) * 64));
     if (h_counters_[C_SEGOVF]) {
+      const unsigned gW = unsigned((nleaves + kWalkWarps - 1) / kWalkWarps);
       k_walk<1><<<gW, 32 * kWalkWarps, 0, s>>>(nodes_, nnodes, leaf_ids_, nleaves, cfg, n, nullptr,
                                                nullptr, seg_base, list_base, segs_, nullptr,
                                                walk_err_, counters_);
@@ -3734,14 +3789,14 @@ cudaError_t DeviceTree::build(const TreeConfig &cfg, int64_t n, const float4 *po
                                                    idx_list_, kept);
     }
     ++info_.launches;
-    k_leaf_desc<<<unsigned((nleaves + 127) / 128), 128, 0, s>>>(
-        nodes_, leaf_ids_, nleaves, list_len, kept, list_base, leafdesc_, counters_);
+    k_leaf_items<true><<<unsigned((nleaves + 127) / 128), 128, 0, s>>>(
+        nodes_, leaf_ids_, nleaves, list_len, kept, list_base, leafdesc_, jsplit, group_, counters_);
     ++info_.launches;
   }
   DT_CHECK(cudaGetLastError());
 
   // ---- work items ----
-  DT_CHECK(make_items(n, jsplit, s));
+  DT_CHECK(fill_items(jsplit, s));
   lists_ms_ = std::chrono::duration<double, std::milli>(std::chrono::steady_clock::now() - t1).count();
   return cudaSuccess;
 }
@@ -3762,37 +3817,32 @@ cudaError_t DeviceTree::scan_counted(const int64_t *in, int64_t *out, int64_t n,
 cudaError_t DeviceTree::regroup(int group, int64_t jsplit, cudaStream_t s) {
   if (group != 16 && group != 32) return cudaErrorInvalidValue;
   group_ = group;
-  return make_items(n_, jsplit, s);
+  const int64_t nleaves = info_.processed_leaves;
+  DT_CHECK(cudaMemsetAsync(counters_ + C_BUCKET, 0, 32 * sizeof(int64_t), s));
+  DT_CHECK(cudaMemsetAsync(counters_ + C_TICKET, 0, sizeof(int64_t), s));
+  if (nleaves > 0) {
+    DT_CHECK(launch_groups(nleaves, group, s));
+    k_leaf_items<false><<<unsigned((nleaves + 127) / 128), 128, 0, s>>>(
+        nullptr, nullptr, nleaves, nullptr, nullptr, nullptr, leafdesc_, jsplit, group, counters_);
+    ++info_.launches;
+  }
+  return fill_items(jsplit, s);
 }
 
-cudaError_t DeviceTree::launch_groups(int64_t nleaves, int G, cudaStream_t s) {
-  k_groups_warp<<<unsigned((nleaves + kGWarps - 1) / kGWarps), 32 * kGWarps, 0, s>>>(
-      nodes_, leaf_ids_, nleaves, epos_, gidx_, G);
-  k_groups<<<unsigned(nleaves), kGroupThreads, 0, s>>>(nodes_, leaf_ids_, nleaves, epos_, gidx_, G);
+cudaError_t DeviceTree::launch_groups(int64_t max_leaves, int G, cudaStream_t s) {
+  k_groups_warp<<<unsigned((max_leaves + kGWarps - 1) / kGWarps), 32 * kGWarps, 0, s>>>(
+      nodes_, leaf_ids_, counters_ + C_NLEAF, epos_, gidx_, G);
+  k_groups<<<unsigned((max_leaves + kGroupThreads - 1) / kGroupThreads), kGroupThreads, 0, s>>>(
+      nodes_, leaf_ids_, counters_ + C_NLEAF, epos_, gidx_, G);
   info_.launches += 2;
   return cudaGetLastError();
 }
 
-cudaError_t DeviceTree::make_items(int64_t n, int64_t jsplit, cudaStream_t s) {
+// The items of the leaves whose buckets k_leaf_items placed; joins the groups.
+cudaError_t DeviceTree::fill_items(int64_t jsplit, cudaStream_t s) {
   const int64_t nleaves = info_.processed_leaves;
-  const int G = group_;
-  DT_CHECK(grow(gidx_, cap_gidx_, size_t(std::max<int64_t>(n, 1)), s));
-  DT_CHECK(cudaMemsetAsync(counters_ + C_BUCKET, 0, 32 * sizeof(int64_t), s));
-  if (nleaves > 0) {
-    if (groups_ready_ == G) {
-      DT_CHECK(cudaStreamWaitEvent(s, ev_groups_, 0));  // launched by build()
-    } else {
-      if (groups_ready_) DT_CHECK(cudaStreamWaitEvent(s, ev_groups_, 0));
-      DT_CHECK(launch_groups(nleaves, G, s));
-    }
-    groups_ready_ = 0;
-    k_item_hist<<<unsigned((nleaves + 127) / 128), 128, 0, s>>>(leafdesc_, nleaves, jsplit, G,
-                                                                counters_);
-    ++info_.launches;
-    k_item_bases<<<1, 32, 0, s>>>(counters_);
-    ++info_.launches;
-  }
-  DT_CHECK(cudaGetLastError());
+  if (groups_ready_) DT_CHECK(cudaStreamWaitEvent(s, ev_groups_, 0));  // launched by build()
+  groups_ready_ = 0;
   DT_CHECK(cudaMemcpyAsync(h_counters_, counters_, C_COUNT * sizeof(int64_t), cudaMemcpyDeviceToHost, s));
   DT_CHECK(cudaStreamSynchronize(s));
   const int64_t nitems = nleaves > 0 ? h_counters_[C_NITEMS] : 0;
@@ -3801,13 +3851,11 @@ cudaError_t DeviceTree::make_items(int64_t n, int64_t jsplit, cudaStream_t s) {
   padded_pairs_ = h_counters_[C_PADDED];
   DT_CHECK(grow(items_, cap_items_, size_t(std::max<int64_t>(nitems, 1)), s));
   if (nitems > 0) {
-    k_item_fill<<<unsigned((nleaves + 127) / 128), 128, 0, s>>>(leafdesc_, nleaves, jsplit, G,
+    k_item_fill<<<unsigned((nleaves + 127) / 128), 128, 0, s>>>(leafdesc_, nleaves, jsplit, group_,
                                                                counters_, items_);
     ++info_.launches;
   }
-  DT_CHECK(cudaGetLastError());
-  DT_CHECK(cudaStreamSynchronize(s));
-  return cudaSuccess;
+  return cudaGetLastError();
 }
 
 cudaError_t launch_gather_f32(const float *in, const int32_t *perm, float *out, int64_t n,

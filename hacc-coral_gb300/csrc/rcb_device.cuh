@@ -106,7 +106,7 @@ class DeviceTree {
  private:
   template <typename T>
   cudaError_t grow(T *&p, size_t &cap, size_t count, cudaStream_t s, bool keep = false);
-  cudaError_t make_items(int64_t n, int64_t jsplit, cudaStream_t s);
+  cudaError_t fill_items(int64_t jsplit, cudaStream_t s);
   // exclusive_scan_i64, adding its kernels to info_.launches
   cudaError_t scan_counted(const int64_t *in, int64_t *out, int64_t n, int64_t *total, int64_t *tmp,
                            cudaStream_t s);
@@ -121,8 +121,7 @@ class DeviceTree {
   cudaStream_t aux_ = nullptr;
   cudaEvent_t ev_fork_ = nullptr, ev_groups_ = nullptr;
   int groups_ready_ = 0;  // G of groups launched on aux_ and not yet joined
-  cudaError_t launch_groups(int64_t nleaves, int G, cudaStream_t s);
-  int64_t n_ = 0;
+  cudaError_t launch_groups(int64_t max_leaves, int G, cudaStream_t s);
   // elements: current and scratch (x, y, z, m) + input index
   float4 *epos_ = nullptr, *tpos_ = nullptr;
   int32_t *oid_ = nullptr, *toid_ = nullptr, *idx_ = nullptr;
@@ -156,8 +155,9 @@ class DeviceTree {
   // lists
   int32_t *leaf_ids_ = nullptr;
   size_t cap_leaf_ = 0;
-  int64_t *leaf_tmp_ = nullptr;
-  size_t cap_lt_ = 0;
+  int2 *up_ = nullptr;             // per node: parent, arrivals from below
+  int32_t *processed_ = nullptr;   // per node: processed leaves below it
+  size_t cap_up_ = 0, cap_pr_ = 0;
   LeafDesc *leafdesc_ = nullptr;
   size_t cap_ld_ = 0;
   SegDesc *segs_ = nullptr;
