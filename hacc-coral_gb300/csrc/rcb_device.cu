@@ -43,24 +43,18 @@ __device__ __forceinline__ int lsb_exp(float t) {
 
 constexpr int kChunk = 4096;        // elements per statistics / partition chunk
 constexpr int kChunkThreads = 256;  // threads per chunk (16 elements each)
-constexpr int kNodeMax = 16384;     // largest node the one-block partition takes
-constexpr int kChainSteps = 32;     // chain steps before the one-block partition jumps pointers
+constexpr int kChainSteps = 32;     // chain steps before a subtree block jumps pointers
 constexpr int kPlainSteps = 4;      // single chain steps before the chunk partition jumps runs
 
-enum { C_NCHUNK = 0, C_NSPLIT = 1, C_NFALLBACK = 2, C_NLEAF = 3, C_NSEG = 4, C_NENT = 5,
+enum { C_NFALLBACK = 2, C_NLEAF = 3, C_NSEG = 4, C_NENT = 5,
        C_PAIRS = 6, C_PADDED = 7, C_NITEMS = 8, C_MAXLEN = 9, C_TDONE1 = 10, C_TDONE2 = 11,
-       C_NTIGHT = 12, C_SEGOVF = 13, C_MAXCNT = 14, C_ERR = 15, C_BUCKET = 16, C_FILL = 48,
-       C_SUBFB = 80, C_CHAINS = 81, C_TICKET = 82, C_COUNT = 83 };
+       C_NTIGHT = 12, C_SEGOVF = 13, C_ERR = 15, C_BUCKET = 16, C_FILL = 48,
+       C_SUBFB = 80, C_CHAINS = 81, C_TICKET = 82, C_SEQ = 83, C_COUNT = 84 };
 
 // Segments a leaf's walk can leave in its own region of the one-pass walk (8
 // bytes each); a leaf with more sends the build to a second, placing walk.
 constexpr int kLocalSegs = 256;
 
-__device__ __forceinline__ double warp_sum(double v) {
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-  return v;
-}
 __device__ __forceinline__ float warp_min(float v) {
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) v = fminf(v, __shfl_xor_sync(0xffffffffu, v, o));
@@ -157,20 +151,6 @@ namespace {
 // Level kernels
 // ---------------------------------------------------------------------------
 
-// Number of chunks of each node of the level [nb, ne).
-__global__ void k_chunk_counts(const DNode *nodes, int32_t nb, int32_t ne, int64_t *cnt) {
-  const int32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (nb + i < ne) cnt[i] = (int64_t(nodes[nb + i].count) + kChunk - 1) / kChunk;
-}
-
-__global__ void k_chunk_fill(const DNode *nodes, int32_t nb, int32_t ne, const int64_t *base,
-                             int32_t *chunk_node) {
-  const int32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (nb + i >= ne) return;
-  const int64_t c = (int64_t(nodes[nb + i].count) + kChunk - 1) / kChunk;
-  for (int64_t k = 0; k < c; ++k) chunk_node[base[i] + k] = nb + i;
-}
-
 // Exclusive scan over one block of kScanThreads threads, kScanPer values each
 // (v in, out out); returns the block total to every thread.
 __device__ __forceinline__ int64_t block_exclusive_scan(const int64_t (&v)[kScanPer],
@@ -237,30 +217,101 @@ __global__ void __launch_bounds__(kScanThreads)
   }
 }
 
-// Levels of at most kScanBlock nodes, in one block: the chunks of every node
-// (k_chunk_counts, the scan and k_chunk_fill), the total into *nchunk.
-__global__ void __launch_bounds__(kScanThreads)
-    k_chunk_setup_small(const DNode *nodes, int32_t nb, int32_t ne, int64_t *base,
-                        int32_t *chunk_node, int64_t *counters) {
-  int64_t c[kScanPer], b[kScanPer];
-  const int32_t i0 = int32_t(threadIdx.x) * kScanPer;
+__device__ __forceinline__ float key_of(const float4 &p, int d) {
+  return d == 0 ? p.x : (d == 1 ? p.y : p.z);
+}
+
+// Block-wide exclusive scan of one int per thread.
+__device__ __forceinline__ int block_excl_scan(int v, int *sh_warp, int *total) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  int x = v;
 #pragma unroll
-  for (int k = 0; k < kScanPer; ++k)
-    c[k] = nb + i0 + k < ne ? (int64_t(nodes[nb + i0 + k].count) + kChunk - 1) / kChunk : 0;
-  const int64_t total = block_exclusive_scan(c, b);
+  for (int o = 1; o < 32; o <<= 1) {
+    const int y = __shfl_up_sync(0xffffffffu, x, o);
+    if (lane >= o) x += y;
+  }
+  if (lane == 31) sh_warp[warp] = x;
+  __syncthreads();
+  if (warp == 0) {
+    int w = lane < (int)(blockDim.x >> 5) ? sh_warp[lane] : 0;
 #pragma unroll
-  for (int k = 0; k < kScanPer; ++k) {
-    if (nb + i0 + k >= ne) break;
-    base[i0 + k] = b[k];
-    for (int64_t q = 0; q < c[k]; ++q) chunk_node[b[k] + q] = nb + i0 + k;
+    for (int o = 1; o < 32; o <<= 1) {
+      const int y = __shfl_up_sync(0xffffffffu, w, o);
+      if (lane >= o) w += y;
+    }
+    sh_warp[lane] = w;
   }
-  if (threadIdx.x == 0) {
-    counters[C_NCHUNK] = total;
-    counters[C_NFALLBACK] = 0;  // the level's centre-of-mass lists start empty
-    counters[C_NTIGHT] = 0;
-    counters[C_MAXCNT] = 0;     // the next level's largest node, from the children
-    counters[C_CHAINS] = 0;     // the level's queue of long swap chains
-  }
+  __syncthreads();
+  const int excl = x - v + (warp > 0 ? sh_warp[warp - 1] : 0);
+  *total = sh_warp[(blockDim.x >> 5) - 1];
+  __syncthreads();
+  return excl;
+}
+
+// ---------------------------------------------------------------------------
+// The levels of large nodes.
+//
+// A level is five launches: statistics (k_level_stats), left counts
+// (k_level_count), left elements (k_part_left), right elements
+// (k_part_right) and the long swap chains (k_part_chains), a block per chunk of
+// kChunk elements.  What follows a node's last chunk -- its split decision, the
+// scan of its chunks' left counts -- and what follows the level's last chunk --
+// the children, their chunks -- is done by the block that finishes last, and
+// the level's extent lives in device memory (LevelCtl), so the host launches
+// the levels that the particle count calls for and waits once for all of them.
+// (Seventeen launches and a synchronisation a level took 100 us a level at
+// 32^3 particles and 160 at 128^3.)
+// A level whose centre-of-mass bounds leave a node undecided raises `abort`:
+// the launches after it do nothing, and the host runs the certification
+// kernels for it and goes on from there.
+// ---------------------------------------------------------------------------
+struct LevelSpan {
+  int32_t level;  // which level this slot describes
+  int32_t run;    // 0: no level here (every node fits a subtree, or none is left)
+  int32_t nb, ne;  // its nodes
+  int32_t nchunk;  // chunks of its nodes
+  int32_t maxcnt;  // its largest node
+  int32_t pad[2];
+};
+constexpr int kCtlLevels = 64;
+struct LevelCtl {
+  LevelSpan lev[2];    // by level parity
+  int32_t abort;       // level + 1 of a level with undecided nodes, or 0
+  int32_t sub_ready;   // every node of [sub_nb, sub_ne) fits a subtree block
+  int32_t sub_nb, sub_ne;
+  int32_t sub_parity;  // the element buffer that holds them
+  int32_t done;        // no node was split: the tree is complete
+  unsigned mx_term, mx_mass;  // largest |w x|, |w y|, |w z| and |w|, as bits
+  unsigned ticket;     // chunks of the level counted
+  int32_t next_level;  // the level made last
+  int32_t pad[2];
+  int32_t begin[kCtlLevels];  // first node of a level, by level modulo kCtlLevels
+};
+__device__ __forceinline__ int32_t chunks_of(int32_t count) { return (count + kChunk - 1) / kChunk; }
+
+// Whether level `level` is to be worked on, and its extent.  (Blocks of its
+// statistics may start after another has raised abort for the same level.)
+__device__ __forceinline__ bool level_runs(const LevelCtl *ctl, int32_t level, LevelSpan &S,
+                                           bool stats = false) {
+  S = ctl->lev[level & 1];
+  const int32_t a = *reinterpret_cast<const volatile int32_t *>(&ctl->abort);
+  return S.run && S.level == level && (a == 0 || (stats && a == level + 1));
+}
+
+struct ChunkRange {
+  int32_t node, begin, len, local;  // local: first element's position inside the node
+};
+
+__device__ __forceinline__ ChunkRange chunk_range(const DNode *nodes, const int32_t *chunk_node,
+                                                  const int32_t *chunk_base, int32_t nb,
+                                                  int32_t chunk) {
+  ChunkRange r;
+  r.node = chunk_node[chunk];
+  const DNode &N = nodes[r.node];
+  r.local = (chunk - chunk_base[r.node - nb]) * kChunk;
+  r.begin = N.offset + r.local;
+  r.len = min(kChunk, N.count - r.local);
+  return r;
 }
 
 // Child s (0 left, 1 right) of split node N, as four 16-byte stores.
@@ -284,348 +335,152 @@ __device__ __forceinline__ void write_child(DNode &dst, const DNode &N, int s) {
   for (int w = 0; w < 4; ++w) out[w] = src[w];
 }
 
-// Levels of at most kScanBlock nodes, in one block: k_split_flags, the scan
-// and k_children; the number of split nodes into *nsplit.
-__global__ void __launch_bounds__(kScanThreads)
-    k_children_small(DNode *nodes, int32_t nb, int32_t ne, int64_t *nsplit, int64_t *maxcnt) {
-  int64_t f[kScanPer], r[kScanPer];
-  unsigned m = 0;  // largest child count of this thread's nodes
-  const int32_t i0 = int32_t(threadIdx.x) * kScanPer;
-#pragma unroll
-  for (int k = 0; k < kScanPer; ++k) {
-    f[k] = 0;
-    if (nb + i0 + k < ne) {
-      const DNode &N = nodes[nb + i0 + k];
-      f[k] = (N.split_dim >= 0 && N.nleft > 0 && N.nleft < N.count) ? 1 : 0;
-    }
-  }
-  const int64_t total = block_exclusive_scan(f, r);
-#pragma unroll
-  for (int k = 0; k < kScanPer; ++k) {
-    if (nb + i0 + k >= ne) break;
-    DNode &N = nodes[nb + i0 + k];
-    if (!f[k]) {
-      N.cl = N.cr = 0;
-      continue;
-    }
-    const int32_t cl = ne + 2 * int32_t(r[k]), cr = cl + 1;
-    N.cl = cl;
-    N.cr = cr;
-    m = max(m, unsigned(max(N.nleft, N.count - N.nleft)));
-    // one block writes every child: whole 16-byte words, not field by field
-    for (int s = 0; s < 2; ++s) write_child(nodes[s == 0 ? cl : cr], N, s);
-  }
-  if (threadIdx.x == 0) *nsplit = total;
-  m = __reduce_max_sync(0xffffffffu, m);
-  if ((threadIdx.x & 31) == 0 && m) atomicMax(reinterpret_cast<unsigned long long *>(maxcnt), m);
+// Order-preserving map of a float to an unsigned integer.
+__device__ __forceinline__ uint32_t f2o(float v) {
+  const uint32_t b = __float_as_uint(v);
+  return (b & 0x80000000u) ? ~b : (b | 0x80000000u);
+}
+__device__ __forceinline__ float o2f(uint32_t o) {
+  return __uint_as_float((o & 0x80000000u) ? (o & 0x7fffffffu) : ~o);
 }
 
-struct ChunkRange {
-  int32_t node, begin, len, local;  // local: first element's position inside the node
+// ---------------------------------------------------------------------------
+// Exact sums of float terms on the FP32 and integer pipes.
+//
+// With every |t| below 2^(k-2), the sum v = t + 1.5 2^k stays in one binade, so
+// its bits count t rounded to multiples of 2^(k-23), h = v - 1.5 2^k is exact,
+// and r = t - h (exact, |r| <= 2^(k-24)) goes the same way onto multiples of
+// 2^(k-45): t = iv 2^(k-23) + iv2 2^(k-45) with |iv| <= 2^21, |iv2| <= 2^21, and
+// what is left (terms with bits below 2^(k-45)) marks the node's sums as
+// truncated, by at most half a unit a term.  Sums of the two integers are exact
+// in any order.  Eleven single-rate operations a term; shifting each term into
+// 128-bit fixed point took more than twice as many, and FP64, and every
+// conversion to or from a 64-bit type, runs at a small fraction of that rate on
+// this part.  One scale for the three coordinates' terms and one for the masses,
+// from the largest of the whole set.
+// ---------------------------------------------------------------------------
+struct SumScale {
+  int k;        // the scale's exponent
+  float m1, m2;  // 1.5 2^k and 1.5 2^(k-22)
+  __device__ __forceinline__ explicit SumScale(unsigned mx) {
+    const int e = int(mx >> 23) - 127;  // mx < 2^(e+1); subnormal or zero: -127
+    k = max(e + 3, -80);
+    m1 = __uint_as_float((unsigned(k + 127) << 23) | 0x400000u);
+    m2 = __uint_as_float((unsigned(k - 22 + 127) << 23) | 0x400000u);
+  }
+  // terms too large for the scale's arithmetic, infinities and NaN
+  __device__ static __forceinline__ bool bad(unsigned mx) { return mx >= (247u << 23); }
 };
 
-__device__ __forceinline__ ChunkRange chunk_range(const DNode *nodes, const int32_t *chunk_node,
-                                                  const int64_t *chunk_base, int32_t nb,
-                                                  int64_t chunk) {
-  ChunkRange r;
-  r.node = chunk_node[chunk];
-  const DNode &N = nodes[r.node];
-  const int64_t c = chunk - chunk_base[r.node - nb];
-  r.local = int32_t(c * kChunk);
-  r.begin = N.offset + r.local;
-  r.len = min(kChunk, N.count - r.local);
-  return r;
-}
+// Reduced statistics of a set of elements (a node, a warp's share).
+struct alignas(16) NodeAcc {
+  long long h[4], l[4];     // sums of iv and iv2 (x, y, z, m)
+  unsigned o1[4], o2[4];    // ors of their bits: the terms' least significant one
+  unsigned lo[3], hi[3];    // bounding box (f2o)
+  unsigned wmin;            // smallest mass (f2o)
+  unsigned trunc;           // some term had bits below 2^(k-45)
+};
+static_assert(sizeof(NodeAcc) == 128, "NodeAcc is eight 16-byte words");
 
-// Exact sums in 128-bit fixed point.  A float term t is the integer
-// t 2^-kFix in units of 2^kFix: exact when t's least significant bit is at
-// least 2^kFix, truncated toward zero otherwise (an error below one unit per
-// term, counted in the bound).  Terms below 2^14 convert in hardware
-// (t 2^48 < 2^62 fits an int64); larger ones take a shift, and terms of
-// 2^46 or more flag the chunk (its node takes the sequential sum), which keeps
-// a sum of 2^31 terms below 2^125.  Integer adds avoid the FP64 pipe, which
-// runs at a small fraction of the FP32 rate on this part.
-constexpr int kFix = -48;
-constexpr int kFixMaxShift = 70;  // |t| < 2^(70 + 24 + kFix) = 2^46
-
-// Adds t 2^-kFix to acc; ors |t 2^-kFix| into bits (its lowest set bit is the
-// least significant bit of all terms, when none is truncated).  |t| < 2^14
-// takes a 64-bit shift on the integer pipe; larger terms the 128-bit one.
-// (Conversions to and from 64-bit types run on the FP64 pipe, slow here.)
-__device__ __forceinline__ void fix_add(__int128 &acc, unsigned __int128 &bits, float t,
-                                        bool &overflow, bool &trunc) {
-  const uint32_t b = __float_as_uint(t);
-  const uint32_t a = b & 0x7fffffffu;
-  if (a == 0) return;
-  int e = int(a >> 23);
-  uint32_t m = a & 0x7fffffu;
-  if (e == 0) e = 1;
-  else m |= 0x800000u;
-  const int sh = e - 150 - kFix;
-  unsigned __int128 v;
-  if (sh >= 0 && sh <= 39) {
-    v = (unsigned __int128)((unsigned long long)m << sh);
-  } else if (sh > 39) {
-    if (sh > kFixMaxShift || e == 255) overflow = true;
-    v = (unsigned __int128)m << min(sh, kFixMaxShift);
-  } else {
-    const int r = -sh;
-    const uint32_t kept = r < 32 ? m >> r : 0u;
-    if ((r < 32 ? (kept << r) : 0u) != m) trunc = true;
-    v = kept;
+__device__ __forceinline__ void acc_zero(NodeAcc &a) {
+  for (int q = 0; q < 4; ++q) {
+    a.h[q] = a.l[q] = 0;
+    a.o1[q] = a.o2[q] = 0u;
   }
-  bits |= v;
-  acc += (b >> 31) ? -__int128(v) : __int128(v);
+  for (int d = 0; d < 3; ++d) {
+    a.lo[d] = 0xffffffffu;
+    a.hi[d] = 0u;
+  }
+  a.wmin = 0xffffffffu;
+  a.trunc = 0u;
 }
 
-__device__ __forceinline__ int lsb_of(unsigned __int128 v) {
-  const unsigned long long lo = (unsigned long long)v, hi = (unsigned long long)(v >> 64);
-  if (lo) return __ffsll((long long)lo) - 1;
-  if (hi) return 64 + __ffsll((long long)hi) - 1;
-  return -1;
-}
-
-// The same sum on the integer pipe.  A term t 2^-kFix with 0 <= shift <= 34
-// (2^-24 <= |t| < 2^10, the common case) is m << shift < 2^58, added to a
-// signed 64-bit partial sum; fold() moves the partial sum into the 128-bit
-// sum (four 32-bit limbs, two's complement, least significant first) and is
-// called at least every kFoldTerms adds, so the partial sum stays below 2^62.
-// Other terms take fix_add's wide path straight into the limbs.
-// lsb: the least significant set bit over the terms' magnitudes (in units of
-// 2^kFix), INT_MAX while no term has one.
-constexpr int kFoldTerms = 16;
-struct FixAcc {
-  uint32_t l[4];  // the sum
-  long long acc;  // fast-path terms since the last fold
-  int lsb;
+// One lane's share.
+struct LaneAcc {
+  unsigned h[4], l[4], o1[4], o2[4];  // sums of the bits of v and v2 (modulo 2^32)
+  float lo[3], hi[3], wmin, left;
   __device__ __forceinline__ void zero() {
 #pragma unroll
-    for (int k = 0; k < 4; ++k) l[k] = 0u;
-    acc = 0;
-    lsb = INT_MAX;
-  }
-  __device__ __forceinline__ void add_limbs(uint32_t v0, uint32_t v1, uint32_t v2, uint32_t v3) {
-    asm("add.cc.u32 %0, %0, %4;\n\taddc.cc.u32 %1, %1, %5;\n\taddc.cc.u32 %2, %2, %6;\n\t"
-        "addc.u32 %3, %3, %7;"
-        : "+r"(l[0]), "+r"(l[1]), "+r"(l[2]), "+r"(l[3])
-        : "r"(v0), "r"(v1), "r"(v2), "r"(v3));
-  }
-  __device__ __forceinline__ void fold() {
-    const uint32_t sx = uint32_t(acc >> 63);  // sign extension: 0 or all ones
-    add_limbs(uint32_t(acc), uint32_t((unsigned long long)acc >> 32), sx, sx);
-    acc = 0;
-  }
-  __device__ __forceinline__ void add(float t, bool &overflow, bool &trunc) {
-    const uint32_t bb = __float_as_uint(t);
-    const uint32_t a = bb & 0x7fffffffu;
-    if (a == 0) return;
-    int e = int(a >> 23);
-    uint32_t m = a & 0x7fffffu;
-    if (e == 0) e = 1;
-    else m |= 0x800000u;
-    const int sh = e - 150 - kFix;
-    if (unsigned(sh) <= 34u) {
-      lsb = min(lsb, sh + __ffs(int(m)) - 1);  // m != 0 here
-      const long long v = (long long)((unsigned long long)m << sh);
-      acc += (bb >> 31) ? -v : v;
-    } else {
-      __int128 w = 0;
-      unsigned __int128 wb = 0;
-      fix_add(w, wb, t, overflow, trunc);
-      if (wb) lsb = min(lsb, lsb_of(wb));
-      const unsigned __int128 u = (unsigned __int128)w;  // +/- v in two's complement
-      add_limbs(uint32_t(u), uint32_t(u >> 32), uint32_t(u >> 64), uint32_t(u >> 96));
+    for (int q = 0; q < 4; ++q) h[q] = l[q] = o1[q] = o2[q] = 0u;
+#pragma unroll
+    for (int d = 0; d < 3; ++d) {
+      lo[d] = INFINITY;
+      hi[d] = -INFINITY;
     }
+    wmin = INFINITY;
+    left = 0.f;
   }
-  // the 128-bit sum (after a fold)
-  __device__ __forceinline__ __int128 sum() const {
-    const unsigned __int128 u = ((unsigned __int128)l[3] << 96) | ((unsigned __int128)l[2] << 64) |
-                                ((unsigned __int128)l[1] << 32) | (unsigned __int128)l[0];
-    return __int128(u);
+  __device__ __forceinline__ void term(int q, float t, float m1, float m2) {
+    const float v = __fadd_rn(t, m1);
+    const float r = __fsub_rn(t, __fsub_rn(v, m1));
+    const float v2 = __fadd_rn(r, m2);
+    left = fmaxf(left, fabsf(__fsub_rn(__fsub_rn(v2, m2), r)));
+    h[q] += __float_as_uint(v);
+    l[q] += __float_as_uint(v2);
+    o1[q] |= __float_as_uint(v);
+    o2[q] |= __float_as_uint(v2);
+  }
+  __device__ __forceinline__ void add(const float4 &p, const SumScale &sc, const SumScale &sm) {
+    term(0, fmul_(p.w, p.x), sc.m1, sc.m2);
+    term(1, fmul_(p.w, p.y), sc.m1, sc.m2);
+    term(2, fmul_(p.w, p.z), sc.m1, sc.m2);
+    term(3, p.w, sm.m1, sm.m2);
+    lo[0] = fminf(lo[0], p.x); hi[0] = fmaxf(hi[0], p.x);
+    lo[1] = fminf(lo[1], p.y); hi[1] = fmaxf(hi[1], p.y);
+    lo[2] = fminf(lo[2], p.z); hi[2] = fmaxf(hi[2], p.z);
+    wmin = fminf(wmin, p.w);
+  }
+  // The warp's sum, the same on every lane; cnt: this lane's elements (at most
+  // 512), few: the warp's are at most 1023 (an int holds their sums).
+  __device__ __forceinline__ void reduce(NodeAcc &a, int cnt, bool few, const SumScale &sc,
+                                         const SumScale &sm) const {
+    const unsigned full = 0xffffffffu;
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+      const SumScale &s = q < 3 ? sc : sm;
+      const int hv = int(h[q] - unsigned(cnt) * __float_as_uint(s.m1));
+      const int lv = int(l[q] - unsigned(cnt) * __float_as_uint(s.m2));
+      if (few) {
+        a.h[q] = __reduce_add_sync(full, hv);
+        a.l[q] = __reduce_add_sync(full, lv);
+      } else {
+        a.h[q] = (long long)(__reduce_add_sync(full, hv >> 16)) * 65536 +
+                 __reduce_add_sync(full, unsigned(hv) & 0xffffu);
+        a.l[q] = (long long)(__reduce_add_sync(full, lv >> 16)) * 65536 +
+                 __reduce_add_sync(full, unsigned(lv) & 0xffffu);
+      }
+      a.o1[q] = __reduce_or_sync(full, o1[q]);
+      a.o2[q] = __reduce_or_sync(full, o2[q]);
+    }
+#pragma unroll
+    for (int d = 0; d < 3; ++d) {
+      a.lo[d] = __reduce_min_sync(full, f2o(lo[d]));
+      a.hi[d] = __reduce_max_sync(full, f2o(hi[d]));
+    }
+    a.wmin = __reduce_min_sync(full, f2o(wmin));
+    a.trunc = __any_sync(full, left != 0.f) ? 1u : 0u;
   }
 };
 
-__device__ __forceinline__ __int128 shfl_xor_i128(__int128 v, int o) {
-  const unsigned long long lo = (unsigned long long)v, hi = (unsigned long long)(v >> 64);
-  const unsigned long long l2 = __shfl_xor_sync(0xffffffffu, lo, o);
-  const unsigned long long h2 = __shfl_xor_sync(0xffffffffu, hi, o);
-  return (__int128(h2) << 64) | __int128(l2);
+__device__ __forceinline__ double pow2(int e) {  // normal range
+  return __longlong_as_double((long long)(e + 1023) << 52);
 }
 
-// Correctly rounded double of v 2^kFix: the top 63 bits of |v| with the
-// rest folded into a sticky bit, rounded once by the conversion.
-__device__ double fix_to_double(__int128 v) {
+// Correctly rounded double of h 2^(k-23) + l 2^(k-45).
+__device__ double sum_to_double(long long h, long long l, int k) {
+  const double unit = pow2(k - 45);
+  if (h < (1ll << 40) && h > -(1ll << 40)) return __dmul_rn(__ll2double_rn((h << 22) + l), unit);
+  const __int128 v = (__int128(h) << 22) + l;
   const bool neg = v < 0;
   const unsigned __int128 u = neg ? (unsigned __int128)(-v) : (unsigned __int128)v;
   const unsigned long long hi = (unsigned long long)(u >> 64), lo = (unsigned long long)u;
-  const int bits = hi ? 128 - __clzll((long long)hi) : (lo ? 64 - __clzll((long long)lo) : 0);
-  const int k = bits > 63 ? bits - 63 : 0;
-  unsigned long long m = (unsigned long long)(u >> k);
-  if (k > 0 && (u & ((((unsigned __int128)1) << k) - 1)) != 0) m |= 1ull;
-  const double r = ldexp(__ull2double_rn(m), k + kFix);
+  const int bits = hi ? 128 - __clzll((long long)hi) : 64 - __clzll((long long)lo);
+  const int sh = bits > 63 ? bits - 63 : 0;
+  // the top 63 bits with the rest folded into a sticky bit, rounded once
+  unsigned long long m = (unsigned long long)(u >> sh);
+  if (sh > 0 && (u & ((((unsigned __int128)1) << sh) - 1)) != 0) m |= 1ull;
+  const double r = __dmul_rn(__dmul_rn(__ull2double_rn(m), pow2(sh)), unit);
   return neg ? -r : r;
-}
-
-// Layout of a chunk's partial record (in 8-byte words): sums of the terms
-// (x, y, z, m) as 4 x int128, upper bounds of the sums of |terms| (4 doubles),
-// the bounding box (6 floats), the least significant exponents (4 ints) and
-// an overflow flag.
-constexpr int kPartWords = 18;
-
-// The chunk kernels run a block per chunk, or (WM, on deep levels where
-// nodes are small) a warp per chunk, 8 chunks per block.
-#define CHUNK_PROLOGUE                                                                  \
-  const int lane_ = threadIdx.x & 31;                                                 \
-  const int64_t chunk =                                                               \
-      WM ? int64_t(blockIdx.x) * (kChunkThreads / 32) + (threadIdx.x >> 5) : int64_t(blockIdx.x); \
-  const int tid = WM ? lane_ : int(threadIdx.x);                                      \
-  constexpr int NT = WM ? 32 : kChunkThreads;                                         \
-  (void)lane_;                                                                        \
-  (void)tid;                                                                          \
-  (void)NT;                                                                           \
-  if (chunk >= *nchunk) return;
-
-// Partial sums of one chunk and its bounding box.  Fixed thread-to-element
-// map and reduction tree.
-template <bool WM>
-__global__ void __launch_bounds__(kChunkThreads, 4)
-    k_stats_partial(const float4 *__restrict__ pos, const DNode *nodes,
-                    const int32_t *chunk_node, const int64_t *chunk_base, int32_t nb,
-                    const int64_t *nchunk, double *part) {
-  CHUNK_PROLOGUE
-  const ChunkRange R = chunk_range(nodes, chunk_node, chunk_base, nb, chunk);
-  __int128 s[4] = {0, 0, 0, 0};
-  float fa[4] = {0.f, 0.f, 0.f, 0.f};
-  float lo[3] = {INFINITY, INFINITY, INFINITY}, hi[3] = {-INFINITY, -INFINITY, -INFINITY};
-  bool ovf = false;
-  bool trn[4] = {false, false, false, false};
-  // four loads in flight per thread; the elements are then taken in the same
-  // order as one at a time
-  constexpr int kU = 2;
-  FixAcc fx[4];
-#pragma unroll
-  for (int q = 0; q < 4; ++q) fx[q].zero();
-  int it = 0;
-  for (int k0 = tid; k0 < R.len; k0 += NT * kU, ++it) {
-    float4 pu[kU];
-#pragma unroll
-    for (int u = 0; u < kU; ++u)
-      if (k0 + u * NT < R.len) pu[u] = pos[R.begin + k0 + u * NT];
-#pragma unroll
-    for (int u = 0; u < kU; ++u) {
-      if (k0 + u * NT >= R.len) break;
-      const float4 p = pu[u];
-      const float w = p.w;
-      const float t[4] = {fmul_(w, p.x), fmul_(w, p.y), fmul_(w, p.z), w};
-#pragma unroll
-      for (int q = 0; q < 4; ++q) {
-        fx[q].add(t[q], ovf, trn[q]);
-        fa[q] = __fadd_ru(fa[q], fabsf(t[q]));
-      }
-      lo[0] = fminf(lo[0], p.x); hi[0] = fmaxf(hi[0], p.x);
-      lo[1] = fminf(lo[1], p.y); hi[1] = fmaxf(hi[1], p.y);
-      lo[2] = fminf(lo[2], p.z); hi[2] = fmaxf(hi[2], p.z);
-    }
-    if ((it + 1) % (kFoldTerms / kU) == 0) {
-#pragma unroll
-      for (int q = 0; q < 4; ++q) fx[q].fold();
-    }
-  }
-  int lsb[4];
-#pragma unroll
-  for (int q = 0; q < 4; ++q) {
-    fx[q].fold();
-    s[q] = fx[q].sum();
-    lsb[q] = __reduce_min_sync(0xffffffffu, fx[q].lsb);
-  }
-  double a[4];
-  int emin[4];
-#pragma unroll
-  for (int q = 0; q < 4; ++q) {
-    for (int o = 16; o > 0; o >>= 1) {
-      s[q] += shfl_xor_i128(s[q], o);
-      fa[q] = __fadd_ru(fa[q], __shfl_xor_sync(0xffffffffu, fa[q], o));
-    }
-    a[q] = double(fa[q]);
-    const bool tq = __any_sync(0xffffffffu, trn[q]);
-    // least significant exponent of the warp's terms; below kFix if any term
-    // lost bits to the truncation, INT_MAX if all are zero
-    emin[q] = tq ? kFix - 1 : (lsb[q] == INT_MAX ? INT_MAX : kFix + lsb[q]);
-  }
-#pragma unroll
-  for (int d = 0; d < 3; ++d) {
-    lo[d] = warp_min(lo[d]);
-    hi[d] = warp_max(hi[d]);
-  }
-  const bool wovf = __any_sync(0xffffffffu, ovf);
-  if (WM) {
-    if (lane_ == 0) {
-      double *o = part + chunk * kPartWords;
-      __int128 *os = reinterpret_cast<__int128 *>(o);
-      for (int q = 0; q < 4; ++q) os[q] = s[q];
-      for (int q = 0; q < 4; ++q) o[8 + q] = a[q];
-      float *ob = reinterpret_cast<float *>(o + 12);
-      for (int d = 0; d < 3; ++d) {
-        ob[d] = lo[d];
-        ob[3 + d] = hi[d];
-      }
-      int *oe = reinterpret_cast<int *>(o + 15);
-      for (int q = 0; q < 4; ++q) oe[q] = emin[q];
-      oe[4] = wovf ? 1 : 0;
-    }
-    return;
-  }
-  __shared__ __int128 shs[kChunkThreads / 32][4];
-  __shared__ double sha[kChunkThreads / 32][4];
-  __shared__ float shb[kChunkThreads / 32][6];
-  __shared__ int she[kChunkThreads / 32][5];
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  if (lane == 0) {
-    for (int q = 0; q < 4; ++q) {
-      shs[warp][q] = s[q];
-      sha[warp][q] = a[q];
-      she[warp][q] = emin[q];
-    }
-    for (int d = 0; d < 3; ++d) {
-      shb[warp][d] = lo[d];
-      shb[warp][3 + d] = hi[d];
-    }
-    she[warp][4] = wovf ? 1 : 0;
-  }
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    __int128 ts[4];
-    double ta[4];
-    float tb[6];
-    int te[5];
-    for (int q = 0; q < 4; ++q) {
-      ts[q] = shs[0][q];
-      ta[q] = sha[0][q];
-      te[q] = she[0][q];
-    }
-    for (int d = 0; d < 6; ++d) tb[d] = shb[0][d];
-    te[4] = she[0][4];
-    for (int w = 1; w < kChunkThreads / 32; ++w) {
-      for (int q = 0; q < 4; ++q) {
-        ts[q] += shs[w][q];
-        ta[q] += sha[w][q];
-        te[q] = min(te[q], she[w][q]);
-      }
-      for (int d = 0; d < 3; ++d) {
-        tb[d] = fminf(tb[d], shb[w][d]);
-        tb[3 + d] = fmaxf(tb[3 + d], shb[w][3 + d]);
-      }
-      te[4] |= she[w][4];
-    }
-    double *o = part + chunk * kPartWords;
-    __int128 *os = reinterpret_cast<__int128 *>(o);
-    for (int q = 0; q < 4; ++q) os[q] = ts[q];
-    for (int q = 0; q < 4; ++q) o[8 + q] = ta[q];
-    float *ob = reinterpret_cast<float *>(o + 12);
-    for (int d = 0; d < 6; ++d) ob[d] = tb[d];
-    int *oe = reinterpret_cast<int *>(o + 15);
-    for (int q = 0; q < 5; ++q) oe[q] = te[q];
-  }
 }
 
 // Float that the reference's (float)(sx / sm) gives, if the bounds decide it.
@@ -646,16 +501,15 @@ __device__ bool certify(double sx, double bx, double sm, double bm, float *out) 
   return true;
 }
 
-// Sets a node's bounding box and, where decided, its centre of mass from the
-// reduced sums; lists it for the tight certification otherwise.
 // The node's box, split axis and (where the bounds decide it) centre of mass
-// from the reduced sums; false when the centre of mass is left undecided.
-__device__ bool decide_node(DNode &N, const __int128 *s, double *a, const float *lo,
-                            const float *hi, const int *emin, bool ovf, int32_t force_fallback,
-                            int32_t nd) {
+// from its reduced statistics; false when the centre of mass is left undecided.
+// One FP64 division a coordinate: the quotient's error bound is taken in float,
+// rounded up.
+__device__ bool decide_node(DNode &N, const NodeAcc &A, const SumScale &sc, const SumScale &sm,
+                            bool bad, int32_t force_fallback, int32_t nd) {
   for (int d = 0; d < 3; ++d) {
-    N.xmin[d] = lo[d];
-    N.xmax[d] = hi[d];
+    N.xmin[d] = o2f(A.lo[d]);
+    N.xmax[d] = o2f(A.hi[d]);
   }
   // leaf by size, or the split axis: the longest box edge, ties to the later
   // axis (RCBForceTree.cxx:837-852); it needs the box only, not the centre
@@ -667,186 +521,564 @@ __device__ bool decide_node(DNode &N, const __int128 *s, double *a, const float 
                 l2 = fsub_(N.xmax[2], N.xmin[2]);
     N.split_dim = (l0 > l1 && l0 > l2) ? 0 : (l1 > l2 ? 1 : 2);
   }
-  // Sums of |terms|: float partials rounded up, added in double; the factor
-  // covers the double additions' rounding.
-  for (int q = 0; q < 4; ++q) a[q] *= 1.0 + 0x1p-30;
+  if (force_fallback != 0 || bad) return false;
   const double n = double(N.count);
   // The reference's sequential sum lies within (n - 1) u sum|terms| of the
   // exact sum, to first order; 2 (n + 64) u covers the rest.  This sum is
-  // exact except for the truncation of terms with bits below 2^kFix (under
-  // 2^kFix each) and its rounding to double.
+  // exact except for truncated terms (half a unit each) and its rounding to
+  // double.
   const double g = 2.0 * (n + 64.0) * 0x1p-53;
-  double sd[4];
-  bool exact_ok[4];
+  const bool wpos = o2f(A.wmin) >= 0.f;
+  double sd[4], bd[4];
+  bool exact[4];
+#pragma unroll
   for (int q = 0; q < 4; ++q) {
-    sd[q] = fix_to_double(s[q]);
+    const int k = q < 3 ? sc.k : sm.k;
+    sd[q] = sum_to_double(A.h[q], A.l[q], k);
+    const double slack = A.trunc ? n * pow2(k - 45) : 0.0;
+    // sum of |terms|: the sum itself where none is negative, else n times the
+    // scale's largest term
+    const bool pos = wpos && (q == 3 || o2f(A.lo[q]) >= 0.f);
+    const double a = pos ? fabs(sd[q]) * (1.0 + 0x1p-50) + slack : n * pow2(k - 2);
     // Exact: every term a multiple of 2^emin (none truncated) and the
     // magnitudes summing below 2^(53 + emin) -- then the reference's
     // sequential sum and this one are the same exact value, a double.
-    if (emin[q] == INT_MAX) exact_ok[q] = true;  // all terms zero
-    else exact_ok[q] = emin[q] >= kFix && a[q] < ldexp(1.0, 53 + emin[q]);
+    const unsigned b2 = A.o2[q] & 0x3fffffu, b1 = A.o1[q] & 0x3fffffu;
+    const int emin = b2 ? k - 45 + __ffs(int(b2)) - 1 : (b1 ? k - 23 + __ffs(int(b1)) - 1 : 1000);
+    exact[q] = !A.trunc && (emin == 1000 || a < pow2(min(53 + emin, 1000)));
+    bd[q] = g * a + fabs(sd[q]) * 0x1p-52 + slack;
   }
-  bool ok = force_fallback == 0 && !ovf;
-  for (int d = 0; d < 3 && ok; ++d) {
-    float v;
-    if (exact_ok[3] && exact_ok[d] && sd[3] != 0.0) {
-      N.xc[d] = __double2float_rn(__ddiv_rn(sd[d], sd[3]));
+  bool ok = true;
+#pragma unroll
+  for (int d = 0; d < 3; ++d) {
+    const double q = __ddiv_rn(sd[d], sd[3]);
+    const float f = __double2float_rn(q);
+    if (exact[3] && exact[d] && sd[3] != 0.0) {
+      N.xc[d] = f;
       continue;
     }
-    double bd[2];
-    const int qs[2] = {d, 3};
-    for (int t = 0; t < 2; ++t) {
-      const int q = qs[t];
-      const bool trunc = emin[q] != INT_MAX && emin[q] < kFix;
-      bd[t] = g * a[q] + fabs(sd[q]) * 0x1p-52 + (trunc ? n * ldexp(1.0, kFix) : 0.0);
+    // |reference quotient - q| <= (bx + |q| bm) / (sm - bm), and both
+    // quotients' own rounding
+    const double ml = sd[3] - bd[3];
+    if (!(ml > 0.0) || !isfinite(q)) {
+      ok = false;
+      continue;
     }
-    if (certify(sd[d], bd[0], sd[3], bd[1], &v)) N.xc[d] = v;
+    const float qa = __double2float_ru(fabs(q));
+    const float num = __fmaf_ru(qa, __double2float_ru(bd[3]), __double2float_ru(bd[d]));
+    const float e = __fadd_ru(__fdiv_ru(num, __double2float_rd(ml)), __fmul_ru(qa, 0x1p-50f));
+    const double w = double(e) * (1.0 + 0x1p-20);
+    const float fl = __double2float_rn(__dadd_rd(q, -w)), fh = __double2float_rn(__dadd_ru(q, w));
+    if (fl == fh) N.xc[d] = fl;
     else ok = false;
   }
   return ok;
 }
 
-__device__ void finish_node(DNode &N, int32_t node, const __int128 *s, double *a, const float *lo,
-                            const float *hi, const int *emin, bool ovf, int32_t *fallback,
-                            int64_t *counters, int32_t force_fallback, int32_t nd) {
-  if (!decide_node(N, s, a, lo, hi, emin, ovf, force_fallback, nd)) {
-    const unsigned long long k = atomicAdd((unsigned long long *)&counters[C_NFALLBACK], 1ull);
-    fallback[k] = node;
-  }
-}
-
-__device__ __forceinline__ void read_part(const double *p, __int128 *s, double *a, float *lo,
-                                          float *hi, int *emin, int &ovf) {
-  const __int128 *ps = reinterpret_cast<const __int128 *>(p);
-  const float *pb = reinterpret_cast<const float *>(p + 12);
-  const int *pe = reinterpret_cast<const int *>(p + 15);
-  for (int q = 0; q < 4; ++q) {
-    s[q] += ps[q];
-    a[q] += p[8 + q];
-    emin[q] = min(emin[q], pe[q]);
-  }
-  for (int d = 0; d < 3; ++d) {
-    lo[d] = fminf(lo[d], pb[d]);
-    hi[d] = fmaxf(hi[d], pb[3 + d]);
-  }
-  ovf |= pe[4];
-}
-
-// One warp per node of more than one chunk: reduce the chunk partials and
-// finish the node.
-__global__ void k_stats_final(DNode *nodes, int32_t nb, int32_t ne, const int64_t *chunk_base,
-                              const double *part, int32_t *fallback, int64_t *counters,
-                              int32_t force_fallback, int32_t nd, bool all) {
-  const int32_t wid = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-  const int lane = threadIdx.x & 31;
-  const int32_t node = nb + wid;
-  if (node >= ne) return;
-  DNode &N = nodes[node];
-  const int64_t nc = (int64_t(N.count) + kChunk - 1) / kChunk;
-  if (N.count <= 0 || (nc <= 1 && !all)) return;  // k_stats_final_one (unless `all`)
-  const int64_t cb = chunk_base[wid];
-  __int128 s[4] = {0, 0, 0, 0};
-  double a[4] = {0, 0, 0, 0};
-  float lo[3] = {INFINITY, INFINITY, INFINITY}, hi[3] = {-INFINITY, -INFINITY, -INFINITY};
-  int emin[4] = {INT_MAX, INT_MAX, INT_MAX, INT_MAX};
-  int ovf = 0;
-  for (int64_t c = lane; c < nc; c += 32) read_part(part + (cb + c) * kPartWords, s, a, lo, hi, emin, ovf);
-  for (int q = 0; q < 4; ++q) {
-    for (int o = 16; o > 0; o >>= 1) s[q] += shfl_xor_i128(s[q], o);
-    a[q] = warp_sum(a[q]);
-  }
-  for (int d = 0; d < 3; ++d) {
-    lo[d] = warp_min(lo[d]);
-    hi[d] = warp_max(hi[d]);
-  }
-  for (int q = 0; q < 4; ++q)
-    for (int o = 16; o > 0; o >>= 1) emin[q] = min(emin[q], __shfl_xor_sync(0xffffffffu, emin[q], o));
-  ovf = __any_sync(0xffffffffu, ovf != 0);
-  if (lane != 0) return;
-  finish_node(N, node, s, a, lo, hi, emin, ovf != 0, fallback, counters, force_fallback, nd);
-}
-
-// One block per node, for the top levels (nodes of many chunks): the warps
-// reduce strided chunk subsets, thread 0 the warps' results, then finishes.
+// The elements into the first buffer, their input indices, and the largest
+// terms for the sums' scale.
 __global__ void __launch_bounds__(256)
-    k_stats_final_block(DNode *nodes, int32_t nb, int32_t ne, const int64_t *chunk_base,
-                        const double *part, int32_t *fallback, int64_t *counters,
-                        int32_t force_fallback, int32_t nd) {
-  const int32_t node = nb + int32_t(blockIdx.x);
-  if (node >= ne) return;
-  DNode &N = nodes[node];
-  if (N.count <= 0) return;
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const int64_t nc = (int64_t(N.count) + kChunk - 1) / kChunk;
-  const int64_t cb = chunk_base[blockIdx.x];
-  __int128 s[4] = {0, 0, 0, 0};
-  double a[4] = {0, 0, 0, 0};
-  float lo[3] = {INFINITY, INFINITY, INFINITY}, hi[3] = {-INFINITY, -INFINITY, -INFINITY};
-  int emin[4] = {INT_MAX, INT_MAX, INT_MAX, INT_MAX};
-  int ovf = 0;
-  for (int64_t c = threadIdx.x; c < nc; c += 256)
-    read_part(part + (cb + c) * kPartWords, s, a, lo, hi, emin, ovf);
-  for (int q = 0; q < 4; ++q) {
-    for (int o = 16; o > 0; o >>= 1) s[q] += shfl_xor_i128(s[q], o);
-    a[q] = warp_sum(a[q]);
-    for (int o = 16; o > 0; o >>= 1) emin[q] = min(emin[q], __shfl_xor_sync(0xffffffffu, emin[q], o));
+    k_elements(const float4 *__restrict__ in, int64_t n, float4 *__restrict__ pos,
+               int32_t *__restrict__ oid, LevelCtl *ctl) {
+  unsigned mt = 0, mm = 0;
+  for (int64_t i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x; i < n;
+       i += int64_t(gridDim.x) * blockDim.x) {
+    const float4 p = in[i];
+    pos[i] = p;
+    oid[i] = int32_t(i);
+    mt = max(mt, __float_as_uint(fmul_(p.w, p.x)) & 0x7fffffffu);
+    mt = max(mt, __float_as_uint(fmul_(p.w, p.y)) & 0x7fffffffu);
+    mt = max(mt, __float_as_uint(fmul_(p.w, p.z)) & 0x7fffffffu);
+    mm = max(mm, __float_as_uint(p.w) & 0x7fffffffu);
   }
-  for (int d = 0; d < 3; ++d) {
-    lo[d] = warp_min(lo[d]);
-    hi[d] = warp_max(hi[d]);
-  }
-  ovf = __any_sync(0xffffffffu, ovf != 0);
-  __shared__ __int128 ws[8][4];
-  __shared__ double wa[8][4];
-  __shared__ float wb[8][6];
-  __shared__ int we[8][5];
-  if (lane == 0) {
-    for (int q = 0; q < 4; ++q) {
-      ws[warp][q] = s[q];
-      wa[warp][q] = a[q];
-      we[warp][q] = emin[q];
-    }
-    for (int d = 0; d < 3; ++d) {
-      wb[warp][d] = lo[d];
-      wb[warp][3 + d] = hi[d];
-    }
-    we[warp][4] = ovf;
+  mt = __reduce_max_sync(0xffffffffu, mt);
+  mm = __reduce_max_sync(0xffffffffu, mm);
+  __shared__ unsigned sh[2];
+  if (threadIdx.x < 2) sh[threadIdx.x] = 0u;
+  __syncthreads();
+  if ((threadIdx.x & 31) == 0) {
+    atomicMax(&sh[0], mt);
+    atomicMax(&sh[1], mm);
   }
   __syncthreads();
-  if (threadIdx.x != 0) return;
-  for (int w = 1; w < 8; ++w) {
-    for (int q = 0; q < 4; ++q) {
-      s[q] += ws[w][q];
-      a[q] += wa[w][q];
-      emin[q] = min(emin[q], we[w][q]);
-    }
-    for (int d = 0; d < 3; ++d) {
-      lo[d] = fminf(lo[d], wb[w][d]);
-      hi[d] = fmaxf(hi[d], wb[w][3 + d]);
-    }
-    ovf |= we[w][4];
+  if (threadIdx.x == 0) {
+    atomicMax(&ctl->mx_term, sh[0]);
+    atomicMax(&ctl->mx_mass, sh[1]);
   }
-  finish_node(N, node, s, a, lo, hi, emin, ovf != 0, fallback, counters, force_fallback, nd);
 }
 
-// One thread per node of a single chunk (most nodes of the deep levels): the
-// per-node arithmetic, much of it FP64, then fills whole warps.
-__global__ void k_stats_final_one(DNode *nodes, int32_t nb, int32_t ne, const int64_t *chunk_base,
-                                  const double *part, int32_t *fallback, int64_t *counters,
-                                  int32_t force_fallback, int32_t nd) {
-  const int32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-  const int32_t node = nb + i;
-  if (node >= ne) return;
-  DNode &N = nodes[node];
-  if (N.count <= 0 || N.count > kChunk) return;
-  __int128 s[4] = {0, 0, 0, 0};
-  double a[4] = {0, 0, 0, 0};
-  float lo[3] = {INFINITY, INFINITY, INFINITY}, hi[3] = {-INFINITY, -INFINITY, -INFINITY};
-  int emin[4] = {INT_MAX, INT_MAX, INT_MAX, INT_MAX};
-  int ovf = 0;
-  read_part(part + chunk_base[i] * kPartWords, s, a, lo, hi, emin, ovf);
-  finish_node(N, node, s, a, lo, hi, emin, ovf != 0, fallback, counters, force_fallback, nd);
+// The root, its chunks and the first level.
+__global__ void __launch_bounds__(256)
+    k_root(DNode *nodes, int64_t n, TreeConfig cfg, LevelCtl *ctl, int32_t *chunk_node,
+           int32_t *chunk_base, NodeAcc *acc, unsigned *ticket, int32_t sub_max) {
+  const int32_t nc = chunks_of(int32_t(n));
+  const bool sub = n <= sub_max;
+  if (!sub)
+    for (int32_t c = threadIdx.x; c < nc; c += blockDim.x) chunk_node[c] = 0;
+  if (threadIdx.x != 0) return;
+  DNode &R = nodes[0];
+  R.count = int32_t(n);
+  R.offset = 0;
+  R.cl = R.cr = 0;
+  for (int d = 0; d < 3; ++d) {
+    R.xmin[d] = cfg.min[d];
+    R.xmax[d] = cfg.max[d];
+    R.xc[d] = 0.f;
+  }
+  R.tdr = 0.f;
+  R.split_dim = -1;
+  R.nleft = 0;
+  if (!sub) {
+    chunk_base[0] = 0;
+    acc_zero(acc[0]);
+    ticket[0] = 0u;
+  }
+  ctl->lev[0] = LevelSpan{0, sub ? 0 : 1, 0, 1, nc, int32_t(n), {0, 0}};
+  ctl->lev[1] = LevelSpan{-1, 0, 0, 0, 0, 0, {0, 0}};
+  ctl->begin[0] = 0;
+  ctl->sub_ready = sub;
+  ctl->sub_nb = 0;
+  ctl->sub_ne = 1;
+  ctl->sub_parity = 0;
 }
+
+// Statistics of every node of the level, and its split decision by the block
+// that adds a node's last chunk.
+__global__ void __launch_bounds__(kChunkThreads)
+    k_level_stats(const float4 *__restrict__ pos, DNode *nodes, LevelCtl *ctl, int32_t level,
+                  const int32_t *__restrict__ chunk_node, const int32_t *__restrict__ chunk_base,
+                  NodeAcc *acc, unsigned *ticket, int32_t *fallback, int64_t *counters,
+                  int32_t force_fallback, int32_t nd) {
+  LevelSpan L;
+  if (!level_runs(ctl, level, L, true) || int32_t(blockIdx.x) >= L.nchunk) return;
+  constexpr int kW = kChunkThreads / 32, kPer = kChunk / kChunkThreads, kU = 4;
+  __shared__ NodeAcc part[kW];
+  const ChunkRange R = chunk_range(nodes, chunk_node, chunk_base, L.nb, int32_t(blockIdx.x));
+  const unsigned mt = ctl->mx_term, mm = ctl->mx_mass;
+  const SumScale sc(mt), sm(mm);
+  LaneAcc a;
+  a.zero();
+  int cnt = 0;
+  for (int j0 = 0; j0 < kPer && j0 * kChunkThreads < R.len; j0 += kU) {
+    float4 p[kU];
+#pragma unroll
+    for (int u = 0; u < kU; ++u) {
+      const int e = (j0 + u) * kChunkThreads + threadIdx.x;
+      if (e < R.len) p[u] = pos[R.begin + e];
+    }
+#pragma unroll
+    for (int u = 0; u < kU; ++u) {
+      const int e = (j0 + u) * kChunkThreads + threadIdx.x;
+      if (e < R.len) {
+        a.add(p[u], sc, sm);
+        ++cnt;
+      }
+    }
+  }
+  NodeAcc w;
+  a.reduce(w, cnt, true, sc, sm);  // a warp's share of a chunk is 512 elements
+  if ((threadIdx.x & 31) == 0) part[threadIdx.x >> 5] = w;
+  __syncthreads();
+  if (threadIdx.x >= 32) return;
+  // a thread per word: the warps' records into the node's, one atomic each
+  NodeAcc &T = acc[R.node - L.nb];
+  const int f = threadIdx.x;
+  if (f < 8) {
+    long long s = 0;
+    for (int v = 0; v < kW; ++v) s += f < 4 ? part[v].h[f] : part[v].l[f - 4];
+    atomicAdd(reinterpret_cast<unsigned long long *>(f < 4 ? &T.h[f] : &T.l[f - 4]),
+              (unsigned long long)s);
+  } else if (f < 16) {
+    unsigned s = 0;
+    for (int v = 0; v < kW; ++v) s |= f < 12 ? part[v].o1[f - 8] : part[v].o2[f - 12];
+    atomicOr(f < 12 ? &T.o1[f - 8] : &T.o2[f - 12], s);
+  } else if (f < 22) {
+    unsigned s = f < 19 ? 0xffffffffu : 0u;
+    for (int v = 0; v < kW; ++v) s = f < 19 ? min(s, part[v].lo[f - 16]) : max(s, part[v].hi[f - 19]);
+    if (f < 19) atomicMin(&T.lo[f - 16], s);
+    else atomicMax(&T.hi[f - 19], s);
+  } else if (f == 22) {
+    unsigned s = 0xffffffffu;
+    for (int v = 0; v < kW; ++v) s = min(s, part[v].wmin);
+    atomicMin(&T.wmin, s);
+  } else if (f == 23) {
+    unsigned s = 0;
+    for (int v = 0; v < kW; ++v) s |= part[v].trunc;
+    if (s) atomicOr(&T.trunc, s);
+  }
+  __threadfence();
+  __syncwarp();
+  if (threadIdx.x != 0) return;
+  DNode N = nodes[R.node];
+  if (atomicAdd(&ticket[R.node - L.nb], 1u) + 1u != unsigned(chunks_of(N.count))) return;
+  __threadfence();
+  ticket[R.node - L.nb] = 0u;  // k_level_count counts the chunks again
+  NodeAcc A;
+  const int4 *src = reinterpret_cast<const int4 *>(&T);
+  int4 *dst = reinterpret_cast<int4 *>(&A);
+#pragma unroll
+  for (int q = 0; q < 8; ++q) dst[q] = __ldcg(src + q);
+  if (!decide_node(N, A, sc, sm, SumScale::bad(mt) || SumScale::bad(mm), force_fallback, nd)) {
+    fallback[atomicAdd((unsigned long long *)&counters[C_NFALLBACK], 1ull)] = R.node;
+    atomicExch(&ctl->abort, level + 1);
+  }
+  nodes[R.node] = N;
+}
+
+// Left counts of the level's chunks and each warp's left elements before its
+// share of the chunk (the shares of k_part_left); only the split coordinate is
+// loaded, every lane's loads in flight at once.  The block that counts a node's
+// last chunk scans the node's chunks; the one that counts the level's last
+// chunk makes the children and the next level.
+__global__ void __launch_bounds__(kChunkThreads)
+    k_level_count(const float4 *__restrict__ pos, DNode *nodes, LevelCtl *ctl, int32_t level,
+                  const int32_t *__restrict__ chunk_node, const int32_t *__restrict__ chunk_base,
+                  int32_t *next_chunk_node, int32_t *next_chunk_base, int32_t *left_cnt,
+                  int32_t *left_base, int32_t *wpre, NodeAcc *acc, unsigned *ticket,
+                  int64_t *counters, int32_t sub_max) {
+  LevelSpan L;
+  if (!level_runs(ctl, level, L) || int32_t(blockIdx.x) >= L.nchunk) return;
+  constexpr int kWarps = kChunkThreads / 32, kSub = kChunk / kWarps, kPer = kSub / 32;
+  __shared__ int wt[kWarps];
+  __shared__ int sh_warp[32];
+  __shared__ int last;
+  const int32_t chunk = int32_t(blockIdx.x);
+  const ChunkRange R = chunk_range(nodes, chunk_node, chunk_base, L.nb, chunk);
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int32_t count = nodes[R.node].count, d = nodes[R.node].split_dim;
+  if (d >= 0) {
+    const float split = nodes[R.node].xc[d];
+    const float *key = reinterpret_cast<const float *>(pos + R.begin) + d;
+    float kv[kPer];
+#pragma unroll
+    for (int u = 0; u < kPer; ++u) {
+      const int e = warp * kSub + 32 * u + lane;
+      kv[u] = e < R.len ? key[4 * e] : INFINITY;
+    }
+    int c = 0;
+#pragma unroll
+    for (int u = 0; u < kPer; ++u) c += warp * kSub + 32 * u + lane < R.len && kv[u] < split;
+    c = __reduce_add_sync(0xffffffffu, c);
+    if (lane == 0) wt[warp] = c;
+    __syncthreads();
+    if (threadIdx.x < kWarps) {
+      int pre = 0, tot = 0;
+      for (int w = 0; w < kWarps; ++w) {
+        pre += w < int(threadIdx.x) ? wt[w] : 0;
+        tot += wt[w];
+      }
+      wpre[chunk * kWarps + threadIdx.x] = pre;
+      if (threadIdx.x == 0) left_cnt[chunk] = tot;
+    }
+  }
+  // the node's last chunk: exclusive scan of its chunks' left counts
+  __threadfence();
+  __syncthreads();
+  const int32_t nc = chunks_of(count);
+  if (threadIdx.x == 0) last = atomicAdd(&ticket[R.node - L.nb], 1u) + 1u == unsigned(nc);
+  __syncthreads();
+  if (last && d >= 0) {
+    __threadfence();
+    const int32_t cb = chunk_base[R.node - L.nb];
+    int run = 0;
+    for (int32_t c0 = 0; c0 < nc; c0 += kChunkThreads) {
+      const int32_t c = c0 + int32_t(threadIdx.x);
+      const int v = c < nc ? __ldcg(left_cnt + cb + c) : 0;
+      int total;
+      const int ex = block_excl_scan(v, sh_warp, &total);
+      if (c < nc) left_base[cb + c] = run + ex;
+      run += total;
+    }
+    if (threadIdx.x == 0) nodes[R.node].nleft = run;
+  }
+  // the level's last chunk: children, two per node split into two non-empty
+  // parts, and the next level's chunks
+  __threadfence();
+  __syncthreads();
+  if (threadIdx.x == 0) last = atomicAdd(&ctl->ticket, 1u) + 1u == unsigned(L.nchunk);
+  __syncthreads();
+  if (!last) return;
+  __threadfence();
+  const int32_t nl = L.ne - L.nb;
+  int splits = 0, chunks = 0, largest = 0;
+  for (int32_t i0 = 0; i0 < nl; i0 += kChunkThreads) {
+    const int32_t i = i0 + int32_t(threadIdx.x);
+    DNode N;
+    bool split = false;
+    if (i < nl) {
+      const int4 *src = reinterpret_cast<const int4 *>(nodes + L.nb + i);
+      int4 *dst = reinterpret_cast<int4 *>(&N);
+#pragma unroll
+      for (int q = 0; q < 4; ++q) dst[q] = __ldcg(src + q);
+      split = N.split_dim >= 0 && N.nleft > 0 && N.nleft < N.count;
+    }
+    const int32_t c0 = split ? chunks_of(N.nleft) : 0, c1 = split ? chunks_of(N.count - N.nleft) : 0;
+    int ts, tc;
+    const int rank = splits + block_excl_scan(split ? 1 : 0, sh_warp, &ts);
+    const int32_t cb = chunks + block_excl_scan(c0 + c1, sh_warp, &tc);
+    if (split) {
+      const int32_t cl = L.ne + 2 * rank;
+      write_child(nodes[cl], N, 0);
+      write_child(nodes[cl + 1], N, 1);
+      nodes[L.nb + i].cl = cl;
+      nodes[L.nb + i].cr = cl + 1;
+      next_chunk_base[2 * rank] = cb;
+      next_chunk_base[2 * rank + 1] = cb + c0;
+      for (int32_t c = 0; c < c0; ++c) next_chunk_node[cb + c] = cl;
+      for (int32_t c = 0; c < c1; ++c) next_chunk_node[cb + c0 + c] = cl + 1;
+      largest = max(largest, max(N.nleft, N.count - N.nleft));
+    }
+    if (i < nl) ticket[i] = 0u;
+    splits += ts;
+    chunks += tc;
+  }
+  largest = __reduce_max_sync(0xffffffffu, largest);
+  if (lane == 0) wt[warp] = largest;
+  __syncthreads();
+  for (int32_t i = threadIdx.x; i < 2 * splits; i += kChunkThreads) {
+    acc_zero(acc[i]);
+    ticket[i] = 0u;
+  }
+  if (threadIdx.x != 0) return;
+  for (int w = 0; w < kWarps; ++w) largest = max(largest, wt[w]);
+  const bool sub = splits > 0 && largest <= sub_max;
+  LevelSpan X{level + 1, splits > 0 && !sub ? 1 : 0, L.ne, L.ne + 2 * splits, chunks, largest, {0, 0}};
+  ctl->lev[(level + 1) & 1] = X;
+  ctl->begin[(level + 1) % kCtlLevels] = L.ne;
+  ctl->next_level = level + 1;
+  ctl->ticket = 0u;
+  ctl->sub_ready = sub;
+  ctl->sub_nb = X.nb;
+  ctl->sub_ne = X.ne;
+  ctl->sub_parity = (level + 1) & 1;
+  ctl->done = splits == 0;
+  counters[C_CHAINS] = 0;  // the level's queue of long swap chains
+}
+
+// Left particles go to their rank; idx[rank] records where each came from.
+// Warp w takes the chunk's elements [w * kSub, (w + 1) * kSub) 32 at a time
+// (coalesced), kB steps' loads in flight; ranks follow array order through
+// the warps' left counts before them (k_level_count) and a ballot prefix
+// within each step.
+__global__ void __launch_bounds__(kChunkThreads)
+    k_part_left(const float4 *__restrict__ pos, const int32_t *__restrict__ oid, const DNode *nodes,
+                const LevelCtl *ctl, int32_t level, const int32_t *__restrict__ chunk_node,
+                const int32_t *__restrict__ chunk_base, const int32_t *left_base,
+                const int32_t *wpre, float4 *tpos, int32_t *toid, int32_t *idx, int32_t *ridx) {
+  LevelSpan L;
+  if (!level_runs(ctl, level, L) || int32_t(blockIdx.x) >= L.nchunk) return;
+  constexpr int kWarps = kChunkThreads / 32;
+  constexpr int kSub = kChunk / kWarps;  // a warp's share of the chunk
+  constexpr int kB = 4;
+  const int32_t chunk = int32_t(blockIdx.x);
+  const ChunkRange R = chunk_range(nodes, chunk_node, chunk_base, L.nb, chunk);
+  const DNode &N = nodes[R.node];
+  if (N.split_dim < 0) {
+    // a leaf keeps its elements: copied once into the next level's buffer
+    for (int k = threadIdx.x; k < R.len; k += kChunkThreads) {
+      tpos[R.begin + k] = pos[R.begin + k];
+      toid[R.begin + k] = oid[R.begin + k];
+    }
+    return;
+  }
+  const int d = N.split_dim;
+  const float split = N.xc[d];
+  const int32_t off = N.offset, nleft = N.nleft;
+  const int lane = threadIdx.x & 31, warp = int(threadIdx.x >> 5);
+  const unsigned below = (1u << lane) - 1u;
+  const int sub_end = min(kSub, R.len - warp * kSub);  // elements of this warp's share
+  int r = left_base[chunk] + wpre[chunk * kWarps + warp];
+  for (int j0 = 0; j0 < sub_end; j0 += 32 * kB) {
+    float4 p[kB];
+    int32_t o[kB];
+#pragma unroll
+    for (int u = 0; u < kB; ++u) {
+      const int e = warp * kSub + j0 + 32 * u + lane;
+      if (j0 + 32 * u < sub_end && e < R.len) {
+        p[u] = pos[R.begin + e];
+        o[u] = oid[R.begin + e];
+      } else {
+        p[u] = make_float4(0.f, 0.f, 0.f, 0.f);
+        o[u] = 0;
+      }
+    }
+#pragma unroll
+    for (int u = 0; u < kB; ++u) {
+      if (j0 + 32 * u >= sub_end) break;  // the same for the whole warp
+      const int e = warp * kSub + j0 + 32 * u + lane;
+      const bool in = e < R.len;
+      const bool l = in && key_of(p[u], d) < split;
+      const unsigned bal = __ballot_sync(0xffffffffu, l);
+      const int q = r + __popc(bal & below);  // left elements before this one
+      if (l) {
+        tpos[off + q] = p[u];
+        toid[off + q] = o[u];
+        idx[off + q] = R.local + e;
+      } else if (in) {
+        ridx[off + (R.local + e - q)] = R.local + e;
+        if (R.local + e >= nleft) {
+          // a right element at or after nleft: no swap touches it, it stays
+          tpos[R.begin + e] = p[u];
+          toid[R.begin + e] = o[u];
+        }
+      }
+      r += __popc(bal);
+    }
+  }
+}
+
+// A swap chain still running after the partition's single steps: its
+// position in the node, the node and the element's position in the level's
+// array.
+struct ChainItem {
+  int32_t q, node;
+  int64_t src;
+};
+static_assert(sizeof(ChainItem) == sizeof(int4), "a chain item fills one int4 of the queue");
+
+// One or more steps of the chain q -> idx[q] -> ... (q < nleft): the q-th
+// left element has c = idx[q] - q right elements before it, and so has every
+// left element up to the c-th right element (at ridx[c]), whose ranks run to
+// b = ridx[c] - c.  Within that run each step adds c, so the chain leaves
+// [q, min(b, nleft)) at the first of q + c, q + 2c, ... at or past it.
+// Returns a position > q; *bad on an inconsistent partition.
+__device__ __forceinline__ int32_t chain_jump(int32_t q, int32_t nleft, int32_t nright,
+                                              const int32_t *idx, const int32_t *ridx, bool *bad) {
+  const int32_t c = idx[q] - q;
+  if (c <= 0) {  // cannot happen for a valid partition (a chain never meets a fixed point)
+    *bad = true;
+    return nleft;
+  }
+  int32_t lim = nleft;
+  if (c < nright) {
+    const int32_t b = ridx[c] - c;
+    if (b <= q) {  // cannot happen for a valid partition
+      *bad = true;
+      return nleft;
+    }
+    lim = min(lim, b);
+  }
+  const int32_t k = lim > q + c ? (lim - q + c - 1) / c : 1;
+  return q + k * c;
+}
+
+// The other particles: those at or after position nleft stay (k_part_left
+// writes them); one at p < nleft moves along p -> idx[p] -> ... until it
+// lands at or after nleft (the reference's swap sequence,
+// RCBForceTree.cxx:647-669), taken a run of equal steps at a time
+// (chain_jump).  Positions increase strictly along a chain, so it ends within
+// count jumps.
+__global__ void __launch_bounds__(kChunkThreads)
+    k_part_right(const float4 *__restrict__ pos, const int32_t *__restrict__ oid, const DNode *nodes,
+                 const LevelCtl *ctl, int32_t level, const int32_t *__restrict__ chunk_node,
+                 const int32_t *__restrict__ chunk_base, const int32_t *__restrict__ idx,
+                 float4 *tpos, int32_t *toid, int32_t *err,
+                 int64_t *counters, ChainItem *chains, int64_t chain_cap) {
+  LevelSpan L;
+  if (!level_runs(ctl, level, L) || int32_t(blockIdx.x) >= L.nchunk) return;
+  constexpr int NT = kChunkThreads;
+  const int tid = threadIdx.x;
+  const ChunkRange R = chunk_range(nodes, chunk_node, chunk_base, L.nb, int32_t(blockIdx.x));
+  const DNode &N = nodes[R.node];
+  if (N.split_dim < 0) return;
+  const int d = N.split_dim;
+  const float split = N.xc[d];
+  const int32_t is = N.nleft;
+  const int32_t *nidx = idx + N.offset;
+  if (R.local >= is) return;  // every element here stays (k_part_left)
+  // The thread's 16 elements take their first kPlainSteps steps
+  // in lockstep, so up to 16 independent loads are in flight per step (most
+  // chains end within a few).  The chains still running go to the level's
+  // chain queue (k_part_chains follows them a chain per thread): long chains
+  // gather in a few regions of a level, thousands in one chunk.
+  constexpr int kPerT = kChunk / kChunkThreads;
+  const float *key = reinterpret_cast<const float *>(pos + R.begin) + d;
+  int32_t q[kPerT];
+  unsigned right = 0;
+#pragma unroll
+  for (int j = 0; j < kPerT; ++j) {
+    const int k = tid + j * NT;
+    q[j] = R.local + k;
+    if (k < R.len && q[j] < is && !(key[4 * k] < split)) right |= 1u << j;
+  }
+  unsigned active = right;
+  bool bad = false;
+  for (int32_t step = 0; active && step < kPlainSteps; ++step) {
+    int32_t nq[kPerT];
+#pragma unroll
+    for (int j = 0; j < kPerT; ++j) nq[j] = (active >> j & 1u) ? nidx[q[j]] : q[j];
+#pragma unroll
+    for (int j = 0; j < kPerT; ++j) {
+      if (!(active >> j & 1u)) continue;
+      if (nq[j] <= q[j] || nq[j] >= N.count) {  // cannot happen for a valid partition
+        bad = true;
+        active &= ~(1u << j);
+        right &= ~(1u << j);
+        continue;
+      }
+      q[j] = nq[j];
+      if (nq[j] >= is) active &= ~(1u << j);
+    }
+  }
+  // one queue reservation per warp
+  const int lane = threadIdx.x & 31;
+  const int na = __popc(active);
+  int incl = na;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const int y = __shfl_up_sync(0xffffffffu, incl, o);
+    if (lane >= o) incl += y;
+  }
+  unsigned long long base = 0;
+  if (lane == 31 && incl > 0)
+    base = atomicAdd((unsigned long long *)&counters[C_CHAINS], (unsigned long long)incl);
+  base = __shfl_sync(0xffffffffu, base, 31);
+  int64_t slot = int64_t(base) + incl - na;
+#pragma unroll
+  for (int j = 0; j < kPerT; ++j) {
+    if (!(right >> j & 1u)) continue;
+    const int64_t src = R.begin + tid + j * NT;
+    if (active >> j & 1u) {
+      if (slot < chain_cap) chains[slot] = ChainItem{q[j], R.node, src};
+      else bad = true;  // cannot happen: a chain per element at most
+      ++slot;
+      continue;
+    }
+    tpos[N.offset + q[j]] = pos[src];
+    toid[N.offset + q[j]] = oid[src];
+  }
+  if (bad) atomicExch(err, 2);
+}
+
+// The level's long swap chains, a thread each, a run of equal steps at a
+// time (chain_jump); each lands its element.
+__global__ void __launch_bounds__(256)
+    k_part_chains(const float4 *__restrict__ pos, const int32_t *__restrict__ oid,
+                  const DNode *nodes, const LevelCtl *ctl, int32_t level,
+                  const ChainItem *__restrict__ chains, int64_t chain_cap, const int64_t *counters, const int32_t *__restrict__ idx,
+                  const int32_t *__restrict__ ridx, float4 *tpos, int32_t *toid, int32_t *err) {
+  LevelSpan L;
+  if (!level_runs(ctl, level, L)) return;
+  const int64_t nq = min64(counters[C_CHAINS], chain_cap);
+  for (int64_t c = int64_t(blockIdx.x) * blockDim.x + threadIdx.x; c < nq;
+       c += int64_t(gridDim.x) * blockDim.x) {
+    const ChainItem it = chains[c];
+    const DNode &N = nodes[it.node];
+    const int32_t is = N.nleft, nright = N.count - N.nleft;
+    const int32_t *nidx = idx + N.offset, *nridx = ridx + N.offset;
+    int32_t qq = it.q;
+    bool b = false;
+    for (int32_t k = 0; qq < is && k <= N.count && !b; ++k)
+      qq = chain_jump(qq, is, nright, nidx, nridx, &b);
+    if (b || qq < is || qq >= N.count) {  // cannot happen for a valid partition
+      atomicExch(err, 2);
+      continue;
+    }
+    tpos[N.offset + qq] = pos[it.src];
+    toid[N.offset + qq] = oid[it.src];
+  }
+}
+
 
 // ---------------------------------------------------------------------------
 // Tight certification of the centre of mass for the nodes the loose bound
@@ -1152,512 +1384,11 @@ __global__ void k_cm_fallback(const float4 *__restrict__ pos, DNode *nodes, cons
   }
 }
 
-__device__ __forceinline__ float key_of(const float4 &p, int d) {
-  return d == 0 ? p.x : (d == 1 ? p.y : p.z);
-}
-
-// Block-wide exclusive scan of one int per thread.
-__device__ __forceinline__ int block_excl_scan(int v, int *sh_warp, int *total) {
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  int x = v;
-#pragma unroll
-  for (int o = 1; o < 32; o <<= 1) {
-    const int y = __shfl_up_sync(0xffffffffu, x, o);
-    if (lane >= o) x += y;
-  }
-  if (lane == 31) sh_warp[warp] = x;
-  __syncthreads();
-  if (warp == 0) {
-    int w = lane < (int)(blockDim.x >> 5) ? sh_warp[lane] : 0;
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-      const int y = __shfl_up_sync(0xffffffffu, w, o);
-      if (lane >= o) w += y;
-    }
-    sh_warp[lane] = w;
-  }
-  __syncthreads();
-  const int excl = x - v + (warp > 0 ? sh_warp[warp - 1] : 0);
-  *total = sh_warp[(blockDim.x >> 5) - 1];
-  __syncthreads();
-  return excl;
-}
-
-// Left counts of each chunk of a splitting node; in block mode also each
-// warp's left elements before its share of the chunk (the shares of
-// k_part_left: warp w takes [w * kChunk / 8, (w + 1) * kChunk / 8)).  Only
-// the split coordinate is loaded, every lane's loads in flight at once.
-template <bool WM>
-__global__ void __launch_bounds__(kChunkThreads)
-    k_part_count(const float4 *__restrict__ pos, const DNode *nodes, const int32_t *chunk_node,
-                 const int64_t *chunk_base, int32_t nb, const int64_t *nchunk, int32_t *left_cnt,
-                 int32_t *wpre) {
-  CHUNK_PROLOGUE
-  const ChunkRange R = chunk_range(nodes, chunk_node, chunk_base, nb, chunk);
-  const DNode &N = nodes[R.node];
-  if (N.split_dim < 0) {
-    if (tid == 0) left_cnt[chunk] = 0;
-    return;
-  }
-  const int d = N.split_dim;
-  const float split = N.xc[d];
-  const float *key = reinterpret_cast<const float *>(pos + R.begin) + d;
-  if (WM) {
-    int c = 0;
-    for (int k = tid; k < R.len; k += NT) c += key[4 * k] < split;
-    c = __reduce_add_sync(0xffffffffu, c);
-    if (lane_ == 0) left_cnt[chunk] = c;
-    return;
-  }
-  constexpr int kWarps = kChunkThreads / 32, kSub = kChunk / kWarps, kPer = kSub / 32;
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  float kv[kPer];
-#pragma unroll
-  for (int u = 0; u < kPer; ++u) {
-    const int e = warp * kSub + 32 * u + lane;
-    kv[u] = e < R.len ? key[4 * e] : INFINITY;
-  }
-  int c = 0;
-#pragma unroll
-  for (int u = 0; u < kPer; ++u) c += kv[u] < split;
-  c = __reduce_add_sync(0xffffffffu, c);
-  __shared__ int wt[kWarps];
-  if (lane == 0) wt[warp] = c;
-  __syncthreads();
-  if (threadIdx.x < kWarps) {
-    int pre = 0, tot = 0;
-    for (int w = 0; w < kWarps; ++w) {
-      pre += w < int(threadIdx.x) ? wt[w] : 0;
-      tot += wt[w];
-    }
-    wpre[chunk * kWarps + threadIdx.x] = pre;
-    if (threadIdx.x == 0) left_cnt[chunk] = tot;
-  }
-}
-
-// Per splitting node, a warp each: exclusive scan of its chunks' left counts
-// (in chunk order) and the node's total.
-__global__ void k_part_node_scan(DNode *nodes, int32_t nb, int32_t ne, const int64_t *chunk_base,
-                                 const int32_t *left_cnt, int64_t *left_base) {
-  const int32_t w = int32_t((int64_t(blockIdx.x) * blockDim.x + threadIdx.x) >> 5);
-  const int lane = threadIdx.x & 31;
-  if (nb + w >= ne) return;  // whole warps
-  DNode &N = nodes[nb + w];
-  if (N.split_dim < 0) return;
-  const int64_t cb = chunk_base[w];
-  const int64_t nc = (int64_t(N.count) + kChunk - 1) / kChunk;
-  int64_t run = 0;
-  for (int64_t c0 = 0; c0 < nc; c0 += 32) {
-    const int64_t c = c0 + lane;
-    const int64_t v = c < nc ? left_cnt[cb + c] : 0;
-    int64_t x = v;
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-      const int64_t y = __shfl_up_sync(0xffffffffu, x, o);
-      if (lane >= o) x += y;
-    }
-    if (c < nc) left_base[cb + c] = run + x - v;
-    run += __shfl_sync(0xffffffffu, x, 31);
-  }
-  if (lane == 0) N.nleft = int32_t(run);
-}
-
-// Left particles go to their rank; idx[rank] records where each came from.
-// Warp w takes the chunk's elements [w * kSub, (w + 1) * kSub) 32 at a time
-// (coalesced), kB steps' loads in flight; ranks follow array order through
-// the warps' left counts before them (k_part_count) and a ballot prefix
-// within each step.
-template <bool WM>
-__global__ void __launch_bounds__(kChunkThreads)
-    k_part_left(const float4 *__restrict__ pos, const int32_t *__restrict__ oid, const DNode *nodes,
-                const int32_t *chunk_node, const int64_t *chunk_base, int32_t nb,
-                const int64_t *nchunk, const int64_t *left_base, const int32_t *wpre, float4 *tpos,
-                int32_t *toid, int32_t *idx, int32_t *ridx) {
-  constexpr int kWarps = kChunkThreads / 32;
-  constexpr int kSub = WM ? kChunk : kChunk / kWarps;  // a warp's share of the chunk
-  constexpr int kB = 4;
-  CHUNK_PROLOGUE
-  const ChunkRange R = chunk_range(nodes, chunk_node, chunk_base, nb, chunk);
-  const DNode &N = nodes[R.node];
-  if (N.split_dim < 0) {
-    // a leaf keeps its elements: copied once into the next level's buffer
-    for (int k = tid; k < R.len; k += NT) {
-      tpos[R.begin + k] = pos[R.begin + k];
-      toid[R.begin + k] = oid[R.begin + k];
-    }
-    return;
-  }
-  const int d = N.split_dim;
-  const float split = N.xc[d];
-  const int32_t off = N.offset, nleft = N.nleft;
-  const int lane = threadIdx.x & 31, warp = WM ? 0 : int(threadIdx.x >> 5);
-  const unsigned below = (1u << lane) - 1u;
-  const int sub_end = min(kSub, R.len - warp * kSub);  // elements of this warp's share
-  int r = int(left_base[chunk]) + (WM ? 0 : wpre[chunk * kWarps + warp]);
-  for (int j0 = 0; j0 < sub_end; j0 += 32 * kB) {
-    float4 p[kB];
-    int32_t o[kB];
-#pragma unroll
-    for (int u = 0; u < kB; ++u) {
-      const int e = warp * kSub + j0 + 32 * u + lane;
-      if (j0 + 32 * u < sub_end && e < R.len) {
-        p[u] = pos[R.begin + e];
-        o[u] = oid[R.begin + e];
-      } else {
-        p[u] = make_float4(0.f, 0.f, 0.f, 0.f);
-        o[u] = 0;
-      }
-    }
-#pragma unroll
-    for (int u = 0; u < kB; ++u) {
-      if (j0 + 32 * u >= sub_end) break;  // the same for the whole warp
-      const int e = warp * kSub + j0 + 32 * u + lane;
-      const bool in = e < R.len;
-      const bool l = in && key_of(p[u], d) < split;
-      const unsigned bal = __ballot_sync(0xffffffffu, l);
-      const int q = r + __popc(bal & below);  // left elements before this one
-      if (l) {
-        tpos[off + q] = p[u];
-        toid[off + q] = o[u];
-        idx[off + q] = R.local + e;
-      } else if (in) {
-        ridx[off + (R.local + e - q)] = R.local + e;
-        if (R.local + e >= nleft) {
-          // a right element at or after nleft: no swap touches it, it stays
-          tpos[R.begin + e] = p[u];
-          toid[R.begin + e] = o[u];
-        }
-      }
-      r += __popc(bal);
-    }
-  }
-}
-
-// A swap chain still running after the partition's single steps: its
-// position in the node, the node and the element's position in the level's
-// array.
-struct ChainItem {
-  int32_t q, node;
-  int64_t src;
-};
-static_assert(sizeof(ChainItem) == sizeof(int4), "a chain item fills one int4 of the queue");
-
-// One or more steps of the chain q -> idx[q] -> ... (q < nleft): the q-th
-// left element has c = idx[q] - q right elements before it, and so has every
-// left element up to the c-th right element (at ridx[c]), whose ranks run to
-// b = ridx[c] - c.  Within that run each step adds c, so the chain leaves
-// [q, min(b, nleft)) at the first of q + c, q + 2c, ... at or past it.
-// Returns a position > q; *bad on an inconsistent partition.
-__device__ __forceinline__ int32_t chain_jump(int32_t q, int32_t nleft, int32_t nright,
-                                              const int32_t *idx, const int32_t *ridx, bool *bad) {
-  const int32_t c = idx[q] - q;
-  if (c <= 0) {  // cannot happen for a valid partition (a chain never meets a fixed point)
-    *bad = true;
-    return nleft;
-  }
-  int32_t lim = nleft;
-  if (c < nright) {
-    const int32_t b = ridx[c] - c;
-    if (b <= q) {  // cannot happen for a valid partition
-      *bad = true;
-      return nleft;
-    }
-    lim = min(lim, b);
-  }
-  const int32_t k = lim > q + c ? (lim - q + c - 1) / c : 1;
-  return q + k * c;
-}
-
-// The other particles: those at or after position nleft stay (k_part_left
-// writes them); one at p < nleft moves along p -> idx[p] -> ... until it
-// lands at or after nleft (the reference's swap sequence,
-// RCBForceTree.cxx:647-669), taken a run of equal steps at a time
-// (chain_jump).  Positions increase strictly along a chain, so it ends within
-// count jumps.
-template <bool WM>
-__global__ void __launch_bounds__(kChunkThreads)
-    k_part_right(const float4 *__restrict__ pos, const int32_t *__restrict__ oid, const DNode *nodes,
-                 const int32_t *chunk_node, const int64_t *chunk_base, int32_t nb,
-                 const int64_t *nchunk, const int32_t *__restrict__ idx,
-                 const int32_t *__restrict__ ridx, float4 *tpos, int32_t *toid, int32_t *err,
-                 int64_t *counters, ChainItem *chains, int64_t chain_cap) {
-  CHUNK_PROLOGUE
-  const ChunkRange R = chunk_range(nodes, chunk_node, chunk_base, nb, chunk);
-  const DNode &N = nodes[R.node];
-  if (N.split_dim < 0) return;
-  const int d = N.split_dim;
-  const float split = N.xc[d];
-  const int32_t is = N.nleft, nright = N.count - N.nleft;
-  const int32_t *nidx = idx + N.offset, *nridx = ridx + N.offset;
-  if (R.local >= is) return;  // every element here stays (k_part_left)
-  if (WM) {
-    for (int k = tid; k < R.len && R.local + k < is; k += NT) {
-      const int64_t src = R.begin + k;
-      const float4 p = pos[src];
-      if (key_of(p, d) < split) continue;
-      int32_t q = R.local + k;
-      int32_t steps = 0;
-      bool bad = false;
-      while (q < is && steps <= N.count && !bad) {
-        if (steps++ < kPlainSteps) {  // single steps first: most chains end within a few
-          const int32_t nq = nidx[q];
-          if (nq <= q) bad = true;
-          q = nq;
-        } else {
-          q = chain_jump(q, is, nright, nidx, nridx, &bad);
-        }
-      }
-      if (q < is || bad || q >= N.count) {
-        atomicExch(err, 2);
-        continue;
-      }
-      tpos[N.offset + q] = p;
-      toid[N.offset + q] = oid[src];
-    }
-    return;
-  }
-  // Block mode: the thread's 16 elements take their first kPlainSteps steps
-  // in lockstep, so up to 16 independent loads are in flight per step (most
-  // chains end within a few).  The chains still running go to the level's
-  // chain queue (k_part_chains follows them a chain per thread): long chains
-  // gather in a few regions of a level, thousands in one chunk.
-  constexpr int kPerT = kChunk / kChunkThreads;
-  const float *key = reinterpret_cast<const float *>(pos + R.begin) + d;
-  int32_t q[kPerT];
-  unsigned right = 0;
-#pragma unroll
-  for (int j = 0; j < kPerT; ++j) {
-    const int k = tid + j * NT;
-    q[j] = R.local + k;
-    if (k < R.len && q[j] < is && !(key[4 * k] < split)) right |= 1u << j;
-  }
-  unsigned active = right;
-  bool bad = false;
-  for (int32_t step = 0; active && step < kPlainSteps; ++step) {
-    int32_t nq[kPerT];
-#pragma unroll
-    for (int j = 0; j < kPerT; ++j) nq[j] = (active >> j & 1u) ? nidx[q[j]] : q[j];
-#pragma unroll
-    for (int j = 0; j < kPerT; ++j) {
-      if (!(active >> j & 1u)) continue;
-      if (nq[j] <= q[j] || nq[j] >= N.count) {  // cannot happen for a valid partition
-        bad = true;
-        active &= ~(1u << j);
-        right &= ~(1u << j);
-        continue;
-      }
-      q[j] = nq[j];
-      if (nq[j] >= is) active &= ~(1u << j);
-    }
-  }
-  // one queue reservation per warp
-  const int lane = threadIdx.x & 31;
-  const int na = __popc(active);
-  int incl = na;
-#pragma unroll
-  for (int o = 1; o < 32; o <<= 1) {
-    const int y = __shfl_up_sync(0xffffffffu, incl, o);
-    if (lane >= o) incl += y;
-  }
-  unsigned long long base = 0;
-  if (lane == 31 && incl > 0)
-    base = atomicAdd((unsigned long long *)&counters[C_CHAINS], (unsigned long long)incl);
-  base = __shfl_sync(0xffffffffu, base, 31);
-  int64_t slot = int64_t(base) + incl - na;
-#pragma unroll
-  for (int j = 0; j < kPerT; ++j) {
-    if (!(right >> j & 1u)) continue;
-    const int64_t src = R.begin + tid + j * NT;
-    if (active >> j & 1u) {
-      if (slot < chain_cap) chains[slot] = ChainItem{q[j], R.node, src};
-      else bad = true;  // cannot happen: a chain per element at most
-      ++slot;
-      continue;
-    }
-    tpos[N.offset + q[j]] = pos[src];
-    toid[N.offset + q[j]] = oid[src];
-  }
-  if (bad) atomicExch(err, 2);
-}
-
-// The level's long swap chains, a thread each, a run of equal steps at a
-// time (chain_jump); each lands its element.
-__global__ void __launch_bounds__(256)
-    k_part_chains(const float4 *__restrict__ pos, const int32_t *__restrict__ oid,
-                  const DNode *nodes, const ChainItem *__restrict__ chains, int64_t chain_cap,
-                  const int64_t *counters, const int32_t *__restrict__ idx,
-                  const int32_t *__restrict__ ridx, float4 *tpos, int32_t *toid, int32_t *err) {
-  const int64_t nq = min64(counters[C_CHAINS], chain_cap);
-  for (int64_t c = int64_t(blockIdx.x) * blockDim.x + threadIdx.x; c < nq;
-       c += int64_t(gridDim.x) * blockDim.x) {
-    const ChainItem it = chains[c];
-    const DNode &N = nodes[it.node];
-    const int32_t is = N.nleft, nright = N.count - N.nleft;
-    const int32_t *nidx = idx + N.offset, *nridx = ridx + N.offset;
-    int32_t qq = it.q;
-    bool b = false;
-    for (int32_t k = 0; qq < is && k <= N.count && !b; ++k)
-      qq = chain_jump(qq, is, nright, nidx, nridx, &b);
-    if (b || qq < is || qq >= N.count) {  // cannot happen for a valid partition
-      atomicExch(err, 2);
-      continue;
-    }
-    tpos[N.offset + qq] = pos[it.src];
-    toid[N.offset + qq] = oid[it.src];
-  }
-}
-
-// The whole partition of one node in one block, for levels whose nodes hold
-// at most kNodeMax elements: the left elements go to their ranks (warp w
-// takes a contiguous share of the node, ranks in array order through the
-// warps' totals and ballot prefixes), their source positions into shared
-// memory, and every right element before nleft follows p -> idx[p] -> ...
-// there (the reference's swap sequence, RCBForceTree.cxx:647-669).  A chain
-// longer than kChainSteps sends the block to pointer jumping in place over
-// idx (each entry moves along its own chain, so every read sees a point of
-// that chain), which ends in log2(count) + 1 rounds.  Also sets N.nleft and
-// copies leaves' elements.
-template <int NT>
-__global__ void __launch_bounds__(NT)
-    k_part_node(const float4 *__restrict__ pos, const int32_t *__restrict__ oid, DNode *nodes,
-                int32_t nb, int32_t ne, int32_t node_max, float4 *tpos, int32_t *toid,
-                int32_t *err) {
-  extern __shared__ int32_t sidx[];
-  constexpr int kW = NT / 32;
-  __shared__ int wtot[kW];
-  __shared__ int s_long;
-  const int32_t node = nb + int32_t(blockIdx.x);
-  if (node >= ne) return;
-  DNode &N = nodes[node];
-  const int cnt = N.count;
-  if (cnt > node_max) {  // the launch's shared memory does not hold it
-    if (threadIdx.x == 0) atomicExch(err, 3);
-    return;
-  }
-  const int64_t off = N.offset;
-  if (N.split_dim < 0) {
-    for (int e = threadIdx.x; e < cnt; e += NT) {
-      tpos[off + e] = pos[off + e];
-      toid[off + e] = oid[off + e];
-    }
-    return;
-  }
-  const int d = N.split_dim;
-  const float split = N.xc[d];
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const unsigned below = (1u << lane) - 1u;
-  const int sub = (((cnt + kW - 1) / kW) + 31) & ~31;
-  const int beg = warp * sub, end = min(cnt, beg + sub);
-  if (threadIdx.x == 0) s_long = 0;
-  // four loads in flight per lane in both passes
-  constexpr int kU = 4;
-  int c = 0;
-  for (int e0 = beg; e0 < end; e0 += 32 * kU) {
-    float key[kU];
-#pragma unroll
-    for (int u = 0; u < kU; ++u) {
-      const int e = e0 + 32 * u + lane;
-      key[u] = e < end ? key_of(pos[off + e], d) : split;
-    }
-#pragma unroll
-    for (int u = 0; u < kU; ++u) c += __popc(__ballot_sync(0xffffffffu, key[u] < split));
-  }
-  if (lane == 0) wtot[warp] = c;
-  __syncthreads();
-  int r = 0, nleft = 0;
-#pragma unroll
-  for (int w = 0; w < kW; ++w) {
-    const int v = wtot[w];
-    r += w < warp ? v : 0;
-    nleft += v;
-  }
-  for (int e0 = beg; e0 < end; e0 += 32 * kU) {
-    float4 pu[kU];
-    int ou[kU];
-#pragma unroll
-    for (int u = 0; u < kU; ++u) {
-      const int e = e0 + 32 * u + lane;
-      pu[u] = make_float4(0.f, 0.f, 0.f, 0.f);
-      ou[u] = 0;
-      if (e < end) {
-        pu[u] = pos[off + e];
-        ou[u] = oid[off + e];
-      }
-    }
-#pragma unroll
-    for (int u = 0; u < kU; ++u) {
-      const int e = e0 + 32 * u + lane;
-      const bool l = e < end && key_of(pu[u], d) < split;
-      const unsigned bal = __ballot_sync(0xffffffffu, l);
-      if (l) {
-        const int q = r + __popc(bal & below);
-        tpos[off + q] = pu[u];
-        toid[off + q] = ou[u];
-        sidx[q] = e;
-      } else if (e < end && e >= nleft) {
-        // a right element at or after nleft: no swap touches it, it stays
-        tpos[off + e] = pu[u];
-        toid[off + e] = ou[u];
-      }
-      r += __popc(bal);
-    }
-  }
-  if (threadIdx.x == 0) N.nleft = nleft;
-  __syncthreads();
-  for (int e = threadIdx.x; e < nleft; e += NT) {
-    const float4 p = pos[off + e];
-    if (key_of(p, d) < split) continue;
-    int q = e, steps = 0;
-    bool bad = false;
-    while (q < nleft && steps < kChainSteps) {
-      const int nq = sidx[q];
-      if (nq <= q || nq >= cnt) {  // cannot happen for a valid partition
-        bad = true;
-        break;
-      }
-      q = nq;
-      ++steps;
-    }
-    if (bad) {
-      atomicExch(err, 2);
-      continue;
-    }
-    if (q < nleft) {
-      s_long = 1;
-      continue;
-    }
-    tpos[off + q] = p;
-    toid[off + q] = oid[off + e];
-  }
-  __syncthreads();
-  if (!s_long) return;
-  // pointer jumping: afterwards idx[q] is the end of the chain through q
-  for (int round = 0;; ++round) {
-    bool ch = false;
-    for (int q = threadIdx.x; q < nleft; q += NT) {
-      const int j = sidx[q];
-      if (j != q && j < nleft) {  // j == q: a left element that no swap moves
-        sidx[q] = sidx[j];
-        ch = true;
-      }
-    }
-    if (!__syncthreads_or(ch)) break;
-    if (round > 40) {  // cannot happen for a valid partition
-      if (threadIdx.x == 0) atomicExch(err, 2);
-      return;
-    }
-  }
-  for (int e = threadIdx.x; e < nleft; e += NT) {
-    const float4 p = pos[off + e];
-    if (key_of(p, d) < split) continue;
-    const int q = sidx[e];
-    if (q < nleft || q >= cnt) {
-      atomicExch(err, 2);
-      continue;
-    }
-    tpos[off + q] = p;
-    toid[off + q] = oid[off + e];
-  }
+// The level's centres are all decided: the launches after go on.
+__global__ void k_decided(LevelCtl *ctl, int64_t *counters) {
+  counters[C_SEQ] += counters[C_NFALLBACK] - counters[C_NTIGHT];
+  counters[C_NFALLBACK] = counters[C_NTIGHT] = 0;
+  ctl->abort = 0;
 }
 
 // ---------------------------------------------------------------------------
@@ -1684,14 +1415,6 @@ constexpr int kSubThreads = 512;   // two blocks per SM
 constexpr int kSubWarps = kSubThreads / 32;
 constexpr int kSubDepth = 48;        // deepest level below a root; deeper: the level loop
 
-struct SubWarpStats {
-  __int128 s[4];
-  double a[4];
-  float lo[3], hi[3];
-  int emin[4];
-  int ovf;
-};
-
 // Barrier over the warps [w0, w0 + nw) of the block: named barrier 1 + team
 // for teams of several warps (at most 8 teams), __syncwarp for one warp.
 __device__ __forceinline__ void team_sync(int team, int nw) {
@@ -1702,26 +1425,59 @@ __device__ __forceinline__ void team_sync(int team, int nw) {
   }
 }
 
+// The records of a team's warps merged into one, a lane per word.
+__device__ __forceinline__ void merge_records(const NodeAcc *part, int nw, int f, NodeAcc *out) {
+  if (f < 8) {
+    long long s = 0;
+    for (int v = 0; v < nw; ++v) s += f < 4 ? part[v].h[f] : part[v].l[f - 4];
+    (f < 4 ? out->h[f] : out->l[f - 4]) = s;
+  } else if (f < 16) {
+    unsigned s = 0;
+    for (int v = 0; v < nw; ++v) s |= f < 12 ? part[v].o1[f - 8] : part[v].o2[f - 12];
+    (f < 12 ? out->o1[f - 8] : out->o2[f - 12]) = s;
+  } else if (f < 22) {
+    unsigned s = f < 19 ? 0xffffffffu : 0u;
+    for (int v = 0; v < nw; ++v) s = f < 19 ? min(s, part[v].lo[f - 16]) : max(s, part[v].hi[f - 19]);
+    (f < 19 ? out->lo[f - 16] : out->hi[f - 19]) = s;
+  } else if (f == 22) {
+    unsigned s = 0xffffffffu;
+    for (int v = 0; v < nw; ++v) s = min(s, part[v].wmin);
+    out->wmin = s;
+  } else if (f == 23) {
+    unsigned s = 0;
+    for (int v = 0; v < nw; ++v) s |= part[v].trunc;
+    out->trunc = s;
+  }
+}
+
 __global__ void __launch_bounds__(kSubThreads, 2)
-    k_subtree(const DNode *__restrict__ nodes, int32_t nb, int32_t ne, float4 *epos, int32_t *eoid,
-              float4 *tpos, int32_t *toid, DNode *sub, SubWarpStats *sub_stats, int32_t *sub_first,
-              int64_t *hist, int32_t force_fallback, int32_t nd, int64_t *counters) {
+    k_subtree(const DNode *__restrict__ nodes, const LevelCtl *ctl, float4 *pos_a, int32_t *oid_a,
+              float4 *pos_b, int32_t *oid_b, DNode *sub, NodeAcc *sub_stats, int32_t *sub_first,
+              int32_t *hist, int32_t force_fallback, int32_t nd, int64_t *counters) {
   extern __shared__ int32_t sidx[];  // chain table by element position in the subtree
-  __shared__ SubWarpStats wst[kSubWarps];
+  __shared__ NodeAcc wst[kSubWarps];
   __shared__ int wtot[kSubWarps];
   __shared__ int tflag[kSubWarps];      // per team: a chain too long / pointer jumping changed
   __shared__ int first[kSubDepth + 2];  // first local node of each depth
   __shared__ int sh_warp[32];
   __shared__ int s_nsplit;
+  if (!ctl->sub_ready || ctl->abort) return;
   const int32_t r = int32_t(blockIdx.x);
-  const int32_t nroots = ne - nb;
-  const DNode R = nodes[nb + r];
+  if (r >= ctl->sub_ne - ctl->sub_nb) {  // the host launched for the most there can be
+    for (int dd = int(threadIdx.x); dd < kSubDepth; dd += kSubThreads)
+      hist[int64_t(dd) * gridDim.x + r] = 0;
+    return;
+  }
+  const unsigned mt = ctl->mx_term, mm = ctl->mx_mass;
+  const SumScale sc(mt), sm(mm);
+  const bool bad_scale = SumScale::bad(mt) || SumScale::bad(mm);
+  const DNode R = nodes[ctl->sub_nb + r];
   const int rcnt = R.count;
   const int32_t roff = R.offset;
   DNode *loc = sub + 2 * int64_t(roff);  // this root's 2 x count records
   // the reduced statistics of the current level's nodes, by position in the
   // level (a level holds at most count nodes)
-  SubWarpStats *lst = sub_stats + roff;
+  NodeAcc *lst = sub_stats + roff;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const unsigned below = (1u << lane) - 1u;
   if (rcnt > kSubMax) {  // the launch's shared memory does not hold it
@@ -1735,10 +1491,11 @@ __global__ void __launch_bounds__(kSubThreads, 2)
     first[1] = 1;
   }
   __syncthreads();
-  const float4 *src = epos;
-  const int32_t *soid = eoid;
-  float4 *dst = tpos;
-  int32_t *doid = toid;
+  const bool par = ctl->sub_parity != 0;
+  const float4 *src = par ? pos_b : pos_a;
+  const int32_t *soid = par ? oid_b : oid_a;
+  float4 *dst = par ? pos_a : pos_b;
+  int32_t *doid = par ? oid_a : oid_b;
   int f0 = 0, f1 = 1, depth = 0;
   int nfb = 0;  // sequential centre-of-mass sums (thread 0 of a team counts)
   while (f1 > f0) {
@@ -1760,90 +1517,28 @@ __global__ void __launch_bounds__(kSubThreads, 2)
       const DNode N = loc[f];
       const int c = N.count;
       const int64_t o = N.offset;
-      FixAcc fx[4];
+      LaneAcc a;
+      a.zero();
+      int cnt = 0;
+      constexpr int kU = 4;
+      for (int e0 = tl; e0 < c; e0 += kU * TN) {
+        float4 p[kU];
 #pragma unroll
-      for (int q = 0; q < 4; ++q) fx[q].zero();
-      float fa[4] = {0.f, 0.f, 0.f, 0.f};
-      float bl[3] = {INFINITY, INFINITY, INFINITY}, bh[3] = {-INFINITY, -INFINITY, -INFINITY};
-      bool ovf = false;
-      bool trn[4] = {false, false, false, false};
-      int it = 0;
-      for (int e = tl; e < c; e += TN, ++it) {
-        const float4 p = src[o + e];
-        const float w = p.w;
-        const float t[4] = {fmul_(w, p.x), fmul_(w, p.y), fmul_(w, p.z), w};
+        for (int u = 0; u < kU; ++u)
+          if (e0 + u * TN < c) p[u] = src[o + e0 + u * TN];
 #pragma unroll
-        for (int q = 0; q < 4; ++q) {
-          fx[q].add(t[q], ovf, trn[q]);
-          fa[q] = __fadd_ru(fa[q], fabsf(t[q]));
-        }
-        bl[0] = fminf(bl[0], p.x); bh[0] = fmaxf(bh[0], p.x);
-        bl[1] = fminf(bl[1], p.y); bh[1] = fmaxf(bh[1], p.y);
-        bl[2] = fminf(bl[2], p.z); bh[2] = fmaxf(bh[2], p.z);
-        if ((it + 1) % kFoldTerms == 0) {
-#pragma unroll
-          for (int q = 0; q < 4; ++q) fx[q].fold();
-        }
+        for (int u = 0; u < kU; ++u)
+          if (e0 + u * TN < c) {
+            a.add(p[u], sc, sm);
+            ++cnt;
+          }
       }
-      __int128 sq[4];
-      int lsb[4];
-#pragma unroll
-      for (int q = 0; q < 4; ++q) {
-        fx[q].fold();
-        sq[q] = fx[q].sum();
-        lsb[q] = __reduce_min_sync(0xffffffffu, fx[q].lsb);
-      }
-#pragma unroll
-      for (int q = 0; q < 4; ++q) {
-        for (int sft = 16; sft > 0; sft >>= 1) {
-          sq[q] += shfl_xor_i128(sq[q], sft);
-          fa[q] = __fadd_ru(fa[q], __shfl_xor_sync(0xffffffffu, fa[q], sft));
-        }
-      }
-      int em[4];
-#pragma unroll
-      for (int q = 0; q < 4; ++q) {
-        const bool tq = __any_sync(0xffffffffu, trn[q]);
-        em[q] = tq ? kFix - 1 : (lsb[q] == INT_MAX ? INT_MAX : kFix + lsb[q]);
-      }
-#pragma unroll
-      for (int d = 0; d < 3; ++d) {
-        bl[d] = warp_min(bl[d]);
-        bh[d] = warp_max(bh[d]);
-      }
-      const bool wovf = __any_sync(0xffffffffu, ovf);
-      SubWarpStats &W = nw == 1 ? lst[f - f0] : wst[warp];
-      if (lane == 0) {
-        for (int q = 0; q < 4; ++q) {
-          W.s[q] = sq[q];
-          W.a[q] = double(fa[q]);
-          W.emin[q] = em[q];
-        }
-        for (int d = 0; d < 3; ++d) {
-          W.lo[d] = bl[d];
-          W.hi[d] = bh[d];
-        }
-        W.ovf = wovf ? 1 : 0;
-      }
+      NodeAcc w;
+      a.reduce(w, cnt, 32 * ((c + TN - 1) / TN) <= 1023, sc, sm);
+      if (lane == 0) (nw == 1 ? lst[f - f0] : wst[warp]) = w;
       if (nw > 1) {
         team_sync(team, nw);
-        if (tl == 0) {
-          SubWarpStats T = wst[w0];
-          for (int w = 1; w < nw; ++w) {
-            const SubWarpStats &V = wst[w0 + w];
-            for (int q = 0; q < 4; ++q) {
-              T.s[q] += V.s[q];
-              T.a[q] += V.a[q];
-              T.emin[q] = min(T.emin[q], V.emin[q]);
-            }
-            for (int d = 0; d < 3; ++d) {
-              T.lo[d] = fminf(T.lo[d], V.lo[d]);
-              T.hi[d] = fmaxf(T.hi[d], V.hi[d]);
-            }
-            T.ovf |= V.ovf;
-          }
-          lst[f - f0] = T;
-        }
+        if (wi == 0) merge_records(wst + w0, nw, lane, &lst[f - f0]);
         team_sync(team, nw);
       }
     }
@@ -1854,8 +1549,8 @@ __global__ void __launch_bounds__(kSubThreads, 2)
       DNode N = loc[f];
       const int c = N.count;
       if (c == 0) continue;  // an empty root (no particles) stays as it is
-      SubWarpStats T = lst[f - f0];
-      if (!decide_node(N, T.s, T.a, T.lo, T.hi, T.emin, T.ovf != 0, force_fallback, nd)) {
+      const NodeAcc T = lst[f - f0];
+      if (!decide_node(N, T, sc, sm, bad_scale, force_fallback, nd)) {
         // the reference's own sum: double, in array order (BGQCM.c:181-212)
         const int64_t o = N.offset;
         double x = 0, y = 0, z = 0, m = 0;
@@ -1894,12 +1589,21 @@ __global__ void __launch_bounds__(kSubThreads, 2)
       const float split = N.xc[d];
       const int share = (((c + nw - 1) / nw) + 31) & ~31;
       const int beg = wi * share, end = min(c, beg + share);
+      // four loads in flight per lane in every pass
+      constexpr int kU = 4;
+      const float *key = reinterpret_cast<const float *>(src + o) + d;
       int cl = 0;
-      for (int e0 = beg; e0 < end; e0 += 32) {
-        const int e = e0 + lane;
-        const bool l = e < end && key_of(src[o + e], d) < split;
-        cl += __popc(__ballot_sync(0xffffffffu, l));
+      for (int e0 = beg; e0 < end; e0 += 32 * kU) {
+        float kv[kU];
+#pragma unroll
+        for (int u = 0; u < kU; ++u) {
+          const int e = e0 + 32 * u + lane;
+          kv[u] = e < end ? key[4 * e] : INFINITY;
+        }
+#pragma unroll
+        for (int u = 0; u < kU; ++u) cl += e0 + 32 * u + lane < end && kv[u] < split;
       }
+      cl = __reduce_add_sync(0xffffffffu, cl);
       if (lane == 0) wtot[warp] = cl;
       team_sync(team, nw);
       int rank = 0, nleft = 0;
@@ -1908,53 +1612,76 @@ __global__ void __launch_bounds__(kSubThreads, 2)
         rank += w < wi ? v : 0;
         nleft += v;
       }
-      for (int e0 = beg; e0 < end; e0 += 32) {
-        const int e = e0 + lane;
-        float4 p = make_float4(0.f, 0.f, 0.f, 0.f);
-        int32_t id = 0;
-        if (e < end) {
-          p = src[o + e];
-          id = soid[o + e];
+      for (int e0 = beg; e0 < end; e0 += 32 * kU) {
+        float4 p[kU];
+        int32_t id[kU];
+#pragma unroll
+        for (int u = 0; u < kU; ++u) {
+          const int e = e0 + 32 * u + lane;
+          p[u] = make_float4(0.f, 0.f, 0.f, 0.f);
+          id[u] = 0;
+          if (e < end) {
+            p[u] = src[o + e];
+            id[u] = soid[o + e];
+          }
         }
-        const bool l = e < end && key_of(p, d) < split;
-        const unsigned bal = __ballot_sync(0xffffffffu, l);
-        if (l) {
-          const int q = rank + __popc(bal & below);
-          dst[o + q] = p;
-          doid[o + q] = id;
-          sidx[lo_off + q] = e;
-        } else if (e < end && e >= nleft) {
-          // a right element at or after nleft: no swap touches it
-          dst[o + e] = p;
-          doid[o + e] = id;
+#pragma unroll
+        for (int u = 0; u < kU; ++u) {
+          if (e0 + 32 * u >= end) break;  // the same for the whole warp
+          const int e = e0 + 32 * u + lane;
+          const bool l = e < end && key_of(p[u], d) < split;
+          const unsigned bal = __ballot_sync(0xffffffffu, l);
+          if (l) {
+            const int q = rank + __popc(bal & below);
+            dst[o + q] = p[u];
+            doid[o + q] = id[u];
+            sidx[lo_off + q] = e;
+          } else if (e < end && e >= nleft) {
+            // a right element at or after nleft: no swap touches it
+            dst[o + e] = p[u];
+            doid[o + e] = id[u];
+          }
+          rank += __popc(bal);
         }
-        rank += __popc(bal);
       }
       team_sync(team, nw);
-      for (int e = tl; e < nleft; e += TN) {
-        const float4 p = src[o + e];
-        if (key_of(p, d) < split) continue;
-        int q = e, steps = 0;
-        bool bad = false;
-        while (q < nleft && steps < kChainSteps) {
-          const int nq = sidx[lo_off + q];
-          if (nq <= q || nq >= c) {  // cannot happen for a valid partition
-            bad = true;
-            break;
+      for (int e0 = tl; e0 < nleft; e0 += kU * TN) {
+        float4 pu[kU];
+        int32_t iu[kU];
+#pragma unroll
+        for (int u = 0; u < kU; ++u)
+          if (e0 + u * TN < nleft) {
+            pu[u] = src[o + e0 + u * TN];
+            iu[u] = soid[o + e0 + u * TN];
           }
-          q = nq;
-          ++steps;
+#pragma unroll
+        for (int u = 0; u < kU; ++u) {
+          const int e = e0 + u * TN;
+          if (e >= nleft) break;
+          const float4 p = pu[u];
+          if (key_of(p, d) < split) continue;
+          int q = e, steps = 0;
+          bool bad = false;
+          while (q < nleft && steps < kChainSteps) {
+            const int nq = sidx[lo_off + q];
+            if (nq <= q || nq >= c) {  // cannot happen for a valid partition
+              bad = true;
+              break;
+            }
+            q = nq;
+            ++steps;
+          }
+          if (bad) {
+            atomicExch(reinterpret_cast<int32_t *>(counters + C_ERR), 2);
+            continue;
+          }
+          if (q < nleft) {
+            tflag[team] = 1;
+            continue;
+          }
+          dst[o + q] = p;
+          doid[o + q] = iu[u];
         }
-        if (bad) {
-          atomicExch(reinterpret_cast<int32_t *>(counters + C_ERR), 2);
-          continue;
-        }
-        if (q < nleft) {
-          tflag[team] = 1;
-          continue;
-        }
-        dst[o + q] = p;
-        doid[o + q] = soid[o + e];
       }
       team_sync(team, nw);
       if (tflag[team]) {
@@ -2051,38 +1778,53 @@ __global__ void __launch_bounds__(kSubThreads, 2)
   for (int dd = int(threadIdx.x); dd <= kSubDepth + 1; dd += kSubThreads)
     sub_first[int64_t(r) * (kSubDepth + 2) + dd] = dd <= depth + 1 ? first[min(dd, depth + 1)] : f1;
   for (int dd = 1 + int(threadIdx.x); dd <= kSubDepth; dd += kSubThreads)
-    hist[int64_t(dd - 1) * nroots + r] = dd <= depth ? first[dd + 1] - first[dd] : 0;
+    hist[int64_t(dd - 1) * gridDim.x + r] = dd <= depth ? first[dd + 1] - first[dd] : 0;
 }
 
-// Node totals of every depth below the subtree roots, into tot[0..kSubDepth).
-__global__ void k_subtree_totals(const int64_t *hist, int32_t nroots, int64_t *tot) {
-  const int dd = blockIdx.x;
-  int64_t v = 0;
-  for (int32_t r = threadIdx.x; r < nroots; r += blockDim.x) v += hist[int64_t(dd) * nroots + r];
-  for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-  __shared__ int64_t part[32];
-  if ((threadIdx.x & 31) == 0) part[threadIdx.x >> 5] = v;
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    int64_t t = 0;
-    for (int w = 0; w < int(blockDim.x >> 5); ++w) t += part[w];
-    tot[dd] = t;
+// Per depth below the subtree roots (a block each): every root's first node
+// among that depth's (exclusive scan over the roots) and the depth's total.
+__global__ void __launch_bounds__(kScanThreads)
+    k_subtree_scan(const LevelCtl *ctl, int32_t *hist, int32_t max_roots, int64_t *tot) {
+  __shared__ int sh_warp[32];
+  int32_t *row = hist + int64_t(blockIdx.x) * max_roots;
+  const int32_t nr = ctl->sub_ready && !ctl->abort ? ctl->sub_ne - ctl->sub_nb : 0;
+  int run = 0;
+  for (int32_t r0 = 0; r0 < nr; r0 += kScanThreads) {
+    const int32_t r = r0 + int32_t(threadIdx.x);
+    int total;
+    const int ex = block_excl_scan(r < nr ? row[r] : 0, sh_warp, &total);
+    if (r < nr) row[r] = run + ex;
+    run += total;
   }
+  if (threadIdx.x == 0) tot[blockIdx.x] = run;
 }
 
 // Copies every subtree node to its place among the levels: depth d below the
 // roots is level nb-level + d, ordered by root (i.e. by offset) and, within a
 // root, by the block's breadth-first order (also by offset).  pos holds the
-// exclusive scan of hist (depth-major), ne the first index after the roots'
-// level.
-__global__ void k_subtree_place(DNode *nodes, int32_t nb, int32_t ne, const DNode *sub,
-                                const int32_t *sub_first, const int64_t *pos) {
+// scans of k_subtree_scan; the first index after the roots' level is sub_ne.
+// Does nothing when the node array is too small (the host grows it and
+// launches this again).
+__global__ void __launch_bounds__(256)
+    k_subtree_place(DNode *nodes, const LevelCtl *ctl, const DNode *sub, const int32_t *sub_first,
+                    const int32_t *pos, int32_t max_roots, const int64_t *tot, int64_t node_cap) {
   __shared__ int fs[kSubDepth + 2];
+  __shared__ int64_t base[kSubDepth + 1];
   const int32_t r = int32_t(blockIdx.x);
-  const int32_t nroots = ne - nb;
+  if (!ctl->sub_ready || ctl->abort || r >= ctl->sub_ne - ctl->sub_nb) return;
+  const int32_t nb = ctl->sub_nb;
   for (int dd = threadIdx.x; dd <= kSubDepth + 1; dd += blockDim.x)
     fs[dd] = sub_first[int64_t(r) * (kSubDepth + 2) + dd];
+  if (threadIdx.x == 0) {
+    int64_t at = ctl->sub_ne;
+    for (int dd = 0; dd < kSubDepth; ++dd) {
+      base[dd] = at;
+      at += tot[dd];
+    }
+    base[kSubDepth] = at;
+  }
   __syncthreads();
+  if (base[kSubDepth] > node_cap) return;
   const int32_t roff = nodes[nb + r].offset;
   const DNode *loc = sub + 2 * int64_t(roff);
   const int total = fs[kSubDepth + 1];
@@ -2092,7 +1834,7 @@ __global__ void k_subtree_place(DNode *nodes, int32_t nb, int32_t ne, const DNod
     return dd;
   };
   auto global = [&](int j, int dd) {
-    return int32_t(ne + pos[int64_t(dd - 1) * nroots + r] + (j - fs[dd]));
+    return int32_t(base[dd - 1] + pos[int64_t(dd - 1) * max_roots + r] + (j - fs[dd]));
   };
   for (int j = 1 + int(threadIdx.x); j < total; j += blockDim.x) {
     const int dd = depth_of(j);
@@ -2111,53 +1853,6 @@ __global__ void k_subtree_place(DNode *nodes, int32_t nb, int32_t ne, const DNod
       N.cr = global(N.cr, 1);
     }
     nodes[nb + r] = N;
-  }
-}
-
-// 1 for nodes whose split produced two non-empty children.  (The element
-// buffers alternate between levels; a leaf's elements are copied once into
-// the next level's buffer by k_part_left, after which both buffers hold them
-// and later levels write only inside splitting nodes.)
-__global__ void k_split_flags(const DNode *nodes, int32_t nb, int32_t ne, int64_t *flag) {
-  const int32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (nb + i >= ne) return;
-  const DNode &N = nodes[nb + i];
-  flag[i] = (N.split_dim >= 0 && N.nleft > 0 && N.nleft < N.count) ? 1 : 0;
-}
-
-__global__ void k_children(DNode *nodes, int32_t nb, int32_t ne, const int64_t *rank,
-                           int64_t *maxcnt) {
-  const int32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-  unsigned m = 0;
-  if (nb + i < ne) {
-    const DNode &N = nodes[nb + i];
-    if (N.split_dim >= 0 && N.nleft > 0 && N.nleft < N.count)
-      m = unsigned(max(N.nleft, N.count - N.nleft));
-  }
-  m = __reduce_max_sync(0xffffffffu, m);
-  if ((threadIdx.x & 31) == 0 && m) atomicMax(reinterpret_cast<unsigned long long *>(maxcnt), m);
-  if (nb + i >= ne) return;
-  DNode &N = nodes[nb + i];
-  if (!(N.split_dim >= 0 && N.nleft > 0 && N.nleft < N.count)) {
-    N.cl = N.cr = 0;
-    return;
-  }
-  const int32_t cl = ne + 2 * int32_t(rank[i]), cr = cl + 1;
-  N.cl = cl;
-  N.cr = cr;
-  for (int s = 0; s < 2; ++s) {
-    DNode &C = nodes[s == 0 ? cl : cr];
-    C.count = s == 0 ? N.nleft : N.count - N.nleft;
-    C.offset = s == 0 ? N.offset : N.offset + N.nleft;
-    C.cl = C.cr = 0;
-    for (int d = 0; d < 3; ++d) {
-      C.xmin[d] = N.xmin[d];
-      C.xmax[d] = N.xmax[d];
-      C.xc[d] = 0.f;
-    }
-    C.tdr = 0.f;
-    C.split_dim = -1;
-    C.nleft = 0;
   }
 }
 
@@ -2658,15 +2353,6 @@ constexpr int kGroupSort = 1024;
 constexpr int kGW = 256;     // leaves up to this size are grouped by one warp
 constexpr int kGWarps = 4;   // warps (leaves) per block of k_groups_warp
 constexpr int kGroupThreads = 256;
-
-// Order-preserving map of a float to an unsigned integer.
-__device__ __forceinline__ uint32_t f2o(float v) {
-  const uint32_t b = __float_as_uint(v);
-  return (b & 0x80000000u) ? ~b : (b | 0x80000000u);
-}
-__device__ __forceinline__ float o2f(uint32_t o) {
-  return __uint_as_float((o & 0x80000000u) ? (o & 0x7fffffffu) : ~o);
-}
 
 // Splits a leaf into groups of G particles (the last one shorter) by recursive
 // median splits along the longest axis, left parts a multiple of G: the
@@ -3352,27 +3038,6 @@ __global__ void k_quad_adj_paths(const DNode *__restrict__ nodes, int32_t nnodes
   }
 }
 
-__global__ void k_iota(int32_t *p, int64_t n) {
-  for (int64_t i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x; i < n;
-       i += int64_t(gridDim.x) * blockDim.x)
-    p[i] = int32_t(i);
-}
-
-__global__ void k_root(DNode *nodes, int64_t n, TreeConfig cfg) {
-  DNode &R = nodes[0];
-  R.count = int32_t(n);
-  R.offset = 0;
-  R.cl = R.cr = 0;
-  for (int d = 0; d < 3; ++d) {
-    R.xmin[d] = cfg.min[d];
-    R.xmax[d] = cfg.max[d];
-    R.xc[d] = 0.f;
-  }
-  R.tdr = 0.f;
-  R.split_dim = -1;
-  R.nleft = 0;
-}
-
 inline unsigned grid_for(int64_t n, int threads, int64_t cap = 0) {
   if (cap <= 0) cap = int64_t(sm_count()) * 32;
   int64_t b = (n + threads - 1) / threads;
@@ -3385,20 +3050,17 @@ inline unsigned grid_for(int64_t n, int threads, int64_t cap = 0) {
 // Host orchestration
 // ---------------------------------------------------------------------------
 
-// Deep levels (nodes of ~2048 elements or fewer on average): the chunk
-// kernels run a warp per chunk.
-inline bool wm_level(int64_t L, int64_t n) { return L * 2048 >= n; }
-
 DeviceTree::~DeviceTree() {
-  void *ptrs[] = {epos_, tpos_, oid_, toid_, idx_, nodes_, ppm_, chunk_node_, chunk_base_, part_,
-                  left_cnt_, left_base_, scan_tmp_, node_tmp_, fallback_, counters_, leaf_ids_,
+  void *ptrs[] = {epos_, tpos_, oid_, toid_, idx_, nodes_, ppm_, chunk_node_, chunk_base_,
+                  left_cnt_, left_base_, acc_, ticket_, ctl_, scan_tmp_, node_tmp_, fallback_, counters_, leaf_ids_,
                   up_, processed_, leafdesc_, segs_, idx_list_, table_, items_, items_tmp_, gidx_,
                   tight_chunks_, tight_nodes_, segs_local_, ridx_, sub_nodes_, sub_first_,
-                  sub_hist_, sub_pos_, sub_tot_, sub_stats_, wpre_, chains_};
+                  sub_hist_, sub_tot_, sub_stats_, wpre_, chains_};
   for (void *p : ptrs)
     if (p) cudaFree(p);
   if (h_counters_) cudaFreeHost(h_counters_);
   if (h_sub_) cudaFreeHost(h_sub_);
+  if (h_ctl_) cudaFreeHost(h_ctl_);
   if (aux_) {
     cudaStreamSynchronize(aux_);
     cudaStreamDestroy(aux_);
@@ -3459,229 +3121,183 @@ cudaError_t DeviceTree::build(const TreeConfig &cfg, int64_t n, const float4 *po
     // the kernels' error flag lives in a counter slot: read back with the counters
     walk_err_ = reinterpret_cast<int32_t *>(counters_ + C_ERR);
   }
+  auto *ctl = reinterpret_cast<LevelCtl *>(ctl_);
+  if (!ctl) {
+    DT_CHECK(cudaMalloc(&ctl_, sizeof(LevelCtl)));
+    DT_CHECK(cudaHostAlloc(&h_ctl_, sizeof(LevelCtl), cudaHostAllocDefault));
+    DT_CHECK(cudaHostAlloc(&h_sub_, kSubDepth * sizeof(int64_t), cudaHostAllocDefault));
+    DT_CHECK(cudaMalloc(&sub_tot_, kSubDepth * sizeof(int64_t)));
+    DT_CHECK(cudaFuncSetAttribute(k_subtree, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                  kSubMax * int(sizeof(int32_t))));
+    ctl = reinterpret_cast<LevelCtl *>(ctl_);
+  }
+  auto *hc = reinterpret_cast<LevelCtl *>(h_ctl_);
   DT_CHECK(cudaMemsetAsync(counters_, 0, C_COUNT * sizeof(int64_t), s));
+  DT_CHECK(cudaMemsetAsync(ctl_, 0, sizeof(LevelCtl), s));
+  const size_t want_nodes = size_t(std::max<int64_t>(64, 4 * n / std::max(1, cfg.nd) + 64));
+  DT_CHECK(grow(nodes_, cap_nodes_, want_nodes, s));
   if (n > 0) {
-    DT_CHECK(cudaMemcpyAsync(epos_, pos_in, size_t(n) * sizeof(float4), cudaMemcpyDeviceToDevice, s));
-    k_iota<<<grid_for(n, 256), 256, 0, s>>>(oid_, n);
+    k_elements<<<grid_for(n, 256, int64_t(sm_count()) * 8), 256, 0, s>>>(pos_in, n, epos_, oid_, ctl);
     ++info_.launches;
   }
-  size_t want_nodes = size_t(std::max<int64_t>(64, 4 * n / std::max(1, cfg.nd) + 64));
-  DT_CHECK(grow(nodes_, cap_nodes_, want_nodes, s));
-  k_root<<<1, 1, 0, s>>>(nodes_, n, cfg);
-  ++info_.launches;
-  DT_CHECK(cudaGetLastError());
 
   // ---- levels ----
+  // Nodes of at most sub_max elements are built whole, a block each; with the
+  // tight-certification hook, or after a subtree deeper than a block's
+  // bookkeeping, every level runs here.
+  const bool subtrees = n == 0 || (!sub_off_ && cfg.force_cm_fallback != 2);
+  const int32_t sub_max = subtrees ? kSubMax : -1;
   std::vector<int32_t> level_begin{0};
-  int32_t nb = 0, ne = 1;
-  int64_t level_max = n;  // the level's largest node
-  if (!node_attr_) {
-    DT_CHECK(cudaFuncSetAttribute(k_part_node<256>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                  kNodeMax * int(sizeof(int32_t))));
-    DT_CHECK(cudaFuncSetAttribute(k_part_node<1024>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                  kNodeMax * int(sizeof(int32_t))));
-    node_attr_ = true;
-  }
-  while (ne > nb) {
-    const int32_t L = ne - nb;
-    if (!sub_off_ && cfg.force_cm_fallback != 2 && level_max <= kSubMax) {
-      // every node of this level fits one block: each builds its whole subtree
+  int64_t level_nodes = 1, level_max = n;  // the next level's extent
+  int32_t level = 0, level_ne = 1;
+  bool counted = true;  // false: the level's statistics are there, its centres just decided
+  for (bool started = false;;) {
+    // as many levels as halve the largest node down to a subtree; few when the
+    // level is already wide (a deep, uneven tree)
+    int batch = 0;
+    if (!(subtrees && level_max <= sub_max)) {
+      batch = 1;
+      const int64_t goal = subtrees ? sub_max : std::max<int64_t>(cfg.nd, 1);
+      while ((level_max >> batch) > goal && batch < 16 && (level_nodes << batch) < 2048) ++batch;
+    }
+    const int64_t widest = std::min<int64_t>(level_nodes << std::max(0, batch - 1), std::max<int64_t>(n, 1));
+    const int64_t after = std::min<int64_t>(level_nodes << batch, std::max<int64_t>(n, 1));
+    const size_t max_chunks = size_t(n / kChunk + after + 1);
+    const size_t nodes_most =
+        std::min<size_t>(size_t(2 * n + 1), size_t(level_ne) + size_t(level_nodes << (batch + 1)));
+    DT_CHECK(grow(nodes_, cap_nodes_, nodes_most, s, true));
+    if (!started || max_chunks > cap_cn_ / 2 || size_t(after) + 1 > cap_ac_) {
+      // the chunk maps and accumulators of the level in progress move along
+      DT_CHECK(grow_chunks(max_chunks, size_t(after) + 1, s));
+    }
+    int32_t *cn[2] = {chunk_node_, chunk_node_ + cap_cn_ / 2};
+    int32_t *cb[2] = {chunk_base_, chunk_base_ + cap_cb_ / 2};
+    DT_CHECK(grow(left_cnt_, cap_lc_, max_chunks, s));
+    DT_CHECK(grow(left_base_, cap_lb_, max_chunks, s));
+    DT_CHECK(grow(wpre_, cap_wp_, max_chunks * (kChunkThreads / 32), s));
+    DT_CHECK(grow(fallback_, cap_fb_, size_t(widest) + 1, s));
+    if (batch > 0) DT_CHECK(grow(chains_, cap_ch_, size_t(std::max<int64_t>(n, 1)), s));
+    auto *acc = reinterpret_cast<NodeAcc *>(acc_);
+    if (!started) {
+      k_root<<<1, 256, 0, s>>>(nodes_, n, cfg, ctl, cn[0], cb[0], acc, ticket_, sub_max);
+      ++info_.launches;
+      started = true;
+    }
+    float4 *pb[2] = {epos_, tpos_};
+    int32_t *ob[2] = {oid_, toid_};
+    for (int i = 0; i < batch; ++i) {
+      const int32_t l = level + i;
+      const int from = l & 1, to = from ^ 1;
+      const unsigned grid =
+          unsigned(n / kChunk + std::min<int64_t>(level_nodes << i, std::max<int64_t>(n, 1)) + 1);
+      if (counted) {
+        k_level_stats<<<grid, kChunkThreads, 0, s>>>(pb[from], nodes_, ctl, l, cn[from], cb[from],
+                                                     acc, ticket_, fallback_, counters_,
+                                                     cfg.force_cm_fallback, cfg.nd);
+        ++info_.launches;
+      }
+      counted = true;
+      k_level_count<<<grid, kChunkThreads, 0, s>>>(pb[from], nodes_, ctl, l, cn[from], cb[from],
+                                                   cn[to], cb[to], left_cnt_, left_base_, wpre_,
+                                                   acc, ticket_, counters_, sub_max);
+      k_part_left<<<grid, kChunkThreads, 0, s>>>(pb[from], ob[from], nodes_, ctl, l, cn[from],
+                                                 cb[from], left_base_, wpre_, pb[to], ob[to], idx_,
+                                                 ridx_);
+      k_part_right<<<grid, kChunkThreads, 0, s>>>(pb[from], ob[from], nodes_, ctl, l, cn[from],
+                                                  cb[from], idx_, pb[to], ob[to], walk_err_,
+                                                  counters_, reinterpret_cast<ChainItem *>(chains_),
+                                                  int64_t(cap_ch_));
+      k_part_chains<<<unsigned(4 * sm_count()), 256, 0, s>>>(
+          pb[from], ob[from], nodes_, ctl, l, reinterpret_cast<const ChainItem *>(chains_),
+          int64_t(cap_ch_), counters_, idx_, ridx_, pb[to], ob[to], walk_err_);
+      info_.launches += 4;
+    }
+    const int64_t max_roots = after;
+    if (subtrees) {
       DT_CHECK(grow(sub_nodes_, cap_sub_, size_t(2 * std::max<int64_t>(n, 1)), s));
-      DT_CHECK(grow(sub_stats_, cap_ss_, size_t(std::max<int64_t>(n, 1)) * sizeof(SubWarpStats), s));
-      DT_CHECK(grow(sub_first_, cap_sf_, size_t(L) * (kSubDepth + 2), s));
-      DT_CHECK(grow(sub_hist_, cap_sh_, size_t(L) * kSubDepth + 1, s));
-      DT_CHECK(grow(sub_pos_, cap_sp_, size_t(L) * kSubDepth + 1, s));
-      DT_CHECK(grow(sub_tot_, cap_st_, size_t(kSubDepth), s));
-      DT_CHECK(grow(scan_tmp_, cap_scan_, size_t(scan_tmp_size(int64_t(L) * kSubDepth)), s));
-      if (!h_sub_) DT_CHECK(cudaHostAlloc(&h_sub_, kSubDepth * sizeof(int64_t), cudaHostAllocDefault));
-      if (!sub_attr_) {
-        DT_CHECK(cudaFuncSetAttribute(k_subtree, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                      kSubMax * int(sizeof(int32_t))));
-        sub_attr_ = true;
-      }
-      const size_t smem = size_t(std::max<int64_t>(level_max, 1)) * sizeof(int32_t);
-      k_subtree<<<unsigned(L), kSubThreads, smem, s>>>(
-          nodes_, nb, ne, epos_, oid_, tpos_, toid_, sub_nodes_,
-          reinterpret_cast<SubWarpStats *>(sub_stats_), sub_first_, sub_hist_,
-          cfg.force_cm_fallback, cfg.nd, counters_);
-      ++info_.launches;
-      DT_CHECK(cudaGetLastError());
-      DT_CHECK(scan_counted(sub_hist_, sub_pos_, int64_t(L) * kSubDepth, nullptr, scan_tmp_, s));
-      k_subtree_totals<<<kSubDepth, 256, 0, s>>>(sub_hist_, L, sub_tot_);
-      ++info_.launches;
-      DT_CHECK(cudaGetLastError());
+      DT_CHECK(grow(sub_stats_, cap_ss_, size_t(std::max<int64_t>(n, 1)) * sizeof(NodeAcc), s));
+      DT_CHECK(grow(sub_first_, cap_sf_, size_t(max_roots) * (kSubDepth + 2), s));
+      DT_CHECK(grow(sub_hist_, cap_sh_, size_t(max_roots) * kSubDepth, s));
+      const size_t smem = size_t(std::max<int64_t>(std::min<int64_t>(n, sub_max), 1)) * sizeof(int32_t);
+      k_subtree<<<unsigned(max_roots), kSubThreads, smem, s>>>(
+          nodes_, ctl, epos_, oid_, tpos_, toid_, sub_nodes_, reinterpret_cast<NodeAcc *>(sub_stats_),
+          sub_first_, sub_hist_, cfg.force_cm_fallback, cfg.nd, counters_);
+      k_subtree_scan<<<kSubDepth, kScanThreads, 0, s>>>(ctl, sub_hist_, int32_t(max_roots), sub_tot_);
+      k_subtree_place<<<unsigned(max_roots), 256, 0, s>>>(nodes_, ctl, sub_nodes_, sub_first_,
+                                                          sub_hist_, int32_t(max_roots), sub_tot_,
+                                                          int64_t(cap_nodes_));
+      info_.launches += 3;
       DT_CHECK(cudaMemcpyAsync(h_sub_, sub_tot_, kSubDepth * sizeof(int64_t), cudaMemcpyDeviceToHost, s));
-      DT_CHECK(cudaMemcpyAsync(h_counters_, counters_, C_COUNT * sizeof(int64_t),
-                               cudaMemcpyDeviceToHost, s));
-      DT_CHECK(cudaStreamSynchronize(s));
-      const int32_t serr = *reinterpret_cast<const int32_t *>(h_counters_ + C_ERR);
-      if (serr == 4) {
-        // a subtree deeper than kSubDepth levels: build again level by level
-        sub_off_ = true;
-        const cudaError_t e = build(cfg, n, pos_in, jsplit, s);
-        sub_off_ = false;
-        return e;
-      }
-      if (serr) {
-        err_ = serr == 3 ? "subtree: a node outgrew the block's shared memory"
-                         : "partition chain check failed";
-        return cudaErrorUnknown;
-      }
-      info_.cm_fallbacks += h_counters_[C_SUBFB];
-      int64_t total = ne;
+    }
+    DT_CHECK(cudaGetLastError());
+    DT_CHECK(cudaMemcpyAsync(hc, ctl_, sizeof(LevelCtl), cudaMemcpyDeviceToHost, s));
+    DT_CHECK(cudaMemcpyAsync(h_counters_, counters_, C_COUNT * sizeof(int64_t),
+                             cudaMemcpyDeviceToHost, s));
+    DT_CHECK(cudaStreamSynchronize(s));
+    const int32_t err = *reinterpret_cast<const int32_t *>(h_counters_ + C_ERR);
+    if (err == 4) {
+      // a subtree deeper than kSubDepth levels: build again level by level
+      sub_off_ = true;
+      const cudaError_t e = build(cfg, n, pos_in, jsplit, s);
+      sub_off_ = false;
+      return e;
+    }
+    if (err) {
+      err_ = err == 3 ? "subtree: a node outgrew the block's shared memory"
+                      : "partition chain check failed";
+      return cudaErrorUnknown;
+    }
+    // the levels made so far, and the extent of the one that is next
+    while (int32_t(level_begin.size()) <= hc->next_level)
+      level_begin.push_back(hc->begin[level_begin.size() % kCtlLevels]);
+    level = hc->next_level;
+    const LevelSpan &X = hc->lev[level & 1];
+    level_nodes = X.ne - X.nb;
+    level_ne = X.ne;
+    level_max = X.maxcnt;
+    if (hc->abort) {
+      // undecided centres of mass in this level: certify them, or sum as the
+      // reference does, then go on from its left counts
+      k_cm_tight_sums<<<tight_blocks(), kTightThreads, 0, s>>>(
+          pb[level & 1], nodes_, fallback_, counters_, reinterpret_cast<TightChunk *>(tight_chunks_),
+          reinterpret_cast<TightNode *>(tight_nodes_), cfg.force_cm_fallback == 1);
+      k_cm_tight_bound<<<tight_blocks(), kTightThreads, 0, s>>>(
+          pb[level & 1], nodes_, fallback_, counters_,
+          reinterpret_cast<const TightChunk *>(tight_chunks_),
+          reinterpret_cast<TightNode *>(tight_nodes_), cfg.force_cm_fallback == 1);
+      k_cm_fallback<<<unsigned(std::min<int64_t>((level_nodes + 127) / 128, 1024)), 128, 0, s>>>(
+          pb[level & 1], nodes_, fallback_, counters_);
+      k_decided<<<1, 1, 0, s>>>(ctl, counters_);
+      info_.launches += 4;
+      DT_CHECK(cudaGetLastError());
+      counted = false;
+      continue;
+    }
+    if (hc->sub_ready) {
+      int64_t total = hc->sub_ne;
       for (int d = 0; d < kSubDepth; ++d) total += h_sub_[d];
       if (total > INT32_MAX) return cudaErrorInvalidValue;
-      DT_CHECK(grow(nodes_, cap_nodes_, size_t(total), s, true));
-      k_subtree_place<<<unsigned(L), 256, 0, s>>>(nodes_, nb, ne, sub_nodes_, sub_first_, sub_pos_);
-      ++info_.launches;
-      DT_CHECK(cudaGetLastError());
-      int64_t at = ne;
-      level_begin.push_back(ne);
+      if (size_t(total) > cap_nodes_) {
+        DT_CHECK(grow(nodes_, cap_nodes_, size_t(total), s, true));
+        k_subtree_place<<<unsigned(max_roots), 256, 0, s>>>(nodes_, ctl, sub_nodes_, sub_first_,
+                                                            sub_hist_, int32_t(max_roots), sub_tot_,
+                                                            int64_t(cap_nodes_));
+        ++info_.launches;
+        DT_CHECK(cudaGetLastError());
+      }
+      int64_t at = hc->sub_ne;
+      level_begin.push_back(int32_t(at));
       for (int d = 0; d < kSubDepth && h_sub_[d] > 0; ++d) {
         at += h_sub_[d];
         level_begin.push_back(int32_t(at));
       }
-      nb = ne = int32_t(total);
+      level_ne = int32_t(total);
       break;
     }
-    if (size_t(ne) + 2 * size_t(L) > cap_nodes_)
-      DT_CHECK(grow(nodes_, cap_nodes_, size_t(ne) + 2 * size_t(L), s, true));
-    DT_CHECK(grow(node_tmp_, cap_nt_, size_t(L) + 1, s));
-    DT_CHECK(grow(chunk_base_, cap_cb_, size_t(L) + 1, s));
-    DT_CHECK(grow(scan_tmp_, cap_scan_, size_t(scan_tmp_size(std::max<int64_t>(L, n + 1))), s));
-    DT_CHECK(grow(fallback_, cap_fb_, size_t(L), s));
-    const int64_t max_chunks = n / kChunk + L + 1;
-    DT_CHECK(grow(chunk_node_, cap_cn_, size_t(max_chunks), s));
-    DT_CHECK(grow(part_, cap_part_, size_t(max_chunks) * kPartWords, s));
-    DT_CHECK(grow(left_cnt_, cap_lc_, size_t(max_chunks), s));
-    DT_CHECK(grow(left_base_, cap_lb_, size_t(max_chunks), s));
-    DT_CHECK(grow(wpre_, cap_wp_, size_t(max_chunks) * (kChunkThreads / 32), s));
-    if (level_max > kNodeMax && !wm_level(L, n))
-      DT_CHECK(grow(chains_, cap_ch_, size_t(std::max<int64_t>(n, 1)), s));
-    const unsigned gL = unsigned((L + 127) / 128);
-    const bool small = int64_t(L) <= kScanBlock;
-    if (small) {
-      k_chunk_setup_small<<<1, kScanThreads, 0, s>>>(nodes_, nb, ne, chunk_base_, chunk_node_,
-                                                     counters_);
-      ++info_.launches;
-    } else {
-      DT_CHECK(cudaMemsetAsync(counters_ + C_NFALLBACK, 0, sizeof(int64_t), s));
-      DT_CHECK(cudaMemsetAsync(counters_ + C_NTIGHT, 0, sizeof(int64_t), s));
-      DT_CHECK(cudaMemsetAsync(counters_ + C_MAXCNT, 0, sizeof(int64_t), s));
-      DT_CHECK(cudaMemsetAsync(counters_ + C_CHAINS, 0, sizeof(int64_t), s));
-      k_chunk_counts<<<gL, 128, 0, s>>>(nodes_, nb, ne, node_tmp_);
-      ++info_.launches;
-      DT_CHECK(scan_counted(node_tmp_, chunk_base_, L, counters_ + C_NCHUNK, scan_tmp_, s));
-      k_chunk_fill<<<gL, 128, 0, s>>>(nodes_, nb, ne, chunk_base_, chunk_node_);
-      ++info_.launches;
-    }
-    // deep levels (nodes of ~2048 elements or fewer on average): a warp per chunk
-    const bool wm = wm_level(L, n);
-    const unsigned gC = wm ? unsigned((max_chunks + 7) / 8) : unsigned(max_chunks);
-#define CHUNK_LAUNCH(kern, ...)                                                  \
-  do {                                                                           \
-    if (wm) kern<true><<<gC, kChunkThreads, 0, s>>>(__VA_ARGS__);                \
-    else kern<false><<<gC, kChunkThreads, 0, s>>>(__VA_ARGS__);                  \
-    ++info_.launches;                                                            \
-  } while (0)
-    CHUNK_LAUNCH(k_stats_partial, epos_, nodes_, chunk_node_, chunk_base_, nb, counters_ + C_NCHUNK,
-                 part_);
-    // one thread finishes each single-chunk node, a warp each larger one; a
-    // small level with larger nodes has a warp finish every node in one launch
-    const bool one_chunk = level_max <= kChunk;
-    const bool big_nodes = L <= 16 && level_max > 32 * int64_t(kChunk);
-    if (big_nodes) {
-      // the top levels: a block per node (every node of the level)
-      k_stats_final_block<<<unsigned(L), 256, 0, s>>>(nodes_, nb, ne, chunk_base_, part_, fallback_,
-                                                      counters_, cfg.force_cm_fallback, cfg.nd);
-      ++info_.launches;
-    } else if (!small || one_chunk) {
-      k_stats_final_one<<<gL, 128, 0, s>>>(nodes_, nb, ne, chunk_base_, part_, fallback_,
-                                            counters_, cfg.force_cm_fallback, cfg.nd);
-      ++info_.launches;
-    }
-    if (!one_chunk && !big_nodes) {
-      k_stats_final<<<unsigned((int64_t(L) * 32 + 255) / 256), 256, 0, s>>>(
-          nodes_, nb, ne, chunk_base_, part_, fallback_, counters_, cfg.force_cm_fallback, cfg.nd,
-          small);
-      ++info_.launches;
-    }
-    k_cm_tight_sums<<<tight_blocks(), kTightThreads, 0, s>>>(
-        epos_, nodes_, fallback_, counters_, reinterpret_cast<TightChunk *>(tight_chunks_),
-        reinterpret_cast<TightNode *>(tight_nodes_), cfg.force_cm_fallback == 1);
-    ++info_.launches;
-    k_cm_tight_bound<<<tight_blocks(), kTightThreads, 0, s>>>(
-        epos_, nodes_, fallback_, counters_, reinterpret_cast<const TightChunk *>(tight_chunks_),
-        reinterpret_cast<TightNode *>(tight_nodes_), cfg.force_cm_fallback == 1);
-    ++info_.launches;
-    k_cm_fallback<<<unsigned(std::min<int64_t>((L + 127) / 128, 1024)), 128, 0, s>>>(
-        epos_, nodes_, fallback_, counters_);
-    ++info_.launches;
-    if (level_max <= kNodeMax) {
-      // every node fits one block's shared memory: the whole partition in one launch
-      const size_t smem = size_t(std::max<int64_t>(level_max, 1)) * sizeof(int32_t);
-      // few large nodes: 1024 threads a node; many (most of them small, as in
-      // clustered sets): 256
-      if (level_max > 2048 && L <= 1024)
-        k_part_node<1024><<<unsigned(L), 1024, smem, s>>>(epos_, oid_, nodes_, nb, ne,
-                                                          int32_t(level_max), tpos_, toid_, walk_err_);
-      else
-        k_part_node<256><<<unsigned(L), 256, smem, s>>>(epos_, oid_, nodes_, nb, ne,
-                                                        int32_t(level_max), tpos_, toid_, walk_err_);
-      ++info_.launches;
-    } else {
-      CHUNK_LAUNCH(k_part_count, epos_, nodes_, chunk_node_, chunk_base_, nb, counters_ + C_NCHUNK,
-                   left_cnt_, wpre_);
-      k_part_node_scan<<<unsigned((int64_t(L) * 32 + 127) / 128), 128, 0, s>>>(
-          nodes_, nb, ne, chunk_base_, left_cnt_, left_base_);
-      ++info_.launches;
-      CHUNK_LAUNCH(k_part_left, epos_, oid_, nodes_, chunk_node_, chunk_base_, nb,
-                   counters_ + C_NCHUNK, left_base_, wpre_, tpos_, toid_, idx_, ridx_);
-      CHUNK_LAUNCH(k_part_right, epos_, oid_, nodes_, chunk_node_, chunk_base_, nb,
-                   counters_ + C_NCHUNK, idx_, ridx_, tpos_, toid_, walk_err_, counters_,
-                   reinterpret_cast<ChainItem *>(chains_), int64_t(cap_ch_));
-      if (!wm) {
-        k_part_chains<<<unsigned(4 * sm_count()), 256, 0, s>>>(
-            epos_, oid_, nodes_, reinterpret_cast<const ChainItem *>(chains_), int64_t(cap_ch_),
-            counters_, idx_, ridx_, tpos_, toid_, walk_err_);
-        ++info_.launches;
-      }
-    }
-#undef CHUNK_LAUNCH
-    std::swap(epos_, tpos_);
-    std::swap(cap_e_, cap_t_);
-    std::swap(oid_, toid_);
-    std::swap(cap_o_, cap_to_);
-    // one block sets up the children of a level of up to 1024 nodes; above
-    // that its stores alone take longer than the three-kernel path
-    if (L <= 1024) {
-      k_children_small<<<1, kScanThreads, 0, s>>>(nodes_, nb, ne, counters_ + C_NSPLIT,
-                                                  counters_ + C_MAXCNT);
-      ++info_.launches;
-    } else {
-      k_split_flags<<<gL, 128, 0, s>>>(nodes_, nb, ne, node_tmp_);
-      ++info_.launches;
-      DT_CHECK(scan_counted(node_tmp_, node_tmp_, L, counters_ + C_NSPLIT, scan_tmp_, s));
-      k_children<<<gL, 128, 0, s>>>(nodes_, nb, ne, node_tmp_, counters_ + C_MAXCNT);
-      ++info_.launches;
-    }
-    DT_CHECK(cudaGetLastError());
-    DT_CHECK(cudaMemcpyAsync(h_counters_, counters_, (C_ERR + 1) * sizeof(int64_t),
-                             cudaMemcpyDeviceToHost, s));
-    DT_CHECK(cudaStreamSynchronize(s));
-    const int32_t perr = *reinterpret_cast<const int32_t *>(h_counters_ + C_ERR);
-    if (perr) {
-      err_ = perr == 3 ? "partition: a node outgrew the one-block partition's shared memory"
-                       : "partition chain check failed";
-      return cudaErrorUnknown;
-    }
-    info_.cm_fallbacks += h_counters_[C_NFALLBACK] - h_counters_[C_NTIGHT];
-    const int64_t nsplit = h_counters_[C_NSPLIT];
-    level_max = h_counters_[C_MAXCNT];
-    nb = ne;
-    ne = int32_t(ne + 2 * nsplit);
-    level_begin.push_back(nb);
+    if (hc->done) break;
   }
+  info_.cm_fallbacks = h_counters_[C_SUBFB] + h_counters_[C_SEQ];
+  const int32_t ne = level_ne;
   levels_ = level_begin;
   const int32_t nnodes = ne;
   info_.nodes = nnodes;
@@ -3798,6 +3414,33 @@ cudaError_t DeviceTree::build(const TreeConfig &cfg, int64_t n, const float4 *po
   // ---- work items ----
   DT_CHECK(fill_items(jsplit, s));
   lists_ms_ = std::chrono::duration<double, std::milli>(std::chrono::steady_clock::now() - t1).count();
+  return cudaSuccess;
+}
+
+// Room for `chunks` chunks a level (two maps, by level parity) and `nodes`
+// nodes' accumulators and tickets, what is there kept.
+cudaError_t DeviceTree::grow_chunks(size_t chunks, size_t nodes, cudaStream_t s) {
+  if (2 * chunks > cap_cn_) {
+    const size_t half = chunks + chunks / 4 + 128, old = cap_cn_ / 2;
+    for (int32_t **p : {&chunk_node_, &chunk_base_}) {
+      int32_t *q = nullptr;
+      DT_CHECK(cudaMalloc(&q, 2 * half * sizeof(int32_t)));
+      if (*p) {
+        for (int m = 0; m < 2; ++m)
+          DT_CHECK(cudaMemcpyAsync(q + m * half, *p + m * old, old * sizeof(int32_t),
+                                   cudaMemcpyDeviceToDevice, s));
+        DT_CHECK(cudaStreamSynchronize(s));
+        cudaFree(*p);
+      }
+      *p = q;
+    }
+    cap_cn_ = cap_cb_ = 2 * half;
+  }
+  size_t bytes = cap_ac_ * sizeof(NodeAcc);
+  DT_CHECK(grow(acc_, bytes, nodes * sizeof(NodeAcc), s, true));
+  size_t tickets = cap_ac_;
+  DT_CHECK(grow(ticket_, tickets, nodes, s, true));
+  cap_ac_ = std::min(bytes / sizeof(NodeAcc), tickets);
   return cudaSuccess;
 }
 

@@ -132,13 +132,14 @@ class DeviceTree {
   float *ppm_ = nullptr;
   size_t cap_ppm_ = 0;
   // per-level work
-  int32_t *chunk_node_ = nullptr;
-  int64_t *chunk_base_ = nullptr;
+  int32_t *chunk_node_ = nullptr, *chunk_base_ = nullptr;  // two maps each, by level parity
   size_t cap_cn_ = 0, cap_cb_ = 0;
-  double *part_ = nullptr;   // per-chunk partial sums
-  size_t cap_part_ = 0;
-  int32_t *left_cnt_ = nullptr;
-  int64_t *left_base_ = nullptr;
+  unsigned char *acc_ = nullptr;  // per node: statistics in the making
+  unsigned *ticket_ = nullptr;    // per node: its chunks done
+  size_t cap_ac_ = 0;
+  unsigned char *ctl_ = nullptr, *h_ctl_ = nullptr;  // the levels' extents, and a pinned copy
+  cudaError_t grow_chunks(size_t chunks, size_t nodes, cudaStream_t s);
+  int32_t *left_cnt_ = nullptr, *left_base_ = nullptr;
   int32_t *wpre_ = nullptr;  // per chunk: each warp's left elements before its share
   int4 *chains_ = nullptr;    // the level's long swap chains (16 bytes each)
   size_t cap_lc_ = 0, cap_lb_ = 0, cap_wp_ = 0, cap_ch_ = 0;
@@ -162,7 +163,6 @@ class DeviceTree {
   size_t cap_ld_ = 0;
   SegDesc *segs_ = nullptr;
   size_t cap_seg_ = 0;
-  bool node_attr_ = false;         // k_part_node's shared-memory limit raised
   int2 *segs_local_ = nullptr;     // the one-pass walk's per-leaf regions (start, count)
   size_t cap_segl_ = 0;
   int32_t *idx_list_ = nullptr;
@@ -180,10 +180,10 @@ class DeviceTree {
   unsigned char *sub_stats_ = nullptr;  // reduced statistics of a level's nodes
   size_t cap_ss_ = 0;
   int32_t *sub_first_ = nullptr;
-  int64_t *sub_hist_ = nullptr, *sub_pos_ = nullptr, *sub_tot_ = nullptr;
-  size_t cap_sub_ = 0, cap_sf_ = 0, cap_sh_ = 0, cap_sp_ = 0, cap_st_ = 0;
+  int32_t *sub_hist_ = nullptr;
+  int64_t *sub_tot_ = nullptr;
+  size_t cap_sub_ = 0, cap_sf_ = 0, cap_sh_ = 0;
   int64_t *h_sub_ = nullptr;
-  bool sub_attr_ = false;
   bool sub_off_ = false;  // when set, every level runs in the level loop
 };
 
