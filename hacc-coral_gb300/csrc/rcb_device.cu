@@ -261,30 +261,32 @@ __device__ __forceinline__ int block_excl_scan(int v, int *sh_warp, int *total) 
 // the levels that the particle count calls for and waits once for all of them.
 // (Seventeen launches and a synchronisation a level took 100 us a level at
 // 32^3 particles and 160 at 128^3.)
+// A child small enough for a subtree block becomes a root of k_subtree at
+// once, whatever its level, and takes no chunk of the levels below: in a
+// clustered set the last halos take several levels more than the rest.
 // A level whose centre-of-mass bounds leave a node undecided raises `abort`:
 // the launches after it do nothing, and the host runs the certification
 // kernels for it and goes on from there.
 // ---------------------------------------------------------------------------
 struct LevelSpan {
   int32_t level;  // which level this slot describes
-  int32_t run;    // 0: no level here (every node fits a subtree, or none is left)
-  int32_t nb, ne;  // its nodes
-  int32_t nchunk;  // chunks of its nodes
-  int32_t maxcnt;  // its largest node
-  int32_t pad[2];
+  int32_t run;    // 0: no level here (no node is left for the level loop)
+  int32_t nb, ne;  // its nodes, subtree roots among them
+  int32_t nchunk;  // chunks of the others
+  int32_t live;    // the others
+  int32_t maxcnt;  // the largest of them
+  int32_t pad;
 };
 constexpr int kCtlLevels = 64;
 struct LevelCtl {
   LevelSpan lev[2];    // by level parity
   int32_t abort;       // level + 1 of a level with undecided nodes, or 0
-  int32_t sub_ready;   // every node of [sub_nb, sub_ne) fits a subtree block
-  int32_t sub_nb, sub_ne;
-  int32_t sub_parity;  // the element buffer that holds them
-  int32_t done;        // no node was split: the tree is complete
+  int32_t nroots;      // subtree roots so far
+  int32_t done;        // no node is left for the level loop
+  int32_t node_end;    // nodes of all levels
   unsigned mx_term, mx_mass;  // largest |w x|, |w y|, |w z| and |w|, as bits
   unsigned ticket;     // chunks of the level counted
   int32_t next_level;  // the level made last
-  int32_t pad[2];
   int32_t begin[kCtlLevels];  // first node of a level, by level modulo kCtlLevels
 };
 __device__ __forceinline__ int32_t chunks_of(int32_t count) { return (count + kChunk - 1) / kChunk; }
@@ -465,11 +467,11 @@ struct LaneAcc {
 __device__ __forceinline__ double pow2(int e) {  // normal range
   return __longlong_as_double((long long)(e + 1023) << 52);
 }
+__device__ __forceinline__ float pow2f(int e) { return __uint_as_float(unsigned(e + 127) << 23); }
 
-// Correctly rounded double of h 2^(k-23) + l 2^(k-45).
-__device__ double sum_to_double(long long h, long long l, int k) {
-  const double unit = pow2(k - 45);
-  if (h < (1ll << 40) && h > -(1ll << 40)) return __dmul_rn(__ll2double_rn((h << 22) + l), unit);
+// Correctly rounded double of h 2^22 + l (units of 2^(k-45)).
+__device__ double units_to_double(long long h, long long l) {
+  if (h < (1ll << 40) && h > -(1ll << 40)) return __ll2double_rn((h << 22) + l);
   const __int128 v = (__int128(h) << 22) + l;
   const bool neg = v < 0;
   const unsigned __int128 u = neg ? (unsigned __int128)(-v) : (unsigned __int128)v;
@@ -479,7 +481,7 @@ __device__ double sum_to_double(long long h, long long l, int k) {
   // the top 63 bits with the rest folded into a sticky bit, rounded once
   unsigned long long m = (unsigned long long)(u >> sh);
   if (sh > 0 && (u & ((((unsigned __int128)1) << sh) - 1)) != 0) m |= 1ull;
-  const double r = __dmul_rn(__dmul_rn(__ull2double_rn(m), pow2(sh)), unit);
+  const double r = __dmul_rn(__ull2double_rn(m), pow2(sh));
   return neg ? -r : r;
 }
 
@@ -501,10 +503,80 @@ __device__ bool certify(double sx, double bx, double sm, double bm, float *out) 
   return true;
 }
 
+// The sums of a node's terms and what bounds their distance from the
+// reference's sequential ones, in units of 2^(k-45).
+struct NodeSums {
+  double x[4];   // the exact sums, rounded to double
+  float abs[4];  // at least sum |terms|
+  float err[4];  // at least |reference sum - x|
+  bool exact[4];  // the reference's sum is exactly x
+};
+
+__device__ __forceinline__ NodeSums node_sums(const NodeAcc &A, int32_t count) {
+  NodeSums S;
+  // The reference's sequential sum lies within (n - 1) u sum|terms| of the
+  // exact sum, to first order; (n + 64) u (1 + 2^-20) covers the rest.  The sums
+  // here are exact except for truncated terms (half a unit each) and their
+  // rounding to double.
+  const float n = __int2float_ru(count);
+  const float g = __fmul_ru(__fmul_ru(__fadd_ru(n, 64.f), 0x1p-53f), 1.f + 0x1p-20f);
+  const float slack = A.trunc ? n : 0.f;
+  const bool wpos = o2f(A.wmin) >= 0.f;
+#pragma unroll
+  for (int q = 0; q < 4; ++q) {
+    S.x[q] = units_to_double(A.h[q], A.l[q]);
+    const float xa = __double2float_ru(fabs(S.x[q]));
+    // sum of |terms|: the sum itself where none is negative, else n times the
+    // scale's largest term (2^(k-2))
+    const bool pos = wpos && (q == 3 || o2f(A.lo[q]) >= 0.f);
+    S.abs[q] = pos ? __fadd_ru(xa, slack) : __fmul_ru(n, 0x1p43f);
+    // Exact: every term a multiple of 2^emin (none truncated) and the
+    // magnitudes summing below 2^(53 + emin) -- then the reference's
+    // sequential sum and this one are the same exact value, a double.
+    const unsigned b2 = A.o2[q] & 0x3fffffu, b1 = A.o1[q] & 0x3fffffu;
+    const int emin = b2 ? __ffs(int(b2)) - 1 : (b1 ? 21 + __ffs(int(b1)) : 64);
+    S.exact[q] = !A.trunc && ((b1 | b2) == 0u || S.abs[q] < pow2f(53 + emin));
+    S.err[q] = S.exact[q] ? 0.f : __fadd_ru(__fmaf_ru(g, S.abs[q], slack), __fmul_ru(xa, 0x1p-52f));
+  }
+  return S;
+}
+
+// The floats that the reference's (float)(x / m) gives, where the bounds decide
+// them: false where one is left open.  One reciprocal a node and three FP64
+// multiply-adds a coordinate: a Newton step takes the float reciprocal to 46
+// bits, the quotient is corrected by its residual (within 2^-52 of x / m), and
+// the error bounds are taken in float, rounded up.
+__device__ __forceinline__ bool quotients(const NodeSums &S, int kx, int km, float *xc) {
+  const float ml = __fsub_rd(__double2float_rd(S.x[3]), S.err[3]);
+  if (!(ml > 0.f)) return false;
+  const float ri = __frcp_ru(ml);
+  const double m = S.x[3];
+  double r = double(__frcp_rn(__double2float_rn(m)));
+  r = __fma_rn(r, __fma_rn(-m, r, 1.0), r);
+  const double scale = pow2(kx - km);
+  bool ok = true;
+#pragma unroll
+  for (int d = 0; d < 3; ++d) {
+    const double x = S.x[d];
+    double q = __dmul_rn(x, r);
+    q = __fma_rn(__fma_rn(-q, m, x), r, q);
+    // |reference quotient - q| <= (err_x + |q| err_m) / (m - err_m), plus both
+    // quotients' own rounding
+    const float qa = __fmul_ru(__double2float_ru(fabs(x)), ri);
+    const float e = __fmul_ru(__fmaf_ru(qa, S.err[3], S.err[d]), ri);
+    const double w = double(__fmaf_ru(qa, 0x1p-50f, e));
+    const float lo = __double2float_rn(__dmul_rn(__dsub_rn(q, w), scale)),
+                hi = __double2float_rn(__dmul_rn(__dadd_rn(q, w), scale));
+    if (lo == hi) xc[d] = lo;
+    else if (S.exact[d] && S.exact[3])
+      xc[d] = __double2float_rn(__dmul_rn(__ddiv_rn(x, m), scale));
+    else ok = false;
+  }
+  return ok;
+}
+
 // The node's box, split axis and (where the bounds decide it) centre of mass
 // from its reduced statistics; false when the centre of mass is left undecided.
-// One FP64 division a coordinate: the quotient's error bound is taken in float,
-// rounded up.
 __device__ bool decide_node(DNode &N, const NodeAcc &A, const SumScale &sc, const SumScale &sm,
                             bool bad, int32_t force_fallback, int32_t nd) {
   for (int d = 0; d < 3; ++d) {
@@ -522,57 +594,27 @@ __device__ bool decide_node(DNode &N, const NodeAcc &A, const SumScale &sc, cons
     N.split_dim = (l0 > l1 && l0 > l2) ? 0 : (l1 > l2 ? 1 : 2);
   }
   if (force_fallback != 0 || bad) return false;
-  const double n = double(N.count);
-  // The reference's sequential sum lies within (n - 1) u sum|terms| of the
-  // exact sum, to first order; 2 (n + 64) u covers the rest.  This sum is
-  // exact except for truncated terms (half a unit each) and its rounding to
-  // double.
-  const double g = 2.0 * (n + 64.0) * 0x1p-53;
-  const bool wpos = o2f(A.wmin) >= 0.f;
-  double sd[4], bd[4];
-  bool exact[4];
+  return quotients(node_sums(A, N.count), sc.k, sm.k, N.xc);
+}
+
+// A tighter bound for sums that node_sums leaves open: an addition rounds only
+// where the term, or the running sum since an earlier such term, has bits below
+// the last place U of the running sum; so with `low` such terms (bits below U,
+// U = the last place of twice sum |terms|) the sequential sum is within
+// 2 (low + 32) U of the exact one.
+__device__ __forceinline__ int last_place(float abs_units) {  // exponent of U, in units
+  return int(__float_as_uint(abs_units) >> 23) - 127 + 1 - 52;
+}
+__device__ __forceinline__ void tighten(NodeSums &S, const int *low, const NodeAcc &A, int32_t count) {
 #pragma unroll
   for (int q = 0; q < 4; ++q) {
-    const int k = q < 3 ? sc.k : sm.k;
-    sd[q] = sum_to_double(A.h[q], A.l[q], k);
-    const double slack = A.trunc ? n * pow2(k - 45) : 0.0;
-    // sum of |terms|: the sum itself where none is negative, else n times the
-    // scale's largest term
-    const bool pos = wpos && (q == 3 || o2f(A.lo[q]) >= 0.f);
-    const double a = pos ? fabs(sd[q]) * (1.0 + 0x1p-50) + slack : n * pow2(k - 2);
-    // Exact: every term a multiple of 2^emin (none truncated) and the
-    // magnitudes summing below 2^(53 + emin) -- then the reference's
-    // sequential sum and this one are the same exact value, a double.
-    const unsigned b2 = A.o2[q] & 0x3fffffu, b1 = A.o1[q] & 0x3fffffu;
-    const int emin = b2 ? k - 45 + __ffs(int(b2)) - 1 : (b1 ? k - 23 + __ffs(int(b1)) - 1 : 1000);
-    exact[q] = !A.trunc && (emin == 1000 || a < pow2(min(53 + emin, 1000)));
-    bd[q] = g * a + fabs(sd[q]) * 0x1p-52 + slack;
+    if (S.exact[q]) continue;
+    const float e = __fadd_ru(
+        __fmul_ru(2.f * (float(low[q]) + 33.f), pow2f(max(-126, last_place(S.abs[q])))),
+        __fadd_ru(A.trunc ? __int2float_ru(count) : 0.f,
+                  __fmul_ru(__double2float_ru(fabs(S.x[q])), 0x1p-52f)));
+    S.err[q] = fminf(S.err[q], e);
   }
-  bool ok = true;
-#pragma unroll
-  for (int d = 0; d < 3; ++d) {
-    const double q = __ddiv_rn(sd[d], sd[3]);
-    const float f = __double2float_rn(q);
-    if (exact[3] && exact[d] && sd[3] != 0.0) {
-      N.xc[d] = f;
-      continue;
-    }
-    // |reference quotient - q| <= (bx + |q| bm) / (sm - bm), and both
-    // quotients' own rounding
-    const double ml = sd[3] - bd[3];
-    if (!(ml > 0.0) || !isfinite(q)) {
-      ok = false;
-      continue;
-    }
-    const float qa = __double2float_ru(fabs(q));
-    const float num = __fmaf_ru(qa, __double2float_ru(bd[3]), __double2float_ru(bd[d]));
-    const float e = __fadd_ru(__fdiv_ru(num, __double2float_rd(ml)), __fmul_ru(qa, 0x1p-50f));
-    const double w = double(e) * (1.0 + 0x1p-20);
-    const float fl = __double2float_rn(__dadd_rd(q, -w)), fh = __double2float_rn(__dadd_ru(q, w));
-    if (fl == fh) N.xc[d] = fl;
-    else ok = false;
-  }
-  return ok;
 }
 
 // The elements into the first buffer, their input indices, and the largest
@@ -610,7 +652,7 @@ __global__ void __launch_bounds__(256)
 // The root, its chunks and the first level.
 __global__ void __launch_bounds__(256)
     k_root(DNode *nodes, int64_t n, TreeConfig cfg, LevelCtl *ctl, int32_t *chunk_node,
-           int32_t *chunk_base, NodeAcc *acc, unsigned *ticket, int32_t sub_max) {
+           int32_t *chunk_base, NodeAcc *acc, unsigned *ticket, int2 *roots, int32_t sub_max) {
   const int32_t nc = chunks_of(int32_t(n));
   const bool sub = n <= sub_max;
   if (!sub)
@@ -633,13 +675,13 @@ __global__ void __launch_bounds__(256)
     acc_zero(acc[0]);
     ticket[0] = 0u;
   }
-  ctl->lev[0] = LevelSpan{0, sub ? 0 : 1, 0, 1, nc, int32_t(n), {0, 0}};
-  ctl->lev[1] = LevelSpan{-1, 0, 0, 0, 0, 0, {0, 0}};
+  ctl->lev[0] = LevelSpan{0, sub ? 0 : 1, 0, 1, nc, 1, int32_t(n), 0};
+  ctl->lev[1] = LevelSpan{-1, 0, 0, 0, 0, 0, 0, 0};
   ctl->begin[0] = 0;
-  ctl->sub_ready = sub;
-  ctl->sub_nb = 0;
-  ctl->sub_ne = 1;
-  ctl->sub_parity = 0;
+  if (sub) roots[0] = make_int2(0, 0);
+  ctl->nroots = sub ? 1 : 0;
+  ctl->done = sub;
+  ctl->node_end = 1;
 }
 
 // Statistics of every node of the level, and its split decision by the block
@@ -734,7 +776,7 @@ __global__ void __launch_bounds__(kChunkThreads)
     k_level_count(const float4 *__restrict__ pos, DNode *nodes, LevelCtl *ctl, int32_t level,
                   const int32_t *__restrict__ chunk_node, const int32_t *__restrict__ chunk_base,
                   int32_t *next_chunk_node, int32_t *next_chunk_base, int32_t *left_cnt,
-                  int32_t *left_base, int32_t *wpre, NodeAcc *acc, unsigned *ticket,
+                  int32_t *left_base, int32_t *wpre, NodeAcc *acc, unsigned *ticket, int2 *roots,
                   int64_t *counters, int32_t sub_max) {
   LevelSpan L;
   if (!level_runs(ctl, level, L) || int32_t(blockIdx.x) >= L.nchunk) return;
@@ -799,8 +841,8 @@ __global__ void __launch_bounds__(kChunkThreads)
   __syncthreads();
   if (!last) return;
   __threadfence();
-  const int32_t nl = L.ne - L.nb;
-  int splits = 0, chunks = 0, largest = 0;
+  const int32_t nl = L.ne - L.nb, nroots = ctl->nroots;
+  int splits = 0, chunks = 0, subs = 0, largest = 0;
   for (int32_t i0 = 0; i0 < nl; i0 += kChunkThreads) {
     const int32_t i = i0 + int32_t(threadIdx.x);
     DNode N;
@@ -812,10 +854,13 @@ __global__ void __launch_bounds__(kChunkThreads)
       for (int q = 0; q < 4; ++q) dst[q] = __ldcg(src + q);
       split = N.split_dim >= 0 && N.nleft > 0 && N.nleft < N.count;
     }
-    const int32_t c0 = split ? chunks_of(N.nleft) : 0, c1 = split ? chunks_of(N.count - N.nleft) : 0;
-    int ts, tc;
+    const int32_t n0 = split ? N.nleft : 0, n1 = split ? N.count - N.nleft : 0;
+    const bool s0 = split && n0 <= sub_max, s1 = split && n1 <= sub_max;  // subtree roots
+    const int32_t c0 = s0 ? 0 : chunks_of(n0), c1 = s1 ? 0 : chunks_of(n1);
+    int ts, tc, tr;
     const int rank = splits + block_excl_scan(split ? 1 : 0, sh_warp, &ts);
     const int32_t cb = chunks + block_excl_scan(c0 + c1, sh_warp, &tc);
+    const int32_t rb = nroots + subs + block_excl_scan(int(s0) + int(s1), sh_warp, &tr);
     if (split) {
       const int32_t cl = L.ne + 2 * rank;
       write_child(nodes[cl], N, 0);
@@ -826,11 +871,15 @@ __global__ void __launch_bounds__(kChunkThreads)
       next_chunk_base[2 * rank + 1] = cb + c0;
       for (int32_t c = 0; c < c0; ++c) next_chunk_node[cb + c] = cl;
       for (int32_t c = 0; c < c1; ++c) next_chunk_node[cb + c0 + c] = cl + 1;
-      largest = max(largest, max(N.nleft, N.count - N.nleft));
+      if (s0) roots[rb] = make_int2(cl, (level + 1) & 1);
+      if (s1) roots[rb + int(s0)] = make_int2(cl + 1, (level + 1) & 1);
+      if (!s0) largest = max(largest, n0);
+      if (!s1) largest = max(largest, n1);
     }
     if (i < nl) ticket[i] = 0u;
     splits += ts;
     chunks += tc;
+    subs += tr;
   }
   largest = __reduce_max_sync(0xffffffffu, largest);
   if (lane == 0) wt[warp] = largest;
@@ -841,17 +890,15 @@ __global__ void __launch_bounds__(kChunkThreads)
   }
   if (threadIdx.x != 0) return;
   for (int w = 0; w < kWarps; ++w) largest = max(largest, wt[w]);
-  const bool sub = splits > 0 && largest <= sub_max;
-  LevelSpan X{level + 1, splits > 0 && !sub ? 1 : 0, L.ne, L.ne + 2 * splits, chunks, largest, {0, 0}};
-  ctl->lev[(level + 1) & 1] = X;
+  const int32_t ne = L.ne + 2 * splits;
+  ctl->lev[(level + 1) & 1] =
+      LevelSpan{level + 1, chunks > 0 ? 1 : 0, L.ne, ne, chunks, 2 * splits - subs, largest, 0};
   ctl->begin[(level + 1) % kCtlLevels] = L.ne;
   ctl->next_level = level + 1;
   ctl->ticket = 0u;
-  ctl->sub_ready = sub;
-  ctl->sub_nb = X.nb;
-  ctl->sub_ne = X.ne;
-  ctl->sub_parity = (level + 1) & 1;
-  ctl->done = splits == 0;
+  ctl->nroots = nroots + subs;
+  ctl->done = chunks == 0;
+  ctl->node_end = ne;
   counters[C_CHAINS] = 0;  // the level's queue of long swap chains
 }
 
@@ -1392,31 +1439,34 @@ __global__ void k_decided(LevelCtl *ctl, int64_t *counters) {
 }
 
 // ---------------------------------------------------------------------------
-// Whole subtrees in one block.  Once every node of a level holds at most
-// kSubMax elements, one block per node builds that node's entire subtree:
-// level by level inside the block, each node's statistics (box, exact
-// fixed-point centre-of-mass sums and their certification, the reference's
-// sequential sum where the bounds leave it open), the split decision, the
-// partition at the centre of mass (left elements to their ranks, right
-// elements along the swap chains kept in shared memory, pointer jumping for
-// long chains -- the reference's swap sequence, RCBForceTree.cxx:623-672) and
-// the children.  The level's nodes are shared out to teams of warps: a whole
-// block for one node, down to a warp per node on deep levels.  Elements
-// alternate between the two element buffers as in the level loop (a leaf's
-// elements are copied into the other buffer once, so both end up holding
-// every leaf).  The subtree's nodes go to a scratch region (2 x count
-// records per root, at twice the root's element offset) in per-root
-// breadth-first order; k_subtree_place later numbers all of them by level
-// and offset, as the level loop would have.  One launch and no host
-// synchronisation replace the deep levels' kernels.
+// Whole subtrees in one block.  One block per node of at most kSubMax elements
+// that the level loop leaves builds that node's entire subtree with its
+// positions in shared memory, read once: level by level, each node's
+// statistics (box, exact centre-of-mass sums and their certification, the
+// reference's sequential sum where the bounds leave it open), the split
+// decision, the partition at the centre of mass (left elements to their ranks,
+// right elements along the swap chains, pointer jumping for long chains -- the
+// reference's swap sequence, RCBForceTree.cxx:623-672) and the children.  What
+// a partition moves is each element's 16-bit index, not its 20 bytes; the
+// elements are written once, in tree order, at the end.  Every step of a level
+// is a few dependent shared-memory accesses: with the elements in L2, and moved
+// at every level, a level cost 20-60 us of latency whatever its size (a block of
+// 4780 elements took 231 us, 256 blocks of 10 thousand 455 us).
+// The level's nodes are shared out to teams of warps: a whole block for one
+// node, down to a warp per node on deep levels, kSubBatch nodes at a time.  The
+// subtree's nodes go to a scratch region (2 x count records per root, at twice
+// the root's element offset) in per-root breadth-first order; k_subtree_place
+// later numbers all of them by level and offset.
 // ---------------------------------------------------------------------------
-constexpr int kSubMax = 16384;       // largest subtree root (elements)
-constexpr int kSubThreads = 512;   // two blocks per SM
+constexpr int kSubMax = 8192;        // largest subtree root (elements)
+constexpr int kSubThreads = 1024;    // one block per SM
 constexpr int kSubWarps = kSubThreads / 32;
+constexpr int kSubBatch = 256;       // nodes of a level taken at a time
 constexpr int kSubDepth = 48;        // deepest level below a root; deeper: the level loop
+constexpr int kSubBytes = 16 + 3 * 2;  // shared memory an element
 
-// Barrier over the warps [w0, w0 + nw) of the block: named barrier 1 + team
-// for teams of several warps (at most 8 teams), __syncwarp for one warp.
+// Barrier over the warps of a team: named barrier 1 + team for teams of
+// several warps (at most 8 teams), __syncwarp for one warp.
 __device__ __forceinline__ void team_sync(int team, int nw) {
   if (nw == 1) {
     __syncwarp();
@@ -1450,20 +1500,35 @@ __device__ __forceinline__ void merge_records(const NodeAcc *part, int nw, int f
   }
 }
 
-__global__ void __launch_bounds__(kSubThreads, 2)
-    k_subtree(const DNode *__restrict__ nodes, const LevelCtl *ctl, float4 *pos_a, int32_t *oid_a,
-              float4 *pos_b, int32_t *oid_b, DNode *sub, NodeAcc *sub_stats, int32_t *sub_first,
-              int32_t *hist, int32_t force_fallback, int32_t nd, int64_t *counters) {
-  extern __shared__ int32_t sidx[];  // chain table by element position in the subtree
+// Node of the batch in progress.
+struct SubNode {
+  int32_t lo, count;  // its elements: [lo, lo + count) of the subtree
+  int32_t dim;        // split axis, -1: a leaf by size
+  float split;
+  int32_t nleft;
+};
+
+__global__ void __launch_bounds__(kSubThreads, 1)
+    k_subtree(const DNode *__restrict__ nodes, const LevelCtl *ctl, const int2 *__restrict__ roots,
+              float4 *pos_a, int32_t *oid_a,
+              const float4 *pos_b, const int32_t *oid_b, DNode *sub, int32_t *sub_first,
+              int32_t *hist, int32_t cap, int32_t force_fallback, int32_t nd, int64_t *counters) {
+  extern __shared__ float4 P[];  // positions by input slot; then the 16-bit tables
+  uint16_t *cur = reinterpret_cast<uint16_t *>(P + cap);  // input slot by position
+  uint16_t *nxt = cur + cap;
+  uint16_t *const chain = nxt + cap;  // swap chains: source position of the q-th left element
+  __shared__ NodeAcc st[kSubBatch];
   __shared__ NodeAcc wst[kSubWarps];
+  __shared__ SubNode H[kSubBatch];
   __shared__ int wtot[kSubWarps];
-  __shared__ int tflag[kSubWarps];      // per team: a chain too long / pointer jumping changed
+  __shared__ int tflag[8];                // per team of several warps: a chain too long / jumping changed
   __shared__ int first[kSubDepth + 2];  // first local node of each depth
   __shared__ int sh_warp[32];
-  __shared__ int s_nsplit;
-  if (!ctl->sub_ready || ctl->abort) return;
+  __shared__ int open_[kSubBatch];      // nodes whose centre is undecided
+  __shared__ int nopen;
+  if (!ctl->done || ctl->abort) return;
   const int32_t r = int32_t(blockIdx.x);
-  if (r >= ctl->sub_ne - ctl->sub_nb) {  // the host launched for the most there can be
+  if (r >= ctl->nroots) {  // the host launched for the most there can be
     for (int dd = int(threadIdx.x); dd < kSubDepth; dd += kSubThreads)
       hist[int64_t(dd) * gridDim.x + r] = 0;
     return;
@@ -1471,199 +1536,191 @@ __global__ void __launch_bounds__(kSubThreads, 2)
   const unsigned mt = ctl->mx_term, mm = ctl->mx_mass;
   const SumScale sc(mt), sm(mm);
   const bool bad_scale = SumScale::bad(mt) || SumScale::bad(mm);
-  const DNode R = nodes[ctl->sub_nb + r];
+  const int2 root = roots[r];
+  const DNode R = nodes[root.x];
   const int rcnt = R.count;
   const int32_t roff = R.offset;
   DNode *loc = sub + 2 * int64_t(roff);  // this root's 2 x count records
-  // the reduced statistics of the current level's nodes, by position in the
-  // level (a level holds at most count nodes)
-  NodeAcc *lst = sub_stats + roff;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const unsigned below = (1u << lane) - 1u;
-  if (rcnt > kSubMax) {  // the launch's shared memory does not hold it
+  if (rcnt > cap) {  // the launch's shared memory does not hold it
     if (threadIdx.x == 0) atomicExch(reinterpret_cast<int32_t *>(counters + C_ERR), 3);
     return;
+  }
+  const bool par = root.y != 0;  // the buffer that holds its elements
+  const int32_t *src_id = (par ? oid_b : oid_a) + roff;
+  constexpr int kPerT = kSubMax / kSubThreads;
+  {
+    const float4 *src = (par ? pos_b : pos_a) + roff;
+#pragma unroll
+    for (int u = 0; u < kPerT; ++u) {
+      const int i = u * kSubThreads + int(threadIdx.x);
+      if (i < rcnt) {
+        P[i] = src[i];
+        cur[i] = uint16_t(i);
+      }
+    }
   }
   if (threadIdx.x == 0) {
     loc[0] = R;
     loc[0].cl = loc[0].cr = 0;
     first[0] = 0;
     first[1] = 1;
+    nopen = 0;
   }
   __syncthreads();
-  const bool par = ctl->sub_parity != 0;
-  const float4 *src = par ? pos_b : pos_a;
-  const int32_t *soid = par ? oid_b : oid_a;
-  float4 *dst = par ? pos_a : pos_b;
-  int32_t *doid = par ? oid_a : oid_b;
+  const float *const Pf = reinterpret_cast<const float *>(P);
   int f0 = 0, f1 = 1, depth = 0;
-  int nfb = 0;  // sequential centre-of-mass sums (thread 0 of a team counts)
   while (f1 > f0) {
-    const int F = f1 - f0;
-    // teams: the whole block for one node, halving per doubling of the level
-    // to a warp per node from 9 nodes on (at most 8 teams of several warps,
-    // named barriers 1-8)
-    int nw = 1;
-    if (F <= 8) {
-      int p2 = 1;
-      while (p2 < F) p2 <<= 1;
-      nw = kSubWarps / p2;
-    }
-    const int nteams = kSubWarps / nw;
-    const int team = warp / nw, w0 = team * nw, wi = warp - w0;
-    const int tl = wi * 32 + lane, TN = nw * 32;
-    // ---- statistics: a team per node, reduced into the level's scratch ----
-    for (int f = f0 + team; f < f1; f += nteams) {
-      const DNode N = loc[f];
-      const int c = N.count;
-      const int64_t o = N.offset;
-      LaneAcc a;
-      a.zero();
-      int cnt = 0;
-      constexpr int kU = 4;
-      for (int e0 = tl; e0 < c; e0 += kU * TN) {
-        float4 p[kU];
+    int base = f1;  // the next level's nodes made so far end here
+    for (int b0 = f0; b0 < f1; b0 += kSubBatch) {
+      const int F = min(kSubBatch, f1 - b0);
+      // teams: the whole block for one node, halving per doubling of the batch
+      // to a warp per node from 9 nodes on (at most 8 teams of several warps,
+      // named barriers 1-8)
+      int nw = 1;
+      if (F <= 8) {
+        int p2 = 1;
+        while (p2 < F) p2 <<= 1;
+        nw = kSubWarps / p2;
+      }
+      const int nteams = kSubWarps / nw;
+      const int team = warp / nw, w0 = team * nw, wi = warp - w0;
+      const int tl = wi * 32 + lane, TN = nw * 32;
+      if (int(threadIdx.x) < F) {
+        const DNode &N = loc[b0 + threadIdx.x];
+        H[threadIdx.x] = SubNode{N.offset - roff, N.count, -1, 0.f, 0};
+      }
+      __syncthreads();
+      // ---- statistics: a team per node ----
+      for (int f = team; f < F; f += nteams) {
+        const int c = H[f].count, lo = H[f].lo;
+        LaneAcc a;
+        a.zero();
+        int cnt = 0;
+        for (int e = tl; e < c; e += TN, ++cnt) a.add(P[cur[lo + e]], sc, sm);
+        NodeAcc w;
+        a.reduce(w, cnt, 32 * ((c + TN - 1) / TN) <= 1023, sc, sm);
+        if (lane == 0) (nw == 1 ? st[f] : wst[warp]) = w;
+        if (nw > 1) {
+          team_sync(team, nw);
+          if (wi == 0) merge_records(wst + w0, nw, lane, &st[f]);
+          team_sync(team, nw);
+        }
+      }
+      __syncthreads();
+      // ---- decisions, a thread per node (FP64 runs on whole warps) ----
+      if (int(threadIdx.x) < F && H[threadIdx.x].count > 0) {  // an empty root stays as it is
+        const int f = threadIdx.x;
+        DNode N = loc[b0 + f];
+        if (!decide_node(N, st[f], sc, sm, bad_scale, force_fallback, nd))
+          open_[atomicAdd(&nopen, 1)] = f;
+        H[f].dim = N.split_dim;
+        if (N.split_dim >= 0) H[f].split = N.xc[N.split_dim];
+        loc[b0 + f] = N;
+      }
+      __syncthreads();
+      const int no = nopen;
+      if (no > 0) {
+        // undecided: a warp each counts the terms that can round (tighten),
+        // and where that is not enough lane 0 sums as the reference does
+        // (double, in array order, BGQCM.c:181-212)
+        for (int k = warp; k < no; k += kSubWarps) {
+          const int f = open_[k];
+          const int c = H[f].count, lo = H[f].lo;
+          float xc[3];
+          bool ok = false;
+          if (force_fallback == 0 && !bad_scale) {
+            NodeSums S = node_sums(st[f], c);
+            int low[4] = {0, 0, 0, 0};
+            const int ux = sc.k - 45, um = sm.k - 45;
+            for (int e = lane; e < c; e += 32) {
+              const float4 p = P[cur[lo + e]];
+              low[0] += lsb_exp(fmul_(p.w, p.x)) < last_place(S.abs[0]) + ux;
+              low[1] += lsb_exp(fmul_(p.w, p.y)) < last_place(S.abs[1]) + ux;
+              low[2] += lsb_exp(fmul_(p.w, p.z)) < last_place(S.abs[2]) + ux;
+              low[3] += lsb_exp(p.w) < last_place(S.abs[3]) + um;
+            }
 #pragma unroll
-        for (int u = 0; u < kU; ++u)
-          if (e0 + u * TN < c) p[u] = src[o + e0 + u * TN];
-#pragma unroll
-        for (int u = 0; u < kU; ++u)
-          if (e0 + u * TN < c) {
-            a.add(p[u], sc, sm);
-            ++cnt;
+            for (int q = 0; q < 4; ++q) low[q] = __reduce_add_sync(0xffffffffu, low[q]);
+            tighten(S, low, st[f], c);
+            ok = quotients(S, sc.k, sm.k, xc);
           }
-      }
-      NodeAcc w;
-      a.reduce(w, cnt, 32 * ((c + TN - 1) / TN) <= 1023, sc, sm);
-      if (lane == 0) (nw == 1 ? lst[f - f0] : wst[warp]) = w;
-      if (nw > 1) {
-        team_sync(team, nw);
-        if (wi == 0) merge_records(wst + w0, nw, lane, &lst[f - f0]);
-        team_sync(team, nw);
-      }
-    }
-    __syncthreads();
-    // ---- the level's decisions, a thread per node (the FP64 certification
-    // runs on whole warps) ----
-    for (int f = f0 + int(threadIdx.x); f < f1; f += kSubThreads) {
-      DNode N = loc[f];
-      const int c = N.count;
-      if (c == 0) continue;  // an empty root (no particles) stays as it is
-      const NodeAcc T = lst[f - f0];
-      if (!decide_node(N, T, sc, sm, bad_scale, force_fallback, nd)) {
-        // the reference's own sum: double, in array order (BGQCM.c:181-212)
-        const int64_t o = N.offset;
-        double x = 0, y = 0, z = 0, m = 0;
-        for (int i = 0; i < c; ++i) {
-          const float4 p = src[o + i];
-          x = __dadd_rn(x, double(fmul_(p.w, p.x)));
-          y = __dadd_rn(y, double(fmul_(p.w, p.y)));
-          z = __dadd_rn(z, double(fmul_(p.w, p.z)));
-          m = __dadd_rn(m, double(p.w));
-        }
-        N.xc[0] = __double2float_rn(__ddiv_rn(x, m));
-        N.xc[1] = __double2float_rn(__ddiv_rn(y, m));
-        N.xc[2] = __double2float_rn(__ddiv_rn(z, m));
-        ++nfb;
-      }
-      loc[f] = N;
-    }
-    __syncthreads();
-    // ---- partition at the centre of mass: a team per node ----
-    for (int f = f0 + team; f < f1; f += nteams) {
-      DNode N = loc[f];
-      const int c = N.count;
-      if (c == 0) continue;
-      const int64_t o = N.offset;
-      const int lo_off = int(o - roff);  // the node's first element in the subtree
-      const int d = N.split_dim;
-      if (d < 0) {
-        // a leaf: its elements into the other buffer as well
-        for (int e = tl; e < c; e += TN) {
-          dst[o + e] = src[o + e];
-          doid[o + e] = soid[o + e];
-        }
-        continue;
-      }
-      if (tl == 0) tflag[team] = 0;
-      const float split = N.xc[d];
-      const int share = (((c + nw - 1) / nw) + 31) & ~31;
-      const int beg = wi * share, end = min(c, beg + share);
-      // four loads in flight per lane in every pass
-      constexpr int kU = 4;
-      const float *key = reinterpret_cast<const float *>(src + o) + d;
-      int cl = 0;
-      for (int e0 = beg; e0 < end; e0 += 32 * kU) {
-        float kv[kU];
-#pragma unroll
-        for (int u = 0; u < kU; ++u) {
-          const int e = e0 + 32 * u + lane;
-          kv[u] = e < end ? key[4 * e] : INFINITY;
-        }
-#pragma unroll
-        for (int u = 0; u < kU; ++u) cl += e0 + 32 * u + lane < end && kv[u] < split;
-      }
-      cl = __reduce_add_sync(0xffffffffu, cl);
-      if (lane == 0) wtot[warp] = cl;
-      team_sync(team, nw);
-      int rank = 0, nleft = 0;
-      for (int w = 0; w < nw; ++w) {
-        const int v = wtot[w0 + w];
-        rank += w < wi ? v : 0;
-        nleft += v;
-      }
-      for (int e0 = beg; e0 < end; e0 += 32 * kU) {
-        float4 p[kU];
-        int32_t id[kU];
-#pragma unroll
-        for (int u = 0; u < kU; ++u) {
-          const int e = e0 + 32 * u + lane;
-          p[u] = make_float4(0.f, 0.f, 0.f, 0.f);
-          id[u] = 0;
-          if (e < end) {
-            p[u] = src[o + e];
-            id[u] = soid[o + e];
+          if (lane == 0) {
+            if (!ok) {
+              double x = 0, y = 0, z = 0, m = 0;
+              for (int i = 0; i < c; ++i) {
+                const float4 p = P[cur[lo + i]];
+                x = __dadd_rn(x, double(fmul_(p.w, p.x)));
+                y = __dadd_rn(y, double(fmul_(p.w, p.y)));
+                z = __dadd_rn(z, double(fmul_(p.w, p.z)));
+                m = __dadd_rn(m, double(p.w));
+              }
+              xc[0] = __double2float_rn(__ddiv_rn(x, m));
+              xc[1] = __double2float_rn(__ddiv_rn(y, m));
+              xc[2] = __double2float_rn(__ddiv_rn(z, m));
+              atomicAdd((unsigned long long *)&counters[C_SUBFB], 1ull);
+            }
+            for (int d = 0; d < 3; ++d) loc[b0 + f].xc[d] = xc[d];
+            if (H[f].dim >= 0) H[f].split = xc[H[f].dim];
           }
         }
-#pragma unroll
-        for (int u = 0; u < kU; ++u) {
-          if (e0 + 32 * u >= end) break;  // the same for the whole warp
-          const int e = e0 + 32 * u + lane;
-          const bool l = e < end && key_of(p[u], d) < split;
+        __syncthreads();
+        if (threadIdx.x == 0) nopen = 0;
+      }
+      // ---- partition at the centre of mass: a team per node ----
+      for (int f = team; f < F; f += nteams) {
+        const int c = H[f].count, lo = H[f].lo, d = H[f].dim;
+        if (d < 0) {
+          // a leaf: its order into the other table as well
+          for (int e = tl; e < c; e += TN) nxt[lo + e] = cur[lo + e];
+          continue;
+        }
+        const float split = H[f].split;
+        const uint16_t *const in = cur + lo;
+        uint16_t *const out = nxt + lo, *const ch = chain + lo;
+        const int share = (((c + nw - 1) / nw) + 31) & ~31;
+        const int beg = min(c, wi * share), end = min(c, beg + share);
+        int rank = 0, nleft = 0;
+        if (nw > 1) {
+          int cl = 0;
+          for (int e = beg + lane; e < end; e += 32) cl += Pf[4 * in[e] + d] < split;
+          cl = __reduce_add_sync(0xffffffffu, cl);
+          if (lane == 0) wtot[warp] = cl;
+          if (tl == 0) tflag[team] = 0;
+          team_sync(team, nw);
+          // the team's totals: a lane a warp
+          const int v = lane < nw ? wtot[w0 + lane] : 0;
+          nleft = __reduce_add_sync(0xffffffffu, v);
+          rank = __reduce_add_sync(0xffffffffu, lane < wi ? v : 0);
+        } else {
+          int cl = 0;
+          for (int e = lane; e < c; e += 32) cl += Pf[4 * in[e] + d] < split;
+          nleft = __reduce_add_sync(0xffffffffu, cl);
+        }
+        for (int e0 = beg; e0 < end; e0 += 32) {
+          const int e = e0 + lane;
+          const bool on = e < end;
+          const int s = on ? in[e] : 0;
+          const bool l = on && Pf[4 * s + d] < split;
           const unsigned bal = __ballot_sync(0xffffffffu, l);
           if (l) {
             const int q = rank + __popc(bal & below);
-            dst[o + q] = p[u];
-            doid[o + q] = id[u];
-            sidx[lo_off + q] = e;
-          } else if (e < end && e >= nleft) {
-            // a right element at or after nleft: no swap touches it
-            dst[o + e] = p[u];
-            doid[o + e] = id[u];
+            out[q] = uint16_t(s);
+            ch[q] = uint16_t(e);
+          } else if (on && e >= nleft) {
+            out[e] = uint16_t(s);  // a right element at or after nleft: no swap touches it
           }
           rank += __popc(bal);
         }
-      }
-      team_sync(team, nw);
-      for (int e0 = tl; e0 < nleft; e0 += kU * TN) {
-        float4 pu[kU];
-        int32_t iu[kU];
-#pragma unroll
-        for (int u = 0; u < kU; ++u)
-          if (e0 + u * TN < nleft) {
-            pu[u] = src[o + e0 + u * TN];
-            iu[u] = soid[o + e0 + u * TN];
-          }
-#pragma unroll
-        for (int u = 0; u < kU; ++u) {
-          const int e = e0 + u * TN;
-          if (e >= nleft) break;
-          const float4 p = pu[u];
-          if (key_of(p, d) < split) continue;
+        team_sync(team, nw);
+        bool any_long = false, bad = false;
+        for (int e = tl; e < nleft; e += TN) {
+          const int s = in[e];
+          if (Pf[4 * s + d] < split) continue;
           int q = e, steps = 0;
-          bool bad = false;
           while (q < nleft && steps < kChainSteps) {
-            const int nq = sidx[lo_off + q];
+            const int nq = ch[q];
             if (nq <= q || nq >= c) {  // cannot happen for a valid partition
               bad = true;
               break;
@@ -1671,114 +1728,116 @@ __global__ void __launch_bounds__(kSubThreads, 2)
             q = nq;
             ++steps;
           }
-          if (bad) {
-            atomicExch(reinterpret_cast<int32_t *>(counters + C_ERR), 2);
-            continue;
-          }
-          if (q < nleft) {
-            tflag[team] = 1;
-            continue;
-          }
-          dst[o + q] = p;
-          doid[o + q] = iu[u];
+          if (q < nleft) any_long = !bad;
+          else out[q] = uint16_t(s);
         }
-      }
-      team_sync(team, nw);
-      if (tflag[team]) {
-        // pointer jumping: afterwards sidx[q] is the end of the chain through q
-        for (int round = 0;; ++round) {
+        if (bad) atomicExch(reinterpret_cast<int32_t *>(counters + C_ERR), 2);
+        bool jump = __any_sync(0xffffffffu, any_long);
+        if (nw > 1) {
+          if (jump && lane == 0) tflag[team] = 1;
           team_sync(team, nw);
-          if (tl == 0) tflag[team] = 0;
-          team_sync(team, nw);
-          bool ch = false;
-          for (int q = tl; q < nleft; q += TN) {
-            const int j = sidx[lo_off + q];
-            if (j != q && j < nleft) {  // j == q: a left element no swap moves
-              sidx[lo_off + q] = sidx[lo_off + j];
-              ch = true;
+          jump = tflag[team] != 0;
+        }
+        if (jump) {
+          // pointer jumping: afterwards ch[q] is the end of the chain through q
+          // (each entry moves along its own chain, so every read sees a point of
+          // that chain): log2(count) + 1 rounds
+          for (int round = 0; round < 40; ++round) {
+            team_sync(team, nw);
+            if (nw > 1 && tl == 0) tflag[team] = 0;
+            team_sync(team, nw);
+            bool changed = false;
+            for (int q = tl; q < nleft; q += TN) {
+              const int j = ch[q];
+              if (j != q && j < nleft) {  // j == q: a left element no swap moves
+                ch[q] = ch[j];
+                changed = true;
+              }
             }
+            changed = __any_sync(0xffffffffu, changed);
+            if (nw > 1) {
+              if (changed && lane == 0) tflag[team] = 1;
+              team_sync(team, nw);
+              changed = tflag[team] != 0;
+            }
+            if (!changed) break;
           }
-          if (__any_sync(0xffffffffu, ch) && lane == 0) tflag[team] = 1;
           team_sync(team, nw);
-          if (!tflag[team]) break;
-          if (round > 40) {  // cannot happen for a valid partition
-            if (tl == 0) atomicExch(reinterpret_cast<int32_t *>(counters + C_ERR), 2);
-            break;
+          for (int e = tl; e < nleft; e += TN) {
+            const int s = in[e];
+            if (Pf[4 * s + d] < split) continue;
+            const int q = ch[e];
+            if (q < nleft || q >= c) {  // cannot happen for a valid partition
+              atomicExch(reinterpret_cast<int32_t *>(counters + C_ERR), 2);
+              continue;
+            }
+            out[q] = uint16_t(s);
           }
         }
-        for (int e = tl; e < nleft; e += TN) {
-          const float4 p = src[o + e];
-          if (key_of(p, d) < split) continue;
-          const int q = sidx[lo_off + e];
-          if (q < nleft || q >= c) {
-            atomicExch(reinterpret_cast<int32_t *>(counters + C_ERR), 2);
-            continue;
-          }
-          dst[o + q] = p;
-          doid[o + q] = soid[o + e];
-        }
+        if (tl == 0) H[f].nleft = nleft;
+        team_sync(team, nw);
       }
-      if (tl == 0) {
-        N.nleft = nleft;
-        loc[f] = N;
-      }
-      team_sync(team, nw);
-    }
-    __syncthreads();
-    // ---- children: two per node split into two non-empty parts ----
-    int base = f1;
-    for (int c0 = f0; c0 < f1; c0 += kSubThreads) {
-      const int f = c0 + int(threadIdx.x);
+      __syncthreads();
+      // ---- children: two per node split into two non-empty parts ----
+      const int f = int(threadIdx.x);
       int flag = 0;
-      DNode N;
-      if (f < f1) {
-        N = loc[f];
-        flag = (N.split_dim >= 0 && N.nleft > 0 && N.nleft < N.count) ? 1 : 0;
-      }
+      if (f < F && H[f].dim >= 0) flag = H[f].nleft > 0 && H[f].nleft < H[f].count;
       int tot = 0;
       const int rk = block_excl_scan(flag, sh_warp, &tot);
-      if (f < f1) {
+      if (f < F) {
+        DNode N = loc[b0 + f];
+        N.nleft = H[f].nleft;
         if (flag) {
           const int cl = base + 2 * rk;
-          N.cl = cl;
-          N.cr = cl + 1;
           write_child(loc[cl], N, 0);
           write_child(loc[cl + 1], N, 1);
+          N.cl = cl;
+          N.cr = cl + 1;
         } else {
           N.cl = N.cr = 0;
         }
-        loc[f].cl = N.cl;
-        loc[f].cr = N.cr;
+        loc[b0 + f].cl = N.cl;
+        loc[b0 + f].cr = N.cr;
+        loc[b0 + f].nleft = N.nleft;
       }
       base += 2 * tot;
+      __syncthreads();
     }
-    if (threadIdx.x == 0) s_nsplit = (base - f1) / 2;
-    __syncthreads();
-    const int nsplit = s_nsplit;
     f0 = f1;
-    f1 += 2 * nsplit;
+    f1 = base;
     ++depth;
     if (threadIdx.x == 0) first[depth + 1] = f1;
     if (f1 > f0 && depth >= kSubDepth) {  // deeper than the bookkeeping holds
       if (threadIdx.x == 0) atomicExch(reinterpret_cast<int32_t *>(counters + C_ERR), 4);
       return;
     }
-    {
-      const float4 *t = src;
-      src = dst;
-      dst = const_cast<float4 *>(t);
-      const int32_t *u = soid;
-      soid = doid;
-      doid = const_cast<int32_t *>(u);
-    }
+    uint16_t *const t = cur;
+    cur = nxt;
+    nxt = t;
     __syncthreads();
   }
-  if (nfb) atomicAdd((unsigned long long *)&counters[C_SUBFB], (unsigned long long)nfb);
   // per depth: first local node and count (depth 0 is the root)
   for (int dd = int(threadIdx.x); dd <= kSubDepth + 1; dd += kSubThreads)
     sub_first[int64_t(r) * (kSubDepth + 2) + dd] = dd <= depth + 1 ? first[min(dd, depth + 1)] : f1;
   for (int dd = 1 + int(threadIdx.x); dd <= kSubDepth; dd += kSubThreads)
     hist[int64_t(dd - 1) * gridDim.x + r] = dd <= depth ? first[dd + 1] - first[dd] : 0;
+  // the elements in tree order, into the first buffer (which may be the one
+  // read: the ids are gathered before any is written)
+  int32_t ids[kPerT];
+#pragma unroll
+  for (int u = 0; u < kPerT; ++u) {
+    const int i = u * kSubThreads + int(threadIdx.x);
+    ids[u] = i < rcnt ? src_id[cur[i]] : 0;
+  }
+  __syncthreads();
+#pragma unroll
+  for (int u = 0; u < kPerT; ++u) {
+    const int i = u * kSubThreads + int(threadIdx.x);
+    if (i < rcnt) {
+      pos_a[roff + i] = P[cur[i]];
+      oid_a[roff + i] = ids[u];
+    }
+  }
 }
 
 // Per depth below the subtree roots (a block each): every root's first node
@@ -1787,7 +1846,7 @@ __global__ void __launch_bounds__(kScanThreads)
     k_subtree_scan(const LevelCtl *ctl, int32_t *hist, int32_t max_roots, int64_t *tot) {
   __shared__ int sh_warp[32];
   int32_t *row = hist + int64_t(blockIdx.x) * max_roots;
-  const int32_t nr = ctl->sub_ready && !ctl->abort ? ctl->sub_ne - ctl->sub_nb : 0;
+  const int32_t nr = ctl->done && !ctl->abort ? ctl->nroots : 0;
   int run = 0;
   for (int32_t r0 = 0; r0 < nr; r0 += kScanThreads) {
     const int32_t r = r0 + int32_t(threadIdx.x);
@@ -1799,24 +1858,25 @@ __global__ void __launch_bounds__(kScanThreads)
   if (threadIdx.x == 0) tot[blockIdx.x] = run;
 }
 
-// Copies every subtree node to its place among the levels: depth d below the
-// roots is level nb-level + d, ordered by root (i.e. by offset) and, within a
-// root, by the block's breadth-first order (also by offset).  pos holds the
-// scans of k_subtree_scan; the first index after the roots' level is sub_ne.
+// Copies every subtree node to its place after the level loop's nodes: by
+// depth below its root, then by root, then in the block's breadth-first order,
+// so a node always comes after its parent.  pos holds the scans of
+// k_subtree_scan.
 // Does nothing when the node array is too small (the host grows it and
 // launches this again).
 __global__ void __launch_bounds__(256)
-    k_subtree_place(DNode *nodes, const LevelCtl *ctl, const DNode *sub, const int32_t *sub_first,
+    k_subtree_place(DNode *nodes, const LevelCtl *ctl, const int2 *__restrict__ roots,
+                    const DNode *sub, const int32_t *sub_first,
                     const int32_t *pos, int32_t max_roots, const int64_t *tot, int64_t node_cap) {
   __shared__ int fs[kSubDepth + 2];
   __shared__ int64_t base[kSubDepth + 1];
   const int32_t r = int32_t(blockIdx.x);
-  if (!ctl->sub_ready || ctl->abort || r >= ctl->sub_ne - ctl->sub_nb) return;
-  const int32_t nb = ctl->sub_nb;
+  if (!ctl->done || ctl->abort || r >= ctl->nroots) return;
+  const int32_t root = roots[r].x;
   for (int dd = threadIdx.x; dd <= kSubDepth + 1; dd += blockDim.x)
     fs[dd] = sub_first[int64_t(r) * (kSubDepth + 2) + dd];
   if (threadIdx.x == 0) {
-    int64_t at = ctl->sub_ne;
+    int64_t at = ctl->node_end;
     for (int dd = 0; dd < kSubDepth; ++dd) {
       base[dd] = at;
       at += tot[dd];
@@ -1825,7 +1885,7 @@ __global__ void __launch_bounds__(256)
   }
   __syncthreads();
   if (base[kSubDepth] > node_cap) return;
-  const int32_t roff = nodes[nb + r].offset;
+  const int32_t roff = nodes[root].offset;
   const DNode *loc = sub + 2 * int64_t(roff);
   const int total = fs[kSubDepth + 1];
   auto depth_of = [&](int j) {
@@ -1852,7 +1912,7 @@ __global__ void __launch_bounds__(256)
       N.cl = global(N.cl, 1);
       N.cr = global(N.cr, 1);
     }
-    nodes[nb + r] = N;
+    nodes[root] = N;
   }
 }
 
@@ -3053,9 +3113,9 @@ inline unsigned grid_for(int64_t n, int threads, int64_t cap = 0) {
 DeviceTree::~DeviceTree() {
   void *ptrs[] = {epos_, tpos_, oid_, toid_, idx_, nodes_, ppm_, chunk_node_, chunk_base_,
                   left_cnt_, left_base_, acc_, ticket_, ctl_, scan_tmp_, node_tmp_, fallback_, counters_, leaf_ids_,
-                  up_, processed_, leafdesc_, segs_, idx_list_, table_, items_, items_tmp_, gidx_,
+                  up_, processed_, roots_, leafdesc_, segs_, idx_list_, table_, items_, items_tmp_, gidx_,
                   tight_chunks_, tight_nodes_, segs_local_, ridx_, sub_nodes_, sub_first_,
-                  sub_hist_, sub_tot_, sub_stats_, wpre_, chains_};
+                  sub_hist_, sub_tot_, wpre_, chains_};
   for (void *p : ptrs)
     if (p) cudaFree(p);
   if (h_counters_) cudaFreeHost(h_counters_);
@@ -3128,7 +3188,7 @@ cudaError_t DeviceTree::build(const TreeConfig &cfg, int64_t n, const float4 *po
     DT_CHECK(cudaHostAlloc(&h_sub_, kSubDepth * sizeof(int64_t), cudaHostAllocDefault));
     DT_CHECK(cudaMalloc(&sub_tot_, kSubDepth * sizeof(int64_t)));
     DT_CHECK(cudaFuncSetAttribute(k_subtree, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                  kSubMax * int(sizeof(int32_t))));
+                                  kSubMax * kSubBytes));
     ctl = reinterpret_cast<LevelCtl *>(ctl_);
   }
   auto *hc = reinterpret_cast<LevelCtl *>(h_ctl_);
@@ -3148,7 +3208,7 @@ cudaError_t DeviceTree::build(const TreeConfig &cfg, int64_t n, const float4 *po
   const bool subtrees = n == 0 || (!sub_off_ && cfg.force_cm_fallback != 2);
   const int32_t sub_max = subtrees ? kSubMax : -1;
   std::vector<int32_t> level_begin{0};
-  int64_t level_nodes = 1, level_max = n;  // the next level's extent
+  int64_t live = 1, level_max = n, nroots = 0;  // the next level's nodes and the roots so far
   int32_t level = 0, level_ne = 1;
   bool counted = true;  // false: the level's statistics are there, its centres just decided
   for (bool started = false;;) {
@@ -3158,28 +3218,33 @@ cudaError_t DeviceTree::build(const TreeConfig &cfg, int64_t n, const float4 *po
     if (!(subtrees && level_max <= sub_max)) {
       batch = 1;
       const int64_t goal = subtrees ? sub_max : std::max<int64_t>(cfg.nd, 1);
-      while ((level_max >> batch) > goal && batch < 16 && (level_nodes << batch) < 2048) ++batch;
+      while ((level_max >> batch) > goal && batch < 16 && (live << batch) < 2048) ++batch;
     }
-    const int64_t widest = std::min<int64_t>(level_nodes << std::max(0, batch - 1), std::max<int64_t>(n, 1));
-    const int64_t after = std::min<int64_t>(level_nodes << batch, std::max<int64_t>(n, 1));
-    const size_t max_chunks = size_t(n / kChunk + after + 1);
+    // nodes after i more levels that take chunks there: more than sub_max
+    // elements each
+    auto wide = [&](int i) {
+      return std::min<int64_t>(live << i, subtrees ? n / sub_max + 1 : std::max<int64_t>(n, 1));
+    };
+    const int64_t after = live << batch;  // nodes that the last level can make
+    const size_t max_chunks = size_t(n / kChunk + wide(batch) + 1);
     const size_t nodes_most =
-        std::min<size_t>(size_t(2 * n + 1), size_t(level_ne) + size_t(level_nodes << (batch + 1)));
+        std::min<size_t>(size_t(2 * n + 1), size_t(level_ne) + size_t(live << (batch + 1)));
+    const int64_t max_roots = nroots + after;
     DT_CHECK(grow(nodes_, cap_nodes_, nodes_most, s, true));
-    if (!started || max_chunks > cap_cn_ / 2 || size_t(after) + 1 > cap_ac_) {
-      // the chunk maps and accumulators of the level in progress move along
-      DT_CHECK(grow_chunks(max_chunks, size_t(after) + 1, s));
-    }
+    DT_CHECK(grow(roots_, cap_ro_, size_t(max_roots), s, true));
+    // (the chunk maps and accumulators of the level in progress move along)
+    DT_CHECK(grow_chunks(std::max(max_chunks, size_t(after)), size_t(after) + 1, s));
     int32_t *cn[2] = {chunk_node_, chunk_node_ + cap_cn_ / 2};
     int32_t *cb[2] = {chunk_base_, chunk_base_ + cap_cb_ / 2};
     DT_CHECK(grow(left_cnt_, cap_lc_, max_chunks, s));
     DT_CHECK(grow(left_base_, cap_lb_, max_chunks, s));
     DT_CHECK(grow(wpre_, cap_wp_, max_chunks * (kChunkThreads / 32), s));
-    DT_CHECK(grow(fallback_, cap_fb_, size_t(widest) + 1, s));
+    DT_CHECK(grow(fallback_, cap_fb_, size_t(after) + 1, s));
     if (batch > 0) DT_CHECK(grow(chains_, cap_ch_, size_t(std::max<int64_t>(n, 1)), s));
     auto *acc = reinterpret_cast<NodeAcc *>(acc_);
     if (!started) {
-      k_root<<<1, 256, 0, s>>>(nodes_, n, cfg, ctl, cn[0], cb[0], acc, ticket_, sub_max);
+      k_root<<<1, 256, 0, s>>>(nodes_, n, cfg, ctl, cn[0], cb[0], acc, ticket_, roots_,
+                              sub_max);
       ++info_.launches;
       started = true;
     }
@@ -3188,8 +3253,7 @@ cudaError_t DeviceTree::build(const TreeConfig &cfg, int64_t n, const float4 *po
     for (int i = 0; i < batch; ++i) {
       const int32_t l = level + i;
       const int from = l & 1, to = from ^ 1;
-      const unsigned grid =
-          unsigned(n / kChunk + std::min<int64_t>(level_nodes << i, std::max<int64_t>(n, 1)) + 1);
+      const unsigned grid = unsigned(n / kChunk + wide(i) + 1);
       if (counted) {
         k_level_stats<<<grid, kChunkThreads, 0, s>>>(pb[from], nodes_, ctl, l, cn[from], cb[from],
                                                      acc, ticket_, fallback_, counters_,
@@ -3199,7 +3263,7 @@ cudaError_t DeviceTree::build(const TreeConfig &cfg, int64_t n, const float4 *po
       counted = true;
       k_level_count<<<grid, kChunkThreads, 0, s>>>(pb[from], nodes_, ctl, l, cn[from], cb[from],
                                                    cn[to], cb[to], left_cnt_, left_base_, wpre_,
-                                                   acc, ticket_, counters_, sub_max);
+                                                   acc, ticket_, roots_, counters_, sub_max);
       k_part_left<<<grid, kChunkThreads, 0, s>>>(pb[from], ob[from], nodes_, ctl, l, cn[from],
                                                  cb[from], left_base_, wpre_, pb[to], ob[to], idx_,
                                                  ridx_);
@@ -3212,18 +3276,16 @@ cudaError_t DeviceTree::build(const TreeConfig &cfg, int64_t n, const float4 *po
           int64_t(cap_ch_), counters_, idx_, ridx_, pb[to], ob[to], walk_err_);
       info_.launches += 4;
     }
-    const int64_t max_roots = after;
     if (subtrees) {
       DT_CHECK(grow(sub_nodes_, cap_sub_, size_t(2 * std::max<int64_t>(n, 1)), s));
-      DT_CHECK(grow(sub_stats_, cap_ss_, size_t(std::max<int64_t>(n, 1)) * sizeof(NodeAcc), s));
       DT_CHECK(grow(sub_first_, cap_sf_, size_t(max_roots) * (kSubDepth + 2), s));
       DT_CHECK(grow(sub_hist_, cap_sh_, size_t(max_roots) * kSubDepth, s));
-      const size_t smem = size_t(std::max<int64_t>(std::min<int64_t>(n, sub_max), 1)) * sizeof(int32_t);
-      k_subtree<<<unsigned(max_roots), kSubThreads, smem, s>>>(
-          nodes_, ctl, epos_, oid_, tpos_, toid_, sub_nodes_, reinterpret_cast<NodeAcc *>(sub_stats_),
-          sub_first_, sub_hist_, cfg.force_cm_fallback, cfg.nd, counters_);
+      const int32_t cap = int32_t((std::min<int64_t>(n, sub_max) + 7) & ~int64_t(7));
+      k_subtree<<<unsigned(max_roots), kSubThreads, size_t(cap) * kSubBytes, s>>>(
+          nodes_, ctl, roots_, epos_, oid_, tpos_, toid_, sub_nodes_, sub_first_, sub_hist_, cap,
+          cfg.force_cm_fallback, cfg.nd, counters_);
       k_subtree_scan<<<kSubDepth, kScanThreads, 0, s>>>(ctl, sub_hist_, int32_t(max_roots), sub_tot_);
-      k_subtree_place<<<unsigned(max_roots), 256, 0, s>>>(nodes_, ctl, sub_nodes_, sub_first_,
+      k_subtree_place<<<unsigned(max_roots), 256, 0, s>>>(nodes_, ctl, roots_, sub_nodes_, sub_first_,
                                                           sub_hist_, int32_t(max_roots), sub_tot_,
                                                           int64_t(cap_nodes_));
       info_.launches += 3;
@@ -3252,8 +3314,9 @@ cudaError_t DeviceTree::build(const TreeConfig &cfg, int64_t n, const float4 *po
       level_begin.push_back(hc->begin[level_begin.size() % kCtlLevels]);
     level = hc->next_level;
     const LevelSpan &X = hc->lev[level & 1];
-    level_nodes = X.ne - X.nb;
-    level_ne = X.ne;
+    live = X.live;
+    nroots = hc->nroots;
+    level_ne = hc->node_end;
     level_max = X.maxcnt;
     if (hc->abort) {
       // undecided centres of mass in this level: certify them, or sum as the
@@ -3265,7 +3328,7 @@ cudaError_t DeviceTree::build(const TreeConfig &cfg, int64_t n, const float4 *po
           pb[level & 1], nodes_, fallback_, counters_,
           reinterpret_cast<const TightChunk *>(tight_chunks_),
           reinterpret_cast<TightNode *>(tight_nodes_), cfg.force_cm_fallback == 1);
-      k_cm_fallback<<<unsigned(std::min<int64_t>((level_nodes + 127) / 128, 1024)), 128, 0, s>>>(
+      k_cm_fallback<<<unsigned(std::min<int64_t>((live + 127) / 128, 1024)), 128, 0, s>>>(
           pb[level & 1], nodes_, fallback_, counters_);
       k_decided<<<1, 1, 0, s>>>(ctl, counters_);
       info_.launches += 4;
@@ -3273,19 +3336,22 @@ cudaError_t DeviceTree::build(const TreeConfig &cfg, int64_t n, const float4 *po
       counted = false;
       continue;
     }
-    if (hc->sub_ready) {
-      int64_t total = hc->sub_ne;
+    if (hc->done) {
+      if (!subtrees) break;
+      int64_t total = level_ne;
       for (int d = 0; d < kSubDepth; ++d) total += h_sub_[d];
       if (total > INT32_MAX) return cudaErrorInvalidValue;
       if (size_t(total) > cap_nodes_) {
         DT_CHECK(grow(nodes_, cap_nodes_, size_t(total), s, true));
-        k_subtree_place<<<unsigned(max_roots), 256, 0, s>>>(nodes_, ctl, sub_nodes_, sub_first_,
+        k_subtree_place<<<unsigned(max_roots), 256, 0, s>>>(nodes_, ctl, roots_, sub_nodes_, sub_first_,
                                                             sub_hist_, int32_t(max_roots), sub_tot_,
                                                             int64_t(cap_nodes_));
         ++info_.launches;
         DT_CHECK(cudaGetLastError());
       }
-      int64_t at = hc->sub_ne;
+      // the ranges that hold every node after its parent: levels, then subtree
+      // depths
+      int64_t at = level_ne;
       level_begin.push_back(int32_t(at));
       for (int d = 0; d < kSubDepth && h_sub_[d] > 0; ++d) {
         at += h_sub_[d];
@@ -3294,7 +3360,6 @@ cudaError_t DeviceTree::build(const TreeConfig &cfg, int64_t n, const float4 *po
       level_ne = int32_t(total);
       break;
     }
-    if (hc->done) break;
   }
   info_.cm_fallbacks = h_counters_[C_SUBFB] + h_counters_[C_SEQ];
   const int32_t ne = level_ne;

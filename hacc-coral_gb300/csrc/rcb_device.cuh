@@ -93,7 +93,8 @@ class DeviceTree {
   const int32_t *gidx() const { return gidx_; }
   const DNode *nodes() const { return nodes_; }
   const float *ppm() const { return ppm_; }
-  // First node of each tree level (BFS order), plus the node count at the end.
+  // Ranges of nodes that hold every node after its parent: their first nodes,
+  // plus the node count at the end.
   const std::vector<int32_t> &levels() const { return levels_; }
   const int32_t *leaf_nodes() const { return leaf_ids_; }
   int64_t padded_pairs() const { return padded_pairs_; }
@@ -177,9 +178,9 @@ class DeviceTree {
   // whole subtrees in one block (k_subtree): node scratch, per-root depth
   // bookkeeping, placement offsets, per-depth totals (and their pinned copy)
   DNode *sub_nodes_ = nullptr;
-  unsigned char *sub_stats_ = nullptr;  // reduced statistics of a level's nodes
-  size_t cap_ss_ = 0;
   int32_t *sub_first_ = nullptr;
+  int2 *roots_ = nullptr;  // subtree roots: node, element buffer
+  size_t cap_ro_ = 0;
   int32_t *sub_hist_ = nullptr;
   int64_t *sub_tot_ = nullptr;
   size_t cap_sub_ = 0, cap_sf_ = 0, cap_sh_ = 0;
