@@ -157,18 +157,20 @@ __global__ void __launch_bounds__(kThreads)
 // ng / 2 pi times larger beside the gradient's than before: below 1e-13 at the
 // largest grid, with the fields rounded to float (6e-8).  Single precision has
 // no such room and keeps the three spectra.
-// A thread per (y, z) column marches kGradSpan cells along x with its five
-// x values in registers; the y and z neighbours come through L1.
+// A thread per (y, z) column marches `span` cells along x with its five x values
+// in registers; the y and z neighbours come through L1.  Up to 16 cells, fewer
+// where that would leave SMs without a block: a march is a chain of L2 loads
+// (16 cells a thread at 24^3 took 16 us, a cell a thread 3).
 constexpr int kGradSpan = 16;
 constexpr double kD1 = 2.0 / 3.0, kD2 = -1.0 / 12.0;
 
 __device__ __forceinline__ int wrap(int i, int ng) { return i < 0 ? i + ng : (i >= ng ? i - ng : i); }
 
 __global__ void __launch_bounds__(256)
-    k_gradient(int ng, const double *__restrict__ phi, float4 *__restrict__ out) {
+    k_gradient(int ng, int span, const double *__restrict__ phi, float4 *__restrict__ out) {
   const int z = int(blockIdx.x) * 32 + int(threadIdx.x), y = int(blockIdx.y) * 8 + int(threadIdx.y);
   if (z >= ng || y >= ng) return;
-  const int x0 = int(blockIdx.z) * kGradSpan, x1 = min(ng, x0 + kGradSpan);
+  const int x0 = int(blockIdx.z) * span, x1 = min(ng, x0 + span);
   const int64_t plane = int64_t(ng) * ng;
   const int64_t row = int64_t(y) * ng;
   const int64_t yp1 = int64_t(wrap(y + 1, ng)) * ng, ym1 = int64_t(wrap(y - 1, ng)) * ng;
@@ -596,9 +598,11 @@ bool Solver::solve(cudaStream_t s, std::string *err) {
     if (!fft_ok(cufftExecZ2D(inv_, (cufftDoubleComplex *)spec_, (cufftDoubleReal *)real_),
                 "pm inverse transform", err))
       return false;
-    k_gradient<<<dim3(unsigned((ng + 31) / 32), unsigned((ng + 7) / 8),
-                      unsigned((ng + kGradSpan - 1) / kGradSpan)),
-                 dim3(32, 8), 0, s>>>(ng, (const double *)real_, grad_);
+    const int gz = (ng + 31) / 32, gy = (ng + 7) / 8;
+    int span = kGradSpan;
+    while (span > 1 && int64_t(gz) * gy * ((ng + span - 1) / span) < 2 * hsr::sm_count()) span /= 2;
+    k_gradient<<<dim3(unsigned(gz), unsigned(gy), unsigned((ng + span - 1) / span)), dim3(32, 8), 0,
+                 s>>>(ng, span, (const double *)real_, grad_);
   } else {
     if (!fft_ok(cufftExecR2C(fwd_, (cufftReal *)rho_, (cufftComplex *)spec_), "pm forward transform",
                 err))
