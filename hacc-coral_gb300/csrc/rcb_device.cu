@@ -41,8 +41,7 @@ __device__ __forceinline__ int lsb_exp(float t) {
   return e - 150 + (__ffs(int(m)) - 1);
 }
 
-constexpr int kChunk = 4096;        // elements per statistics / partition chunk
-constexpr int kChunkThreads = 256;  // threads per chunk (16 elements each)
+constexpr int kChunkThreads = 256;  // threads per statistics / partition chunk
 constexpr int kChainSteps = 32;     // chain steps before a subtree block jumps pointers
 constexpr int kPlainSteps = 4;      // single chain steps before the chunk partition jumps runs
 
@@ -254,7 +253,7 @@ __device__ __forceinline__ int block_excl_scan(int v, int *sh_warp, int *total) 
 // A level is five launches: statistics (k_level_stats), left counts
 // (k_level_count), left elements (k_part_left), right elements
 // (k_part_right) and the long swap chains (k_part_chains), a block per chunk of
-// kChunk elements.  What follows a node's last chunk -- its split decision, the
+// a few thousand elements.  What follows a node's last chunk -- its split decision, the
 // scan of its chunks' left counts -- and what follows the level's last chunk --
 // the children, their chunks -- is done by the block that finishes last, and
 // the level's extent lives in device memory (LevelCtl), so the host launches
@@ -285,11 +284,23 @@ struct LevelCtl {
   int32_t done;        // no node is left for the level loop
   int32_t node_end;    // nodes of all levels
   unsigned mx_term, mx_mass;  // largest |w x|, |w y|, |w z| and |w|, as bits
+  unsigned mn_mass;    // smallest w by its bits, complemented
   unsigned ticket;     // chunks of the level counted
   int32_t next_level;  // the level made last
   int32_t begin[kCtlLevels];  // first node of a level, by level modulo kCtlLevels
 };
-__device__ __forceinline__ int32_t chunks_of(int32_t count) { return (count + kChunk - 1) / kChunk; }
+// A chunk is PT elements a thread of its block: 16 (4096 elements) keep the
+// per-block work (reductions, tickets) small beside the elements where there
+// are enough of them to fill the GPU; sets of up to kSmallSet take 4, four
+// times as many blocks whose threads go through a quarter of the dependent
+// loads (a level of 68 thousand elements: 62 us with 16).
+constexpr int64_t kSmallSet = 1 << 20;
+template <int PT>
+__host__ __device__ constexpr int32_t chunk_size() { return PT * kChunkThreads; }
+template <int PT>
+__device__ __forceinline__ int32_t chunks_of(int32_t count) {
+  return (count + chunk_size<PT>() - 1) / chunk_size<PT>();
+}
 
 // Whether level `level` is to be worked on, and its extent.  (Blocks of its
 // statistics may start after another has raised abort for the same level.)
@@ -304,15 +315,16 @@ struct ChunkRange {
   int32_t node, begin, len, local;  // local: first element's position inside the node
 };
 
+template <int PT>
 __device__ __forceinline__ ChunkRange chunk_range(const DNode *nodes, const int32_t *chunk_node,
                                                   const int32_t *chunk_base, int32_t nb,
                                                   int32_t chunk) {
   ChunkRange r;
   r.node = chunk_node[chunk];
   const DNode &N = nodes[r.node];
-  r.local = (chunk - chunk_base[r.node - nb]) * kChunk;
+  r.local = (chunk - chunk_base[r.node - nb]) * chunk_size<PT>();
   r.begin = N.offset + r.local;
-  r.len = min(kChunk, N.count - r.local);
+  r.len = min(chunk_size<PT>(), N.count - r.local);
   return r;
 }
 
@@ -377,17 +389,18 @@ struct SumScale {
 // Reduced statistics of a set of elements (a node, a warp's share).
 struct alignas(16) NodeAcc {
   long long h[4], l[4];     // sums of iv and iv2 (x, y, z, m)
-  unsigned o1[4], o2[4];    // ors of their bits: the terms' least significant one
+  unsigned o[4];            // ors of iv2's bits: the terms' least significant one
   unsigned lo[3], hi[3];    // bounding box (f2o)
   unsigned wmin;            // smallest mass (f2o)
   unsigned trunc;           // some term had bits below 2^(k-45)
 };
-static_assert(sizeof(NodeAcc) == 128, "NodeAcc is eight 16-byte words");
+constexpr int kAccWords16 = int(sizeof(NodeAcc) / 16);
+static_assert(sizeof(NodeAcc) == 112, "NodeAcc is seven 16-byte words");
 
 __device__ __forceinline__ void acc_zero(NodeAcc &a) {
   for (int q = 0; q < 4; ++q) {
     a.h[q] = a.l[q] = 0;
-    a.o1[q] = a.o2[q] = 0u;
+    a.o[q] = 0u;
   }
   for (int d = 0; d < 3; ++d) {
     a.lo[d] = 0xffffffffu;
@@ -397,13 +410,69 @@ __device__ __forceinline__ void acc_zero(NodeAcc &a) {
   a.trunc = 0u;
 }
 
+// The scales of a set's terms, and its mass where all are the same (the
+// simulation's own kicks set them all to 1): the mass sums then follow from the
+// counts and cost nothing.
+struct SumScales {
+  SumScale c, m;
+  bool uniform, bad;
+  unsigned h1, l1;  // iv and iv2 of the one mass
+  unsigned wbits;
+  __device__ __forceinline__ SumScales(unsigned mx_term, unsigned mx_mass, unsigned mn_mass)
+      : c(mx_term), m(mx_mass) {
+    // (raw bits: equal only where sign and value are)
+    uniform = mx_mass == mn_mass;
+    bad = SumScale::bad(mx_term) || SumScale::bad(mx_mass);
+    wbits = mn_mass;
+    const float v = __fadd_rn(__uint_as_float(wbits), m.m1);
+    const float r = __fsub_rn(__uint_as_float(wbits), __fsub_rn(v, m.m1));
+    h1 = __float_as_uint(v) - __float_as_uint(m.m1);
+    l1 = __float_as_uint(__fadd_rn(r, m.m2)) - __float_as_uint(m.m2);
+  }
+  // The mass words of a node of `count` elements.
+  __device__ __forceinline__ void masses(NodeAcc &a, int32_t count) const {
+    if (!uniform) return;
+    a.h[3] = (long long)int(h1) * count;
+    a.l[3] = (long long)int(l1) * count;
+    a.o[3] = l1;
+    a.wmin = f2o(__uint_as_float(wbits));
+  }
+};
+
+// Values reduced over a warp (W = 32) or over each eight lanes (W = 8): lane l
+// ends with value l & 7 (reduce8) or l & 3 (reduce4).  Each of the first steps
+// exchanges half of the values that are left, so eight reductions take 9
+// shuffles, not 40.
+template <typename T, typename Op>
+__device__ __forceinline__ T reduce_half(T a, T b, int m, Op op) {
+  const bool up = threadIdx.x & m;  // keeps a on lanes without bit m, b on the others
+  const T mine = up ? b : a, theirs = up ? a : b;
+  return op(mine, __shfl_xor_sync(0xffffffffu, theirs, m));
+}
+template <int W, typename T, typename Op>
+__device__ __forceinline__ T reduce4(T v0, T v1, T v2, T v3, Op op) {
+  T c = reduce_half(reduce_half(v0, v1, 1, op), reduce_half(v2, v3, 1, op), 2, op);
+#pragma unroll
+  for (int o = 4; o < W; o <<= 1) c = op(c, __shfl_xor_sync(0xffffffffu, c, o));
+  return c;
+}
+template <int W, typename T, typename Op>
+__device__ __forceinline__ T reduce8(T v0, T v1, T v2, T v3, T v4, T v5, T v6, T v7, Op op) {
+  const T b0 = reduce_half(reduce_half(v0, v1, 1, op), reduce_half(v2, v3, 1, op), 2, op);
+  const T b1 = reduce_half(reduce_half(v4, v5, 1, op), reduce_half(v6, v7, 1, op), 2, op);
+  T c = reduce_half(b0, b1, 4, op);
+#pragma unroll
+  for (int o = 8; o < W; o <<= 1) c = op(c, __shfl_xor_sync(0xffffffffu, c, o));
+  return c;
+}
+
 // One lane's share.
 struct LaneAcc {
-  unsigned h[4], l[4], o1[4], o2[4];  // sums of the bits of v and v2 (modulo 2^32)
+  unsigned h[4], l[4], o[4];  // sums of the bits of v and v2 (modulo 2^32), ors of v2's
   float lo[3], hi[3], wmin, left;
   __device__ __forceinline__ void zero() {
 #pragma unroll
-    for (int q = 0; q < 4; ++q) h[q] = l[q] = o1[q] = o2[q] = 0u;
+    for (int q = 0; q < 4; ++q) h[q] = l[q] = o[q] = 0u;
 #pragma unroll
     for (int d = 0; d < 3; ++d) {
       lo[d] = INFINITY;
@@ -412,57 +481,87 @@ struct LaneAcc {
     wmin = INFINITY;
     left = 0.f;
   }
-  __device__ __forceinline__ void term(int q, float t, float m1, float m2) {
-    const float v = __fadd_rn(t, m1);
-    const float r = __fsub_rn(t, __fsub_rn(v, m1));
-    const float v2 = __fadd_rn(r, m2);
-    left = fmaxf(left, fabsf(__fsub_rn(__fsub_rn(v2, m2), r)));
+  __device__ __forceinline__ void term(int q, float t, const SumScale &s) {
+    const float v = __fadd_rn(t, s.m1);
+    const float r = __fsub_rn(t, __fsub_rn(v, s.m1));
+    const float v2 = __fadd_rn(r, s.m2);
+    left = fmaxf(left, fabsf(__fsub_rn(__fsub_rn(v2, s.m2), r)));
     h[q] += __float_as_uint(v);
     l[q] += __float_as_uint(v2);
-    o1[q] |= __float_as_uint(v);
-    o2[q] |= __float_as_uint(v2);
+    o[q] |= __float_as_uint(v2);
   }
-  __device__ __forceinline__ void add(const float4 &p, const SumScale &sc, const SumScale &sm) {
-    term(0, fmul_(p.w, p.x), sc.m1, sc.m2);
-    term(1, fmul_(p.w, p.y), sc.m1, sc.m2);
-    term(2, fmul_(p.w, p.z), sc.m1, sc.m2);
-    term(3, p.w, sm.m1, sm.m2);
+  __device__ __forceinline__ void add(const float4 &p, const SumScales &S) {
+    term(0, fmul_(p.w, p.x), S.c);
+    term(1, fmul_(p.w, p.y), S.c);
+    term(2, fmul_(p.w, p.z), S.c);
+    if (!S.uniform) {
+      term(3, p.w, S.m);
+      wmin = fminf(wmin, p.w);
+    }
     lo[0] = fminf(lo[0], p.x); hi[0] = fmaxf(hi[0], p.x);
     lo[1] = fminf(lo[1], p.y); hi[1] = fmaxf(hi[1], p.y);
     lo[2] = fminf(lo[2], p.z); hi[2] = fmaxf(hi[2], p.z);
-    wmin = fminf(wmin, p.w);
   }
-  // The warp's sum, the same on every lane; cnt: this lane's elements (at most
-  // 512), few: the warp's are at most 1023 (an int holds their sums).
-  __device__ __forceinline__ void reduce(NodeAcc &a, int cnt, bool few, const SumScale &sc,
-                                         const SumScale &sm) const {
-    const unsigned full = 0xffffffffu;
+  // The sums of a warp (W = 32; of each eight lanes, W = 8) into *out, word by
+  // word from different lanes; cnt: this lane's elements (at most 512), few: the
+  // warp's are at most 1023 (an int holds their sums).
+  template <int W>
+  __device__ __forceinline__ void reduce(NodeAcc *out, bool write, int cnt, bool few,
+                                         const SumScales &S) const {
+    int hv[4], lv[4];
 #pragma unroll
-    for (int q = 0; q < 4; ++q) {
-      const SumScale &s = q < 3 ? sc : sm;
-      const int hv = int(h[q] - unsigned(cnt) * __float_as_uint(s.m1));
-      const int lv = int(l[q] - unsigned(cnt) * __float_as_uint(s.m2));
-      if (few) {
-        a.h[q] = __reduce_add_sync(full, hv);
-        a.l[q] = __reduce_add_sync(full, lv);
-      } else {
-        a.h[q] = (long long)(__reduce_add_sync(full, hv >> 16)) * 65536 +
-                 __reduce_add_sync(full, unsigned(hv) & 0xffffu);
-        a.l[q] = (long long)(__reduce_add_sync(full, lv >> 16)) * 65536 +
-                 __reduce_add_sync(full, unsigned(lv) & 0xffffu);
-      }
-      a.o1[q] = __reduce_or_sync(full, o1[q]);
-      a.o2[q] = __reduce_or_sync(full, o2[q]);
+    for (int q = 0; q < 3; ++q) {
+      hv[q] = int(h[q] - unsigned(cnt) * __float_as_uint(S.c.m1));
+      lv[q] = int(l[q] - unsigned(cnt) * __float_as_uint(S.c.m2));
     }
-#pragma unroll
-    for (int d = 0; d < 3; ++d) {
-      a.lo[d] = __reduce_min_sync(full, f2o(lo[d]));
-      a.hi[d] = __reduce_max_sync(full, f2o(hi[d]));
+    hv[3] = S.uniform ? 0 : int(h[3] - unsigned(cnt) * __float_as_uint(S.m.m1));
+    lv[3] = S.uniform ? 0 : int(l[3] - unsigned(cnt) * __float_as_uint(S.m.m2));
+    long long sum;
+    if (few) {
+      sum = reduce8<W>(hv[0], hv[1], hv[2], hv[3], lv[0], lv[1], lv[2], lv[3],
+                       [](int a, int b) { return a + b; });
+    } else {
+      using LL = long long;
+      sum = reduce8<W>(LL(hv[0]), LL(hv[1]), LL(hv[2]), LL(hv[3]), LL(lv[0]), LL(lv[1]), LL(lv[2]),
+                       LL(lv[3]), [](LL a, LL b) { return a + b; });
     }
-    a.wmin = __reduce_min_sync(full, f2o(wmin));
-    a.trunc = __any_sync(full, left != 0.f) ? 1u : 0u;
+    const unsigned bits = reduce4<W>(o[0], o[1], o[2], o[3], [](unsigned a, unsigned b) { return a | b; });
+    // minima; the upper bounds complemented, and 0 where a term was truncated
+    const unsigned mn = reduce8<W>(f2o(lo[0]), f2o(lo[1]), f2o(lo[2]), ~f2o(hi[0]), ~f2o(hi[1]),
+                                   ~f2o(hi[2]), f2o(wmin), left != 0.f ? 0u : 1u,
+                                   [](unsigned a, unsigned b) { return min(a, b); });
+    const int f = threadIdx.x & (W - 1);
+    if (write && f < 8) {
+      (f < 4 ? out->h[f] : out->l[f - 4]) = sum;
+      if (f < 4) out->o[f] = bits;
+      if (f < 3) out->lo[f] = mn;
+      else if (f < 6) out->hi[f - 3] = ~mn;
+      else if (f == 6) out->wmin = mn;
+      else out->trunc = 1u - mn;
+    }
   }
 };
+
+// Word f of n records merged, a lane a word: sums 0-7 (into *sum), then o, lo,
+// hi, wmin and trunc (into *bits).
+constexpr int kAccWords = 20;
+__device__ __forceinline__ bool acc_or(int f) { return f < 12 || f == 19; }
+__device__ __forceinline__ bool acc_max(int f) { return f >= 15 && f < 18; }
+__device__ __forceinline__ void merge_word(const NodeAcc *part, int n, int f, long long *sum,
+                                           unsigned *bits) {
+  long long s = 0;
+  unsigned u = acc_or(f) || acc_max(f) ? 0u : 0xffffffffu;
+  for (int v = 0; v < n; ++v) {
+    if (f < 8) {
+      s += reinterpret_cast<const long long *>(part + v)[f];
+    } else {
+      const unsigned w = reinterpret_cast<const unsigned *>(part + v)[f + 8];
+      u = acc_or(f) ? (u | w) : (acc_max(f) ? max(u, w) : min(u, w));
+    }
+  }
+  *sum = s;
+  *bits = u;
+}
 
 __device__ __forceinline__ double pow2(int e) {  // normal range
   return __longlong_as_double((long long)(e + 1023) << 52);
@@ -533,12 +632,87 @@ __device__ __forceinline__ NodeSums node_sums(const NodeAcc &A, int32_t count) {
     // Exact: every term a multiple of 2^emin (none truncated) and the
     // magnitudes summing below 2^(53 + emin) -- then the reference's
     // sequential sum and this one are the same exact value, a double.
-    const unsigned b2 = A.o2[q] & 0x3fffffu, b1 = A.o1[q] & 0x3fffffu;
-    const int emin = b2 ? __ffs(int(b2)) - 1 : (b1 ? 21 + __ffs(int(b1)) : 64);
-    S.exact[q] = !A.trunc && ((b1 | b2) == 0u || S.abs[q] < pow2f(53 + emin));
+    const unsigned b = A.o[q] & 0x3fffffu;
+    const int emin = b ? __ffs(int(b)) - 1 : 22;  // no iv2: whole multiples of 2^22 units
+    S.exact[q] = !A.trunc && S.abs[q] < pow2f(53 + emin);
     S.err[q] = S.exact[q] ? 0.f : __fadd_ru(__fmaf_ru(g, S.abs[q], slack), __fmul_ru(xa, 0x1p-52f));
   }
   return S;
+}
+
+// A node's exact sum h 2^22 + l as an unevaluated sum of two floats, within err
+// of it (2^-45 of it where its two parts do not cancel); |h| and |l| below 2^46.
+__device__ __forceinline__ void two_sum_f(float a, float b, float &s, float &e) {
+  s = __fadd_rn(a, b);
+  const float bb = __fsub_rn(s, a);
+  e = __fadd_rn(__fsub_rn(a, __fsub_rn(s, bb)), __fsub_rn(b, bb));
+}
+__device__ __forceinline__ void sum_pair(long long h, long long l, float &hi, float &lo, float &err) {
+  const float ha = __int2float_rn(int(h >> 24)) * 0x1p46f, hb = __int2float_rn(int(h & 0xffffff)) * 0x1p22f;
+  const float la = __int2float_rn(int(l >> 24)) * 0x1p24f, lb = __int2float_rn(int(l & 0xffffff));
+  float a, ea, b, eb, s, es;
+  two_sum_f(ha, hb, a, ea);
+  two_sum_f(la, lb, b, eb);
+  two_sum_f(a, b, s, es);
+  two_sum_f(s, __fadd_rn(es, __fadd_rn(ea, eb)), hi, lo);
+  err = __fmul_ru(__fadd_ru(fabsf(a), fabsf(b)), 0x1p-46f);
+}
+
+// The centre of mass on the FP32 pipe alone: the sums as float pairs, the
+// quotient as q0 + q1 with its residual from fused multiply-adds (within 2^-43
+// of x / m), decided where q0 + q1 -/+ the error bound round to one float.  (FP64
+// leaves a chain of 5000 cycles to every level of a subtree.)  What it leaves
+// open goes to the FP64 sums.
+__device__ __forceinline__ bool quotients_f32(const NodeAcc &A, int32_t count, int kx, int km,
+                                              float *xc) {
+  const float n = __int2float_ru(count);
+  const float g = __fmul_ru(__fmul_ru(__fadd_ru(n, 64.f), 0x1p-53f), 1.f + 0x1p-20f);
+  const float slack = A.trunc ? n : 0.f;
+  const bool wpos = o2f(A.wmin) >= 0.f;
+  float hi[4], lo[4], err[4];
+  bool exact[4];
+#pragma unroll
+  for (int q = 0; q < 4; ++q) {
+    const long long lim = 1ll << 46;
+    if (A.h[q] >= lim || A.h[q] <= -lim || A.l[q] >= lim || A.l[q] <= -lim) return false;
+    float pair_err;
+    sum_pair(A.h[q], A.l[q], hi[q], lo[q], pair_err);
+    // as in node_sums, whose comments give the reasons
+    const float xa = __fadd_ru(__fmul_ru(fabsf(hi[q]), 1.f + 0x1p-20f), pair_err);
+    const bool pos = wpos && (q == 3 || o2f(A.lo[q]) >= 0.f);
+    const float sabs = pos ? __fadd_ru(xa, slack) : __fmul_ru(n, 0x1p43f);
+    const unsigned b = A.o[q] & 0x3fffffu;
+    const int emin = b ? __ffs(int(b)) - 1 : 22;
+    exact[q] = !A.trunc && sabs < pow2f(53 + emin);
+    err[q] = __fadd_ru(pair_err, exact[q] ? 0.f : __fmaf_ru(g, sabs, slack));
+  }
+  const float ml = __fsub_rd(__fmul_rd(hi[3], 1.f - 0x1p-20f), err[3]);
+  const int ks = kx - km;
+  if (!(ml > 0.f) || ks < -60 || ks > 60) return false;
+  const float ri = __frcp_ru(ml), r = __frcp_rn(hi[3]), scale = pow2f(ks);
+  bool ok = true;
+#pragma unroll
+  for (int d = 0; d < 3; ++d) {
+    const float q0 = __fmul_rn(hi[d], r);
+    // x - q0 m: the products' high parts cancel exactly in the fused operation
+    float rem = __fmaf_rn(-q0, hi[3], hi[d]);
+    rem = __fadd_rn(rem, __fmaf_rn(-q0, lo[3], lo[d]));
+    const float q1 = __fmul_rn(rem, r);
+    float f, e;
+    two_sum_f(q0, q1, f, e);
+    const float qa = __fmul_ru(fabsf(hi[d]), __fmul_ru(ri, 1.f + 0x1p-20f));
+    const float w = __fmaf_ru(qa, 0x1p-42f, __fmul_ru(__fmaf_ru(qa, err[3], err[d]), ri));
+    const float fl = __fadd_rn(f, __fsub_rd(e, w)), fh = __fadd_rn(f, __fadd_ru(e, w));
+    const float v = __fmul_rn(fl, scale);
+    // (a scaled result near the subnormals would round again)
+    if (fl == fh && (fl == 0.f || fabsf(v) > 0x1p-100f)) xc[d] = v;
+    // exact sums whose quotient is a tie between two floats (an even count)
+    else if (exact[d] && exact[3])
+      xc[d] = __double2float_rn(__dmul_rn(
+          __ddiv_rn(units_to_double(A.h[d], A.l[d]), units_to_double(A.h[3], A.l[3])), pow2(ks)));
+    else ok = false;
+  }
+  return ok;
 }
 
 // The floats that the reference's (float)(x / m) gives, where the bounds decide
@@ -577,8 +751,8 @@ __device__ __forceinline__ bool quotients(const NodeSums &S, int kx, int km, flo
 
 // The node's box, split axis and (where the bounds decide it) centre of mass
 // from its reduced statistics; false when the centre of mass is left undecided.
-__device__ bool decide_node(DNode &N, const NodeAcc &A, const SumScale &sc, const SumScale &sm,
-                            bool bad, int32_t force_fallback, int32_t nd) {
+__device__ bool decide_node(DNode &N, const NodeAcc &A, const SumScales &S, int32_t force_fallback,
+                            int32_t nd) {
   for (int d = 0; d < 3; ++d) {
     N.xmin[d] = o2f(A.lo[d]);
     N.xmax[d] = o2f(A.hi[d]);
@@ -593,8 +767,9 @@ __device__ bool decide_node(DNode &N, const NodeAcc &A, const SumScale &sc, cons
                 l2 = fsub_(N.xmax[2], N.xmin[2]);
     N.split_dim = (l0 > l1 && l0 > l2) ? 0 : (l1 > l2 ? 1 : 2);
   }
-  if (force_fallback != 0 || bad) return false;
-  return quotients(node_sums(A, N.count), sc.k, sm.k, N.xc);
+  if (force_fallback != 0 || S.bad) return false;
+  return quotients_f32(A, N.count, S.c.k, S.m.k, N.xc) ||
+         quotients(node_sums(A, N.count), S.c.k, S.m.k, N.xc);
 }
 
 // A tighter bound for sums that node_sums leaves open: an addition rounds only
@@ -622,7 +797,7 @@ __device__ __forceinline__ void tighten(NodeSums &S, const int *low, const NodeA
 __global__ void __launch_bounds__(256)
     k_elements(const float4 *__restrict__ in, int64_t n, float4 *__restrict__ pos,
                int32_t *__restrict__ oid, LevelCtl *ctl) {
-  unsigned mt = 0, mm = 0;
+  unsigned mt = 0, mm = 0, mn = 0xffffffffu;
   for (int64_t i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x; i < n;
        i += int64_t(gridDim.x) * blockDim.x) {
     const float4 p = in[i];
@@ -632,28 +807,33 @@ __global__ void __launch_bounds__(256)
     mt = max(mt, __float_as_uint(fmul_(p.w, p.y)) & 0x7fffffffu);
     mt = max(mt, __float_as_uint(fmul_(p.w, p.z)) & 0x7fffffffu);
     mm = max(mm, __float_as_uint(p.w) & 0x7fffffffu);
+    mn = min(mn, __float_as_uint(p.w));
   }
   mt = __reduce_max_sync(0xffffffffu, mt);
   mm = __reduce_max_sync(0xffffffffu, mm);
-  __shared__ unsigned sh[2];
-  if (threadIdx.x < 2) sh[threadIdx.x] = 0u;
+  mn = __reduce_min_sync(0xffffffffu, mn);
+  __shared__ unsigned sh[3];
+  if (threadIdx.x < 3) sh[threadIdx.x] = threadIdx.x < 2 ? 0u : 0xffffffffu;
   __syncthreads();
   if ((threadIdx.x & 31) == 0) {
     atomicMax(&sh[0], mt);
     atomicMax(&sh[1], mm);
+    atomicMin(&sh[2], mn);
   }
   __syncthreads();
   if (threadIdx.x == 0) {
     atomicMax(&ctl->mx_term, sh[0]);
     atomicMax(&ctl->mx_mass, sh[1]);
+    atomicMax(&ctl->mn_mass, ~sh[2]);  // the control block starts as zeros
   }
 }
 
 // The root, its chunks and the first level.
+template <int PT>
 __global__ void __launch_bounds__(256)
     k_root(DNode *nodes, int64_t n, TreeConfig cfg, LevelCtl *ctl, int32_t *chunk_node,
            int32_t *chunk_base, NodeAcc *acc, unsigned *ticket, int2 *roots, int32_t sub_max) {
-  const int32_t nc = chunks_of(int32_t(n));
+  const int32_t nc = chunks_of<PT>(int32_t(n));
   const bool sub = n <= sub_max;
   if (!sub)
     for (int32_t c = threadIdx.x; c < nc; c += blockDim.x) chunk_node[c] = 0;
@@ -686,6 +866,7 @@ __global__ void __launch_bounds__(256)
 
 // Statistics of every node of the level, and its split decision by the block
 // that adds a node's last chunk.
+template <int PT>
 __global__ void __launch_bounds__(kChunkThreads)
     k_level_stats(const float4 *__restrict__ pos, DNode *nodes, LevelCtl *ctl, int32_t level,
                   const int32_t *__restrict__ chunk_node, const int32_t *__restrict__ chunk_base,
@@ -693,15 +874,14 @@ __global__ void __launch_bounds__(kChunkThreads)
                   int32_t force_fallback, int32_t nd) {
   LevelSpan L;
   if (!level_runs(ctl, level, L, true) || int32_t(blockIdx.x) >= L.nchunk) return;
-  constexpr int kW = kChunkThreads / 32, kPer = kChunk / kChunkThreads, kU = 4;
+  constexpr int kW = kChunkThreads / 32, kU = 4;
   __shared__ NodeAcc part[kW];
-  const ChunkRange R = chunk_range(nodes, chunk_node, chunk_base, L.nb, int32_t(blockIdx.x));
-  const unsigned mt = ctl->mx_term, mm = ctl->mx_mass;
-  const SumScale sc(mt), sm(mm);
+  const ChunkRange R = chunk_range<PT>(nodes, chunk_node, chunk_base, L.nb, int32_t(blockIdx.x));
+  const SumScales S(ctl->mx_term, ctl->mx_mass, ~ctl->mn_mass);
   LaneAcc a;
   a.zero();
   int cnt = 0;
-  for (int j0 = 0; j0 < kPer && j0 * kChunkThreads < R.len; j0 += kU) {
+  for (int j0 = 0; j0 < PT && j0 * kChunkThreads < R.len; j0 += kU) {
     float4 p[kU];
 #pragma unroll
     for (int u = 0; u < kU; ++u) {
@@ -712,55 +892,41 @@ __global__ void __launch_bounds__(kChunkThreads)
     for (int u = 0; u < kU; ++u) {
       const int e = (j0 + u) * kChunkThreads + threadIdx.x;
       if (e < R.len) {
-        a.add(p[u], sc, sm);
+        a.add(p[u], S);
         ++cnt;
       }
     }
   }
-  NodeAcc w;
-  a.reduce(w, cnt, true, sc, sm);  // a warp's share of a chunk is 512 elements
-  if ((threadIdx.x & 31) == 0) part[threadIdx.x >> 5] = w;
+  a.reduce<32>(&part[threadIdx.x >> 5], true, cnt, true, S);  // a warp has at most 512 elements
   __syncthreads();
   if (threadIdx.x >= 32) return;
   // a thread per word: the warps' records into the node's, one atomic each
   NodeAcc &T = acc[R.node - L.nb];
   const int f = threadIdx.x;
-  if (f < 8) {
-    long long s = 0;
-    for (int v = 0; v < kW; ++v) s += f < 4 ? part[v].h[f] : part[v].l[f - 4];
-    atomicAdd(reinterpret_cast<unsigned long long *>(f < 4 ? &T.h[f] : &T.l[f - 4]),
-              (unsigned long long)s);
-  } else if (f < 16) {
-    unsigned s = 0;
-    for (int v = 0; v < kW; ++v) s |= f < 12 ? part[v].o1[f - 8] : part[v].o2[f - 12];
-    atomicOr(f < 12 ? &T.o1[f - 8] : &T.o2[f - 12], s);
-  } else if (f < 22) {
-    unsigned s = f < 19 ? 0xffffffffu : 0u;
-    for (int v = 0; v < kW; ++v) s = f < 19 ? min(s, part[v].lo[f - 16]) : max(s, part[v].hi[f - 19]);
-    if (f < 19) atomicMin(&T.lo[f - 16], s);
-    else atomicMax(&T.hi[f - 19], s);
-  } else if (f == 22) {
-    unsigned s = 0xffffffffu;
-    for (int v = 0; v < kW; ++v) s = min(s, part[v].wmin);
-    atomicMin(&T.wmin, s);
-  } else if (f == 23) {
-    unsigned s = 0;
-    for (int v = 0; v < kW; ++v) s |= part[v].trunc;
-    if (s) atomicOr(&T.trunc, s);
+  if (f < kAccWords) {
+    long long sum;
+    unsigned bits;
+    merge_word(part, kW, f, &sum, &bits);
+    unsigned *word = reinterpret_cast<unsigned *>(&T) + 8 + f;
+    if (f < 8) atomicAdd(reinterpret_cast<unsigned long long *>(&T) + f, (unsigned long long)sum);
+    else if (acc_or(f)) atomicOr(word, bits);
+    else if (acc_max(f)) atomicMax(word, bits);
+    else atomicMin(word, bits);
   }
   __threadfence();
   __syncwarp();
   if (threadIdx.x != 0) return;
   DNode N = nodes[R.node];
-  if (atomicAdd(&ticket[R.node - L.nb], 1u) + 1u != unsigned(chunks_of(N.count))) return;
+  if (atomicAdd(&ticket[R.node - L.nb], 1u) + 1u != unsigned(chunks_of<PT>(N.count))) return;
   __threadfence();
   ticket[R.node - L.nb] = 0u;  // k_level_count counts the chunks again
   NodeAcc A;
   const int4 *src = reinterpret_cast<const int4 *>(&T);
   int4 *dst = reinterpret_cast<int4 *>(&A);
 #pragma unroll
-  for (int q = 0; q < 8; ++q) dst[q] = __ldcg(src + q);
-  if (!decide_node(N, A, sc, sm, SumScale::bad(mt) || SumScale::bad(mm), force_fallback, nd)) {
+  for (int q = 0; q < kAccWords16; ++q) dst[q] = __ldcg(src + q);
+  S.masses(A, N.count);
+  if (!decide_node(N, A, S, force_fallback, nd)) {
     fallback[atomicAdd((unsigned long long *)&counters[C_NFALLBACK], 1ull)] = R.node;
     atomicExch(&ctl->abort, level + 1);
   }
@@ -772,6 +938,7 @@ __global__ void __launch_bounds__(kChunkThreads)
 // loaded, every lane's loads in flight at once.  The block that counts a node's
 // last chunk scans the node's chunks; the one that counts the level's last
 // chunk makes the children and the next level.
+template <int PT>
 __global__ void __launch_bounds__(kChunkThreads)
     k_level_count(const float4 *__restrict__ pos, DNode *nodes, LevelCtl *ctl, int32_t level,
                   const int32_t *__restrict__ chunk_node, const int32_t *__restrict__ chunk_base,
@@ -780,26 +947,26 @@ __global__ void __launch_bounds__(kChunkThreads)
                   int64_t *counters, int32_t sub_max) {
   LevelSpan L;
   if (!level_runs(ctl, level, L) || int32_t(blockIdx.x) >= L.nchunk) return;
-  constexpr int kWarps = kChunkThreads / 32, kSub = kChunk / kWarps, kPer = kSub / 32;
+  constexpr int kWarps = kChunkThreads / 32, kSub = 32 * PT;
   __shared__ int wt[kWarps];
   __shared__ int sh_warp[32];
   __shared__ int last;
   const int32_t chunk = int32_t(blockIdx.x);
-  const ChunkRange R = chunk_range(nodes, chunk_node, chunk_base, L.nb, chunk);
+  const ChunkRange R = chunk_range<PT>(nodes, chunk_node, chunk_base, L.nb, chunk);
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int32_t count = nodes[R.node].count, d = nodes[R.node].split_dim;
   if (d >= 0) {
     const float split = nodes[R.node].xc[d];
     const float *key = reinterpret_cast<const float *>(pos + R.begin) + d;
-    float kv[kPer];
+    float kv[PT];
 #pragma unroll
-    for (int u = 0; u < kPer; ++u) {
+    for (int u = 0; u < PT; ++u) {
       const int e = warp * kSub + 32 * u + lane;
       kv[u] = e < R.len ? key[4 * e] : INFINITY;
     }
     int c = 0;
 #pragma unroll
-    for (int u = 0; u < kPer; ++u) c += warp * kSub + 32 * u + lane < R.len && kv[u] < split;
+    for (int u = 0; u < PT; ++u) c += warp * kSub + 32 * u + lane < R.len && kv[u] < split;
     c = __reduce_add_sync(0xffffffffu, c);
     if (lane == 0) wt[warp] = c;
     __syncthreads();
@@ -816,7 +983,7 @@ __global__ void __launch_bounds__(kChunkThreads)
   // the node's last chunk: exclusive scan of its chunks' left counts
   __threadfence();
   __syncthreads();
-  const int32_t nc = chunks_of(count);
+  const int32_t nc = chunks_of<PT>(count);
   if (threadIdx.x == 0) last = atomicAdd(&ticket[R.node - L.nb], 1u) + 1u == unsigned(nc);
   __syncthreads();
   if (last && d >= 0) {
@@ -856,7 +1023,7 @@ __global__ void __launch_bounds__(kChunkThreads)
     }
     const int32_t n0 = split ? N.nleft : 0, n1 = split ? N.count - N.nleft : 0;
     const bool s0 = split && n0 <= sub_max, s1 = split && n1 <= sub_max;  // subtree roots
-    const int32_t c0 = s0 ? 0 : chunks_of(n0), c1 = s1 ? 0 : chunks_of(n1);
+    const int32_t c0 = s0 ? 0 : chunks_of<PT>(n0), c1 = s1 ? 0 : chunks_of<PT>(n1);
     int ts, tc, tr;
     const int rank = splits + block_excl_scan(split ? 1 : 0, sh_warp, &ts);
     const int32_t cb = chunks + block_excl_scan(c0 + c1, sh_warp, &tc);
@@ -907,6 +1074,7 @@ __global__ void __launch_bounds__(kChunkThreads)
 // (coalesced), kB steps' loads in flight; ranks follow array order through
 // the warps' left counts before them (k_level_count) and a ballot prefix
 // within each step.
+template <int PT>
 __global__ void __launch_bounds__(kChunkThreads)
     k_part_left(const float4 *__restrict__ pos, const int32_t *__restrict__ oid, const DNode *nodes,
                 const LevelCtl *ctl, int32_t level, const int32_t *__restrict__ chunk_node,
@@ -915,10 +1083,10 @@ __global__ void __launch_bounds__(kChunkThreads)
   LevelSpan L;
   if (!level_runs(ctl, level, L) || int32_t(blockIdx.x) >= L.nchunk) return;
   constexpr int kWarps = kChunkThreads / 32;
-  constexpr int kSub = kChunk / kWarps;  // a warp's share of the chunk
+  constexpr int kSub = 32 * PT;  // a warp's share of the chunk
   constexpr int kB = 4;
   const int32_t chunk = int32_t(blockIdx.x);
-  const ChunkRange R = chunk_range(nodes, chunk_node, chunk_base, L.nb, chunk);
+  const ChunkRange R = chunk_range<PT>(nodes, chunk_node, chunk_base, L.nb, chunk);
   const DNode &N = nodes[R.node];
   if (N.split_dim < 0) {
     // a leaf keeps its elements: copied once into the next level's buffer
@@ -1015,6 +1183,7 @@ __device__ __forceinline__ int32_t chain_jump(int32_t q, int32_t nleft, int32_t 
 // RCBForceTree.cxx:647-669), taken a run of equal steps at a time
 // (chain_jump).  Positions increase strictly along a chain, so it ends within
 // count jumps.
+template <int PT>
 __global__ void __launch_bounds__(kChunkThreads)
     k_part_right(const float4 *__restrict__ pos, const int32_t *__restrict__ oid, const DNode *nodes,
                  const LevelCtl *ctl, int32_t level, const int32_t *__restrict__ chunk_node,
@@ -1025,7 +1194,7 @@ __global__ void __launch_bounds__(kChunkThreads)
   if (!level_runs(ctl, level, L) || int32_t(blockIdx.x) >= L.nchunk) return;
   constexpr int NT = kChunkThreads;
   const int tid = threadIdx.x;
-  const ChunkRange R = chunk_range(nodes, chunk_node, chunk_base, L.nb, int32_t(blockIdx.x));
+  const ChunkRange R = chunk_range<PT>(nodes, chunk_node, chunk_base, L.nb, int32_t(blockIdx.x));
   const DNode &N = nodes[R.node];
   if (N.split_dim < 0) return;
   const int d = N.split_dim;
@@ -1033,12 +1202,12 @@ __global__ void __launch_bounds__(kChunkThreads)
   const int32_t is = N.nleft;
   const int32_t *nidx = idx + N.offset;
   if (R.local >= is) return;  // every element here stays (k_part_left)
-  // The thread's 16 elements take their first kPlainSteps steps
-  // in lockstep, so up to 16 independent loads are in flight per step (most
+  // The thread's PT elements take their first kPlainSteps steps in lockstep,
+  // so up to PT independent loads are in flight per step (most
   // chains end within a few).  The chains still running go to the level's
   // chain queue (k_part_chains follows them a chain per thread): long chains
   // gather in a few regions of a level, thousands in one chunk.
-  constexpr int kPerT = kChunk / kChunkThreads;
+  constexpr int kPerT = PT;
   const float *key = reinterpret_cast<const float *>(pos + R.begin) + d;
   int32_t q[kPerT];
   unsigned right = 0;
@@ -1081,18 +1250,31 @@ __global__ void __launch_bounds__(kChunkThreads)
     base = atomicAdd((unsigned long long *)&counters[C_CHAINS], (unsigned long long)incl);
   base = __shfl_sync(0xffffffffu, base, 31);
   int64_t slot = int64_t(base) + incl - na;
+  // the landed elements, four loads in flight at a time
+  const unsigned landed = right & ~active;
+#pragma unroll
+  for (int j0 = 0; j0 < kPerT; j0 += 4) {
+    float4 p[4];
+    int32_t o[4];
+#pragma unroll
+    for (int u = 0; u < 4; ++u)
+      if (landed >> (j0 + u) & 1u) {
+        p[u] = pos[R.begin + tid + (j0 + u) * NT];
+        o[u] = oid[R.begin + tid + (j0 + u) * NT];
+      }
+#pragma unroll
+    for (int u = 0; u < 4; ++u)
+      if (landed >> (j0 + u) & 1u) {
+        tpos[N.offset + q[j0 + u]] = p[u];
+        toid[N.offset + q[j0 + u]] = o[u];
+      }
+  }
 #pragma unroll
   for (int j = 0; j < kPerT; ++j) {
-    if (!(right >> j & 1u)) continue;
-    const int64_t src = R.begin + tid + j * NT;
-    if (active >> j & 1u) {
-      if (slot < chain_cap) chains[slot] = ChainItem{q[j], R.node, src};
-      else bad = true;  // cannot happen: a chain per element at most
-      ++slot;
-      continue;
-    }
-    tpos[N.offset + q[j]] = pos[src];
-    toid[N.offset + q[j]] = oid[src];
+    if (!(active >> j & 1u)) continue;
+    if (slot < chain_cap) chains[slot] = ChainItem{q[j], R.node, R.begin + tid + j * NT};
+    else bad = true;  // cannot happen: a chain per element at most
+    ++slot;
   }
   if (bad) atomicExch(err, 2);
 }
@@ -1462,6 +1644,7 @@ constexpr int kSubMax = 8192;        // largest subtree root (elements)
 constexpr int kSubThreads = 1024;    // one block per SM
 constexpr int kSubWarps = kSubThreads / 32;
 constexpr int kSubBatch = 256;       // nodes of a level taken at a time
+constexpr int kSubLevel = 512;       // level whose nodes stay in shared memory
 constexpr int kSubDepth = 48;        // deepest level below a root; deeper: the level loop
 constexpr int kSubBytes = 16 + 3 * 2;  // shared memory an element
 
@@ -1475,44 +1658,19 @@ __device__ __forceinline__ void team_sync(int team, int nw) {
   }
 }
 
-// The records of a team's warps merged into one, a lane per word.
-__device__ __forceinline__ void merge_records(const NodeAcc *part, int nw, int f, NodeAcc *out) {
-  if (f < 8) {
-    long long s = 0;
-    for (int v = 0; v < nw; ++v) s += f < 4 ? part[v].h[f] : part[v].l[f - 4];
-    (f < 4 ? out->h[f] : out->l[f - 4]) = s;
-  } else if (f < 16) {
-    unsigned s = 0;
-    for (int v = 0; v < nw; ++v) s |= f < 12 ? part[v].o1[f - 8] : part[v].o2[f - 12];
-    (f < 12 ? out->o1[f - 8] : out->o2[f - 12]) = s;
-  } else if (f < 22) {
-    unsigned s = f < 19 ? 0xffffffffu : 0u;
-    for (int v = 0; v < nw; ++v) s = f < 19 ? min(s, part[v].lo[f - 16]) : max(s, part[v].hi[f - 19]);
-    (f < 19 ? out->lo[f - 16] : out->hi[f - 19]) = s;
-  } else if (f == 22) {
-    unsigned s = 0xffffffffu;
-    for (int v = 0; v < nw; ++v) s = min(s, part[v].wmin);
-    out->wmin = s;
-  } else if (f == 23) {
-    unsigned s = 0;
-    for (int v = 0; v < nw; ++v) s |= part[v].trunc;
-    out->trunc = s;
-  }
-}
-
 // Node of the batch in progress.
 struct SubNode {
   int32_t lo, count;  // its elements: [lo, lo + count) of the subtree
   int32_t dim;        // split axis, -1: a leaf by size
-  float split;
   int32_t nleft;
+  float xc[3];
 };
 
 __global__ void __launch_bounds__(kSubThreads, 1)
     k_subtree(const DNode *__restrict__ nodes, const LevelCtl *ctl, const int2 *__restrict__ roots,
-              float4 *pos_a, int32_t *oid_a,
-              const float4 *pos_b, const int32_t *oid_b, DNode *sub, int32_t *sub_first,
-              int32_t *hist, int32_t cap, int32_t force_fallback, int32_t nd, int64_t *counters) {
+              float4 *pos_a, int32_t *oid_a, const float4 *pos_b, const int32_t *oid_b, DNode *sub,
+              int32_t *sub_first, int32_t *hist, int32_t cap, int32_t force_fallback, int32_t nd,
+              int64_t *counters) {
   extern __shared__ float4 P[];  // positions by input slot; then the 16-bit tables
   uint16_t *cur = reinterpret_cast<uint16_t *>(P + cap);  // input slot by position
   uint16_t *nxt = cur + cap;
@@ -1520,12 +1678,13 @@ __global__ void __launch_bounds__(kSubThreads, 1)
   __shared__ NodeAcc st[kSubBatch];
   __shared__ NodeAcc wst[kSubWarps];
   __shared__ SubNode H[kSubBatch];
+  __shared__ uint16_t lv_lo[2][kSubLevel], lv_count[2][kSubLevel];  // nodes of this level, the next
   __shared__ int wtot[kSubWarps];
-  __shared__ int tflag[8];                // per team of several warps: a chain too long / jumping changed
+  __shared__ int tflag[8];              // per team of several warps: a chain too long / jumping changed
   __shared__ int first[kSubDepth + 2];  // first local node of each depth
   __shared__ int sh_warp[32];
   __shared__ int open_[kSubBatch];      // nodes whose centre is undecided
-  __shared__ int nopen;
+  __shared__ int nopen, largest;
   if (!ctl->done || ctl->abort) return;
   const int32_t r = int32_t(blockIdx.x);
   if (r >= ctl->nroots) {  // the host launched for the most there can be
@@ -1533,16 +1692,12 @@ __global__ void __launch_bounds__(kSubThreads, 1)
       hist[int64_t(dd) * gridDim.x + r] = 0;
     return;
   }
-  const unsigned mt = ctl->mx_term, mm = ctl->mx_mass;
-  const SumScale sc(mt), sm(mm);
-  const bool bad_scale = SumScale::bad(mt) || SumScale::bad(mm);
+  const SumScales S(ctl->mx_term, ctl->mx_mass, ~ctl->mn_mass);
   const int2 root = roots[r];
-  const DNode R = nodes[root.x];
-  const int rcnt = R.count;
-  const int32_t roff = R.offset;
+  const int rcnt = nodes[root.x].count;
+  const int32_t roff = nodes[root.x].offset;
   DNode *loc = sub + 2 * int64_t(roff);  // this root's 2 x count records
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const unsigned below = (1u << lane) - 1u;
   if (rcnt > cap) {  // the launch's shared memory does not hold it
     if (threadIdx.x == 0) atomicExch(reinterpret_cast<int32_t *>(counters + C_ERR), 3);
     return;
@@ -1562,63 +1717,99 @@ __global__ void __launch_bounds__(kSubThreads, 1)
     }
   }
   if (threadIdx.x == 0) {
-    loc[0] = R;
-    loc[0].cl = loc[0].cr = 0;
+    lv_lo[0][0] = 0;
+    lv_count[0][0] = uint16_t(rcnt);
     first[0] = 0;
     first[1] = 1;
     nopen = 0;
+    largest = 0;
   }
   __syncthreads();
   const float *const Pf = reinterpret_cast<const float *>(P);
   int f0 = 0, f1 = 1, depth = 0;
   while (f1 > f0) {
     int base = f1;  // the next level's nodes made so far end here
+    const int lv = depth & 1;
     for (int b0 = f0; b0 < f1; b0 += kSubBatch) {
       const int F = min(kSubBatch, f1 - b0);
+      int count = 0;
+      if (int(threadIdx.x) < F) {
+        const int i = b0 - f0 + int(threadIdx.x);
+        int lo;
+        if (f1 - f0 <= kSubLevel) {
+          lo = lv_lo[lv][i];
+          count = lv_count[lv][i];
+        } else {
+          lo = loc[f0 + i].offset - roff;
+          count = loc[f0 + i].count;
+        }
+        H[threadIdx.x] = SubNode{lo, count, -1, 0, {0.f, 0.f, 0.f}};
+      }
+      if (warp * 32 < F) {
+        const int m = __reduce_max_sync(0xffffffffu, count);
+        if (lane == 0) atomicMax(&largest, m);
+      }
+      __syncthreads();
       // teams: the whole block for one node, halving per doubling of the batch
       // to a warp per node from 9 nodes on (at most 8 teams of several warps,
-      // named barriers 1-8)
+      // named barriers 1-8), and eight lanes per node where there are more than
+      // warps and none is large
+      const bool oct = F > kSubWarps && largest <= 512;
       int nw = 1;
       if (F <= 8) {
         int p2 = 1;
         while (p2 < F) p2 <<= 1;
         nw = kSubWarps / p2;
       }
-      const int nteams = kSubWarps / nw;
       const int team = warp / nw, w0 = team * nw, wi = warp - w0;
-      const int tl = wi * 32 + lane, TN = nw * 32;
-      if (int(threadIdx.x) < F) {
-        const DNode &N = loc[b0 + threadIdx.x];
-        H[threadIdx.x] = SubNode{N.offset - roff, N.count, -1, 0.f, 0};
-      }
-      __syncthreads();
-      // ---- statistics: a team per node ----
-      for (int f = team; f < F; f += nteams) {
-        const int c = H[f].count, lo = H[f].lo;
+      const int sl = oct ? lane & 7 : lane;               // lane of the node's in this warp
+      const int lanes = oct ? 8 : 32;                     // of the node in this warp
+      const int tl = wi * 32 + sl, TN = oct ? 8 : nw * 32;  // of the node in the block
+      const int fstep = oct ? kSubWarps * 4 : kSubWarps / nw;
+      const int fbase = oct ? warp * 4 : team, fsub = oct ? lane >> 3 : 0;
+      // ---- statistics ----
+      for (int fb = fbase; fb < F; fb += fstep) {
+        const int f = fb + fsub;
+        const int c = f < F ? H[f].count : 0, lo = f < F ? H[f].lo : 0;
+        // few enough warps that a lane has about 8 elements: what a warp's
+        // reduction costs is some 4 elements a lane
+        const int uw = nw == 1 ? 1 : min(nw, max(1, c / 256));
         LaneAcc a;
         a.zero();
         int cnt = 0;
-        for (int e = tl; e < c; e += TN, ++cnt) a.add(P[cur[lo + e]], sc, sm);
-        NodeAcc w;
-        a.reduce(w, cnt, 32 * ((c + TN - 1) / TN) <= 1023, sc, sm);
-        if (lane == 0) (nw == 1 ? st[f] : wst[warp]) = w;
+        if (oct) {
+          for (int e = sl; e < c; e += 8, ++cnt) a.add(P[cur[lo + e]], S);
+          __syncwarp();
+          a.reduce<8>(&st[min(f, kSubBatch - 1)], f < F, cnt, true, S);
+        } else if (wi < uw) {
+          for (int e = tl; e < c; e += uw * 32, ++cnt) a.add(P[cur[lo + e]], S);
+          __syncwarp();
+          a.reduce<32>(uw == 1 ? &st[f] : &wst[warp], true, cnt, 32 * ((c + uw * 32 - 1) / (uw * 32)) <= 1023, S);
+        }
         if (nw > 1) {
           team_sync(team, nw);
-          if (wi == 0) merge_records(wst + w0, nw, lane, &st[f]);
+          if (uw > 1 && wi == 0 && lane < kAccWords) {
+            long long sum;
+            unsigned bits;
+            merge_word(wst + w0, uw, lane, &sum, &bits);
+            if (lane < 8) reinterpret_cast<long long *>(&st[f])[lane] = sum;
+            else reinterpret_cast<unsigned *>(&st[f])[lane + 8] = bits;
+          }
           team_sync(team, nw);
         }
       }
       __syncthreads();
-      // ---- decisions, a thread per node (FP64 runs on whole warps) ----
+      // ---- decisions, a thread per node ----
       if (int(threadIdx.x) < F && H[threadIdx.x].count > 0) {  // an empty root stays as it is
         const int f = threadIdx.x;
-        DNode N = loc[b0 + f];
-        if (!decide_node(N, st[f], sc, sm, bad_scale, force_fallback, nd))
-          open_[atomicAdd(&nopen, 1)] = f;
+        DNode N;
+        N.count = H[f].count;
+        S.masses(st[f], N.count);
+        if (!decide_node(N, st[f], S, force_fallback, nd)) open_[atomicAdd(&nopen, 1)] = f;
         H[f].dim = N.split_dim;
-        if (N.split_dim >= 0) H[f].split = N.xc[N.split_dim];
-        loc[b0 + f] = N;
+        for (int d = 0; d < 3; ++d) H[f].xc[d] = N.xc[d];
       }
+      if (threadIdx.x == 0) largest = 0;
       __syncthreads();
       const int no = nopen;
       if (no > 0) {
@@ -1630,21 +1821,22 @@ __global__ void __launch_bounds__(kSubThreads, 1)
           const int c = H[f].count, lo = H[f].lo;
           float xc[3];
           bool ok = false;
-          if (force_fallback == 0 && !bad_scale) {
-            NodeSums S = node_sums(st[f], c);
+          if (force_fallback == 0 && !S.bad) {
+            NodeSums Q = node_sums(st[f], c);
             int low[4] = {0, 0, 0, 0};
-            const int ux = sc.k - 45, um = sm.k - 45;
+            const int ux = S.c.k - 45, um = S.m.k - 45;
             for (int e = lane; e < c; e += 32) {
               const float4 p = P[cur[lo + e]];
-              low[0] += lsb_exp(fmul_(p.w, p.x)) < last_place(S.abs[0]) + ux;
-              low[1] += lsb_exp(fmul_(p.w, p.y)) < last_place(S.abs[1]) + ux;
-              low[2] += lsb_exp(fmul_(p.w, p.z)) < last_place(S.abs[2]) + ux;
-              low[3] += lsb_exp(p.w) < last_place(S.abs[3]) + um;
+              low[0] += lsb_exp(fmul_(p.w, p.x)) < last_place(Q.abs[0]) + ux;
+              low[1] += lsb_exp(fmul_(p.w, p.y)) < last_place(Q.abs[1]) + ux;
+              low[2] += lsb_exp(fmul_(p.w, p.z)) < last_place(Q.abs[2]) + ux;
+              low[3] += lsb_exp(p.w) < last_place(Q.abs[3]) + um;
             }
+            __syncwarp();
 #pragma unroll
             for (int q = 0; q < 4; ++q) low[q] = __reduce_add_sync(0xffffffffu, low[q]);
-            tighten(S, low, st[f], c);
-            ok = quotients(S, sc.k, sm.k, xc);
+            tighten(Q, low, st[f], c);
+            ok = quotients(Q, S.c.k, S.m.k, xc);
           }
           if (lane == 0) {
             if (!ok) {
@@ -1661,49 +1853,59 @@ __global__ void __launch_bounds__(kSubThreads, 1)
               xc[2] = __double2float_rn(__ddiv_rn(z, m));
               atomicAdd((unsigned long long *)&counters[C_SUBFB], 1ull);
             }
-            for (int d = 0; d < 3; ++d) loc[b0 + f].xc[d] = xc[d];
-            if (H[f].dim >= 0) H[f].split = xc[H[f].dim];
+            for (int d = 0; d < 3; ++d) H[f].xc[d] = xc[d];
           }
         }
         __syncthreads();
         if (threadIdx.x == 0) nopen = 0;
       }
-      // ---- partition at the centre of mass: a team per node ----
-      for (int f = team; f < F; f += nteams) {
-        const int c = H[f].count, lo = H[f].lo, d = H[f].dim;
-        if (d < 0) {
-          // a leaf: its order into the other table as well
-          for (int e = tl; e < c; e += TN) nxt[lo + e] = cur[lo + e];
-          continue;
-        }
-        const float split = H[f].split;
+      // ---- partition at the centre of mass ----
+      for (int fb = fbase; fb < F; fb += fstep) {
+        const int f = fb + fsub;
+        const bool have = f < F;
+        const int c = have ? H[f].count : 0, lo = have ? H[f].lo : 0, dim = have ? H[f].dim : -1;
         const uint16_t *const in = cur + lo;
         uint16_t *const out = nxt + lo, *const ch = chain + lo;
-        const int share = (((c + nw - 1) / nw) + 31) & ~31;
-        const int beg = min(c, wi * share), end = min(c, beg + share);
+        // a leaf: its order into the other table as well
+        if (dim < 0)
+          for (int e = tl; e < c; e += TN) out[e] = in[e];
+        if (!oct && dim < 0) continue;  // the whole team
+        const int d = max(dim, 0);
+        const float split = have ? H[f].xc[d] : 0.f;
+        const int cp = dim < 0 ? 0 : c;  // elements to partition
+        const int share = oct ? cp : (((cp + nw - 1) / nw) + 31) & ~31;
+        const int beg = oct ? 0 : min(cp, wi * share), end = min(cp, beg + share);
+        // the same number of steps for the lanes of a warp
+        const int steps = __reduce_max_sync(0xffffffffu, (end - beg + lanes - 1) / lanes);
+        const int shift = oct ? lane & 24 : 0;
+        const unsigned mask = oct ? 0xffu : 0xffffffffu, below = (1u << sl) - 1u;
         int rank = 0, nleft = 0;
+        for (int k = 0; k < steps; ++k) {
+          const int e = beg + k * lanes + sl;
+          const unsigned bal = __ballot_sync(0xffffffffu, e < end && Pf[4 * in[e] + d] < split);
+          nleft += __popc(bal >> shift & mask);
+        }
         if (nw > 1) {
-          int cl = 0;
-          for (int e = beg + lane; e < end; e += 32) cl += Pf[4 * in[e] + d] < split;
-          cl = __reduce_add_sync(0xffffffffu, cl);
-          if (lane == 0) wtot[warp] = cl;
+          const int mine = nleft;
+          if (lane == 0) wtot[warp] = mine;
           if (tl == 0) tflag[team] = 0;
           team_sync(team, nw);
-          // the team's totals: a lane a warp
-          const int v = lane < nw ? wtot[w0 + lane] : 0;
-          nleft = __reduce_add_sync(0xffffffffu, v);
-          rank = __reduce_add_sync(0xffffffffu, lane < wi ? v : 0);
-        } else {
-          int cl = 0;
-          for (int e = lane; e < c; e += 32) cl += Pf[4 * in[e] + d] < split;
-          nleft = __reduce_add_sync(0xffffffffu, cl);
+          // the team's totals, a lane a warp: inclusive scan
+          int v = lane < nw ? wtot[w0 + lane] : 0;
+#pragma unroll
+          for (int o = 1; o < 32; o <<= 1) {
+            const int y = __shfl_up_sync(0xffffffffu, v, o);
+            if (lane >= o) v += y;
+          }
+          nleft = __shfl_sync(0xffffffffu, v, 31);
+          rank = __shfl_sync(0xffffffffu, v, wi) - mine;
         }
-        for (int e0 = beg; e0 < end; e0 += 32) {
-          const int e = e0 + lane;
+        for (int k = 0; k < steps; ++k) {
+          const int e = beg + k * lanes + sl;
           const bool on = e < end;
           const int s = on ? in[e] : 0;
           const bool l = on && Pf[4 * s + d] < split;
-          const unsigned bal = __ballot_sync(0xffffffffu, l);
+          const unsigned bal = __ballot_sync(0xffffffffu, l) >> shift & mask;
           if (l) {
             const int q = rank + __popc(bal & below);
             out[q] = uint16_t(s);
@@ -1718,20 +1920,21 @@ __global__ void __launch_bounds__(kSubThreads, 1)
         for (int e = tl; e < nleft; e += TN) {
           const int s = in[e];
           if (Pf[4 * s + d] < split) continue;
-          int q = e, steps = 0;
-          while (q < nleft && steps < kChainSteps) {
+          int q = e, hops = 0;
+          while (q < nleft && hops < kChainSteps) {
             const int nq = ch[q];
             if (nq <= q || nq >= c) {  // cannot happen for a valid partition
               bad = true;
               break;
             }
             q = nq;
-            ++steps;
+            ++hops;
           }
           if (q < nleft) any_long = !bad;
           else out[q] = uint16_t(s);
         }
         if (bad) atomicExch(reinterpret_cast<int32_t *>(counters + C_ERR), 2);
+        __syncwarp();
         bool jump = __any_sync(0xffffffffu, any_long);
         if (nw > 1) {
           if (jump && lane == 0) tflag[team] = 1;
@@ -1754,6 +1957,7 @@ __global__ void __launch_bounds__(kSubThreads, 1)
                 changed = true;
               }
             }
+            __syncwarp();
             changed = __any_sync(0xffffffffu, changed);
             if (nw > 1) {
               if (changed && lane == 0) tflag[team] = 1;
@@ -1774,31 +1978,51 @@ __global__ void __launch_bounds__(kSubThreads, 1)
             out[q] = uint16_t(s);
           }
         }
-        if (tl == 0) H[f].nleft = nleft;
+        if (have && dim >= 0 && tl == 0) H[f].nleft = nleft;
         team_sync(team, nw);
       }
       __syncthreads();
-      // ---- children: two per node split into two non-empty parts ----
+      // ---- records and children: two per node split into two non-empty parts ----
       const int f = int(threadIdx.x);
       int flag = 0;
       if (f < F && H[f].dim >= 0) flag = H[f].nleft > 0 && H[f].nleft < H[f].count;
       int tot = 0;
       const int rk = block_excl_scan(flag, sh_warp, &tot);
       if (f < F) {
-        DNode N = loc[b0 + f];
+        DNode N;
+        N.count = H[f].count;
+        N.offset = roff + H[f].lo;
+        const int cl = base + 2 * rk;
+        N.cl = flag ? cl : 0;
+        N.cr = flag ? cl + 1 : 0;
+        for (int d = 0; d < 3; ++d) {
+          N.xmin[d] = H[f].count > 0 ? o2f(st[f].lo[d]) : 0.f;
+          N.xmax[d] = H[f].count > 0 ? o2f(st[f].hi[d]) : 0.f;
+          N.xc[d] = H[f].xc[d];
+        }
+        N.tdr = 0.f;
+        N.split_dim = H[f].dim;
         N.nleft = H[f].nleft;
-        if (flag) {
-          const int cl = base + 2 * rk;
-          write_child(loc[cl], N, 0);
-          write_child(loc[cl + 1], N, 1);
-          N.cl = cl;
-          N.cr = cl + 1;
-        } else {
+        if (H[f].count == 0) {  // an empty set's root keeps the caller's box
+          N = nodes[root.x];
           N.cl = N.cr = 0;
         }
-        loc[b0 + f].cl = N.cl;
-        loc[b0 + f].cr = N.cr;
-        loc[b0 + f].nleft = N.nleft;
+        const int4 *src = reinterpret_cast<const int4 *>(&N);
+        int4 *out = reinterpret_cast<int4 *>(&loc[b0 + f]);
+#pragma unroll
+        for (int w = 0; w < 4; ++w) out[w] = src[w];
+        if (flag) {
+          // the children's extents: for the next level's headers
+          const int n0 = H[f].nleft, n1 = H[f].count - n0, i = cl - f1;
+          *reinterpret_cast<int2 *>(&loc[cl]) = make_int2(n0, N.offset);
+          *reinterpret_cast<int2 *>(&loc[cl + 1]) = make_int2(n1, N.offset + n0);
+          if (i + 1 < kSubLevel) {
+            lv_lo[lv ^ 1][i] = uint16_t(H[f].lo);
+            lv_count[lv ^ 1][i] = uint16_t(n0);
+            lv_lo[lv ^ 1][i + 1] = uint16_t(H[f].lo + n0);
+            lv_count[lv ^ 1][i + 1] = uint16_t(n1);
+          }
+        }
       }
       base += 2 * tot;
       __syncthreads();
@@ -3207,6 +3431,14 @@ cudaError_t DeviceTree::build(const TreeConfig &cfg, int64_t n, const float4 *po
   // bookkeeping, every level runs here.
   const bool subtrees = n == 0 || (!sub_off_ && cfg.force_cm_fallback != 2);
   const int32_t sub_max = subtrees ? kSubMax : -1;
+  const bool small = n <= kSmallSet;
+  const int64_t chunk = small ? chunk_size<4>() : chunk_size<16>();
+#define LEVEL_LAUNCH(kern, grid, ...)                                             \
+  do {                                                                            \
+    if (small) kern<4><<<grid, kChunkThreads, 0, s>>>(__VA_ARGS__);               \
+    else kern<16><<<grid, kChunkThreads, 0, s>>>(__VA_ARGS__);                    \
+    ++info_.launches;                                                             \
+  } while (0)
   std::vector<int32_t> level_begin{0};
   int64_t live = 1, level_max = n, nroots = 0;  // the next level's nodes and the roots so far
   int32_t level = 0, level_ne = 1;
@@ -3226,7 +3458,7 @@ cudaError_t DeviceTree::build(const TreeConfig &cfg, int64_t n, const float4 *po
       return std::min<int64_t>(live << i, subtrees ? n / sub_max + 1 : std::max<int64_t>(n, 1));
     };
     const int64_t after = live << batch;  // nodes that the last level can make
-    const size_t max_chunks = size_t(n / kChunk + wide(batch) + 1);
+    const size_t max_chunks = size_t(n / chunk + wide(batch) + 1);
     const size_t nodes_most =
         std::min<size_t>(size_t(2 * n + 1), size_t(level_ne) + size_t(live << (batch + 1)));
     const int64_t max_roots = nroots + after;
@@ -3243,9 +3475,7 @@ cudaError_t DeviceTree::build(const TreeConfig &cfg, int64_t n, const float4 *po
     if (batch > 0) DT_CHECK(grow(chains_, cap_ch_, size_t(std::max<int64_t>(n, 1)), s));
     auto *acc = reinterpret_cast<NodeAcc *>(acc_);
     if (!started) {
-      k_root<<<1, 256, 0, s>>>(nodes_, n, cfg, ctl, cn[0], cb[0], acc, ticket_, roots_,
-                              sub_max);
-      ++info_.launches;
+      LEVEL_LAUNCH(k_root, 1, nodes_, n, cfg, ctl, cn[0], cb[0], acc, ticket_, roots_, sub_max);
       started = true;
     }
     float4 *pb[2] = {epos_, tpos_};
@@ -3253,28 +3483,22 @@ cudaError_t DeviceTree::build(const TreeConfig &cfg, int64_t n, const float4 *po
     for (int i = 0; i < batch; ++i) {
       const int32_t l = level + i;
       const int from = l & 1, to = from ^ 1;
-      const unsigned grid = unsigned(n / kChunk + wide(i) + 1);
-      if (counted) {
-        k_level_stats<<<grid, kChunkThreads, 0, s>>>(pb[from], nodes_, ctl, l, cn[from], cb[from],
-                                                     acc, ticket_, fallback_, counters_,
-                                                     cfg.force_cm_fallback, cfg.nd);
-        ++info_.launches;
-      }
+      const unsigned grid = unsigned(n / chunk + wide(i) + 1);
+      if (counted)
+        LEVEL_LAUNCH(k_level_stats, grid, pb[from], nodes_, ctl, l, cn[from], cb[from], acc, ticket_,
+                     fallback_, counters_, cfg.force_cm_fallback, cfg.nd);
       counted = true;
-      k_level_count<<<grid, kChunkThreads, 0, s>>>(pb[from], nodes_, ctl, l, cn[from], cb[from],
-                                                   cn[to], cb[to], left_cnt_, left_base_, wpre_,
-                                                   acc, ticket_, roots_, counters_, sub_max);
-      k_part_left<<<grid, kChunkThreads, 0, s>>>(pb[from], ob[from], nodes_, ctl, l, cn[from],
-                                                 cb[from], left_base_, wpre_, pb[to], ob[to], idx_,
-                                                 ridx_);
-      k_part_right<<<grid, kChunkThreads, 0, s>>>(pb[from], ob[from], nodes_, ctl, l, cn[from],
-                                                  cb[from], idx_, pb[to], ob[to], walk_err_,
-                                                  counters_, reinterpret_cast<ChainItem *>(chains_),
-                                                  int64_t(cap_ch_));
+      LEVEL_LAUNCH(k_level_count, grid, pb[from], nodes_, ctl, l, cn[from], cb[from], cn[to], cb[to],
+                   left_cnt_, left_base_, wpre_, acc, ticket_, roots_, counters_, sub_max);
+      LEVEL_LAUNCH(k_part_left, grid, pb[from], ob[from], nodes_, ctl, l, cn[from], cb[from],
+                   left_base_, wpre_, pb[to], ob[to], idx_, ridx_);
+      LEVEL_LAUNCH(k_part_right, grid, pb[from], ob[from], nodes_, ctl, l, cn[from], cb[from], idx_,
+                   pb[to], ob[to], walk_err_, counters_, reinterpret_cast<ChainItem *>(chains_),
+                   int64_t(cap_ch_));
       k_part_chains<<<unsigned(4 * sm_count()), 256, 0, s>>>(
           pb[from], ob[from], nodes_, ctl, l, reinterpret_cast<const ChainItem *>(chains_),
           int64_t(cap_ch_), counters_, idx_, ridx_, pb[to], ob[to], walk_err_);
-      info_.launches += 4;
+      ++info_.launches;
     }
     if (subtrees) {
       DT_CHECK(grow(sub_nodes_, cap_sub_, size_t(2 * std::max<int64_t>(n, 1)), s));
@@ -3361,6 +3585,7 @@ cudaError_t DeviceTree::build(const TreeConfig &cfg, int64_t n, const float4 *po
       break;
     }
   }
+#undef LEVEL_LAUNCH
   info_.cm_fallbacks = h_counters_[C_SUBFB] + h_counters_[C_SEQ];
   const int32_t ne = level_ne;
   levels_ = level_begin;
