@@ -757,6 +757,13 @@ struct ArrayLayout {
     o = up(o + size_t(n) * 2);
     bytes = std::max<size_t>(o, 256);
   }
+  hsr::KickArrays in(char *base) const {
+    hsr::KickArrays k;
+    for (int i = 0; i < 8; ++i) k.f[i] = reinterpret_cast<float *>(base + f[i]);
+    k.id = reinterpret_cast<int64_t *>(base + id);
+    k.mask = reinterpret_cast<uint16_t *>(base + mask);
+    return k;
+  }
 };
 
 // Tree, lists, work items and the kick all on the device (rcb_device.cu).
@@ -768,9 +775,7 @@ hsr_status kick_device_build(hsr_ctx *ctx, const hsr_params *p, int64_t n, float
   float *arr[8] = {x, y, z, vx, vy, vz, mass, phi};
   CU(ctx->d_out.ensure(A.bytes), "cudaMalloc(out)");
   CU(ctx->d_pos4.ensure(size_t(std::max<int64_t>(n, 1)) * 16), "cudaMalloc(pos4)");
-  const float *in[8];
-  const int64_t *in_id;
-  const uint16_t *in_mask;
+  hsr::KickArrays in{{x, y, z, vx, vy, vz, mass, phi}, id, mask};
   char *ob = ctx->d_out.as<char>();
   const auto t_in = clk::now();
   // Host arrays: x, y, z and mass (the tree build's input) are copied on the
@@ -788,11 +793,9 @@ hsr_status kick_device_build(hsr_ctx *ctx, const hsr_params *p, int64_t n, float
   if (mem == HSR_MEM_HOST) {
     CU(ctx->d_in.ensure(A.bytes), "cudaMalloc(in)");
     char *ib = ctx->d_in.as<char>();
-    for (int i = 0; i < 8; ++i) in[i] = reinterpret_cast<const float *>(ib + A.f[i]);
+    in = A.in(ib);
     for (int i : {0, 1, 2, 6})
       CU(cudaMemcpyAsync(ib + A.f[i], arr[i], size_t(n) * 4, cudaMemcpyHostToDevice, s), "H2D positions");
-    in_id = reinterpret_cast<const int64_t *>(ib + A.id);
-    in_mask = reinterpret_cast<const uint16_t *>(ib + A.mask);
     st.h2d_bytes = n * 42;
     if (overlap) {
       if (!ctx->copier) ctx->copier.reset(new (std::nothrow) CopyWorker());
@@ -816,16 +819,12 @@ hsr_status kick_device_build(hsr_ctx *ctx, const hsr_params *p, int64_t n, float
         return e;
       });
     }
-  } else {
-    for (int i = 0; i < 8; ++i) in[i] = arr[i];
-    in_id = id;
-    in_mask = mask;
+    CU(cudaStreamSynchronize(s), "host to device copies");
+    st.t_h2d_ms = ms_since(t_in);
   }
   int64_t launches = 0;
   float4 *pos4 = ctx->d_pos4.as<float4>();
-  CU(cudaStreamSynchronize(s), "host to device copies");
-  st.t_h2d_ms = ms_since(t_in);
-  CU(hsr::launch_pack4(in[0], in[1], in[2], in[6], pos4, n, s), "pack kernel");
+  CU(hsr::launch_pack4(in.f[0], in.f[1], in.f[2], in.f[6], pos4, n, s), "pack kernel");
   ++launches;
   hsr::TreeConfig cfg{};
   for (int i = 0; i < 3; ++i) {
@@ -862,23 +861,16 @@ hsr_status kick_device_build(hsr_ctx *ctx, const hsr_params *p, int64_t n, float
     CU(ctx->copier->wait(), "H2D arrays (copy thread)");
     CU(cudaStreamWaitEvent(s, ctx->ev_in, 0), "wait for the copies");
   }
-  // outputs in tree order: velocities to the kick buffer, the rest to d_out
+  // everything into tree order: velocities to the kick buffer, the rest to
+  // d_out.  For host arrays the positions and masses too, ahead of the pair
+  // kernel (which takes every SM), so that their copies back overlap it.
   Work &w = ctx->work;
   set_work_params(w, p, n, ctx->tune);
-  float *ovx = reinterpret_cast<float *>(ob + A.f[3]), *ovy = reinterpret_cast<float *>(ob + A.f[4]),
-        *ovz = reinterpret_cast<float *>(ob + A.f[5]);
   CU(ctx->d_vel.ensure(size_t(std::max<int64_t>(3 * n, 1)) * 4), "cudaMalloc(vel)");
   float *dv = ctx->d_vel.as<float>();
-  CU(hsr::launch_gather3_f32(in[3], in[4], in[5], perm, dv, n, s), "gather velocities");
-  // the other permuted outputs ahead of the pair kernel (which takes every
-  // SM), so that their copies back overlap it
-  CU(hsr::launch_outputs(ctx->tree.table(), in[7], in_id, in_mask, perm,
-                         reinterpret_cast<float *>(ob + A.f[0]), reinterpret_cast<float *>(ob + A.f[1]),
-                         reinterpret_cast<float *>(ob + A.f[2]), reinterpret_cast<float *>(ob + A.f[6]),
-                         reinterpret_cast<float *>(ob + A.f[7]), reinterpret_cast<int64_t *>(ob + A.id),
-                         reinterpret_cast<uint16_t *>(ob + A.mask), n, s),
-     "gather outputs");
-  launches += 2;
+  const hsr::KickArrays staged = A.in(ob);
+  CU(hsr::launch_outputs(in, ctx->tree.table(), overlap, perm, dv, staged, n, s), "gather outputs");
+  ++launches;
   if (overlap) {
     // the permuted arrays other than the velocities go back now
     CU(cudaEventRecord(ctx->ev_perm, s), "event");
@@ -915,17 +907,16 @@ hsr_status kick_device_build(hsr_ctx *ctx, const hsr_params *p, int64_t n, float
   CU(ctx->launch_pairs(w.kernel), "pair kernel");
   launches += plain ? w.nleaves > 0 : w.nitems > 0;
   CU(cudaEventRecord(ctx->ev1, s), "event");
-  // kicked velocities into the output slots, then everything back
-  CU(cudaMemcpyAsync(ovx, dv, size_t(n) * 4, cudaMemcpyDeviceToDevice, s), "copy vx");
-  CU(cudaMemcpyAsync(ovy, dv + n, size_t(n) * 4, cudaMemcpyDeviceToDevice, s), "copy vy");
-  CU(cudaMemcpyAsync(ovz, dv + 2 * n, size_t(n) * 4, cudaMemcpyDeviceToDevice, s), "copy vz");
-  const cudaMemcpyKind back = mem == HSR_MEM_HOST ? cudaMemcpyDeviceToHost : cudaMemcpyDeviceToDevice;
-  for (int i = 0; i < 8; ++i)
-    if (!overlap || (i >= 3 && i <= 5))
-      CU(cudaMemcpyAsync(arr[i], ob + A.f[i], size_t(n) * 4, back, s), "copy arrays back");
-  if (!overlap) {
-    CU(cudaMemcpyAsync(id, ob + A.id, size_t(n) * 8, back, s), "copy ids back");
-    CU(cudaMemcpyAsync(mask, ob + A.mask, size_t(n) * 2, back, s), "copy masks back");
+  // kicked velocities back to the host, or everything to the device arrays
+  if (mem == HSR_MEM_HOST) {
+    for (int d = 0; d < 3; ++d)
+      CU(cudaMemcpyAsync(arr[3 + d], dv + d * n, size_t(n) * 4, cudaMemcpyDeviceToHost, s),
+         "copy velocities back");
+  } else {
+    CU(hsr::launch_finish(ctx->tree.table(), dv, staged, {{x, y, z, vx, vy, vz, mass, phi}, id, mask},
+                          n, s),
+       "results");
+    launches += n > 0;
   }
   unsigned long long counters[2] = {0, 0};
   if (!plain) CU(cudaMemcpyAsync(counters, ctx->d_queue.p, sizeof(counters), cudaMemcpyDeviceToHost, s),
@@ -962,16 +953,18 @@ namespace {
 hsr_status subcycle_resident(hsr_ctx *ctx, const hsr_subcycle_params *sp, int64_t n, float **f,
                              int64_t *ids, uint16_t *msk, int64_t *inbox, hsr_stats &total) {
   cudaStream_t s = ctx->stream;
-  CU(ctx->d_sort.ensure(hsr::resort_scratch_bytes(n)), "cudaMalloc(sort)");
+  CU(ctx->d_sort.ensure(hsr::resort_scratch_bytes(n, sp->ng)), "cudaMalloc(sort)");
   // map1's prefactor in float, as the reference computes it
   const float pf = std::pow(sp->pp, float(1.0 + 1.0 / sp->alpha));
   const float prefactor = float(1.0 / (sp->alpha * sp->adot * pf));
   const float pt = prefactor * sp->tau;
   for (int32_t step = 0; step < sp->nsub; ++step) {
-    if (!sp->skip_stream) CU(hsr::launch_stream(f[0], f[1], f[2], f[3], f[4], f[5], n, pt, s), "stream");
-    if (!sp->skip_kick) {
-      CU(hsr::resort_by_cell(n, sp->ng, f, ids, msk, ctx->d_sort.p, inbox, s), "resort");
-      CU(hsr::launch_fill(f[6], n, 1.0f, s), "masses");
+    if (sp->skip_kick) {
+      if (!sp->skip_stream) CU(hsr::launch_stream(f[0], f[1], f[2], f[3], f[4], f[5], n, pt, s), "stream");
+    } else {
+      CU(hsr::drift_and_resort(n, sp->ng, {{f[0], f[1], f[2], f[3], f[4], f[5], f[6], f[7]}, ids, msk},
+                               sp->skip_stream ? nullptr : &pt, ctx->d_sort.p, inbox, s),
+         "resort");
       hsr_stats st{};
       hsr_status r = kick_device_build(ctx, &sp->kick, *inbox, f[0], f[1], f[2], f[3], f[4], f[5],
                                        f[6], f[7], ids, msk, HSR_MEM_DEVICE, st);
@@ -1220,19 +1213,16 @@ hsr_status force_fwd_impl(hsr_ctx *ctx, const hsr_params *p, int64_t n, const fl
   CU(ctx->d_out.ensure(3 * nb + 1024), "cudaMalloc(out)");
   float *ob = ctx->d_out.as<float>();
   const size_t stride = ((nb + 255) & ~size_t(255)) / 4;
-  float *outs[3] = {dvx, dvy, dvz};
+  float *outs[3] = {dvx, dvy, dvz}, *o[3];
   for (int d = 0; d < 3; ++d) {
-    float *o = mem == HSR_MEM_HOST ? ob + d * stride : outs[d];
-    if (accumulate) {
-      if (mem == HSR_MEM_HOST)
-        CU(cudaMemcpyAsync(o, outs[d], size_t(n) * 4, cudaMemcpyHostToDevice, s), "H2D v");
-      CU(hsr::launch_scatter_add_f32(dv + d * n, ctx->tree.perm(), o, n, s), "scatter-add dv");
-    } else {
-      CU(hsr::launch_scatter_f32(dv + d * n, ctx->tree.perm(), o, n, s), "scatter dv");
-    }
-    if (mem == HSR_MEM_HOST)
-      CU(cudaMemcpyAsync(outs[d], o, size_t(n) * 4, cudaMemcpyDeviceToHost, s), "D2H dv");
+    o[d] = mem == HSR_MEM_HOST ? ob + d * stride : outs[d];
+    if (accumulate && mem == HSR_MEM_HOST)
+      CU(cudaMemcpyAsync(o[d], outs[d], size_t(n) * 4, cudaMemcpyHostToDevice, s), "H2D v");
   }
+  CU(hsr::launch_scatter3_f32(dv, n, ctx->tree.perm(), o, accumulate, n, s), "scatter dv");
+  if (mem == HSR_MEM_HOST)
+    for (int d = 0; d < 3; ++d)
+      CU(cudaMemcpyAsync(outs[d], o[d], size_t(n) * 4, cudaMemcpyDeviceToHost, s), "D2H dv");
   CU(cudaStreamSynchronize(s), "forward");
   float fms = 0;
   CU(cudaEventElapsedTime(&fms, ctx->ev0, ctx->ev1), "event time");
@@ -1321,14 +1311,12 @@ hsr_status hsr_force_vjp(hsr_ctx *ctx, const float *dvbx, const float *dvby, con
   float *acc = xcbar + sa;
   const float *uin[3] = {dvbx, dvby, dvbz};
   const int32_t *perm = ctx->tree.perm();
-  for (int d = 0; d < 3; ++d) {
-    const float *src = uin[d];
-    if (mem == HSR_MEM_HOST) {
+  if (mem == HSR_MEM_HOST)
+    for (int d = 0; d < 3; ++d) {
       CU(cudaMemcpyAsync(ub + d * sn, uin[d], size_t(n) * 4, cudaMemcpyHostToDevice, s), "H2D cotangent");
-      src = ub + d * sn;
+      uin[d] = ub + d * sn;
     }
-    CU(hsr::launch_gather_f32(src, perm, ut + d * sn, n, s), "gather cotangent");
-  }
+  CU(hsr::launch_gather3_f32(uin[0], uin[1], uin[2], perm, ut, sn, n, s), "gather cotangent");
   CU(cudaMemsetAsync(xb, 0, (quad ? 4 : 3) * st_ * 4, s), "zero xbar");
   CU(ctx->d_queue.ensure(64), "cudaMalloc(queue)");
   CU(cudaMemsetAsync(ctx->d_queue.p, 0, 2 * sizeof(unsigned long long), s), "reset queue");
@@ -1351,13 +1339,12 @@ hsr_status hsr_force_vjp(hsr_ctx *ctx, const float *dvbx, const float *dvby, con
                                   xb + 2 * st_, aerr, s),
        "pseudo-particle adjoint");
   CU(cudaEventRecord(ctx->ev1, s), "event");
-  float *outs[3] = {xbx, xby, xbz};
-  for (int d = 0; d < 3; ++d) {
-    float *o = mem == HSR_MEM_HOST ? ub + d * sn : outs[d];
-    CU(hsr::launch_scatter_f32(xb + d * st_, perm, o, n, s), "scatter xbar");
-    if (mem == HSR_MEM_HOST)
-      CU(cudaMemcpyAsync(outs[d], o, size_t(n) * 4, cudaMemcpyDeviceToHost, s), "D2H xbar");
-  }
+  float *outs[3] = {xbx, xby, xbz}, *o[3];
+  for (int d = 0; d < 3; ++d) o[d] = mem == HSR_MEM_HOST ? ub + d * sn : outs[d];
+  CU(hsr::launch_scatter3_f32(xb, int64_t(st_), perm, o, false, n, s), "scatter xbar");
+  if (mem == HSR_MEM_HOST)
+    for (int d = 0; d < 3; ++d)
+      CU(cudaMemcpyAsync(outs[d], o[d], size_t(n) * 4, cudaMemcpyDeviceToHost, s), "D2H xbar");
   int32_t h_aerr = 0;
   CU(cudaMemcpyAsync(&h_aerr, aerr, sizeof(int32_t), cudaMemcpyDeviceToHost, s), "D2H flag");
   CU(cudaStreamSynchronize(s), "adjoint");
@@ -1531,26 +1518,17 @@ hsr_status hsr_rcb_kick_batch(hsr_ctx *ctx, int32_t nbox, const hsr_params *para
     BCU(B.out.ensure(A.bytes), "cudaMalloc(out)");
     BCU(B.pos4.ensure(size_t(std::max<int64_t>(n, 1)) * 16), "cudaMalloc(pos4)");
     BCU(B.vel.ensure(size_t(std::max<int64_t>(3 * n, 1)) * 4), "cudaMalloc(vel)");
-    const float *in[8];
-    const int64_t *in_id;
-    const uint16_t *in_mask;
+    hsr::KickArrays in{{x[b], y[b], z[b], vx[b], vy[b], vz[b], mass[b], phi[b]}, id[b], mask[b]};
     if (mem == HSR_MEM_HOST) {
       BCU(B.in.ensure(A.bytes), "cudaMalloc(in)");
       char *ib = B.in.as<char>();
-      for (int i = 0; i < 8; ++i) {
+      for (int i = 0; i < 8; ++i)
         BCU(cudaMemcpyAsync(ib + A.f[i], arr[i], size_t(n) * 4, cudaMemcpyHostToDevice, s), "H2D arrays");
-        in[i] = reinterpret_cast<const float *>(ib + A.f[i]);
-      }
       BCU(cudaMemcpyAsync(ib + A.id, id[b], size_t(n) * 8, cudaMemcpyHostToDevice, s), "H2D ids");
       BCU(cudaMemcpyAsync(ib + A.mask, mask[b], size_t(n) * 2, cudaMemcpyHostToDevice, s), "H2D masks");
-      in_id = reinterpret_cast<const int64_t *>(ib + A.id);
-      in_mask = reinterpret_cast<const uint16_t *>(ib + A.mask);
-    } else {
-      for (int i = 0; i < 8; ++i) in[i] = arr[i];
-      in_id = id[b];
-      in_mask = mask[b];
+      in = A.in(ib);
     }
-    BCU(hsr::launch_pack4(in[0], in[1], in[2], in[6], B.pos4.as<float4>(), n, s), "pack kernel");
+    BCU(hsr::launch_pack4(in.f[0], in.f[1], in.f[2], in.f[6], B.pos4.as<float4>(), n, s), "pack kernel");
     hsr::TreeConfig cfg{};
     for (int i = 0; i < 3; ++i) {
       cfg.min[i] = p->min[i];
@@ -1571,14 +1549,9 @@ hsr_status hsr_rcb_kick_batch(hsr_ctx *ctx, int32_t nbox, const hsr_params *para
       return fail(HSR_ERR_CUDA, std::string("device tree build: ") + cudaGetErrorString(e));
     }
     const int32_t *perm = B.tree.perm();
-    char *ob = B.out.as<char>();
     float *dv = B.vel.as<float>();
-    BCU(hsr::launch_gather3_f32(in[3], in[4], in[5], perm, dv, n, s), "gather velocities");
-    BCU(hsr::launch_outputs(B.tree.table(), in[7], in_id, in_mask, perm,
-                            reinterpret_cast<float *>(ob + A.f[0]), reinterpret_cast<float *>(ob + A.f[1]),
-                            reinterpret_cast<float *>(ob + A.f[2]), reinterpret_cast<float *>(ob + A.f[6]),
-                            reinterpret_cast<float *>(ob + A.f[7]), reinterpret_cast<int64_t *>(ob + A.id),
-                            reinterpret_cast<uint16_t *>(ob + A.mask), n, s),
+    BCU(hsr::launch_outputs(in, B.tree.table(), mem == HSR_MEM_HOST, perm, dv,
+                            A.in(B.out.as<char>()), n, s),
         "gather outputs");
     BCU(cudaEventRecord(B.done, s), "box event");
 #undef BCU
@@ -1648,22 +1621,23 @@ hsr_status hsr_rcb_kick_batch(hsr_ctx *ctx, int32_t nbox, const hsr_params *para
                                      ctx->batched_ctas, s),
      "multi-box pair kernel");
   CU(cudaEventRecord(ctx->ev1, s), "event");
-  const cudaMemcpyKind back = mem == HSR_MEM_HOST ? cudaMemcpyDeviceToHost : cudaMemcpyDeviceToDevice;
   for (int32_t b = 0; b < nbox; ++b) {
     BoxState &B = *ctx->boxes[b];
     const int64_t n = B.n;
-    const ArrayLayout A(n);
-    char *ob = B.out.as<char>();
-    float *dv = B.vel.as<float>();
-    float *arr[8] = {x[b], y[b], z[b], vx[b], vy[b], vz[b], mass[b], phi[b]};
-    for (int d = 0; d < 3; ++d)
-      CU(cudaMemcpyAsync(ob + A.f[3 + d], dv + d * n, size_t(n) * 4, cudaMemcpyDeviceToDevice, s),
-         "copy velocities");
+    const hsr::KickArrays staged = ArrayLayout(n).in(B.out.as<char>());
+    const float *dv = B.vel.as<float>();
+    const hsr::KickArrays out{{x[b], y[b], z[b], vx[b], vy[b], vz[b], mass[b], phi[b]}, id[b], mask[b]};
+    if (mem == HSR_MEM_DEVICE) {
+      CU(hsr::launch_finish(B.tree.table(), dv, staged, out, n, s), "results");
+      continue;
+    }
     for (int i = 0; i < 8; ++i)
-      CU(cudaMemcpyAsync(arr[i], ob + A.f[i], size_t(n) * 4, back, s), "copy arrays back");
-    CU(cudaMemcpyAsync(id[b], ob + A.id, size_t(n) * 8, back, s), "copy ids back");
-    CU(cudaMemcpyAsync(mask[b], ob + A.mask, size_t(n) * 2, back, s), "copy masks back");
-    if (mem == HSR_MEM_HOST) st.d2h_bytes += n * 42;
+      CU(cudaMemcpyAsync(out.f[i], i >= 3 && i <= 5 ? dv + (i - 3) * n : staged.f[i], size_t(n) * 4,
+                         cudaMemcpyDeviceToHost, s),
+         "copy arrays back");
+    CU(cudaMemcpyAsync(out.id, staged.id, size_t(n) * 8, cudaMemcpyDeviceToHost, s), "copy ids back");
+    CU(cudaMemcpyAsync(out.mask, staged.mask, size_t(n) * 2, cudaMemcpyDeviceToHost, s), "copy masks back");
+    st.d2h_bytes += n * 42;
   }
   unsigned long long counters[2] = {0, 0};
   CU(cudaMemcpyAsync(counters, ctx->d_queue.p, sizeof(counters), cudaMemcpyDeviceToHost, s),
@@ -1889,20 +1863,17 @@ hsr_status force_batch_impl(hsr_ctx *ctx, int32_t nbox, const hsr_params *params
     const int64_t n = B.n;
     const size_t nb = (size_t(std::max<int64_t>(n, 1)) * 4 + 255) & ~size_t(255);
     float *dv = B.vel.as<float>();
-    float *outs[3] = {dvx[b], dvy[b], dvz[b]};
+    float *outs[3] = {dvx[b], dvy[b], dvz[b]}, *o[3];
     if (mem == HSR_MEM_HOST) CU(B.out.ensure(3 * nb), "cudaMalloc(out)");
     for (int d = 0; d < 3; ++d) {
-      float *o = mem == HSR_MEM_HOST ? reinterpret_cast<float *>(B.out.as<char>() + d * nb) : outs[d];
-      if (accumulate) {
-        if (mem == HSR_MEM_HOST)
-          CU(cudaMemcpyAsync(o, outs[d], size_t(n) * 4, cudaMemcpyHostToDevice, s), "H2D v");
-        CU(hsr::launch_scatter_add_f32(dv + d * n, B.tree.perm(), o, n, s), "scatter-add dv");
-      } else {
-        CU(hsr::launch_scatter_f32(dv + d * n, B.tree.perm(), o, n, s), "scatter dv");
-      }
-      if (mem == HSR_MEM_HOST)
-        CU(cudaMemcpyAsync(outs[d], o, size_t(n) * 4, cudaMemcpyDeviceToHost, s), "D2H dv");
+      o[d] = mem == HSR_MEM_HOST ? reinterpret_cast<float *>(B.out.as<char>() + d * nb) : outs[d];
+      if (accumulate && mem == HSR_MEM_HOST)
+        CU(cudaMemcpyAsync(o[d], outs[d], size_t(n) * 4, cudaMemcpyHostToDevice, s), "H2D v");
     }
+    CU(hsr::launch_scatter3_f32(dv, n, B.tree.perm(), o, accumulate, n, s), "scatter dv");
+    if (mem == HSR_MEM_HOST)
+      for (int d = 0; d < 3; ++d)
+        CU(cudaMemcpyAsync(outs[d], o[d], size_t(n) * 4, cudaMemcpyDeviceToHost, s), "D2H dv");
     if (mem == HSR_MEM_HOST) st.d2h_bytes += n * 12;
   }
   unsigned long long counters[2] = {0, 0};
@@ -1994,15 +1965,14 @@ hsr_status hsr_force_vjp_batch(hsr_ctx *ctx, int32_t nbox, const float *const *d
     float *ut = ub + 3 * sn;
     float *xb = ut + 3 * sn;
     const float *uin[3] = {dvbx[b], dvby[b], dvbz[b]};
-    for (int d = 0; d < 3; ++d) {
-      const float *src = uin[d];
-      if (mem == HSR_MEM_HOST) {
+    if (mem == HSR_MEM_HOST)
+      for (int d = 0; d < 3; ++d) {
         CU(cudaMemcpyAsync(ub + d * sn, uin[d], size_t(n) * 4, cudaMemcpyHostToDevice, s),
            "H2D cotangent");
-        src = ub + d * sn;
+        uin[d] = ub + d * sn;
       }
-      CU(hsr::launch_gather_f32(src, B.tree.perm(), ut + d * sn, n, s), "gather cotangent");
-    }
+    CU(hsr::launch_gather3_f32(uin[0], uin[1], uin[2], B.tree.perm(), ut, int64_t(sn), n, s),
+       "gather cotangent");
     CU(cudaMemsetAsync(xb, 0, (quad ? 4 : 3) * st_ * 4, s), "zero xbar");
     hsr::VjpBoxDesc &D = desc[b];
     D.mb = quad ? xb + 3 * st_ : nullptr;
@@ -2056,13 +2026,12 @@ hsr_status hsr_force_vjp_batch(hsr_ctx *ctx, int32_t nbox, const float *const *d
                                     xb + st_, xb + 2 * st_, aerr, s),
          "pseudo-particle adjoint");
     aerrs.push_back(aerr);
-    float *outs[3] = {xbx[b], xby[b], xbz[b]};
-    for (int d = 0; d < 3; ++d) {
-      float *o = mem == HSR_MEM_HOST ? ub + d * sn : outs[d];
-      CU(hsr::launch_scatter_f32(xb + d * st_, B.tree.perm(), o, n, s), "scatter xbar");
-      if (mem == HSR_MEM_HOST)
-        CU(cudaMemcpyAsync(outs[d], o, size_t(n) * 4, cudaMemcpyDeviceToHost, s), "D2H xbar");
-    }
+    float *outs[3] = {xbx[b], xby[b], xbz[b]}, *o[3];
+    for (int d = 0; d < 3; ++d) o[d] = mem == HSR_MEM_HOST ? ub + d * sn : outs[d];
+    CU(hsr::launch_scatter3_f32(xb, int64_t(st_), B.tree.perm(), o, false, n, s), "scatter xbar");
+    if (mem == HSR_MEM_HOST)
+      for (int d = 0; d < 3; ++d)
+        CU(cudaMemcpyAsync(outs[d], o[d], size_t(n) * 4, cudaMemcpyDeviceToHost, s), "D2H xbar");
   }
   std::vector<int32_t> h_aerrs(aerrs.size(), 0);
   for (size_t b = 0; b < aerrs.size(); ++b)

@@ -3009,51 +3009,71 @@ __global__ void __launch_bounds__(128)
     }
 }
 
-// ---------------------------------------------------------------------------
-// Gathers and packing
-// ---------------------------------------------------------------------------
-template <typename T>
-__global__ void k_gather(const T *__restrict__ in, const int32_t *__restrict__ perm, T *out,
-                         int64_t n) {
-  for (int64_t i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x; i < n;
-       i += int64_t(gridDim.x) * blockDim.x)
-    out[i] = in[perm[i]];
-}
-
-// The three velocity components into tree order, perm read once:
-// out[d n + i] = in_d[perm[i]].
+// Three arrays into tree order, perm read once: out[d stride + i] = in_d[perm[i]].
 __global__ void k_gather3_f32(const float *__restrict__ a, const float *__restrict__ b,
                               const float *__restrict__ c, const int32_t *__restrict__ perm,
-                              float *out, int64_t n) {
+                              float *out, int64_t stride, int64_t n) {
   for (int64_t i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x; i < n;
        i += int64_t(gridDim.x) * blockDim.x) {
     const int32_t j = perm[i];
-    out[i] = a[j];
-    out[n + i] = b[j];
-    out[2 * n + i] = c[j];
+    const float va = a[j], vb = b[j], vc = c[j];
+    out[i] = va;
+    out[stride + i] = vb;
+    out[2 * stride + i] = vc;
   }
 }
 
-// Every permuted output but the velocities in one pass: positions and masses
-// from the tree-ordered table, phi, id and mask through perm.
-__global__ void k_outputs(const float4 *__restrict__ table, const float *__restrict__ phi,
-                          const int64_t *__restrict__ id, const uint16_t *__restrict__ mask,
-                          const int32_t *__restrict__ perm, float *x, float *y, float *z, float *m,
-                          float *ophi, int64_t *oid, uint16_t *omask, int64_t n) {
+// Everything a kick permutes, perm read once: velocities to the kick's
+// buffer, phi, ids and masks to the staging arrays.  TABLE also splits the
+// tree-ordered table into positions and masses, for results that go back to
+// the host while the pairs run; device arrays get those from k_finish.
+template <bool TABLE>
+__global__ void k_outputs(KickArrays in, const float4 *__restrict__ table,
+                          const int32_t *__restrict__ perm, float *__restrict__ vel, KickArrays out,
+                          int64_t n) {
   for (int64_t i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x; i < n;
        i += int64_t(gridDim.x) * blockDim.x) {
     const int32_t j = perm[i];
+    const float v0 = in.f[3][j], v1 = in.f[4][j], v2 = in.f[5][j], h = in.f[7][j];
+    const int64_t d = in.id[j];
+    const uint16_t k = in.mask[j];
+    vel[i] = v0;
+    vel[n + i] = v1;
+    vel[2 * n + i] = v2;
+    out.f[7][i] = h;
+    out.id[i] = d;
+    out.mask[i] = k;
+    if (TABLE) {
+      const float4 p = table[i];
+      out.f[0][i] = p.x;
+      out.f[1][i] = p.y;
+      out.f[2][i] = p.z;
+      out.f[6][i] = p.w;
+    }
+  }
+}
+
+// A kick's results into the caller's device arrays, all ten in one launch
+// (thirteen copies before: 3 us each at a few thousand particles, where they
+// were a tenth of the call).
+__global__ void k_finish(const float4 *__restrict__ table, const float *__restrict__ vel,
+                         KickArrays st, KickArrays out, int64_t n) {
+  for (int64_t i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x; i < n;
+       i += int64_t(gridDim.x) * blockDim.x) {
     const float4 p = table[i];
-    const float f = phi[j];
-    const int64_t d = id[j];
-    const uint16_t k = mask[j];
-    x[i] = p.x;
-    y[i] = p.y;
-    z[i] = p.z;
-    m[i] = p.w;
-    ophi[i] = f;
-    oid[i] = d;
-    omask[i] = k;
+    const float v0 = vel[i], v1 = vel[n + i], v2 = vel[2 * n + i], h = st.f[7][i];
+    const int64_t d = st.id[i];
+    const uint16_t k = st.mask[i];
+    out.f[0][i] = p.x;
+    out.f[1][i] = p.y;
+    out.f[2][i] = p.z;
+    out.f[3][i] = v0;
+    out.f[4][i] = v1;
+    out.f[5][i] = v2;
+    out.f[6][i] = p.w;
+    out.f[7][i] = h;
+    out.id[i] = d;
+    out.mask[i] = k;
   }
 }
 
@@ -3064,18 +3084,27 @@ __global__ void k_pack4(const float *x, const float *y, const float *z, const fl
     out[i] = make_float4(x[i], y[i], z[i], m[i]);
 }
 
-__global__ void k_scatter_f32(const float *__restrict__ in, const int32_t *__restrict__ perm,
-                              float *out, int64_t n) {
+// Three tree-ordered arrays back to the caller's order, perm read once:
+// out_d[perm[i]] = in[d stride + i], or += for ADD.  The outputs may be the
+// same array (each thread's three accesses stay in order).
+template <bool ADD>
+__global__ void k_scatter3_f32(const float *__restrict__ in, int64_t stride,
+                               const int32_t *__restrict__ perm, float *o0, float *o1, float *o2,
+                               int64_t n) {
   for (int64_t i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x; i < n;
-       i += int64_t(gridDim.x) * blockDim.x)
-    out[perm[i]] = in[i];
-}
-
-__global__ void k_scatter_add_f32(const float *__restrict__ in, const int32_t *__restrict__ perm,
-                                  float *out, int64_t n) {
-  for (int64_t i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x; i < n;
-       i += int64_t(gridDim.x) * blockDim.x)
-    out[perm[i]] += in[i];
+       i += int64_t(gridDim.x) * blockDim.x) {
+    const int32_t j = perm[i];
+    const float a = in[i], b = in[stride + i], c = in[2 * stride + i];
+    if (ADD) {
+      o0[j] += a;
+      o1[j] += b;
+      o2[j] += c;
+    } else {
+      o0[j] = a;
+      o1[j] = b;
+      o2[j] = c;
+    }
+  }
 }
 
 // acc holds, per node, sum over it and its ancestors of xbar_P / M_P.
@@ -3791,38 +3820,35 @@ cudaError_t DeviceTree::fill_items(int64_t jsplit, cudaStream_t s) {
   return cudaGetLastError();
 }
 
-cudaError_t launch_gather_f32(const float *in, const int32_t *perm, float *out, int64_t n,
-                              cudaStream_t s) {
-  if (n <= 0) return cudaSuccess;
-  k_gather<float><<<grid_for(n, 256), 256, 0, s>>>(in, perm, out, n);
-  return cudaGetLastError();
-}
 cudaError_t launch_gather3_f32(const float *a, const float *b, const float *c, const int32_t *perm,
-                               float *out, int64_t n, cudaStream_t s) {
+                               float *out, int64_t stride, int64_t n, cudaStream_t s) {
   if (n <= 0) return cudaSuccess;
-  k_gather3_f32<<<grid_for(n, 256), 256, 0, s>>>(a, b, c, perm, out, n);
+  k_gather3_f32<<<grid_for(n, 256), 256, 0, s>>>(a, b, c, perm, out, stride, n);
   return cudaGetLastError();
 }
-cudaError_t launch_outputs(const float4 *table, const float *phi, const int64_t *id,
-                           const uint16_t *mask, const int32_t *perm, float *x, float *y, float *z,
-                           float *m, float *ophi, int64_t *oid, uint16_t *omask, int64_t n,
+cudaError_t launch_outputs(const KickArrays &in, const float4 *table, bool split_table,
+                           const int32_t *perm, float *vel, const KickArrays &out, int64_t n,
                            cudaStream_t s) {
   if (n <= 0) return cudaSuccess;
-  k_outputs<<<grid_for(n, 256), 256, 0, s>>>(table, phi, id, mask, perm, x, y, z, m, ophi, oid,
-                                             omask, n);
+  if (split_table)
+    k_outputs<true><<<grid_for(n, 256), 256, 0, s>>>(in, table, perm, vel, out, n);
+  else
+    k_outputs<false><<<grid_for(n, 256), 256, 0, s>>>(in, table, perm, vel, out, n);
   return cudaGetLastError();
 }
-cudaError_t launch_scatter_f32(const float *in, const int32_t *perm, float *out, int64_t n,
-                               cudaStream_t s) {
+cudaError_t launch_finish(const float4 *table, const float *vel, const KickArrays &staged,
+                          const KickArrays &out, int64_t n, cudaStream_t s) {
   if (n <= 0) return cudaSuccess;
-  k_scatter_f32<<<grid_for(n, 256), 256, 0, s>>>(in, perm, out, n);
+  k_finish<<<grid_for(n, 256), 256, 0, s>>>(table, vel, staged, out, n);
   return cudaGetLastError();
 }
-
-cudaError_t launch_scatter_add_f32(const float *in, const int32_t *perm, float *out, int64_t n,
-                                   cudaStream_t s) {
+cudaError_t launch_scatter3_f32(const float *in, int64_t stride, const int32_t *perm,
+                                float *const out[3], bool add, int64_t n, cudaStream_t s) {
   if (n <= 0) return cudaSuccess;
-  k_scatter_add_f32<<<grid_for(n, 256), 256, 0, s>>>(in, perm, out, n);
+  if (add)
+    k_scatter3_f32<true><<<grid_for(n, 256), 256, 0, s>>>(in, stride, perm, out[0], out[1], out[2], n);
+  else
+    k_scatter3_f32<false><<<grid_for(n, 256), 256, 0, s>>>(in, stride, perm, out[0], out[1], out[2], n);
   return cudaGetLastError();
 }
 

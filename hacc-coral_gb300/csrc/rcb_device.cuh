@@ -188,27 +188,33 @@ class DeviceTree {
   bool sub_off_ = false;  // when set, every level runs in the level loop
 };
 
-// The three velocity components into tree order (out: 3 n floats).
+// The ten arrays of a kick: x, y, z, vx, vy, vz, mass, phi; ids; masks.
+struct KickArrays {
+  float *f[8];
+  int64_t *id;
+  uint16_t *mask;
+};
+
+// out[d stride + i] = in_d[perm[i]] (three arrays into tree order).
 cudaError_t launch_gather3_f32(const float *a, const float *b, const float *c, const int32_t *perm,
-                               float *out, int64_t n, cudaStream_t s);
-// The permuted outputs besides the velocities: x, y, z and mass from the
-// tree-ordered table, phi, id and mask through perm.
-cudaError_t launch_outputs(const float4 *table, const float *phi, const int64_t *id,
-                           const uint16_t *mask, const int32_t *perm, float *x, float *y, float *z,
-                           float *m, float *ophi, int64_t *oid, uint16_t *omask, int64_t n,
+                               float *out, int64_t stride, int64_t n, cudaStream_t s);
+// The arrays of a kick into tree order: velocities to vel (3 n floats), phi,
+// ids and masks to out; with split_table x, y, z and mass from the tree-ordered
+// table to out as well (out's other pointers are not touched).
+cudaError_t launch_outputs(const KickArrays &in, const float4 *table, bool split_table,
+                           const int32_t *perm, float *vel, const KickArrays &out, int64_t n,
                            cudaStream_t s);
-// out[i] = in[perm[i]] (into tree order).
-cudaError_t launch_gather_f32(const float *in, const int32_t *perm, float *out, int64_t n,
-                              cudaStream_t s);
+// The results of a kick into ten device arrays: x, y, z and mass from the
+// table, the velocities from vel, phi, ids and masks from `staged`.
+cudaError_t launch_finish(const float4 *table, const float *vel, const KickArrays &staged,
+                          const KickArrays &out, int64_t n, cudaStream_t s);
 // pos4[i] = (x[i], y[i], z[i], m[i]).
 cudaError_t launch_pack4(const float *x, const float *y, const float *z, const float *m,
                          float4 *out, int64_t n, cudaStream_t s);
-// out[perm[i]] = in[i] (back to the caller's order).
-cudaError_t launch_scatter_f32(const float *in, const int32_t *perm, float *out, int64_t n,
-                               cudaStream_t s);
-// out[perm[i]] += in[i].
-cudaError_t launch_scatter_add_f32(const float *in, const int32_t *perm, float *out, int64_t n,
-                                   cudaStream_t s);
+// out_d[perm[i]] = in[d stride + i] (three arrays back to the caller's
+// order), or += with add.
+cudaError_t launch_scatter3_f32(const float *in, int64_t stride, const int32_t *perm,
+                                float *const out[3], bool add, int64_t n, cudaStream_t s);
 // Monopole pseudo-particle gradients passed to the particles through the
 // nodes' centres of mass: xbar_k += m_k sum_{nodes P containing k} xbar_P / M_P,
 // where xbar_P sits at slot n + P of the 3 arrays and M_P is the pseudo mass.

@@ -25,8 +25,20 @@ __global__ void k_stream(float *x, float *y, float *z, const float *vx, const fl
   }
 }
 
-// Cell key of every particle (Particles::array_index with lo = 0, hi = ng):
-// (floor(x) * ng1 + floor(y)) * ng2 + floor(z), or Ng when outside the box.
+// Cell of a particle (Particles::array_index with lo = 0, hi = ng):
+// (floor(x) * ng1 + floor(y)) * ng2 + floor(z); false when outside the box.
+__device__ __forceinline__ bool cell_of(float x, float y, float z, int32_t ng0, int32_t ng1,
+                                        int32_t ng2, uint32_t *k) {
+  const float fx = floorf(x), fy = floorf(y), fz = floorf(z);
+  // the reference casts floorf to int; compare in float first so huge or
+  // non-finite values land out of the box instead of overflowing the cast
+  const bool in = fx >= 0.f && fx < float(ng0) && fy >= 0.f && fy < float(ng1) && fz >= 0.f &&
+                  fz < float(ng2);
+  if (in) *k = (uint32_t(int(fx)) * uint32_t(ng1) + uint32_t(int(fy))) * uint32_t(ng2) + uint32_t(int(fz));
+  return in;
+}
+
+// Radix keys: the cell, or Ng when outside the box.
 __global__ void k_cell_keys(const float *x, const float *y, const float *z, int64_t n, int32_t ng0,
                             int32_t ng1, int32_t ng2, uint32_t *key, uint32_t *val,
                             unsigned long long *inbox) {
@@ -34,13 +46,9 @@ __global__ void k_cell_keys(const float *x, const float *y, const float *z, int6
   unsigned long long c = 0;
   for (int64_t i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x; i < n;
        i += int64_t(gridDim.x) * blockDim.x) {
-    const float fx = floorf(x[i]), fy = floorf(y[i]), fz = floorf(z[i]);
-    // the reference casts floorf to int; compare in float first so huge or
-    // non-finite values land out of the box instead of overflowing the cast
-    const bool in = fx >= 0.f && fx < float(ng0) && fy >= 0.f && fy < float(ng1) && fz >= 0.f &&
-                    fz < float(ng2);
-    uint32_t k = Ng;
-    if (in) k = (uint32_t(int(fx)) * uint32_t(ng1) + uint32_t(int(fy))) * uint32_t(ng2) + uint32_t(int(fz));
+    uint32_t k;
+    const bool in = cell_of(x[i], y[i], z[i], ng0, ng1, ng2, &k);
+    if (!in) k = Ng;
     key[i] = k;
     val[i] = uint32_t(i);
     c += in;
@@ -122,18 +130,177 @@ __global__ void __launch_bounds__(kRadixThreads)
   }
 }
 
-template <typename T>
-__global__ void k_permute(const T *__restrict__ in, const uint32_t *__restrict__ perm, T *out,
-                          int64_t n) {
+// ---- counting sort by cell --------------------------------------------------
+// Three radix passes and ten permutations with their copies back were 45
+// launches and 210 us at 88,000 particles, most of it launch gaps and 22
+// blocks on 152 SMs.  Here a particle's place is its cell's offset plus its
+// rank among the cell's particles: six launches.  A cell's particles arrive in
+// any order, so each counts the ones of its cell with a smaller index, which
+// makes the sort stable.  Particles outside the box get a pseudo-cell for
+// every 32 indices behind the grid's cells, which keeps their order with the
+// same rule and no long cell.
+constexpr uint32_t kOutRun = 32;       // indices per pseudo-cell
+constexpr int kMaxOcc = 1024;          // longest cell whose ranks are counted
+constexpr int kCellThreads = 256;
+constexpr int kCellPer = 16;
+constexpr int kCellTile = kCellThreads * kCellPer;  // cells per block of the scan
+constexpr int64_t kMaxTiles = 4096;
+
+// Words of counter: in-box particles, longest cell.
+struct CellCount {
+  unsigned long long inbox;
+  unsigned int longest;
+  unsigned int pad;
+};
+
+// The half-stream (DRIFT), each particle's cell and its arrival in the cell.
+template <bool DRIFT>
+__global__ void __launch_bounds__(kCellThreads)
+    k_cell_count(KickArrays A, int64_t n, float pt, int32_t ng0, int32_t ng1, int32_t ng2,
+                 uint32_t *key, uint32_t *slot, uint32_t *cnt, CellCount *out) {
+  const uint32_t Ng = uint32_t(ng0) * uint32_t(ng1) * uint32_t(ng2);
+  unsigned c = 0, most = 0;
   for (int64_t i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x; i < n;
-       i += int64_t(gridDim.x) * blockDim.x)
-    out[i] = in[perm[i]];
+       i += int64_t(gridDim.x) * blockDim.x) {
+    float x = A.f[0][i], y = A.f[1][i], z = A.f[2][i];
+    if (DRIFT) {
+      A.f[0][i] = x = __fadd_rn(x, __fmul_rn(pt, A.f[3][i]));
+      A.f[1][i] = y = __fadd_rn(y, __fmul_rn(pt, A.f[4][i]));
+      A.f[2][i] = z = __fadd_rn(z, __fmul_rn(pt, A.f[5][i]));
+    }
+    uint32_t k;
+    const bool in = cell_of(x, y, z, ng0, ng1, ng2, &k);
+    if (!in) k = Ng + uint32_t(i) / kOutRun;
+    const uint32_t at = atomicAdd(&cnt[k], 1u);
+    key[i] = k;
+    slot[i] = at;
+    c += in;
+    most = max(most, at + 1);
+  }
+  c = __reduce_add_sync(0xffffffffu, c);
+  most = __reduce_max_sync(0xffffffffu, most);
+  if ((threadIdx.x & 31) == 0) {
+    if (c) atomicAdd(&out->inbox, (unsigned long long)c);
+    if (most > kOutRun) atomicMax(&out->longest, most);
+  }
 }
 
-__global__ void k_fill_f32(float *p, int64_t n, float v) {
+__device__ __forceinline__ uint32_t block_sum_u32(uint32_t v, uint32_t *sh) {
+  v = __reduce_add_sync(0xffffffffu, v);
+  if ((threadIdx.x & 31) == 0) sh[threadIdx.x >> 5] = v;
+  __syncthreads();
+  uint32_t t = 0;
+  for (int w = 0; w < kCellThreads / 32; ++w) t += sh[w];
+  __syncthreads();
+  return t;
+}
+
+__global__ void __launch_bounds__(kCellThreads)
+    k_cell_tiles(const uint32_t *__restrict__ cnt, int64_t ncell, uint32_t *tile) {
+  __shared__ uint32_t sh[kCellThreads / 32];
+  const int64_t base = int64_t(blockIdx.x) * kCellTile;
+  uint32_t v = 0;
+#pragma unroll
+  for (int k = 0; k < kCellPer; ++k) {
+    const int64_t i = base + k * kCellThreads + threadIdx.x;
+    v += i < ncell ? cnt[i] : 0u;
+  }
+  v = block_sum_u32(v, sh);
+  if (threadIdx.x == 0) tile[blockIdx.x] = v;
+}
+
+// Each block adds up the tiles before its own (at most kMaxTiles) instead of
+// waiting for a scan of them.
+__global__ void __launch_bounds__(kCellThreads)
+    k_cell_offsets(const uint32_t *__restrict__ cnt, int64_t ncell,
+                   const uint32_t *__restrict__ tile, uint32_t *offs) {
+  __shared__ uint32_t sh[kCellThreads / 32];
+  uint32_t before = 0;
+  for (unsigned t = threadIdx.x; t < blockIdx.x; t += kCellThreads) before += tile[t];
+  before = block_sum_u32(before, sh);
+  const int64_t i0 = int64_t(blockIdx.x) * kCellTile + int64_t(threadIdx.x) * kCellPer;
+  uint32_t v[kCellPer], t = 0;
+#pragma unroll
+  for (int k = 0; k < kCellPer; ++k) {
+    v[k] = i0 + k < ncell ? cnt[i0 + k] : 0u;
+    t += v[k];
+  }
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  uint32_t x = t;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const uint32_t y = __shfl_up_sync(0xffffffffu, x, o);
+    if (lane >= o) x += y;
+  }
+  if (lane == 31) sh[warp] = x;
+  __syncthreads();
+  uint32_t run = before + x - t;
+  for (int w = 0; w < warp; ++w) run += sh[w];
+#pragma unroll
+  for (int k = 0; k < kCellPer; ++k) {
+    if (i0 + k < ncell) offs[i0 + k] = run;
+    run += v[k];
+  }
+}
+
+__global__ void k_cell_place(const uint32_t *__restrict__ key, const uint32_t *__restrict__ slot,
+                             const uint32_t *__restrict__ offs, int64_t n, const CellCount *c,
+                             uint32_t *order) {
+  if (c->longest > kMaxOcc) return;  // the radix sort follows
   for (int64_t i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x; i < n;
        i += int64_t(gridDim.x) * blockDim.x)
-    p[i] = v;
+    order[offs[key[i]] + slot[i]] = uint32_t(i);
+}
+
+__device__ __forceinline__ void move_particle(const KickArrays &A, const KickArrays &S, int64_t i,
+                                              int64_t to) {
+  const float x = A.f[0][i], y = A.f[1][i], z = A.f[2][i], vx = A.f[3][i], vy = A.f[4][i],
+              vz = A.f[5][i], phi = A.f[7][i];
+  const int64_t id = A.id[i];
+  const uint16_t mask = A.mask[i];
+  S.f[0][to] = x;
+  S.f[1][to] = y;
+  S.f[2][to] = z;
+  S.f[3][to] = vx;
+  S.f[4][to] = vy;
+  S.f[5][to] = vz;
+  S.f[7][to] = phi;
+  S.id[to] = id;
+  S.mask[to] = mask;
+}
+
+// Thread p takes the p-th particle by cell, finds its rank in the cell and
+// moves its arrays to their place in the staging copy.
+__global__ void k_cell_move(const uint32_t *__restrict__ order, const uint32_t *__restrict__ key,
+                            const uint32_t *__restrict__ offs, const uint32_t *__restrict__ cnt,
+                            int64_t n, const CellCount *c, KickArrays A, KickArrays S) {
+  if (c->longest > kMaxOcc) return;
+  for (int64_t p = int64_t(blockIdx.x) * blockDim.x + threadIdx.x; p < n;
+       p += int64_t(gridDim.x) * blockDim.x) {
+    const uint32_t i = order[p], k = key[i];
+    const uint32_t lo = offs[k], m = cnt[k];
+    uint32_t rank = 0;
+    if (m > 1)
+      for (uint32_t q = 0; q < m; ++q) rank += order[lo + q] < i;
+    move_particle(A, S, i, int64_t(lo) + rank);
+  }
+}
+
+// The radix sort's permutation applied to the arrays.
+__global__ void k_perm_move(const uint32_t *__restrict__ perm, int64_t n, KickArrays A, KickArrays S) {
+  for (int64_t p = int64_t(blockIdx.x) * blockDim.x + threadIdx.x; p < n;
+       p += int64_t(gridDim.x) * blockDim.x)
+    move_particle(A, S, perm[p], p);
+}
+
+// The staging copy back into the arrays, the masses set to one.
+__global__ void k_move_back(KickArrays S, KickArrays A, int64_t n, const CellCount *c) {
+  if (c && c->longest > kMaxOcc) return;
+  for (int64_t i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x; i < n;
+       i += int64_t(gridDim.x) * blockDim.x) {
+    move_particle(S, A, i, i);
+    A.f[6][i] = 1.0f;
+  }
 }
 
 inline unsigned grid_of(int64_t n, int threads = 256) {
@@ -150,50 +317,122 @@ cudaError_t launch_stream(float *x, float *y, float *z, const float *vx, const f
   return cudaGetLastError();
 }
 
-cudaError_t launch_fill(float *p, int64_t n, float v, cudaStream_t s) {
+namespace {
+
+// Scratch of a resort: staging copies, then either sort's tables in the same
+// space.
+struct ResortLayout {
+  size_t f[8], id, mask, count, tables, bytes;
+  ResortLayout(int64_t n, const int32_t ng[3]) {
+    auto up = [](size_t v) { return (v + 255) & ~size_t(255); };
+    const size_t m = size_t(std::max<int64_t>(n, 1));
+    size_t o = 0;
+    for (int i = 0; i < 8; ++i) {
+      f[i] = o;
+      if (i != 6) o = up(o + m * 4);  // masses are set, not moved
+    }
+    id = o;
+    o = up(o + m * 8);
+    mask = o;
+    o = up(o + m * 2);
+    count = o;
+    o = up(o + sizeof(CellCount));
+    tables = o;
+    // radix sort: keys and values twice, histograms, offsets, scan scratch
+    const int64_t h = 256 * std::max<int64_t>((n + kRadixTile - 1) / kRadixTile, 1);
+    size_t r = 4 * up(m * 4) + 2 * up(size_t(h) * 8) + up(size_t(scan_tmp_size(h)) * 8);
+    // counting sort: keys, slots, order, counts and offsets of the cells, tiles
+    if (counted(n, ng))
+      r = std::max(r, 3 * up(m * 4) + 2 * up(size_t(cells(n, ng)) * 4) + up(size_t(kMaxTiles) * 4));
+    bytes = o + r;
+  }
+  static int64_t grid_cells(const int32_t ng[3]) { return int64_t(ng[0]) * ng[1] * ng[2]; }
+  static int64_t cells(int64_t n, const int32_t ng[3]) {
+    return grid_cells(ng) + (n + kOutRun - 1) / kOutRun;
+  }
+  // The counting sort goes through every cell twice and a radix pass through
+  // every particle three times, so a grid of many more cells than particles
+  // takes the radix sort; so does one of more than 16 M cells, whose tiles
+  // are too many to be added up by each block.
+  static bool counted(int64_t n, const int32_t ng[3]) {
+    return grid_cells(ng) <= 8 * n && cells(n, ng) <= kMaxTiles * kCellTile;
+  }
+  KickArrays staged(char *p) const {
+    KickArrays k;
+    for (int i = 0; i < 8; ++i) k.f[i] = reinterpret_cast<float *>(p + f[i]);
+    k.f[6] = nullptr;
+    k.id = reinterpret_cast<int64_t *>(p + id);
+    k.mask = reinterpret_cast<uint16_t *>(p + mask);
+    return k;
+  }
+};
+
+struct Carve {
+  char *p;
+  template <typename T>
+  T *take(int64_t count) {
+    T *q = reinterpret_cast<T *>(p);
+    p += (size_t(count) * sizeof(T) + 255) & ~size_t(255);
+    return q;
+  }
+};
+
+}  // namespace
+
+size_t resort_scratch_bytes(int64_t n, const int32_t ng[3]) { return ResortLayout(n, ng).bytes; }
+
+cudaError_t drift_and_resort(int64_t n, const int32_t ng[3], const KickArrays &A, const float *pt,
+                             void *scratch, int64_t *n_inbox, cudaStream_t s) {
+  *n_inbox = 0;
   if (n <= 0) return cudaSuccess;
-  k_fill_f32<<<grid_of(n), 256, 0, s>>>(p, n, v);
-  return cudaGetLastError();
-}
-
-size_t resort_scratch_bytes(int64_t n) {
-  const int64_t nblocks = (n + kRadixTile - 1) / kRadixTile;
-  const int64_t h = 256 * std::max<int64_t>(nblocks, 1);
-  size_t b = 4 * size_t(std::max<int64_t>(n, 1)) * 4;          // key, val, key', val'
-  b += size_t(h) * 8 * 2;                                       // histograms, offsets
-  b += size_t(scan_tmp_size(h)) * 8 + 4096;
-  b += size_t(std::max<int64_t>(n, 1)) * 8 + 256;               // staging for one array
-  return b;
-}
-
-cudaError_t resort_by_cell(int64_t n, const int32_t ng[3], float *const arr_f[8], int64_t *ids,
-                           uint16_t *mask, void *scratch, int64_t *n_inbox, cudaStream_t s) {
-  if (n <= 0) {
-    *n_inbox = 0;
-    return cudaSuccess;
+  const ResortLayout L(n, ng);
+  char *base = static_cast<char *>(scratch);
+  const KickArrays S = L.staged(base);
+  CellCount *count = reinterpret_cast<CellCount *>(base + L.count);
+  CellCount got{};
+  cudaError_t e = cudaMemsetAsync(count, 0, sizeof(CellCount), s);
+  if (e != cudaSuccess) return e;
+  const unsigned grid = grid_of(n);
+  if (ResortLayout::counted(n, ng)) {
+    const int64_t ncell = ResortLayout::cells(n, ng);
+    const unsigned tiles = unsigned((ncell + kCellTile - 1) / kCellTile);
+    Carve c{base + L.tables};
+    uint32_t *key = c.take<uint32_t>(n), *slot = c.take<uint32_t>(n), *order = c.take<uint32_t>(n);
+    uint32_t *cnt = c.take<uint32_t>(ncell), *offs = c.take<uint32_t>(ncell);
+    uint32_t *tile = c.take<uint32_t>(kMaxTiles);
+    e = cudaMemsetAsync(cnt, 0, size_t(ncell) * 4, s);
+    if (e != cudaSuccess) return e;
+    if (pt)
+      k_cell_count<true><<<grid, kCellThreads, 0, s>>>(A, n, *pt, ng[0], ng[1], ng[2], key, slot, cnt, count);
+    else
+      k_cell_count<false><<<grid, kCellThreads, 0, s>>>(A, n, 0.f, ng[0], ng[1], ng[2], key, slot, cnt, count);
+    k_cell_tiles<<<tiles, kCellThreads, 0, s>>>(cnt, ncell, tile);
+    k_cell_offsets<<<tiles, kCellThreads, 0, s>>>(cnt, ncell, tile, offs);
+    k_cell_place<<<grid, 256, 0, s>>>(key, slot, offs, n, count, order);
+    k_cell_move<<<grid, 256, 0, s>>>(order, key, offs, cnt, n, count, A, S);
+    k_move_back<<<grid, 256, 0, s>>>(S, A, n, count);
+    e = cudaMemcpyAsync(&got, count, sizeof(got), cudaMemcpyDeviceToHost, s);
+    if (e == cudaSuccess) e = cudaStreamSynchronize(s);
+    if (e != cudaSuccess) return e;
+    *n_inbox = int64_t(got.inbox);
+    if (got.longest <= kMaxOcc) return cudaGetLastError();
+    // a cell of more particles: ranks by counting would take too long
+    e = cudaMemsetAsync(count, 0, sizeof(CellCount), s);
+    if (e != cudaSuccess) return e;
+  } else if (pt) {
+    e = launch_stream(A.f[0], A.f[1], A.f[2], A.f[3], A.f[4], A.f[5], n, *pt, s);
+    if (e != cudaSuccess) return e;
   }
   const int64_t nblocks = (n + kRadixTile - 1) / kRadixTile;
   const int64_t h = 256 * nblocks;
-  char *p = static_cast<char *>(scratch);
-  auto take = [&](size_t bytes) {
-    char *q = p;
-    p += (bytes + 255) & ~size_t(255);
-    return q;
-  };
-  uint32_t *key = reinterpret_cast<uint32_t *>(take(size_t(n) * 4));
-  uint32_t *val = reinterpret_cast<uint32_t *>(take(size_t(n) * 4));
-  uint32_t *key2 = reinterpret_cast<uint32_t *>(take(size_t(n) * 4));
-  uint32_t *val2 = reinterpret_cast<uint32_t *>(take(size_t(n) * 4));
-  int64_t *hist = reinterpret_cast<int64_t *>(take(size_t(h) * 8));
-  int64_t *offs = reinterpret_cast<int64_t *>(take(size_t(h) * 8));
-  int64_t *tmp = reinterpret_cast<int64_t *>(take(size_t(scan_tmp_size(h)) * 8));
-  unsigned long long *cnt = reinterpret_cast<unsigned long long *>(take(64));
-  char *stage = take(size_t(n) * 8);
-  cudaError_t e = cudaMemsetAsync(cnt, 0, 8, s);
-  if (e != cudaSuccess) return e;
-  k_cell_keys<<<grid_of(n), 256, 0, s>>>(arr_f[0], arr_f[1], arr_f[2], n, ng[0], ng[1], ng[2], key,
-                                         val, cnt);
-  const uint64_t Ng = uint64_t(ng[0]) * uint64_t(ng[1]) * uint64_t(ng[2]);
+  Carve c{base + L.tables};
+  uint32_t *key = c.take<uint32_t>(n), *val = c.take<uint32_t>(n), *key2 = c.take<uint32_t>(n),
+           *val2 = c.take<uint32_t>(n);
+  int64_t *hist = c.take<int64_t>(h), *offs = c.take<int64_t>(h);
+  int64_t *tmp = c.take<int64_t>(scan_tmp_size(h));
+  k_cell_keys<<<grid, 256, 0, s>>>(A.f[0], A.f[1], A.f[2], n, ng[0], ng[1], ng[2], key, val,
+                                   &count->inbox);
+  const uint64_t Ng = uint64_t(ResortLayout::grid_cells(ng));
   int bits = 1;
   while ((uint64_t(1) << bits) <= Ng) ++bits;
   for (int shift = 0; shift < bits; shift += 8) {
@@ -205,27 +444,12 @@ cudaError_t resort_by_cell(int64_t n, const int32_t ng[3], float *const arr_f[8]
     std::swap(key, key2);
     std::swap(val, val2);
   }
-  // apply the permutation to the ten arrays
-  float *sf = reinterpret_cast<float *>(stage);
-  for (int a = 0; a < 8; ++a) {
-    k_permute<float><<<grid_of(n), 256, 0, s>>>(arr_f[a], val, sf, n);
-    e = cudaMemcpyAsync(arr_f[a], sf, size_t(n) * 4, cudaMemcpyDeviceToDevice, s);
-    if (e != cudaSuccess) return e;
-  }
-  int64_t *si = reinterpret_cast<int64_t *>(stage);
-  k_permute<int64_t><<<grid_of(n), 256, 0, s>>>(ids, val, si, n);
-  e = cudaMemcpyAsync(ids, si, size_t(n) * 8, cudaMemcpyDeviceToDevice, s);
+  k_perm_move<<<grid, 256, 0, s>>>(val, n, A, S);
+  k_move_back<<<grid, 256, 0, s>>>(S, A, n, nullptr);
+  e = cudaMemcpyAsync(&got, count, sizeof(got), cudaMemcpyDeviceToHost, s);
+  if (e == cudaSuccess) e = cudaStreamSynchronize(s);
   if (e != cudaSuccess) return e;
-  uint16_t *sm = reinterpret_cast<uint16_t *>(stage);
-  k_permute<uint16_t><<<grid_of(n), 256, 0, s>>>(mask, val, sm, n);
-  e = cudaMemcpyAsync(mask, sm, size_t(n) * 2, cudaMemcpyDeviceToDevice, s);
-  if (e != cudaSuccess) return e;
-  unsigned long long h_cnt = 0;
-  e = cudaMemcpyAsync(&h_cnt, cnt, 8, cudaMemcpyDeviceToHost, s);
-  if (e != cudaSuccess) return e;
-  e = cudaStreamSynchronize(s);
-  if (e != cudaSuccess) return e;
-  *n_inbox = int64_t(h_cnt);
+  *n_inbox = int64_t(got.inbox);
   return cudaGetLastError();
 }
 
