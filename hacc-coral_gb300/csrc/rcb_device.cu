@@ -2634,14 +2634,21 @@ __global__ void __launch_bounds__(256)
 // inside the leaf's box) and the batched kernel's work items.
 // ---------------------------------------------------------------------------
 constexpr int kGroupSort = 1024;
+constexpr int kGroupHalf = 16;  // particles of a group with a box of their own
 constexpr int kGW = 256;     // leaves up to this size are grouped by one warp
 constexpr int kGWarps = 4;   // warps (leaves) per block of k_groups_warp
 constexpr int kGroupThreads = 256;
 
+// Where a segment of c > kGroupHalf particles is split: between groups, and a
+// group between its first 16 particles and the rest.
+__device__ __forceinline__ int group_split(int c, int G) {
+  return c > G ? G * (((c + G - 1) / G + 1) / 2) : kGroupHalf;
+}
+
 // Splits a leaf into groups of G particles (the last one shorter) by recursive
-// median splits along the longest axis, left parts a multiple of G: the
-// particles of a group are close, so the batched kernel's box test keeps few
-// list entries.  Every level sorts all segments of the leaf at once by
+// median splits along the longest axis, left parts a multiple of G, and each
+// group of 32 into halves once more: the particles of a half are close, so the
+// pair kernels' box test of each half keeps few list entries.  Every level sorts all segments of the leaf at once by
 // (segment, coordinate along the segment's longest axis).
 __device__ void group_large_leaf(const DNode &T, const float4 *__restrict__ pos, int32_t *gidx,
                                  int G) {
@@ -2677,7 +2684,7 @@ __device__ void group_large_leaf(const DNode &T, const float4 *__restrict__ pos,
     for (int i = threadIdx.x; i < c; i += blockDim.x) {
       int q = 0;
       while (q + 1 < nseg && seg_a[q + 1] <= i) ++q;
-      if (seg_c[q] <= G) continue;
+      if (seg_c[q] <= kGroupHalf) continue;
       const float4 p = pos[val[i]];
       const uint32_t o[3] = {f2o(p.x), f2o(p.y), f2o(p.z)};
       for (int d = 0; d < 3; ++d) {
@@ -2693,7 +2700,7 @@ __device__ void group_large_leaf(const DNode &T, const float4 *__restrict__ pos,
         int q = 0;
         while (q + 1 < nseg && seg_a[q + 1] <= i) ++q;
         uint32_t ko = 0;
-        if (seg_c[q] > G) {
+        if (seg_c[q] > kGroupHalf) {
           float ext[3];
           for (int d = 0; d < 3; ++d) ext[d] = o2f(seg_hi[d][q]) - o2f(seg_lo[d][q]);
           const int ax = (ext[0] >= ext[1] && ext[0] >= ext[2]) ? 0 : (ext[1] >= ext[2] ? 1 : 2);
@@ -2725,24 +2732,24 @@ __device__ void group_large_leaf(const DNode &T, const float4 *__restrict__ pos,
         }
         __syncthreads();
       }
-    // split every segment above G at G * ceil(groups / 2)
+    // split every segment above kGroupHalf
     if (threadIdx.x == 0) {
       int n2 = 0;
       int32_t na[kGroupSort / 16 + 1], nc[kGroupSort / 16 + 1];
       int more = 0;
       for (int q = 0; q < nseg; ++q) {
         const int32_t a0 = seg_a[q], c0 = seg_c[q];
-        if (c0 <= G) {
+        if (c0 <= kGroupHalf) {
           na[n2] = a0;
           nc[n2++] = c0;
           continue;
         }
-        const int32_t ng = (c0 + G - 1) / G, left = G * ((ng + 1) / 2);
+        const int32_t left = group_split(c0, G);
         na[n2] = a0;
         nc[n2++] = left;
         na[n2] = a0 + left;
         nc[n2++] = c0 - left;
-        more |= left > G || c0 - left > G;
+        more |= left > kGroupHalf || c0 - left > kGroupHalf;
       }
       for (int q = 0; q < n2; ++q) {
         seg_a[q] = na[q];
@@ -2781,9 +2788,9 @@ __global__ void __launch_bounds__(kGroupThreads)
 
 // Warp-per-leaf grouping for leaves of at most kGW particles (the usual
 // case; larger leaves take k_groups).  Same median splits as k_groups: per
-// level, every segment above G particles is sorted along its longest axis by
-// ranking (each element counts the keys below its own, ties by position) and
-// split at G * ceil(groups / 2).
+// level, every segment above kGroupHalf particles is sorted along its longest
+// axis by ranking (each element counts the keys below its own, ties by
+// position) and split at group_split().
 __global__ void __launch_bounds__(32 * kGWarps)
     k_groups_warp(const DNode *nodes, const int32_t *leaf_ids, const int64_t *nleaves,
                   const float4 *__restrict__ pos, int32_t *gidx, int G) {
@@ -2798,7 +2805,7 @@ __global__ void __launch_bounds__(32 * kGWarps)
   const DNode &T = nodes[leaf_ids[li]];
   const int c = T.count;
   if (c <= 0 || c > kGW) return;
-  if (c <= G) {
+  if (c <= kGroupHalf) {
     for (int i = lane; i < c; i += 32) gidx[T.offset + i] = T.offset + i;
     return;
   }
@@ -2814,11 +2821,11 @@ __global__ void __launch_bounds__(32 * kGWarps)
   __syncwarp();
   int cur = 0;
   for (int level = 0; level < 16; ++level) {
-    // longest axis of every segment above G
+    // longest axis of every segment to split
     bool any = false;
     for (int q = 0; q < nseg; ++q) {
       const int a0 = seg_a[w][q], c0 = seg_c[w][q];
-      if (c0 <= G) continue;
+      if (c0 <= kGroupHalf) continue;
       any = true;
       float lo[3] = {INFINITY, INFINITY, INFINITY}, hi[3] = {-INFINITY, -INFINITY, -INFINITY};
       for (int i = a0 + lane; i < a0 + c0; i += 32) {
@@ -2839,7 +2846,7 @@ __global__ void __launch_bounds__(32 * kGWarps)
     for (int i = lane; i < c; i += 32) {
       const int q = segid[w][i];
       float k = 0.f;
-      if (seg_c[w][q] > G) {
+      if (seg_c[w][q] > kGroupHalf) {
         const float4 p = pos[val[w][cur][i]];
         const int ax = seg_ax[w][q];
         k = ax == 0 ? p.x : (ax == 1 ? p.y : p.z);
@@ -2851,7 +2858,7 @@ __global__ void __launch_bounds__(32 * kGWarps)
       const int q = segid[w][i];
       const int a0 = seg_a[w][q], c0 = seg_c[w][q];
       int np = i;
-      if (c0 > G) {
+      if (c0 > kGroupHalf) {
         const float ki = key[w][i];
         int r = 0;
         for (int j = a0; j < a0 + c0; ++j) {
@@ -2864,18 +2871,18 @@ __global__ void __launch_bounds__(32 * kGWarps)
     }
     __syncwarp();
     cur ^= 1;
-    // split every segment above G at G * ceil(groups / 2)
+    // split every segment above kGroupHalf
     if (lane == 0) {
       int16_t na[kGW / 16 + 1], nc[kGW / 16 + 1];
       int n2 = 0;
       for (int q = 0; q < nseg; ++q) {
         const int a0 = seg_a[w][q], c0 = seg_c[w][q];
-        if (c0 <= G) {
+        if (c0 <= kGroupHalf) {
           na[n2] = int16_t(a0);
           nc[n2++] = int16_t(c0);
           continue;
         }
-        const int ng = (c0 + G - 1) / G, left = G * ((ng + 1) / 2);
+        const int left = group_split(c0, G);
         na[n2] = int16_t(a0);
         nc[n2++] = int16_t(left);
         na[n2] = int16_t(a0 + left);

@@ -462,33 +462,47 @@ cudaError_t launch_tag_items(const PairItem *in, PairItem *out, int64_t n, int b
 // Adjoint of the batched kernel.  For a pair (i, j) with d = x_j - x_i,
 // r2 = |d|^2 and w = fcoeff m_i m_j:
 //   d dv_i / d x_j = w (g(r2) I + 2 g'(r2) d d^T) =: M,  d dv_i / d x_i = -M,
-// so the pair adds v = M u_i to xbar_j and subtracts it from xbar_i.  Each
-// pair's v is computed once, lanes = the group's particles and two buffered
-// entries per step on packed FP32: the particle side accumulates in
-// registers, and the entry side goes through shared memory -- every lane
-// writes its v into one row per entry, and then one lane per entry sums the
-// entry's row (16-byte loads) and adds it with one atomic triple.  Groups of
-// more than 16 particles take a lane each, 16 buffered entries per transpose;
-// groups of at most 16 run on both half-warps as in k_pairs_batched (half 0
-// the even slot pairs, half 1 the odd ones), 32 entries of 16-column rows per
-// transpose, and their particle sums are added across the halves at the end.
-// Self entries (j = i) are skipped: their two terms cancel.
+// so the pair adds v = M u_i to xbar_j and subtracts it from xbar_i, each
+// pair's terms computed once.  Self entries (j = i) are skipped: their two
+// terms cancel.
+//
+// An item's group is taken as two halves of at most 16 particles, one after
+// the other, each against the entries its own bounding box keeps (23 % fewer
+// pairs than with the box of all 32).  The kept entries are evaluated 16 at a
+// time, a lane per entry: lanes 0-15 run the first half of the particles'
+// pairs, lanes 16-31 the second.  The entry's sums over the particles stay in
+// the lane (one exchange between the half-warps per 16 entries, then the
+// atomics), the particles' sums over the entries stay in registers until the
+// list ends.  With a lane per particle, as before, every entry's sum had to
+// cross the warp through shared memory: a quarter of the kernel's
+// instructions (64^3 Zel'dovich set: 456 us before, 320 us now; eight 96^3
+// boxes: 9.0 ms, 7.1 ms).  What bounds it: dispatch.  A packed operation takes two
+// dispatch slots, 82 of the 98 that a pair of particles against an entry
+// needs here.
 // ---------------------------------------------------------------------------
-constexpr int kVjpRow = 36;   // floats per transpose row: 32 particles, 16-byte rows
-constexpr int kVjpRows = 16;  // entries per transpose
-// half-warp groups: 16 particles per row; a stride of 24 floats puts the two
-// halves' rows (two apart) on disjoint banks
-constexpr int kVjpRowH = 24;
-constexpr int kVjpRowsH = 32;
-constexpr int kVjpWarpFloats = 3 * kVjpRowsH * kVjpRowH > 3 * kVjpRows * kVjpRow
-                                   ? 3 * kVjpRowsH * kVjpRowH
-                                   : 3 * kVjpRows * kVjpRow;
-constexpr size_t kVjpSmem = size_t(kBatchedWarps) * kVjpWarpFloats * sizeof(float);
-// with mass cotangents (12-point pseudo-particles): a fourth component row
-constexpr int kVjpComp = kVjpRowsH * kVjpRowH > kVjpRows * kVjpRow ? kVjpRowsH * kVjpRowH
-                                                                    : kVjpRows * kVjpRow;
-constexpr int kVjpWarpFloatsMB = 4 * kVjpComp;
-constexpr size_t kVjpSmemMB = size_t(kBatchedWarps) * kVjpWarpFloatsMB * sizeof(float);
+constexpr int kHalf = 16;                 // particles of a half, entries of an evaluation
+constexpr int kHalfPairs = kHalf / 2;     // its particle pairs
+constexpr int kLanePairs = kHalfPairs / 2;  // particle pairs per lane
+constexpr int kHalfBuf = kHalf - 1 + 32;  // kept entries waiting: a remainder and a step's
+
+// Sums over the 16 lanes of a half-warp of the lane's 8 particles' values
+// v[pair] = (first, second): every lane receives the sum for the particle of
+// slot (lane >> 1) & 7 (slot = 2 pair + which).
+__device__ __forceinline__ float half_sums(const float2 (&v)[kLanePairs], int lane) {
+  const unsigned full = 0xffffffffu;
+  float2 a[2];
+#pragma unroll
+  for (int i = 0; i < 2; ++i) {
+    const float2 send = (lane & 8) ? v[i] : v[i + 2], keep = (lane & 8) ? v[i + 2] : v[i];
+    a[i].x = keep.x + __shfl_xor_sync(full, send.x, 8);
+    a[i].y = keep.y + __shfl_xor_sync(full, send.y, 8);
+  }
+  const float2 send = (lane & 4) ? a[0] : a[1], keep = (lane & 4) ? a[1] : a[0];
+  const float bx = keep.x + __shfl_xor_sync(full, send.x, 4);
+  const float by = keep.y + __shfl_xor_sync(full, send.y, 4);
+  const float c = ((lane & 2) ? by : bx) + __shfl_xor_sync(full, (lane & 2) ? bx : by, 2);
+  return c + __shfl_xor_sync(full, c, 1);
+}
 
 // MB: also the mass cotangent of every pseudo-particle entry (table index >=
 // npart) into mb_ (the 12-point pseudo-particles' masses depend on positions).
@@ -501,22 +515,15 @@ __global__ void __launch_bounds__(32 * kBatchedWarps, 2)
                 float *__restrict__ xbz_, float fcoeff_, float rsm2_, float rcut2_, float rcull2_,
                 unsigned long long *__restrict__ queue, const VjpBoxDesc *__restrict__ boxes,
                 float *__restrict__ mb_ = nullptr, int64_t npart = 0) {
-  // kept entries, two per slot pair as in k_pairs_batched: (x, x', y, y'),
-  // (z, z', m, m') and their table indices
-  __shared__ float4 bufA[kBatchedWarps][33], bufB[kBatchedWarps][33];
-  __shared__ int32_t bufI[kBatchedWarps][66];
-  // per warp, the entry side's transpose: rows (component, entry) of the 32
-  // particles' v
-  extern __shared__ float4 vjp_rows[];
+  // kept entries as (x, x, y, y) and (z, z, m, m), and their table indices
+  __shared__ float4 ent[kBatchedWarps][kHalfBuf][2];
+  __shared__ int32_t ent_idx[kBatchedWarps][kHalfBuf];
+  __shared__ VjpPair grp[kBatchedWarps][kHalfPairs];
   const int lane = threadIdx.x & 31;
   const int w = threadIdx.x >> 5;
   const unsigned full = 0xffffffffu;
   const unsigned below = (1u << lane) - 1u;
-  float *const fa = reinterpret_cast<float *>(bufA[w]);
-  float *const fb = reinterpret_cast<float *>(bufB[w]);
-  float *const tv =
-      reinterpret_cast<float *>(vjp_rows) + size_t(w) * (MB ? kVjpWarpFloatsMB : kVjpWarpFloats);
-  constexpr int NC = MB ? 4 : 3;  // components summed per entry
+  const int el = lane & (kHalf - 1), hw = lane >> 4;
   for (;;) {
     unsigned long long it = 0;
     if (lane == 0) it = atomicAdd(queue, 1ull);
@@ -548,52 +555,92 @@ __global__ void __launch_bounds__(32 * kBatchedWarps, 2)
       rcut2 = B.rcut2;
       rcull2 = B.rcull2;
     }
-    // groups of at most 16 particles on half-warps (warp-uniform)
-    const bool hm = W.g_count <= 16;
-    const int gl = hm ? (lane & 15) : lane;  // particle of the group
-    const int half = hm ? (lane >> 4) : 0;
-    const bool act = gl < W.g_count;
-    const int pi = gidx[W.g_begin + (act ? gl : 0)];
-    const float4 P = pos[pi];
-    // inactive lanes carry a zero cotangent and weight, so they add nothing
-    const float u0 = act ? ux[pi] : 0.f, u1 = act ? uy[pi] : 0.f, u2 = act ? uz[pi] : 0.f;
-    const float wi = act ? ((LAW == LAW_POLY5_STEP16) ? fcoeff : fcoeff * P.w) : 0.f;
-    float lox = P.x, hix = P.x, loy = P.y, hiy = P.y, loz = P.z, hiz = P.z;
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-      lox = fminf(lox, __shfl_xor_sync(full, lox, o));
-      hix = fmaxf(hix, __shfl_xor_sync(full, hix, o));
-      loy = fminf(loy, __shfl_xor_sync(full, loy, o));
-      hiy = fmaxf(hiy, __shfl_xor_sync(full, hiy, o));
-      loz = fminf(loz, __shfl_xor_sync(full, loz, o));
-      hiz = fmaxf(hiz, __shfl_xor_sync(full, hiz, o));
-    }
-    // centre and half-width, widened by 4 ulps of the coordinates
-    const float hx = fmaf(fmaxf(fabsf(lox), fabsf(hix)), 4.8e-7f, 0.5f * (hix - lox));
-    const float hy = fmaf(fmaxf(fabsf(loy), fabsf(hiy)), 4.8e-7f, 0.5f * (hiy - loy));
-    const float hz = fmaf(fmaxf(fabsf(loz), fabsf(hiz)), 4.8e-7f, 0.5f * (hiz - loz));
-    const float cx = 0.5f * (lox + hix), cy = 0.5f * (loy + hiy), cz = 0.5f * (loz + hiz);
-    const float2 nxi = make_float2(-P.x, -P.x), nyi = make_float2(-P.y, -P.y),
-                 nzi = make_float2(-P.z, -P.z);
-    const float2 wi2 = make_float2(wi, wi), ua = make_float2(u0, u0), ub = make_float2(u1, u1),
-                 uc = make_float2(u2, u2);
-    float2 bx = make_float2(0.f, 0.f), by = bx, bz = bx;  // particle side
     const int32_t *lst = idx + W.j_begin;
     const int len = W.j_len;
-    int nbuf = 0;
-    // software pipeline as in k_pairs_batched: the next step's entry and the
-    // index of the one after it are in flight while this step runs
-    int32_t jtn = 0, in2 = 0;
-    float4 Jn = make_float4(0.f, 0.f, 0.f, 0.f);
-    if (len > 0) {
-      jtn = lst[lane < len ? lane : 0];
-      Jn = pos[jtn];
-      in2 = lst[32 + lane < len ? 32 + lane : 0];
-    }
-    for (int j0 = 0; j0 < len || nbuf > 0; j0 += 32) {
-      if (j0 < len) {
-        const int j = j0 + lane;
-        const bool ok = j < len;
+    for (int g0 = 0; g0 < W.g_count; g0 += kHalf) {
+      const int g = min(W.g_count - g0, kHalf);  // particles of this half, warp-uniform
+      const bool act = el < g;
+      const int pi = gidx[W.g_begin + g0 + (act ? el : 0)];
+      const float4 P = pos[pi];
+      float lox = P.x, hix = P.x, loy = P.y, hiy = P.y, loz = P.z, hiz = P.z;
+#pragma unroll
+      for (int o = kHalf / 2; o > 0; o >>= 1) {
+        lox = fminf(lox, __shfl_xor_sync(full, lox, o));
+        hix = fmaxf(hix, __shfl_xor_sync(full, hix, o));
+        loy = fminf(loy, __shfl_xor_sync(full, loy, o));
+        hiy = fmaxf(hiy, __shfl_xor_sync(full, hiy, o));
+        loz = fminf(loz, __shfl_xor_sync(full, loz, o));
+        hiz = fmaxf(hiz, __shfl_xor_sync(full, hiz, o));
+      }
+      // centre and half-width, widened by 4 ulps of the coordinates
+      const float hx = fmaf(fmaxf(fabsf(lox), fabsf(hix)), 4.8e-7f, 0.5f * (hix - lox));
+      const float hy = fmaf(fmaxf(fabsf(loy), fabsf(hiy)), 4.8e-7f, 0.5f * (hiy - loy));
+      const float hz = fmaf(fmaxf(fabsf(loz), fabsf(hiz)), 4.8e-7f, 0.5f * (hiz - loz));
+      const float cx = 0.5f * (lox + hix), cy = 0.5f * (loy + hiy), cz = 0.5f * (loz + hiz);
+      if (hw == 0) {
+        // absent particles: far away (outside every entry's cutoff), no cotangent
+        const float wi = (LAW == LAW_POLY5_STEP16) ? fcoeff : fcoeff * P.w;
+        VjpPair &G = grp[w][el >> 1];
+        const int o = el & 1;
+        (&G.nxy.x)[o] = act ? -P.x : 1e18f;
+        (&G.nxy.z)[o] = act ? -P.y : 1e18f;
+        (&G.nz_u.x)[o] = act ? -P.z : 1e18f;
+        (&G.nz_u.z)[o] = act ? wi * ux[pi] : 0.f;
+        (&G.u.x)[o] = act ? wi * uy[pi] : 0.f;
+        (&G.u.z)[o] = act ? wi * uz[pi] : 0.f;
+        (&G.idx.x)[o] = act ? pi : -1;
+      }
+      __syncwarp();
+      const int steps = (g + 3) >> 2;  // particle pairs per lane
+      const VjpPair *const mine = grp[w] + hw * steps;
+      float2 px[kLanePairs], py[kLanePairs], pz[kLanePairs];
+#pragma unroll
+      for (int q = 0; q < kLanePairs; ++q) px[q] = py[q] = pz[q] = make_float2(0.f, 0.f);
+      // the entries from `first` on, n <= 16 of them (the rest are far away)
+      auto eval = [&](int first, int n) {
+        const float4 e0 = ent[w][first + el][0], e1 = ent[w][first + el][1];
+        const int jt = ent_idx[w][first + el];
+        const float2 x = make_float2(e0.x, e0.y), y = make_float2(e0.z, e0.w),
+                     z = make_float2(e1.x, e1.y), m = make_float2(e1.z, e1.w);
+        float2 ex = make_float2(0.f, 0.f), ey = ex, ez = ex, mb2 = ex;
+        if (steps == kLanePairs) {
+#pragma unroll
+          for (int q = 0; q < kLanePairs; ++q)
+            vjp_pair_acc<LAW, MB>(mine[q], x, y, z, m, jt, rsm2, rcut2, ex, ey, ez, mb2, px[q],
+                                  py[q], pz[q]);
+        } else {
+#pragma unroll
+          for (int q = 0; q < kLanePairs - 1; ++q)
+            if (q < steps)
+              vjp_pair_acc<LAW, MB>(mine[q], x, y, z, m, jt, rsm2, rcut2, ex, ey, ez, mb2,
+                                    px[q], py[q], pz[q]);
+        }
+        float sx = ex.x + ex.y, sy = ey.x + ey.y, sz = ez.x + ez.y, sm = mb2.x + mb2.y;
+        sx += __shfl_xor_sync(full, sx, 16);
+        sy += __shfl_xor_sync(full, sy, 16);
+        sz += __shfl_xor_sync(full, sz, 16);
+        if (MB) sm += __shfl_xor_sync(full, sm, 16);
+        if (lane < n) {
+          if (sx != 0.f || sy != 0.f || sz != 0.f) {
+            atomicAdd(xbx + jt, sx);
+            atomicAdd(xby + jt, sy);
+            atomicAdd(xbz + jt, sz);
+          }
+          if (MB && mbp && jt >= np && sm != 0.f) atomicAdd(mbp + jt, sm);
+        }
+      };
+      int nbuf = 0;  // entries waiting, warp-uniform
+      // software pipeline as in k_pairs_batched: the next step's entry and the
+      // index of the one after it are in flight while this step runs
+      int32_t jtn = 0, in2 = 0;
+      float4 Jn = make_float4(0.f, 0.f, 0.f, 0.f);
+      if (len > 0) {
+        jtn = lst[lane < len ? lane : 0];
+        Jn = pos[jtn];
+        in2 = lst[32 + lane < len ? 32 + lane : 0];
+      }
+      for (int j0 = 0; j0 < len; j0 += 32) {
+        const bool ok = j0 + lane < len;
         const int32_t jt = jtn;
         const float4 J = Jn;
         if (j0 + 32 < len) {
@@ -609,182 +656,53 @@ __global__ void __launch_bounds__(32 * kBatchedWarps, 2)
         const unsigned keep = __ballot_sync(full, k);
         if (k) {
           const int e = nbuf + __popc(keep & below);
-          const int o = 4 * (e >> 1) + (e & 1);
-          fa[o] = J.x;
-          fa[o + 2] = J.y;
-          fb[o] = J.z;
-          fb[o + 2] = J.w;
-          bufI[w][e] = jt;
+          ent[w][e][0] = make_float4(J.x, J.x, J.y, J.y);
+          ent[w][e][1] = make_float4(J.z, J.z, J.w, J.w);
+          ent_idx[w][e] = jt;
         }
         nbuf += __popc(keep);
-        if (nbuf < 32 && j0 + 32 < len) continue;
-      }
-      // evaluate up to 32 buffered entries (all of them at the end of the list)
-      const int ne = nbuf < 32 ? nbuf : 32;
-      if (lane >= ne && lane < ((ne + 1) & ~1)) {
-        // odd tail: a far-away massless entry of no particle
-        const int o = 4 * (lane >> 1) + (lane & 1);
-        fa[o] = 1e18f;
-        fa[o + 2] = 1e18f;
-        fb[o] = 1e18f;
-        fb[o + 2] = 0.f;
-        bufI[w][lane] = -2;
-      }
-      __syncwarp();
-      // v of slot pair q's two entries against this lane's particle
-      auto eval_pair = [&](int q, float2 &vx, float2 &vy, float2 &vz, float2 &mb2) {
-        const float4 A = bufA[w][q], B = bufB[w][q];
-        const int ja = bufI[w][2 * q], jb = bufI[w][2 * q + 1];
-        const float2 ex = __fadd2_rn(make_float2(A.x, A.y), nxi);
-        const float2 ey = __fadd2_rn(make_float2(A.z, A.w), nyi);
-        const float2 ez = __fadd2_rn(make_float2(B.x, B.y), nzi);
-        const float2 r2 = __ffma2_rn(ex, ex, __ffma2_rn(ey, ey, __fmul2_rn(ez, ez)));
-        const bool on_a = act && ja != pi && in_range<LAW>(r2.x, rcut2);
-        const bool on_b = act && jb != pi && in_range<LAW>(r2.y, rcut2);
-        vjp2_term<LAW, MB>(ex, ey, ez, __fmul2_rn(wi2, make_float2(B.z, B.w)), ua, ub, uc, rsm2,
-                           on_a, on_b, vx, vy, vz, wi2, &mb2);
-        bx = __fadd2_rn(bx, vx);
-        by = __fadd2_rn(by, vy);
-        bz = __fadd2_rn(bz, vz);
-      };
-      if (hm) {
-        // all (up to 32) entries in one transpose: half 0 the even slot
-        // pairs, half 1 the odd ones
-        const int nq = (ne + 1) / 2;
-        for (int q = half; q < nq; q += 2) {
-          float2 vx, vy, vz, mb2;
-          eval_pair(q, vx, vy, vz, mb2);
-          float *row = tv + (2 * q) * kVjpRowH + gl;
-          row[0] = vx.x;
-          row[kVjpRowH] = vx.y;
-          row[kVjpRowsH * kVjpRowH] = vy.x;
-          row[(kVjpRowsH + 1) * kVjpRowH] = vy.y;
-          row[2 * kVjpRowsH * kVjpRowH] = vz.x;
-          row[(2 * kVjpRowsH + 1) * kVjpRowH] = vz.y;
-          if (MB) {
-            row[3 * kVjpRowsH * kVjpRowH] = mb2.x;
-            row[(3 * kVjpRowsH + 1) * kVjpRowH] = mb2.y;
-          }
-        }
         __syncwarp();
-        // entry side: lane e sums entry e's row of each component; rows start
-        // on 4 bank groups only (stride 24), so lanes 4-7 of each quarter-warp
-        // take the row's 16-byte pieces rotated by one, which puts a quarter-
-        // warp's 8 loads on 32 distinct banks
-        if (lane < ne) {
-          float sum[NC];
-          const int rot = (lane >> 2) & 1;
-#pragma unroll
-          for (int c = 0; c < NC; ++c) {
-            const float4 *row =
-                reinterpret_cast<const float4 *>(tv + (c * kVjpRowsH + lane) * kVjpRowH);
-            float2 s2 = make_float2(0.f, 0.f);
-#pragma unroll
-            for (int k = 0; k < 4; ++k) {
-              const float4 t = row[(k + rot) & 3];
-              s2 = __fadd2_rn(s2, __fadd2_rn(make_float2(t.x, t.y), make_float2(t.z, t.w)));
-            }
-            sum[c] = s2.x + s2.y;
-          }
-          const int jt = bufI[w][lane];
-          if (sum[0] != 0.f || sum[1] != 0.f || sum[2] != 0.f) {
-            atomicAdd(xbx + jt, sum[0]);
-            atomicAdd(xby + jt, sum[1]);
-            atomicAdd(xbz + jt, sum[2]);
-          }
-          if (MB && mbp && jt >= np && sum[NC - 1] != 0.f) atomicAdd(mbp + jt, sum[NC - 1]);
+        while (nbuf >= kHalf) {
+          nbuf -= kHalf;
+          eval(nbuf, kHalf);
         }
         __syncwarp();
       }
-      for (int h = 0; !hm && 16 * h < ne; ++h) {
-        // entries 16h .. 16h + 15 of the buffer
-        const int q1 = min(8 * h + 8, (ne + 1) / 2);
-        for (int q = 8 * h; q < q1; ++q) {
-          float2 vx, vy, vz, mb2;
-          eval_pair(q, vx, vy, vz, mb2);
-          float *row = tv + (2 * q - 16 * h) * kVjpRow + lane;
-          row[0] = vx.x;
-          row[kVjpRow] = vx.y;
-          row[kVjpRows * kVjpRow] = vy.x;
-          row[(kVjpRows + 1) * kVjpRow] = vy.y;
-          row[2 * kVjpRows * kVjpRow] = vz.x;
-          row[(2 * kVjpRows + 1) * kVjpRow] = vz.y;
-          if (MB) {
-            row[3 * kVjpRows * kVjpRow] = mb2.x;
-            row[(3 * kVjpRows + 1) * kVjpRow] = mb2.y;
-          }
+      if (nbuf > 0) {
+        // the remainder, filled up with far-away massless entries
+        if (hw == 0 && el >= nbuf) {
+          ent[w][el][0] = make_float4(1e18f, 1e18f, 1e18f, 1e18f);
+          ent[w][el][1] = make_float4(1e18f, 1e18f, 0.f, 0.f);
+          ent_idx[w][el] = -2;
         }
         __syncwarp();
-        // entry side: lanes r and r + 16 sum the two halves of entry 16h + r's
-        // row of each component
-        const int er = lane & 15, e = 16 * h + er, part = lane >> 4;
-        float sum[NC];
-#pragma unroll
-        for (int c = 0; c < NC; ++c) {
-          const float4 *row =
-              reinterpret_cast<const float4 *>(tv + (c * kVjpRows + er) * kVjpRow) + 4 * part;
-          float2 s2 = make_float2(0.f, 0.f);
-#pragma unroll
-          for (int k = 0; k < 4; ++k) {
-            const float4 t = row[k];
-            s2 = __fadd2_rn(s2, __fadd2_rn(make_float2(t.x, t.y), make_float2(t.z, t.w)));
-          }
-          sum[c] = s2.x + s2.y;
-          sum[c] += __shfl_xor_sync(full, sum[c], 16);
-        }
-        if (part == 0 && e < ne) {
-          const int jt = bufI[w][e];
-          if (sum[0] != 0.f || sum[1] != 0.f || sum[2] != 0.f) {
-            atomicAdd(xbx + jt, sum[0]);
-            atomicAdd(xby + jt, sum[1]);
-            atomicAdd(xbz + jt, sum[2]);
-          }
-          if (MB && mbp && jt >= np && sum[NC - 1] != 0.f) atomicAdd(mbp + jt, sum[NC - 1]);
-        }
-        __syncwarp();
+        eval(0, nbuf);
       }
-      // keep what is past the first 32 (slot pairs 16.. move to 0..)
-      if (nbuf > 32) {
-        if (2 * lane < nbuf - 32) {
-          bufA[w][lane] = bufA[w][16 + lane];
-          bufB[w][lane] = bufB[w][16 + lane];
-        }
-        if (lane < nbuf - 32) bufI[w][lane] = bufI[w][32 + lane];
+      const float sx = half_sums(px, lane), sy = half_sums(py, lane), sz = half_sums(pz, lane);
+      const int q = (lane >> 2) & 3, p = 2 * (hw * steps + q) + ((lane >> 1) & 1);
+      const int po = __shfl_sync(full, pi, p & (kHalf - 1));
+      if (!(lane & 1) && q < steps && p < g) {
+        atomicAdd(xbx + po, -sx);
+        atomicAdd(xby + po, -sy);
+        atomicAdd(xbz + po, -sz);
       }
-      nbuf -= ne;
-      __syncwarp();
-      if (j0 >= len && nbuf == 0) break;
-    }
-    float sx = bx.x + bx.y, sy = by.x + by.y, sz = bz.x + bz.y;
-    if (hm) {
-      sx += __shfl_xor_sync(full, sx, 16);
-      sy += __shfl_xor_sync(full, sy, 16);
-      sz += __shfl_xor_sync(full, sz, 16);
-    }
-    if (act && half == 0) {
-      atomicAdd(xbx + pi, -sx);
-      atomicAdd(xby + pi, -sy);
-      atomicAdd(xbz + pi, -sz);
+      __syncwarp();  // the next half's particles take these ones' place
     }
   }
 }
 
 namespace {
-// Shared memory opt-in and resident CTAs of one VJP instantiation (cached
-// per device).
+// Resident CTAs of one VJP instantiation (cached per device).
 template <int LAW, bool MULTI, bool MB = false>
 int vjp_ctas(int64_t nitems) {
   constexpr int kDev = 64;
-  constexpr size_t smem = MB ? kVjpSmemMB : kVjpSmem;
   static int per[kDev] = {};
   int dev = 0;
   cudaGetDevice(&dev);
   int pc = dev >= 0 && dev < kDev ? per[dev] : 0;
   if (pc == 0) {
-    cudaFuncSetAttribute(k_pairs_vjp<LAW, MULTI, MB>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                         int(smem));
     cudaOccupancyMaxActiveBlocksPerMultiprocessor(&pc, k_pairs_vjp<LAW, MULTI, MB>,
-                                                  32 * kBatchedWarps, smem);
+                                                  32 * kBatchedWarps, 0);
     if (pc < 1) pc = 1;
     if (dev >= 0 && dev < kDev) per[dev] = pc;
   }
@@ -800,12 +718,12 @@ void vjp_single(const float4 *pos, const PairItem *items, int64_t nitems, const 
                 unsigned long long *queue, float *mb, int64_t npart, cudaStream_t s) {
   if (mb)
     k_pairs_vjp<LAW, false, true>
-        <<<vjp_ctas<LAW, false, true>(nitems), 32 * kBatchedWarps, kVjpSmemMB, s>>>(
+        <<<vjp_ctas<LAW, false, true>(nitems), 32 * kBatchedWarps, 0, s>>>(
             pos, items, nitems, gidx, idx, ux, uy, uz, xbx, xby, xbz, fcoeff, rsm2, rcut2, rcull2,
             queue, nullptr, mb, npart);
   else
     k_pairs_vjp<LAW, false>
-        <<<vjp_ctas<LAW, false>(nitems), 32 * kBatchedWarps, kVjpSmem, s>>>(
+        <<<vjp_ctas<LAW, false>(nitems), 32 * kBatchedWarps, 0, s>>>(
             pos, items, nitems, gidx, idx, ux, uy, uz, xbx, xby, xbz, fcoeff, rsm2, rcut2, rcull2,
             queue, nullptr);
 }
@@ -833,16 +751,16 @@ cudaError_t launch_pairs_vjp_multi(int law, const VjpBoxDesc *boxes, const PairI
                                    cudaStream_t s, bool mass_cotangents) {
   (void)ctas;
   if (nitems <= 0) return cudaSuccess;
-#define VJP_MULTI(L, MBV, SMEM)                                                                 \
-  k_pairs_vjp<L, true, MBV><<<vjp_ctas<L, true, MBV>(nitems), 32 * kBatchedWarps, SMEM, s>>>(  \
+#define VJP_MULTI(L, MBV)                                                                       \
+  k_pairs_vjp<L, true, MBV><<<vjp_ctas<L, true, MBV>(nitems), 32 * kBatchedWarps, 0, s>>>(     \
       nullptr, items, nitems, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr,   \
       nullptr, 0.f, 0.f, 0.f, 0.f, queue, boxes)
   if (law == LAW_POLY5_STEP16) {
-    if (mass_cotangents) VJP_MULTI(LAW_POLY5_STEP16, true, kVjpSmemMB);
-    else VJP_MULTI(LAW_POLY5_STEP16, false, kVjpSmem);
+    if (mass_cotangents) VJP_MULTI(LAW_POLY5_STEP16, true);
+    else VJP_MULTI(LAW_POLY5_STEP16, false);
   } else {
-    if (mass_cotangents) VJP_MULTI(LAW_POLY6, true, kVjpSmemMB);
-    else VJP_MULTI(LAW_POLY6, false, kVjpSmem);
+    if (mass_cotangents) VJP_MULTI(LAW_POLY6, true);
+    else VJP_MULTI(LAW_POLY6, false);
   }
 #undef VJP_MULTI
   return cudaGetLastError();

@@ -127,31 +127,6 @@ __device__ __forceinline__ float law_g(float r2, float rsm2) {
   return fmaf(y, y * y, neg_poly<LAW>(r2));
 }
 
-// -p'(r2), the derivative of the law's polynomial, negated.
-template <int LAW>
-__device__ __forceinline__ float neg_dpoly(float r2);
-
-template <>
-__device__ __forceinline__ float neg_dpoly<LAW_POLY6>(float r2) {
-  float q = -6.0f * static_cast<float>(0.000000147305);
-  q = fmaf(q, r2, -5.0f * static_cast<float>(-0.00000663394));
-  q = fmaf(q, r2, -4.0f * static_cast<float>(0.000132336));
-  q = fmaf(q, r2, -3.0f * static_cast<float>(-0.00159485));
-  q = fmaf(q, r2, -2.0f * static_cast<float>(0.0133122));
-  q = fmaf(q, r2, -static_cast<float>(-0.0783394));
-  return q;
-}
-
-template <>
-__device__ __forceinline__ float neg_dpoly<LAW_POLY5_STEP16>(float r2) {
-  float q = -5.0f * static_cast<float>(-0.00000147177);
-  q = fmaf(q, r2, -4.0f * static_cast<float>(0.0000605491));
-  q = fmaf(q, r2, -3.0f * static_cast<float>(-0.00109313));
-  q = fmaf(q, r2, -2.0f * static_cast<float>(0.0114808));
-  q = fmaf(q, r2, -static_cast<float>(-0.0750978));
-  return q;
-}
-
 // Whether a pair at squared distance r2 contributes (the reference's
 // updateq and the law's own range, folded into one strict threshold rcut2;
 // Step16_int also drops r2 == 0).
@@ -229,8 +204,8 @@ __device__ __forceinline__ void pair2_acc_s(float2 nxi, float2 nyi, float2 nzi, 
   az = __ffma2_rn(w, dz, az);
 }
 
-// -p(r2) and -p'(r2) of the law on two values at once (packed FP32), the
-// same coefficients and Horner order as neg_poly / neg_dpoly.
+// -p(r2) of the law on two values at once (packed FP32), the same coefficients
+// and Horner order as neg_poly.
 template <int LAW>
 __device__ __forceinline__ float2 neg_poly2(float2 r2);
 template <>
@@ -254,9 +229,10 @@ __device__ __forceinline__ float2 neg_poly2<LAW_POLY5_STEP16>(float2 r2) {
   for (int k = 1; k < 6; ++k) q = __ffma2_rn(q, r2, make_float2(c[k], c[k]));
   return q;
 }
-// -2 p'(r2) of the law on two values at once (packed FP32): neg_dpoly's
-// coefficients doubled (exactly) and its Horner order, so the result is
-// exactly twice neg_dpoly's.
+// -2 p'(r2) of the law on two values at once (packed FP32), Horner, on the
+// float coefficients times small whole numbers.  (Scaled by -1/3, which would
+// save the factor -3 of y^5, the rounded coefficients raise the gradient's
+// error against 64 bits by a tenth.)
 template <int LAW>
 __device__ __forceinline__ float2 neg_dpoly2_x2(float2 r2);
 template <>
@@ -283,40 +259,65 @@ __device__ __forceinline__ float2 neg_dpoly2_x2<LAW_POLY5_STEP16>(float2 r2) {
   return q;
 }
 
-// The adjoint pair term for two pairs at once: with e = x_j - x_i,
-// M = w (g I + 2 g' e e^T), w = w_i m_j, returns M u (u: particle i's
-// cotangent), zero where `on` is false.  Packed FP32 as pair2_acc_s.
-// With MB, *mb also receives the mass cotangent of the two entries,
-// d (u . dv_i) / d m_j = w_i g (d . u) (wi: fcoeff m_i, or fcoeff for Step16).
-template <int LAW, bool MB = false>
-__device__ __forceinline__ void vjp2_term(float2 ex, float2 ey, float2 ez, float2 w, float2 u0,
-                                          float2 u1, float2 u2, float rsm2, bool on_a, bool on_b,
-                                          float2 &vx, float2 &vy, float2 &vz,
-                                          float2 wi = make_float2(0.f, 0.f),
-                                          float2 *mb = nullptr) {
-  const float2 r2 = __ffma2_rn(ex, ex, __ffma2_rn(ey, ey, __fmul2_rn(ez, ez)));
+// A pair of particles of the adjoint kernel: negated positions, cotangents
+// times fcoeff m_i (fcoeff for Step16) and table indices, (first, second).
+struct alignas(16) VjpPair {
+  float4 nxy;   // -x, -x', -y, -y'
+  float4 nz_u;  // -z, -z', u_x, u_x'
+  float4 u;     // u_y, u_y', u_z, u_z'
+  int2 idx;
+  int2 pad;
+};
+
+// The adjoint pair terms of one list entry (m: its mass twice)
+// against a pair of particles, packed FP32 as pair2_acc_s.  With e = x_j - x_i,
+// a = m g and b = 2 m g' (e . u) the pair adds v = a u + b e to the entry and
+// subtracts it from the particle; zero outside the cutoff and for the entry's
+// own particle.  (ex, ey, ez) and (px, py, pz) are the sums of v for the entry
+// and for the particles.  (Sums of a and of b e for the particles need two
+// operations fewer and two registers a pair more: no faster.)  With MB, mb also
+// gets d (u . dv_i) / d m_j = g (e . u).
+template <int LAW, bool MB>
+__device__ __forceinline__ void vjp_pair_acc(const VjpPair &P, float2 x, float2 y, float2 z,
+                                             float2 m, int j, float rsm2, float rcut2,
+                                             float2 &ex, float2 &ey, float2 &ez, float2 &mb,
+                                             float2 &px, float2 &py, float2 &pz) {
+  const float4 nxy = P.nxy, nzu = P.nz_u, u = P.u;
+  const int2 pi = P.idx;
+  const float2 u0 = make_float2(nzu.z, nzu.w), u1 = make_float2(u.x, u.y), u2 = make_float2(u.z, u.w);
+  const float2 dx = __fadd2_rn(x, make_float2(nxy.x, nxy.y));
+  const float2 dy = __fadd2_rn(y, make_float2(nxy.z, nxy.w));
+  const float2 dz = __fadd2_rn(z, make_float2(nzu.x, nzu.y));
+  const float2 r2 = __ffma2_rn(dx, dx, __ffma2_rn(dy, dy, __fmul2_rn(dz, dz)));
+  const bool on_a = pi.x != j && in_range<LAW>(r2.x, rcut2);
+  const bool on_b = pi.y != j && in_range<LAW>(r2.y, rcut2);
   const float2 s = __fadd2_rn(r2, make_float2(rsm2, rsm2));
-  const float2 y = make_float2(rsqrt_ftz(s.x), rsqrt_ftz(s.y));
-  const float2 y2 = __fmul2_rn(y, y);
-  const float2 g = __ffma2_rn(y, y2, neg_poly2<LAW>(r2));
-  // 2 g': the factors 2 folded into the constants (exact)
-  const float2 gp2 = __ffma2_rn(__fmul2_rn(make_float2(-3.f, -3.f), y2), __fmul2_rn(y2, y),
-                                neg_dpoly2_x2<LAW>(r2));
-  const float2 du = __ffma2_rn(ex, u0, __ffma2_rn(ey, u1, __fmul2_rn(ez, u2)));
-  float2 a = __fmul2_rn(w, g);
-  float2 bq = __fmul2_rn(w, __fmul2_rn(gp2, du));
+  const float2 yy = make_float2(rsqrt_ftz(s.x), rsqrt_ftz(s.y));
+  const float2 y2 = __fmul2_rn(yy, yy);
+  const float2 g = __ffma2_rn(yy, y2, neg_poly2<LAW>(r2));
+  // 2 g': the factors 2 are in the coefficients
+  const float2 gp = __ffma2_rn(__fmul2_rn(make_float2(-3.f, -3.f), y2), __fmul2_rn(y2, yy),
+                               neg_dpoly2_x2<LAW>(r2));
+  const float2 du = __ffma2_rn(dx, u0, __ffma2_rn(dy, u1, __fmul2_rn(dz, u2)));
+  float2 a = __fmul2_rn(m, g);
+  float2 b = __fmul2_rn(m, __fmul2_rn(gp, du));
   a.x = on_a ? a.x : 0.f;
   a.y = on_b ? a.y : 0.f;
-  bq.x = on_a ? bq.x : 0.f;
-  bq.y = on_b ? bq.y : 0.f;
-  vx = __ffma2_rn(a, u0, __fmul2_rn(bq, ex));
-  vy = __ffma2_rn(a, u1, __fmul2_rn(bq, ey));
-  vz = __ffma2_rn(a, u2, __fmul2_rn(bq, ez));
+  b.x = on_a ? b.x : 0.f;
+  b.y = on_b ? b.y : 0.f;
+  const float2 vx = __ffma2_rn(a, u0, __fmul2_rn(b, dx));
+  const float2 vy = __ffma2_rn(a, u1, __fmul2_rn(b, dy));
+  const float2 vz = __ffma2_rn(a, u2, __fmul2_rn(b, dz));
+  ex = __fadd2_rn(ex, vx);
+  ey = __fadd2_rn(ey, vy);
+  ez = __fadd2_rn(ez, vz);
+  px = __fadd2_rn(px, vx);
+  py = __fadd2_rn(py, vy);
+  pz = __fadd2_rn(pz, vz);
   if (MB) {
-    float2 t = __fmul2_rn(__fmul2_rn(wi, g), du);
-    t.x = on_a ? t.x : 0.f;
-    t.y = on_b ? t.y : 0.f;
-    *mb = t;
+    const float2 t = __fmul2_rn(g, du);
+    mb.x += on_a ? t.x : 0.f;
+    mb.y += on_b ? t.y : 0.f;
   }
 }
 
