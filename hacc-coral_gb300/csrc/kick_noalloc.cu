@@ -28,21 +28,19 @@ constexpr size_t kItemsOffset = 256;
 constexpr int64_t kMaxItems = int64_t((kScratchBytes - kItemsOffset) / sizeof(hsr::PairItem));
 // Longest list range of one item; longer lists are split over several items.
 constexpr int64_t kSplit = 8192;
-constexpr int kWarps = 8;
 
 static __device__ __align__(256) unsigned char g_scratch[kScratchBytes];
 
 struct ScratchHead {
   unsigned long long queue;      // next item to take
   unsigned long long evaluated;  // pairs evaluated after the box test
-  unsigned long long reserved;   // items reserved by the builder
-  unsigned int overflow;         // set when the items do not fit
+  hsr::BuiltItems built;         // items reserved by the builder
 };
 
-__device__ __forceinline__ ScratchHead *head(unsigned char *scr) {
+__host__ __device__ __forceinline__ ScratchHead *head(unsigned char *scr) {
   return reinterpret_cast<ScratchHead *>(scr);
 }
-__device__ __forceinline__ hsr::PairItem *item_at(unsigned char *scr, int64_t i) {
+__host__ __device__ __forceinline__ hsr::PairItem *item_at(unsigned char *scr, int64_t i) {
   return reinterpret_cast<hsr::PairItem *>(scr + kItemsOffset) + i;
 }
 
@@ -58,9 +56,9 @@ __global__ void k_noalloc_items(unsigned char *scr, const int32_t *leaf_offset,
   const int64_t nch = (int64_t(len) + kSplit - 1) / kSplit;
   const int32_t ng = (cnt + 31) / 32;
   const int64_t need = nch * ng;
-  const unsigned long long at = atomicAdd(&head(scr)->reserved, (unsigned long long)need);
+  const unsigned long long at = atomicAdd(&head(scr)->built.count, (unsigned long long)need);
   if (int64_t(at) + need > kMaxItems) {
-    atomicExch(&head(scr)->overflow, 1u);
+    atomicExch(&head(scr)->built.overflow, 1u);
     return;
   }
   int64_t k = int64_t(at);
@@ -74,78 +72,6 @@ __global__ void k_noalloc_items(unsigned char *scr, const int32_t *leaf_offset,
       it.flags = nch > 1 ? 1 : 0;
       *item_at(scr, k++) = it;
     }
-}
-
-// The batched pair kernel (sr_kernels.cu, k_pairs_batched) with its items and
-// counters in the scratch array and groups of consecutive particles.
-template <int LAW>
-__global__ void __launch_bounds__(32 * kWarps)
-    k_noalloc_pairs(unsigned char *scr, const float4 *__restrict__ table,
-                    const int32_t *__restrict__ idx,
-                    float *__restrict__ vx, float *__restrict__ vy, float *__restrict__ vz,
-                    float fcoeff, float rsm2, float rcut2, float rcull2) {
-  __shared__ float4 slot[kWarps][32];
-  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-  const unsigned full = 0xffffffffu;
-  // items that did not fit: no pair is evaluated, the velocities stay as
-  // they are and the host reports the overflow
-  if (head(scr)->overflow) return;
-  const unsigned long long nitems = head(scr)->reserved;
-  unsigned long long evaluated = 0;
-  for (;;) {
-    unsigned long long it = 0;
-    if (lane == 0) it = atomicAdd(&head(scr)->queue, 1ull);
-    it = __shfl_sync(full, it, 0);
-    if (it >= nitems) break;
-    const hsr::PairItem W = *item_at(scr, int64_t(it));
-    const bool act = lane < W.g_count;
-    const int pi = W.g_begin + (act ? lane : 0);
-    const float4 P = table[pi];
-    float lox = P.x, hix = P.x, loy = P.y, hiy = P.y, loz = P.z, hiz = P.z;
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-      lox = fminf(lox, __shfl_xor_sync(full, lox, o));
-      hix = fmaxf(hix, __shfl_xor_sync(full, hix, o));
-      loy = fminf(loy, __shfl_xor_sync(full, loy, o));
-      hiy = fmaxf(hiy, __shfl_xor_sync(full, hiy, o));
-      loz = fminf(loz, __shfl_xor_sync(full, loz, o));
-      hiz = fmaxf(hiz, __shfl_xor_sync(full, hiz, o));
-    }
-    float ax = 0.f, ay = 0.f, az = 0.f;
-    const int32_t *lst = idx + W.j_begin;
-    for (int j0 = 0; j0 < W.j_len; j0 += 32) {
-      const int j = j0 + lane;
-      const bool ok = j < W.j_len;
-      const float4 J = table[lst[ok ? j : 0]];
-      const float dx = fmaxf(fmaxf(lox - J.x, J.x - hix), 0.f);
-      const float dy = fmaxf(fmaxf(loy - J.y, J.y - hiy), 0.f);
-      const float dz = fmaxf(fmaxf(loz - J.z, J.z - hiz), 0.f);
-      unsigned keep = __ballot_sync(full, ok && fmaf(dx, dx, fmaf(dy, dy, dz * dz)) < rcull2);
-      if (!keep) continue;
-      evaluated += (unsigned long long)__popc(keep) * (unsigned long long)W.g_count;
-      slot[w][lane] = J;
-      __syncwarp();
-      while (keep) {
-        const int b = __ffs(keep) - 1;
-        keep &= keep - 1;
-        hsr::pair_acc<LAW>(P.x, P.y, P.z, slot[w][b], rsm2, rcut2, ax, ay, az);
-      }
-      __syncwarp();
-    }
-    if (act) {
-      const float c = (LAW == hsr::LAW_POLY5_STEP16) ? fcoeff : fcoeff * P.w;
-      if (W.flags & 1) {
-        atomicAdd(vx + pi, c * ax);
-        atomicAdd(vy + pi, c * ay);
-        atomicAdd(vz + pi, c * az);
-      } else {
-        vx[pi] += c * ax;
-        vy[pi] += c * ay;
-        vz[pi] += c * az;
-      }
-    }
-  }
-  if (lane == 0 && evaluated) atomicAdd(&head(scr)->evaluated, evaluated);
 }
 
 // The device address of g_scratch.  In host code the name g_scratch is only a
@@ -214,29 +140,17 @@ extern "C" hsr_status hsr_kick_lists_noalloc(const float *table, int64_t ntab, i
   // persistent grid from the SM count and occupancy alone: the pair kernel
   // reads the item count (and the overflow flag) on the device, and CTAs
   // beyond the work exit at their first queue read
-  int sms = 0, per = 0;
-  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-  if (law == HSR_LAW_POLY5_STEP16)
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_noalloc_pairs<hsr::LAW_POLY5_STEP16>,
-                                                  32 * kWarps, 0);
-  else
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_noalloc_pairs<hsr::LAW_POLY6>,
-                                                  32 * kWarps, 0);
-  const int64_t ctas = int64_t(sms > 0 ? sms : 1) * (per > 0 ? per : 1);
-  const float4 *tab = reinterpret_cast<const float4 *>(table);
-  if (law == HSR_LAW_POLY5_STEP16)
-    k_noalloc_pairs<hsr::LAW_POLY5_STEP16><<<unsigned(ctas), 32 * kWarps, 0, s>>>(
-        scr, tab, list_index, vx, vy, vz, fcoeff, rsm * rsm, rc2, rcull2);
-  else
-    k_noalloc_pairs<hsr::LAW_POLY6><<<unsigned(ctas), 32 * kWarps, 0, s>>>(
-        scr, tab, list_index, vx, vy, vz, fcoeff, rsm * rsm, rc2, rcull2);
-  if (cudaGetLastError() != cudaSuccess) return HSR_ERR_CUDA;
+  if (hsr::launch_pairs_batched_built(law, reinterpret_cast<const float4 *>(table), item_at(scr, 0),
+                                      &head(scr)->built, list_index, vx, vy, vz, fcoeff, rsm * rsm,
+                                      rc2, rcull2, &head(scr)->queue,
+                                      hsr::batched_resident_ctas(dev), s) != cudaSuccess)
+    return HSR_ERR_CUDA;
   // the overflow flag comes back once the kernels are done (a copy into host
   // stack memory, which waits for the stream)
   ScratchHead h{};
   if (cudaMemcpyAsync(&h, base, sizeof(h), cudaMemcpyDeviceToHost, s) != cudaSuccess ||
       cudaStreamSynchronize(s) != cudaSuccess)
     return HSR_ERR_CUDA;
-  if (h.overflow) return HSR_ERR_ARG;  // more work items than the fixed array holds
+  if (h.built.overflow) return HSR_ERR_ARG;  // more work items than the fixed array holds
   return HSR_OK;
 }

@@ -51,6 +51,13 @@ struct alignas(16) PairItem {
   int64_t pad;
 };
 
+// How many items a kernel has built, for a launch sized before they are
+// counted; overflow: they did not fit, and nothing is to be evaluated.
+struct BuiltItems {
+  unsigned long long count;
+  unsigned int overflow;
+};
+
 // The law in terms of s = r2 + rsm^2, for the batched kernel: g = s^-3/2 +
 // q(s) with q(s) = -p(s - rsm^2) re-expanded in s (nb[k], computed in double
 // and rounded), and the cutoff as s < scut (scut = rcut2 + rsm^2 in float).
@@ -229,6 +236,27 @@ __device__ __forceinline__ float2 neg_poly2<LAW_POLY5_STEP16>(float2 r2) {
   for (int k = 1; k < 6; ++k) q = __ffma2_rn(q, r2, make_float2(c[k], c[k]));
   return q;
 }
+// pair2_acc_s with the law in r2, on its own coefficients: one operation more,
+// the error of the scalar pair_acc.
+template <int LAW>
+__device__ __forceinline__ void pair2_acc(float2 nxi, float2 nyi, float2 nzi, const float4 A,
+                                          const float4 B, float rsm2, float rcut2, float2 &ax,
+                                          float2 &ay, float2 &az) {
+  const float2 dx = __fadd2_rn(make_float2(A.x, A.y), nxi);
+  const float2 dy = __fadd2_rn(make_float2(A.z, A.w), nyi);
+  const float2 dz = __fadd2_rn(make_float2(B.x, B.y), nzi);
+  const float2 r2 = __ffma2_rn(dx, dx, __ffma2_rn(dy, dy, __fmul2_rn(dz, dz)));
+  const float2 s = __fadd2_rn(r2, make_float2(rsm2, rsm2));
+  const float2 y = make_float2(rsqrtf(s.x), rsqrtf(s.y));
+  const float2 g = __ffma2_rn(y, __fmul2_rn(y, y), neg_poly2<LAW>(r2));
+  float2 w = __fmul2_rn(make_float2(B.z, B.w), g);
+  w.x = in_range<LAW>(r2.x, rcut2) ? w.x : 0.f;
+  w.y = in_range<LAW>(r2.y, rcut2) ? w.y : 0.f;
+  ax = __ffma2_rn(w, dx, ax);
+  ay = __ffma2_rn(w, dy, ay);
+  az = __ffma2_rn(w, dz, az);
+}
+
 // -2 p'(r2) of the law on two values at once (packed FP32), Horner, on the
 // float coefficients times small whole numbers.  (Scaled by -1/3, which would
 // save the factor -3 of y^5, the rounded coefficients raise the gradient's
@@ -363,6 +391,13 @@ cudaError_t launch_pairs_batched(int law, int group, const float4 *pos, const Pa
                                  float *vx, float *vy, float *vz, float fcoeff, float rsm2,
                                  float rcut2, float rcull2, unsigned long long *queue, int ctas,
                                  cudaStream_t s);
+// The batched kernel over items that the device counts (*built), each a group
+// of at most 32 consecutive particles, with `ctas` CTAs.
+cudaError_t launch_pairs_batched_built(int law, const float4 *pos, const PairItem *items,
+                                       const BuiltItems *built, const int32_t *idx, float *vx,
+                                       float *vy, float *vz, float fcoeff, float rsm2, float rcut2,
+                                       float rcull2, unsigned long long *queue, int ctas,
+                                       cudaStream_t s);
 // The batched kernel over the items of several boxes (items of box b carry
 // b << 8 in flags), one persistent launch; queue as above.
 cudaError_t launch_pairs_batched_multi(int law, int group, const BoxDesc *boxes,
