@@ -1,6 +1,7 @@
 // rcb_device.cu -- RCB tree, interaction lists and batched work items built on
 // the GPU (see rcb_device.cuh for the method).
 #include "rcb_device.cuh"
+#include "chain.cuh"
 #include "device_info.cuh"
 
 #include <algorithm>
@@ -74,6 +75,7 @@ constexpr int64_t kScanBlock = kScanThreads * kScanPer;
 
 __global__ void __launch_bounds__(kScanThreads)
     k_scan_block(const int64_t *in, int64_t *out, int64_t n, int64_t *bsum, int64_t *total) {
+  chain_enter();
   __shared__ int64_t wsum[32];
   const int64_t base = int64_t(blockIdx.x) * kScanBlock + int64_t(threadIdx.x) * kScanPer;
   int64_t v[kScanPer];
@@ -116,6 +118,7 @@ __global__ void __launch_bounds__(kScanThreads)
 }
 
 __global__ void k_scan_add(int64_t *out, int64_t n, const int64_t *boff) {
+  chain_enter();
   const int64_t i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
   if (i < n) out[i] += boff[i / kScanBlock];
 }
@@ -135,12 +138,13 @@ cudaError_t exclusive_scan_i64(const int64_t *in, int64_t *out, int64_t n, int64
     return cudaSuccess;
   }
   const int64_t nb = (n + kScanBlock - 1) / kScanBlock;
-  k_scan_block<<<unsigned(nb), kScanThreads, 0, s>>>(in, out, n, tmp, nb == 1 ? total : nullptr);
+  launch_chained(k_scan_block, unsigned(nb), kScanThreads, 0, s, in, out, n, tmp,
+                 nb == 1 ? total : nullptr);
   if (nb == 1) return cudaGetLastError();
   // scan the block sums in place, then add them
   cudaError_t e = exclusive_scan_i64(tmp, tmp, nb, total, tmp + nb + 1, s);
   if (e != cudaSuccess) return e;
-  k_scan_add<<<unsigned((n + 255) / 256), 256, 0, s>>>(out, n, tmp);
+  launch_chained(k_scan_add, unsigned((n + 255) / 256), 256, 0, s, out, n, tmp);
   return cudaGetLastError();
 }
 
@@ -192,6 +196,7 @@ constexpr int64_t kScanPairMax = 4 * kScanBlock;
 __global__ void __launch_bounds__(kScanThreads)
     k_scan_pair(const int64_t *a, const int64_t *b, int64_t *oa, int64_t *ob, int64_t n,
                 int64_t *ta, int64_t *tb) {
+  chain_enter();
   int64_t ca = 0, cb = 0;
   for (int64_t base = 0; base < n; base += kScanBlock) {
     const int64_t i0 = base + int64_t(threadIdx.x) * kScanPer;
@@ -797,6 +802,7 @@ __device__ __forceinline__ void tighten(NodeSums &S, const int *low, const NodeA
 __global__ void __launch_bounds__(256)
     k_elements(const float4 *__restrict__ in, int64_t n, float4 *__restrict__ pos,
                int32_t *__restrict__ oid, LevelCtl *ctl) {
+  chain_enter();
   unsigned mt = 0, mm = 0, mn = 0xffffffffu;
   for (int64_t i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x; i < n;
        i += int64_t(gridDim.x) * blockDim.x) {
@@ -833,6 +839,7 @@ template <int PT>
 __global__ void __launch_bounds__(256)
     k_root(DNode *nodes, int64_t n, TreeConfig cfg, LevelCtl *ctl, int32_t *chunk_node,
            int32_t *chunk_base, NodeAcc *acc, unsigned *ticket, int2 *roots, int32_t sub_max) {
+  chain_enter();
   const int32_t nc = chunks_of<PT>(int32_t(n));
   const bool sub = n <= sub_max;
   if (!sub)
@@ -872,6 +879,7 @@ __global__ void __launch_bounds__(kChunkThreads)
                   const int32_t *__restrict__ chunk_node, const int32_t *__restrict__ chunk_base,
                   NodeAcc *acc, unsigned *ticket, int32_t *fallback, int64_t *counters,
                   int32_t force_fallback, int32_t nd) {
+  chain_enter();
   LevelSpan L;
   if (!level_runs(ctl, level, L, true) || int32_t(blockIdx.x) >= L.nchunk) return;
   constexpr int kW = kChunkThreads / 32, kU = 4;
@@ -945,6 +953,7 @@ __global__ void __launch_bounds__(kChunkThreads)
                   int32_t *next_chunk_node, int32_t *next_chunk_base, int32_t *left_cnt,
                   int32_t *left_base, int32_t *wpre, NodeAcc *acc, unsigned *ticket, int2 *roots,
                   int64_t *counters, int32_t sub_max) {
+  chain_enter();
   LevelSpan L;
   if (!level_runs(ctl, level, L) || int32_t(blockIdx.x) >= L.nchunk) return;
   constexpr int kWarps = kChunkThreads / 32, kSub = 32 * PT;
@@ -1080,6 +1089,7 @@ __global__ void __launch_bounds__(kChunkThreads)
                 const LevelCtl *ctl, int32_t level, const int32_t *__restrict__ chunk_node,
                 const int32_t *__restrict__ chunk_base, const int32_t *left_base,
                 const int32_t *wpre, float4 *tpos, int32_t *toid, int32_t *idx, int32_t *ridx) {
+  chain_enter();
   LevelSpan L;
   if (!level_runs(ctl, level, L) || int32_t(blockIdx.x) >= L.nchunk) return;
   constexpr int kWarps = kChunkThreads / 32;
@@ -1190,6 +1200,7 @@ __global__ void __launch_bounds__(kChunkThreads)
                  const int32_t *__restrict__ chunk_base, const int32_t *__restrict__ idx,
                  float4 *tpos, int32_t *toid, int32_t *err,
                  int64_t *counters, ChainItem *chains, int64_t chain_cap) {
+  chain_enter();
   LevelSpan L;
   if (!level_runs(ctl, level, L) || int32_t(blockIdx.x) >= L.nchunk) return;
   constexpr int NT = kChunkThreads;
@@ -1286,6 +1297,7 @@ __global__ void __launch_bounds__(256)
                   const DNode *nodes, const LevelCtl *ctl, int32_t level,
                   const ChainItem *__restrict__ chains, int64_t chain_cap, const int64_t *counters, const int32_t *__restrict__ idx,
                   const int32_t *__restrict__ ridx, float4 *tpos, int32_t *toid, int32_t *err) {
+  chain_enter();
   LevelSpan L;
   if (!level_runs(ctl, level, L)) return;
   const int64_t nq = min64(counters[C_CHAINS], chain_cap);
@@ -1671,6 +1683,7 @@ __global__ void __launch_bounds__(kSubThreads, 1)
               float4 *pos_a, int32_t *oid_a, const float4 *pos_b, const int32_t *oid_b, DNode *sub,
               int32_t *sub_first, int32_t *hist, int32_t cap, int32_t force_fallback, int32_t nd,
               int64_t *counters) {
+  chain_enter();
   extern __shared__ float4 P[];  // positions by input slot; then the 16-bit tables
   uint16_t *cur = reinterpret_cast<uint16_t *>(P + cap);  // input slot by position
   uint16_t *nxt = cur + cap;
@@ -2068,6 +2081,7 @@ __global__ void __launch_bounds__(kSubThreads, 1)
 // among that depth's (exclusive scan over the roots) and the depth's total.
 __global__ void __launch_bounds__(kScanThreads)
     k_subtree_scan(const LevelCtl *ctl, int32_t *hist, int32_t max_roots, int64_t *tot) {
+  chain_enter();
   __shared__ int sh_warp[32];
   int32_t *row = hist + int64_t(blockIdx.x) * max_roots;
   const int32_t nr = ctl->done && !ctl->abort ? ctl->nroots : 0;
@@ -2092,6 +2106,7 @@ __global__ void __launch_bounds__(256)
     k_subtree_place(DNode *nodes, const LevelCtl *ctl, const int2 *__restrict__ roots,
                     const DNode *sub, const int32_t *sub_first,
                     const int32_t *pos, int32_t max_roots, const int64_t *tot, int64_t node_cap) {
+  chain_enter();
   __shared__ int fs[kSubDepth + 2];
   __shared__ int64_t base[kSubDepth + 1];
   const int32_t r = int32_t(blockIdx.x);
@@ -2225,6 +2240,7 @@ __device__ __forceinline__ bool leaf_in_force_box(const DNode &T, const TreeConf
 // marks a left child (its sibling is t + 1: children are made in pairs).
 constexpr int kLeftChild = 0x100;
 __global__ void k_links(const DNode *nodes, int32_t nnodes, int2 *up) {
+  chain_enter();
   const int32_t t = blockIdx.x * blockDim.x + threadIdx.x;
   if (t >= nnodes) return;
   const int32_t cl = nodes[t].cl;
@@ -2250,6 +2266,7 @@ template <int K>
 __global__ void __launch_bounds__(128)
     k_pseudo_up(DNode *nodes, int32_t nnodes, int2 *up, const float4 *__restrict__ pos, float *ppm,
                 float4 *table, int64_t n, TreeConfig cfg, int32_t *processed) {
+  chain_enter();
   const unsigned full = 0xffffffffu;
   const int lane = threadIdx.x & 31;
   int32_t t = int32_t((int64_t(blockIdx.x) * blockDim.x + threadIdx.x) >> 5);
@@ -2337,6 +2354,7 @@ __global__ void __launch_bounds__(128)
 // ---------------------------------------------------------------------------
 __global__ void k_leaf_rank(const DNode *nodes, int32_t nnodes, const int2 *up,
                             const int32_t *processed, int32_t *leaf_ids, int64_t *counters) {
+  chain_enter();
   const int32_t t0 = blockIdx.x * blockDim.x + threadIdx.x;
   if (t0 >= nnodes) return;
   if (t0 == 0) counters[C_NLEAF] = processed[0];
@@ -2379,6 +2397,7 @@ __global__ void __launch_bounds__(32 * kWalkWarps)
            int64_t max_leaves, TreeConfig cfg, int64_t n, int64_t *seg_cnt, int64_t *list_len,
            const int64_t *seg_base, const int64_t *list_base, SegDesc *segs, int2 *local,
            int32_t *err, int64_t *counters) {
+  chain_enter();
   static_assert(MODE == 1 || MODE == 2, "walk mode");
   // entries: a node still to decide (x = node, y = 0, or -1 for a child of an
   // ancestor of the leaf, which no distance test drops), or a finished segment
@@ -2552,6 +2571,7 @@ __global__ void __launch_bounds__(256)
                     const int32_t *__restrict__ leaf_ids, int64_t nleaves,
                     const float4 *__restrict__ table, float cull2, int32_t *__restrict__ idx,
                     int64_t *__restrict__ kept) {
+  chain_enter();
   constexpr int kU = 4;
   const unsigned full = 0xffffffffu;
   const int lane = threadIdx.x & 31;
@@ -2917,6 +2937,7 @@ __global__ void __launch_bounds__(128)
     k_leaf_items(const DNode *nodes, const int32_t *leaf_ids, int64_t nleaves,
                  const int64_t *list_len, const int64_t *kept_len, const int64_t *list_base,
                  LeafDesc *ld, int64_t jsplit, int G, int64_t *counters) {
+  chain_enter();
   __shared__ unsigned long long hist[32];
   __shared__ bool last;
   if (threadIdx.x < 32) hist[threadIdx.x] = 0;
@@ -2979,6 +3000,7 @@ __global__ void __launch_bounds__(128)
 __global__ void __launch_bounds__(128)
     k_item_fill(const LeafDesc *ld, int64_t nleaves, int64_t jsplit, int G, int64_t *counters,
                 PairItem *items) {
+  chain_enter();
   // positions inside the block's share of each bucket, then one global
   // reservation a bucket
   __shared__ unsigned long long cnt[32], base[32];
@@ -3020,6 +3042,7 @@ __global__ void __launch_bounds__(128)
 __global__ void k_gather3_f32(const float *__restrict__ a, const float *__restrict__ b,
                               const float *__restrict__ c, const int32_t *__restrict__ perm,
                               float *out, int64_t stride, int64_t n) {
+  chain_enter();
   for (int64_t i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x; i < n;
        i += int64_t(gridDim.x) * blockDim.x) {
     const int32_t j = perm[i];
@@ -3038,6 +3061,7 @@ template <bool TABLE>
 __global__ void k_outputs(KickArrays in, const float4 *__restrict__ table,
                           const int32_t *__restrict__ perm, float *__restrict__ vel, KickArrays out,
                           int64_t n) {
+  chain_enter();
   for (int64_t i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x; i < n;
        i += int64_t(gridDim.x) * blockDim.x) {
     const int32_t j = perm[i];
@@ -3065,6 +3089,7 @@ __global__ void k_outputs(KickArrays in, const float4 *__restrict__ table,
 // were a tenth of the call).
 __global__ void k_finish(const float4 *__restrict__ table, const float *__restrict__ vel,
                          KickArrays st, KickArrays out, int64_t n) {
+  chain_enter();
   for (int64_t i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x; i < n;
        i += int64_t(gridDim.x) * blockDim.x) {
     const float4 p = table[i];
@@ -3086,6 +3111,7 @@ __global__ void k_finish(const float4 *__restrict__ table, const float *__restri
 
 __global__ void k_pack4(const float *x, const float *y, const float *z, const float *m, float4 *out,
                         int64_t n) {
+  chain_enter();
   for (int64_t i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x; i < n;
        i += int64_t(gridDim.x) * blockDim.x)
     out[i] = make_float4(x[i], y[i], z[i], m[i]);
@@ -3098,6 +3124,7 @@ template <bool ADD>
 __global__ void k_scatter3_f32(const float *__restrict__ in, int64_t stride,
                                const int32_t *__restrict__ perm, float *o0, float *o1, float *o2,
                                int64_t n) {
+  chain_enter();
   for (int64_t i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x; i < n;
        i += int64_t(gridDim.x) * blockDim.x) {
     const int32_t j = perm[i];
@@ -3457,7 +3484,8 @@ cudaError_t DeviceTree::build(const TreeConfig &cfg, int64_t n, const float4 *po
   const size_t want_nodes = size_t(std::max<int64_t>(64, 4 * n / std::max(1, cfg.nd) + 64));
   DT_CHECK(grow(nodes_, cap_nodes_, want_nodes, s));
   if (n > 0) {
-    k_elements<<<grid_for(n, 256, int64_t(sm_count()) * 8), 256, 0, s>>>(pos_in, n, epos_, oid_, ctl);
+    launch_chained(k_elements, grid_for(n, 256, int64_t(sm_count()) * 8), 256, 0, s, pos_in, n,
+                   epos_, oid_, ctl);
     ++info_.launches;
   }
 
@@ -3471,8 +3499,8 @@ cudaError_t DeviceTree::build(const TreeConfig &cfg, int64_t n, const float4 *po
   const int64_t chunk = small ? chunk_size<4>() : chunk_size<16>();
 #define LEVEL_LAUNCH(kern, grid, ...)                                             \
   do {                                                                            \
-    if (small) kern<4><<<grid, kChunkThreads, 0, s>>>(__VA_ARGS__);               \
-    else kern<16><<<grid, kChunkThreads, 0, s>>>(__VA_ARGS__);                    \
+    if (small) launch_chained(kern<4>, grid, kChunkThreads, 0, s, __VA_ARGS__);   \
+    else launch_chained(kern<16>, grid, kChunkThreads, 0, s, __VA_ARGS__);        \
     ++info_.launches;                                                             \
   } while (0)
   std::vector<int32_t> level_begin{0};
@@ -3531,9 +3559,9 @@ cudaError_t DeviceTree::build(const TreeConfig &cfg, int64_t n, const float4 *po
       LEVEL_LAUNCH(k_part_right, grid, pb[from], ob[from], nodes_, ctl, l, cn[from], cb[from], idx_,
                    pb[to], ob[to], walk_err_, counters_, reinterpret_cast<ChainItem *>(chains_),
                    int64_t(cap_ch_));
-      k_part_chains<<<unsigned(4 * sm_count()), 256, 0, s>>>(
-          pb[from], ob[from], nodes_, ctl, l, reinterpret_cast<const ChainItem *>(chains_),
-          int64_t(cap_ch_), counters_, idx_, ridx_, pb[to], ob[to], walk_err_);
+      launch_chained(k_part_chains, unsigned(4 * sm_count()), 256, 0, s, pb[from], ob[from], nodes_,
+                     ctl, l, reinterpret_cast<const ChainItem *>(chains_), int64_t(cap_ch_),
+                     counters_, idx_, ridx_, pb[to], ob[to], walk_err_);
       ++info_.launches;
     }
     if (subtrees) {
@@ -3541,13 +3569,14 @@ cudaError_t DeviceTree::build(const TreeConfig &cfg, int64_t n, const float4 *po
       DT_CHECK(grow(sub_first_, cap_sf_, size_t(max_roots) * (kSubDepth + 2), s));
       DT_CHECK(grow(sub_hist_, cap_sh_, size_t(max_roots) * kSubDepth, s));
       const int32_t cap = int32_t((std::min<int64_t>(n, sub_max) + 7) & ~int64_t(7));
-      k_subtree<<<unsigned(max_roots), kSubThreads, size_t(cap) * kSubBytes, s>>>(
-          nodes_, ctl, roots_, epos_, oid_, tpos_, toid_, sub_nodes_, sub_first_, sub_hist_, cap,
-          cfg.force_cm_fallback, cfg.nd, counters_);
-      k_subtree_scan<<<kSubDepth, kScanThreads, 0, s>>>(ctl, sub_hist_, int32_t(max_roots), sub_tot_);
-      k_subtree_place<<<unsigned(max_roots), 256, 0, s>>>(nodes_, ctl, roots_, sub_nodes_, sub_first_,
-                                                          sub_hist_, int32_t(max_roots), sub_tot_,
-                                                          int64_t(cap_nodes_));
+      launch_chained(k_subtree, unsigned(max_roots), kSubThreads, size_t(cap) * kSubBytes, s,
+                     nodes_, ctl, roots_, epos_, oid_, tpos_, toid_, sub_nodes_, sub_first_,
+                     sub_hist_, cap, cfg.force_cm_fallback, cfg.nd, counters_);
+      launch_chained(k_subtree_scan, kSubDepth, kScanThreads, 0, s, ctl, sub_hist_,
+                     int32_t(max_roots), sub_tot_);
+      launch_chained(k_subtree_place, unsigned(max_roots), 256, 0, s, nodes_, ctl, roots_,
+                     sub_nodes_, sub_first_, sub_hist_, int32_t(max_roots), sub_tot_,
+                     int64_t(cap_nodes_));
       info_.launches += 3;
       DT_CHECK(cudaMemcpyAsync(h_sub_, sub_tot_, kSubDepth * sizeof(int64_t), cudaMemcpyDeviceToHost, s));
     }
@@ -3603,9 +3632,9 @@ cudaError_t DeviceTree::build(const TreeConfig &cfg, int64_t n, const float4 *po
       if (total > INT32_MAX) return cudaErrorInvalidValue;
       if (size_t(total) > cap_nodes_) {
         DT_CHECK(grow(nodes_, cap_nodes_, size_t(total), s, true));
-        k_subtree_place<<<unsigned(max_roots), 256, 0, s>>>(nodes_, ctl, roots_, sub_nodes_, sub_first_,
-                                                            sub_hist_, int32_t(max_roots), sub_tot_,
-                                                            int64_t(cap_nodes_));
+        launch_chained(k_subtree_place, unsigned(max_roots), 256, 0, s, nodes_, ctl, roots_,
+                       sub_nodes_, sub_first_, sub_hist_, int32_t(max_roots), sub_tot_,
+                       int64_t(cap_nodes_));
         ++info_.launches;
         DT_CHECK(cudaGetLastError());
       }
@@ -3643,12 +3672,14 @@ cudaError_t DeviceTree::build(const TreeConfig &cfg, int64_t n, const float4 *po
   if (n > 0)
     DT_CHECK(cudaMemcpyAsync(table_, epos_, size_t(n) * sizeof(float4), cudaMemcpyDeviceToDevice, s));
   const unsigned gN = unsigned((nnodes + 127) / 128), gP = unsigned((int64_t(nnodes) * 32 + 127) / 128);
-  k_links<<<gN, 128, 0, s>>>(nodes_, nnodes, up_);
+  launch_chained(k_links, gN, 128, 0, s, nodes_, nnodes, up_);
   if (k == 12)
-    k_pseudo_up<12><<<gP, 128, 0, s>>>(nodes_, nnodes, up_, epos_, ppm_, table_, n, cfg, processed_);
+    launch_chained(k_pseudo_up<12>, gP, 128, 0, s, nodes_, nnodes, up_, epos_, ppm_, table_, n, cfg,
+                   processed_);
   else
-    k_pseudo_up<1><<<gP, 128, 0, s>>>(nodes_, nnodes, up_, epos_, ppm_, table_, n, cfg, processed_);
-  k_leaf_rank<<<gN, 128, 0, s>>>(nodes_, nnodes, up_, processed_, leaf_ids_, counters_);
+    launch_chained(k_pseudo_up<1>, gP, 128, 0, s, nodes_, nnodes, up_, epos_, ppm_, table_, n, cfg,
+                   processed_);
+  launch_chained(k_leaf_rank, gN, 128, 0, s, nodes_, nnodes, up_, processed_, leaf_ids_, counters_);
   info_.launches += 3;
   DT_CHECK(cudaGetLastError());
   // the groups need only the leaves: on the second stream, beside the walk
@@ -3674,17 +3705,17 @@ cudaError_t DeviceTree::build(const TreeConfig &cfg, int64_t n, const float4 *po
   // build to a second, placing walk)
   DT_CHECK(grow(segs_local_, cap_segl_, nlw * kLocalSegs, s));
   DT_CHECK(cudaMemsetAsync(counters_ + C_SEGOVF, 0, sizeof(int64_t), s));
-  k_walk<2><<<unsigned((max_leaves + kWalkWarps - 1) / kWalkWarps), 32 * kWalkWarps, 0, s>>>(
-      nodes_, nnodes, leaf_ids_, max_leaves, cfg, n, seg_cnt, list_len, nullptr, nullptr, nullptr,
-      segs_local_, walk_err_, counters_);
+  launch_chained(k_walk<2>, unsigned((max_leaves + kWalkWarps - 1) / kWalkWarps), 32 * kWalkWarps,
+                 0, s, nodes_, nnodes, leaf_ids_, max_leaves, cfg, n, seg_cnt, list_len, nullptr,
+                 nullptr, nullptr, segs_local_, walk_err_, counters_);
   ++info_.launches;
   // the groups after the walk's blocks, which then have their SMs first
   DT_CHECK(launch_groups(max_leaves, group_, aux_));
   DT_CHECK(cudaEventRecord(ev_groups_, aux_));
   groups_ready_ = group_;
   if (max_leaves <= kScanPairMax) {
-    k_scan_pair<<<1, kScanThreads, 0, s>>>(seg_cnt, list_len, seg_base, list_base, max_leaves,
-                                           counters_ + C_NSEG, counters_ + C_NENT);
+    launch_chained(k_scan_pair, 1, kScanThreads, 0, s, seg_cnt, list_len, seg_base, list_base,
+                   max_leaves, counters_ + C_NSEG, counters_ + C_NENT);
     ++info_.launches;
   } else {
     DT_CHECK(scan_counted(seg_cnt, seg_base, max_leaves, counters_ + C_NSEG, scan_tmp_, s));
@@ -3718,21 +3749,21 @@ cudaError_t DeviceTree::build(const TreeConfig &cfg, int64_t n, const float4 *po
         unsigned(std::min<int64_t>((nleaves + 7) / 8, int64_t(sm_count()) * 64));
     if (h_counters_[C_SEGOVF]) {
       const unsigned gW = unsigned((nleaves + kWalkWarps - 1) / kWalkWarps);
-      k_walk<1><<<gW, 32 * kWalkWarps, 0, s>>>(nodes_, nnodes, leaf_ids_, nleaves, cfg, n, nullptr,
-                                               nullptr, seg_base, list_base, segs_, nullptr,
-                                               walk_err_, counters_);
+      launch_chained(k_walk<1>, gW, 32 * kWalkWarps, 0, s, nodes_, nnodes, leaf_ids_, nleaves, cfg,
+                     n, nullptr, nullptr, seg_base, list_base, segs_, nullptr, walk_err_,
+                     counters_);
       ++info_.launches;
-      k_expand_pruned<false><<<blocks, 256, 0, s>>>(nullptr, segs_, seg_base, seg_cnt, list_base,
-                                                    nodes_, leaf_ids_, nleaves, table_, cfg.prune2,
-                                                    idx_list_, kept);
+      launch_chained(k_expand_pruned<false>, blocks, 256, 0, s, nullptr, segs_, seg_base, seg_cnt,
+                     list_base, nodes_, leaf_ids_, nleaves, table_, cfg.prune2, idx_list_, kept);
     } else {
-      k_expand_pruned<true><<<blocks, 256, 0, s>>>(segs_local_, segs_, seg_base, seg_cnt, list_base,
-                                                   nodes_, leaf_ids_, nleaves, table_, cfg.prune2,
-                                                   idx_list_, kept);
+      launch_chained(k_expand_pruned<true>, blocks, 256, 0, s, segs_local_, segs_, seg_base,
+                     seg_cnt, list_base, nodes_, leaf_ids_, nleaves, table_, cfg.prune2, idx_list_,
+                     kept);
     }
     ++info_.launches;
-    k_leaf_items<true><<<unsigned((nleaves + 127) / 128), 128, 0, s>>>(
-        nodes_, leaf_ids_, nleaves, list_len, kept, list_base, leafdesc_, jsplit, group_, counters_);
+    launch_chained(k_leaf_items<true>, unsigned((nleaves + 127) / 128), 128, 0, s, nodes_,
+                   leaf_ids_, nleaves, list_len, kept, list_base, leafdesc_, jsplit, group_,
+                   counters_);
     ++info_.launches;
   }
   DT_CHECK(cudaGetLastError());
@@ -3791,8 +3822,9 @@ cudaError_t DeviceTree::regroup(int group, int64_t jsplit, cudaStream_t s) {
   DT_CHECK(cudaMemsetAsync(counters_ + C_TICKET, 0, sizeof(int64_t), s));
   if (nleaves > 0) {
     DT_CHECK(launch_groups(nleaves, group, s));
-    k_leaf_items<false><<<unsigned((nleaves + 127) / 128), 128, 0, s>>>(
-        nullptr, nullptr, nleaves, nullptr, nullptr, nullptr, leafdesc_, jsplit, group, counters_);
+    launch_chained(k_leaf_items<false>, unsigned((nleaves + 127) / 128), 128, 0, s, nullptr,
+                   nullptr, nleaves, nullptr, nullptr, nullptr, leafdesc_, jsplit, group,
+                   counters_);
     ++info_.launches;
   }
   return fill_items(jsplit, s);
@@ -3820,8 +3852,8 @@ cudaError_t DeviceTree::fill_items(int64_t jsplit, cudaStream_t s) {
   padded_pairs_ = h_counters_[C_PADDED];
   DT_CHECK(grow(items_, cap_items_, size_t(std::max<int64_t>(nitems, 1)), s));
   if (nitems > 0) {
-    k_item_fill<<<unsigned((nleaves + 127) / 128), 128, 0, s>>>(leafdesc_, nleaves, jsplit, group_,
-                                                               counters_, items_);
+    launch_chained(k_item_fill, unsigned((nleaves + 127) / 128), 128, 0, s, leafdesc_, nleaves,
+                   jsplit, group_, counters_, items_);
     ++info_.launches;
   }
   return cudaGetLastError();
@@ -3830,7 +3862,7 @@ cudaError_t DeviceTree::fill_items(int64_t jsplit, cudaStream_t s) {
 cudaError_t launch_gather3_f32(const float *a, const float *b, const float *c, const int32_t *perm,
                                float *out, int64_t stride, int64_t n, cudaStream_t s) {
   if (n <= 0) return cudaSuccess;
-  k_gather3_f32<<<grid_for(n, 256), 256, 0, s>>>(a, b, c, perm, out, stride, n);
+  launch_chained(k_gather3_f32, grid_for(n, 256), 256, 0, s, a, b, c, perm, out, stride, n);
   return cudaGetLastError();
 }
 cudaError_t launch_outputs(const KickArrays &in, const float4 *table, bool split_table,
@@ -3838,24 +3870,26 @@ cudaError_t launch_outputs(const KickArrays &in, const float4 *table, bool split
                            cudaStream_t s) {
   if (n <= 0) return cudaSuccess;
   if (split_table)
-    k_outputs<true><<<grid_for(n, 256), 256, 0, s>>>(in, table, perm, vel, out, n);
+    launch_chained(k_outputs<true>, grid_for(n, 256), 256, 0, s, in, table, perm, vel, out, n);
   else
-    k_outputs<false><<<grid_for(n, 256), 256, 0, s>>>(in, table, perm, vel, out, n);
+    launch_chained(k_outputs<false>, grid_for(n, 256), 256, 0, s, in, table, perm, vel, out, n);
   return cudaGetLastError();
 }
 cudaError_t launch_finish(const float4 *table, const float *vel, const KickArrays &staged,
                           const KickArrays &out, int64_t n, cudaStream_t s) {
   if (n <= 0) return cudaSuccess;
-  k_finish<<<grid_for(n, 256), 256, 0, s>>>(table, vel, staged, out, n);
+  launch_chained(k_finish, grid_for(n, 256), 256, 0, s, table, vel, staged, out, n);
   return cudaGetLastError();
 }
 cudaError_t launch_scatter3_f32(const float *in, int64_t stride, const int32_t *perm,
                                 float *const out[3], bool add, int64_t n, cudaStream_t s) {
   if (n <= 0) return cudaSuccess;
   if (add)
-    k_scatter3_f32<true><<<grid_for(n, 256), 256, 0, s>>>(in, stride, perm, out[0], out[1], out[2], n);
+    launch_chained(k_scatter3_f32<true>, grid_for(n, 256), 256, 0, s, in, stride, perm, out[0],
+                   out[1], out[2], n);
   else
-    k_scatter3_f32<false><<<grid_for(n, 256), 256, 0, s>>>(in, stride, perm, out[0], out[1], out[2], n);
+    launch_chained(k_scatter3_f32<false>, grid_for(n, 256), 256, 0, s, in, stride, perm, out[0],
+                   out[1], out[2], n);
   return cudaGetLastError();
 }
 
@@ -3896,7 +3930,7 @@ cudaError_t launch_pseudo_adjoint_quad(const DNode *nodes, const std::vector<int
 cudaError_t launch_pack4(const float *x, const float *y, const float *z, const float *m,
                          float4 *out, int64_t n, cudaStream_t s) {
   if (n <= 0) return cudaSuccess;
-  k_pack4<<<grid_for(n, 256), 256, 0, s>>>(x, y, z, m, out, n);
+  launch_chained(k_pack4, grid_for(n, 256), 256, 0, s, x, y, z, m, out, n);
   return cudaGetLastError();
 }
 }  // namespace hsr

@@ -7,6 +7,7 @@
 #include <algorithm>
 
 #include "rcb_device.cuh"
+#include "chain.cuh"
 #include "device_info.cuh"
 
 namespace hsr {
@@ -17,6 +18,7 @@ namespace {
 // reference's x[i] + prefactor * tau * vx[i] with pt = prefactor * tau.
 __global__ void k_stream(float *x, float *y, float *z, const float *vx, const float *vy,
                          const float *vz, int64_t n, float pt) {
+  chain_enter();
   for (int64_t i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x; i < n;
        i += int64_t(gridDim.x) * blockDim.x) {
     x[i] = __fadd_rn(x[i], __fmul_rn(pt, vx[i]));
@@ -42,6 +44,7 @@ __device__ __forceinline__ bool cell_of(float x, float y, float z, int32_t ng0, 
 __global__ void k_cell_keys(const float *x, const float *y, const float *z, int64_t n, int32_t ng0,
                             int32_t ng1, int32_t ng2, uint32_t *key, uint32_t *val,
                             unsigned long long *inbox) {
+  chain_enter();
   const uint32_t Ng = uint32_t(ng0) * uint32_t(ng1) * uint32_t(ng2);
   unsigned long long c = 0;
   for (int64_t i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x; i < n;
@@ -158,6 +161,7 @@ template <bool DRIFT>
 __global__ void __launch_bounds__(kCellThreads)
     k_cell_count(KickArrays A, int64_t n, float pt, int32_t ng0, int32_t ng1, int32_t ng2,
                  uint32_t *key, uint32_t *slot, uint32_t *cnt, CellCount *out) {
+  chain_enter();
   const uint32_t Ng = uint32_t(ng0) * uint32_t(ng1) * uint32_t(ng2);
   unsigned c = 0, most = 0;
   for (int64_t i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x; i < n;
@@ -197,6 +201,7 @@ __device__ __forceinline__ uint32_t block_sum_u32(uint32_t v, uint32_t *sh) {
 
 __global__ void __launch_bounds__(kCellThreads)
     k_cell_tiles(const uint32_t *__restrict__ cnt, int64_t ncell, uint32_t *tile) {
+  chain_enter();
   __shared__ uint32_t sh[kCellThreads / 32];
   const int64_t base = int64_t(blockIdx.x) * kCellTile;
   uint32_t v = 0;
@@ -214,6 +219,7 @@ __global__ void __launch_bounds__(kCellThreads)
 __global__ void __launch_bounds__(kCellThreads)
     k_cell_offsets(const uint32_t *__restrict__ cnt, int64_t ncell,
                    const uint32_t *__restrict__ tile, uint32_t *offs) {
+  chain_enter();
   __shared__ uint32_t sh[kCellThreads / 32];
   uint32_t before = 0;
   for (unsigned t = threadIdx.x; t < blockIdx.x; t += kCellThreads) before += tile[t];
@@ -246,6 +252,7 @@ __global__ void __launch_bounds__(kCellThreads)
 __global__ void k_cell_place(const uint32_t *__restrict__ key, const uint32_t *__restrict__ slot,
                              const uint32_t *__restrict__ offs, int64_t n, const CellCount *c,
                              uint32_t *order) {
+  chain_enter();
   if (c->longest > kMaxOcc) return;  // the radix sort follows
   for (int64_t i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x; i < n;
        i += int64_t(gridDim.x) * blockDim.x)
@@ -274,6 +281,7 @@ __device__ __forceinline__ void move_particle(const KickArrays &A, const KickArr
 __global__ void k_cell_move(const uint32_t *__restrict__ order, const uint32_t *__restrict__ key,
                             const uint32_t *__restrict__ offs, const uint32_t *__restrict__ cnt,
                             int64_t n, const CellCount *c, KickArrays A, KickArrays S) {
+  chain_enter();
   if (c->longest > kMaxOcc) return;
   for (int64_t p = int64_t(blockIdx.x) * blockDim.x + threadIdx.x; p < n;
        p += int64_t(gridDim.x) * blockDim.x) {
@@ -288,6 +296,7 @@ __global__ void k_cell_move(const uint32_t *__restrict__ order, const uint32_t *
 
 // The radix sort's permutation applied to the arrays.
 __global__ void k_perm_move(const uint32_t *__restrict__ perm, int64_t n, KickArrays A, KickArrays S) {
+  chain_enter();
   for (int64_t p = int64_t(blockIdx.x) * blockDim.x + threadIdx.x; p < n;
        p += int64_t(gridDim.x) * blockDim.x)
     move_particle(A, S, perm[p], p);
@@ -295,6 +304,7 @@ __global__ void k_perm_move(const uint32_t *__restrict__ perm, int64_t n, KickAr
 
 // The staging copy back into the arrays, the masses set to one.
 __global__ void k_move_back(KickArrays S, KickArrays A, int64_t n, const CellCount *c) {
+  chain_enter();
   if (c && c->longest > kMaxOcc) return;
   for (int64_t i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x; i < n;
        i += int64_t(gridDim.x) * blockDim.x) {
@@ -313,7 +323,7 @@ inline unsigned grid_of(int64_t n, int threads = 256) {
 cudaError_t launch_stream(float *x, float *y, float *z, const float *vx, const float *vy,
                           const float *vz, int64_t n, float pt, cudaStream_t s) {
   if (n <= 0) return cudaSuccess;
-  k_stream<<<grid_of(n), 256, 0, s>>>(x, y, z, vx, vy, vz, n, pt);
+  launch_chained(k_stream, grid_of(n), 256, 0, s, x, y, z, vx, vy, vz, n, pt);
   return cudaGetLastError();
 }
 
@@ -403,14 +413,16 @@ cudaError_t drift_and_resort(int64_t n, const int32_t ng[3], const KickArrays &A
     e = cudaMemsetAsync(cnt, 0, size_t(ncell) * 4, s);
     if (e != cudaSuccess) return e;
     if (pt)
-      k_cell_count<true><<<grid, kCellThreads, 0, s>>>(A, n, *pt, ng[0], ng[1], ng[2], key, slot, cnt, count);
+      launch_chained(k_cell_count<true>, grid, kCellThreads, 0, s, A, n, *pt, ng[0], ng[1], ng[2],
+                     key, slot, cnt, count);
     else
-      k_cell_count<false><<<grid, kCellThreads, 0, s>>>(A, n, 0.f, ng[0], ng[1], ng[2], key, slot, cnt, count);
-    k_cell_tiles<<<tiles, kCellThreads, 0, s>>>(cnt, ncell, tile);
-    k_cell_offsets<<<tiles, kCellThreads, 0, s>>>(cnt, ncell, tile, offs);
-    k_cell_place<<<grid, 256, 0, s>>>(key, slot, offs, n, count, order);
-    k_cell_move<<<grid, 256, 0, s>>>(order, key, offs, cnt, n, count, A, S);
-    k_move_back<<<grid, 256, 0, s>>>(S, A, n, count);
+      launch_chained(k_cell_count<false>, grid, kCellThreads, 0, s, A, n, 0.f, ng[0], ng[1], ng[2],
+                     key, slot, cnt, count);
+    launch_chained(k_cell_tiles, tiles, kCellThreads, 0, s, cnt, ncell, tile);
+    launch_chained(k_cell_offsets, tiles, kCellThreads, 0, s, cnt, ncell, tile, offs);
+    launch_chained(k_cell_place, grid, 256, 0, s, key, slot, offs, n, count, order);
+    launch_chained(k_cell_move, grid, 256, 0, s, order, key, offs, cnt, n, count, A, S);
+    launch_chained(k_move_back, grid, 256, 0, s, S, A, n, count);
     e = cudaMemcpyAsync(&got, count, sizeof(got), cudaMemcpyDeviceToHost, s);
     if (e == cudaSuccess) e = cudaStreamSynchronize(s);
     if (e != cudaSuccess) return e;
@@ -430,8 +442,8 @@ cudaError_t drift_and_resort(int64_t n, const int32_t ng[3], const KickArrays &A
            *val2 = c.take<uint32_t>(n);
   int64_t *hist = c.take<int64_t>(h), *offs = c.take<int64_t>(h);
   int64_t *tmp = c.take<int64_t>(scan_tmp_size(h));
-  k_cell_keys<<<grid, 256, 0, s>>>(A.f[0], A.f[1], A.f[2], n, ng[0], ng[1], ng[2], key, val,
-                                   &count->inbox);
+  launch_chained(k_cell_keys, grid, 256, 0, s, A.f[0], A.f[1], A.f[2], n, ng[0], ng[1], ng[2], key,
+                 val, &count->inbox);
   const uint64_t Ng = uint64_t(ResortLayout::grid_cells(ng));
   int bits = 1;
   while ((uint64_t(1) << bits) <= Ng) ++bits;
@@ -444,8 +456,8 @@ cudaError_t drift_and_resort(int64_t n, const int32_t ng[3], const KickArrays &A
     std::swap(key, key2);
     std::swap(val, val2);
   }
-  k_perm_move<<<grid, 256, 0, s>>>(val, n, A, S);
-  k_move_back<<<grid, 256, 0, s>>>(S, A, n, nullptr);
+  launch_chained(k_perm_move, grid, 256, 0, s, val, n, A, S);
+  launch_chained(k_move_back, grid, 256, 0, s, S, A, n, nullptr);
   e = cudaMemcpyAsync(&got, count, sizeof(got), cudaMemcpyDeviceToHost, s);
   if (e == cudaSuccess) e = cudaStreamSynchronize(s);
   if (e != cudaSuccess) return e;
