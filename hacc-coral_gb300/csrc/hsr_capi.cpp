@@ -1189,6 +1189,7 @@ hsr_status force_fwd_impl(hsr_ctx *ctx, const hsr_params *p, int64_t n, const fl
   cfg.nd = int32_t(std::min<int64_t>(p->nd, INT32_MAX));
   cfg.tdpts = p->tdpts;
   cfg.group = ctx->tune.group;  // the adjoint kernel takes groups of 16 or 32
+  cfg.halves = true;      // and tests each half of one
   cudaError_t e = ctx->tree.build(cfg, n, pos4, kJSplit, s);
   if (e != cudaSuccess) {
     if (ctx->tree.error()) return ctx->fail(HSR_ERR_UNSUPPORTED, ctx->tree.error());
@@ -1782,6 +1783,7 @@ hsr_status force_batch_impl(hsr_ctx *ctx, int32_t nbox, const hsr_params *params
     cfg.nd = int32_t(std::min<int64_t>(p->nd, INT32_MAX));
     cfg.tdpts = p->tdpts;
     cfg.group = ctx->tune.group;  // the adjoint kernel takes groups of 16 or 32
+    cfg.halves = true;      // and tests each half of one
     cudaError_t e = B.tree.build(cfg, n, B.pos4.as<float4>(), kJSplit, s);
     if (e != cudaSuccess) {
       if (B.tree.error()) return fail(HSR_ERR_UNSUPPORTED, B.tree.error());

@@ -2654,7 +2654,7 @@ __global__ void __launch_bounds__(256)
 // inside the leaf's box) and the batched kernel's work items.
 // ---------------------------------------------------------------------------
 constexpr int kGroupSort = 1024;
-constexpr int kGroupHalf = 16;  // particles of a group with a box of their own
+constexpr int kGroupHalf = 16;  // particles of a group with a box of their own (adjoint)
 constexpr int kGW = 256;     // leaves up to this size are grouped by one warp
 constexpr int kGWarps = 4;   // warps (leaves) per block of k_groups_warp
 constexpr int kGroupThreads = 256;
@@ -2667,11 +2667,12 @@ __device__ __forceinline__ int group_split(int c, int G) {
 
 // Splits a leaf into groups of G particles (the last one shorter) by recursive
 // median splits along the longest axis, left parts a multiple of G, and each
-// group of 32 into halves once more: the particles of a half are close, so the
-// pair kernels' box test of each half keeps few list entries.  Every level sorts all segments of the leaf at once by
+// group once more at `half` (G where the halves do not matter: that level is a
+// third of the time): the particles are close, so the pair kernels' box tests
+// keep few list entries.  Every level sorts all segments of the leaf at once by
 // (segment, coordinate along the segment's longest axis).
 __device__ void group_large_leaf(const DNode &T, const float4 *__restrict__ pos, int32_t *gidx,
-                                 int G) {
+                                 int G, int half) {
   __shared__ uint64_t key[kGroupSort];
   __shared__ int32_t val[kGroupSort];
   __shared__ int32_t seg_a[kGroupSort / 16 + 1], seg_c[kGroupSort / 16 + 1];
@@ -2704,7 +2705,7 @@ __device__ void group_large_leaf(const DNode &T, const float4 *__restrict__ pos,
     for (int i = threadIdx.x; i < c; i += blockDim.x) {
       int q = 0;
       while (q + 1 < nseg && seg_a[q + 1] <= i) ++q;
-      if (seg_c[q] <= kGroupHalf) continue;
+      if (seg_c[q] <= half) continue;
       const float4 p = pos[val[i]];
       const uint32_t o[3] = {f2o(p.x), f2o(p.y), f2o(p.z)};
       for (int d = 0; d < 3; ++d) {
@@ -2720,7 +2721,7 @@ __device__ void group_large_leaf(const DNode &T, const float4 *__restrict__ pos,
         int q = 0;
         while (q + 1 < nseg && seg_a[q + 1] <= i) ++q;
         uint32_t ko = 0;
-        if (seg_c[q] > kGroupHalf) {
+        if (seg_c[q] > half) {
           float ext[3];
           for (int d = 0; d < 3; ++d) ext[d] = o2f(seg_hi[d][q]) - o2f(seg_lo[d][q]);
           const int ax = (ext[0] >= ext[1] && ext[0] >= ext[2]) ? 0 : (ext[1] >= ext[2] ? 1 : 2);
@@ -2752,14 +2753,14 @@ __device__ void group_large_leaf(const DNode &T, const float4 *__restrict__ pos,
         }
         __syncthreads();
       }
-    // split every segment above kGroupHalf
+    // split every segment above `half`
     if (threadIdx.x == 0) {
       int n2 = 0;
       int32_t na[kGroupSort / 16 + 1], nc[kGroupSort / 16 + 1];
       int more = 0;
       for (int q = 0; q < nseg; ++q) {
         const int32_t a0 = seg_a[q], c0 = seg_c[q];
-        if (c0 <= kGroupHalf) {
+        if (c0 <= half) {
           na[n2] = a0;
           nc[n2++] = c0;
           continue;
@@ -2769,7 +2770,7 @@ __device__ void group_large_leaf(const DNode &T, const float4 *__restrict__ pos,
         nc[n2++] = left;
         na[n2] = a0 + left;
         nc[n2++] = c0 - left;
-        more |= left > kGroupHalf || c0 - left > kGroupHalf;
+        more |= left > half || c0 - left > half;
       }
       for (int q = 0; q < n2; ++q) {
         seg_a[q] = na[q];
@@ -2789,7 +2790,7 @@ __device__ void group_large_leaf(const DNode &T, const float4 *__restrict__ pos,
 // leaf, most of them returning at once, took 31 us of a 128^3 kick).
 __global__ void __launch_bounds__(kGroupThreads)
     k_groups(const DNode *nodes, const int32_t *leaf_ids, const int64_t *nleaves,
-             const float4 *__restrict__ pos, int32_t *gidx, int G) {
+             const float4 *__restrict__ pos, int32_t *gidx, int G, int half) {
   __shared__ int32_t big[kGroupThreads];
   __shared__ int nbig;
   if (threadIdx.x == 0) nbig = 0;
@@ -2801,19 +2802,19 @@ __global__ void __launch_bounds__(kGroupThreads)
   }
   __syncthreads();
   for (int b = 0; b < nbig; ++b) {
-    group_large_leaf(nodes[big[b]], pos, gidx, G);
+    group_large_leaf(nodes[big[b]], pos, gidx, G, half);
     __syncthreads();  // the next leaf reuses the shared arrays
   }
 }
 
 // Warp-per-leaf grouping for leaves of at most kGW particles (the usual
 // case; larger leaves take k_groups).  Same median splits as k_groups: per
-// level, every segment above kGroupHalf particles is sorted along its longest
+// level, every segment above `half` particles is sorted along its longest
 // axis by ranking (each element counts the keys below its own, ties by
 // position) and split at group_split().
 __global__ void __launch_bounds__(32 * kGWarps)
     k_groups_warp(const DNode *nodes, const int32_t *leaf_ids, const int64_t *nleaves,
-                  const float4 *__restrict__ pos, int32_t *gidx, int G) {
+                  const float4 *__restrict__ pos, int32_t *gidx, int G, int half) {
   __shared__ float key[kGWarps][kGW];
   __shared__ int32_t val[kGWarps][2][kGW];
   __shared__ uint8_t segid[kGWarps][kGW];
@@ -2825,7 +2826,7 @@ __global__ void __launch_bounds__(32 * kGWarps)
   const DNode &T = nodes[leaf_ids[li]];
   const int c = T.count;
   if (c <= 0 || c > kGW) return;
-  if (c <= kGroupHalf) {
+  if (c <= half) {
     for (int i = lane; i < c; i += 32) gidx[T.offset + i] = T.offset + i;
     return;
   }
@@ -2845,7 +2846,7 @@ __global__ void __launch_bounds__(32 * kGWarps)
     bool any = false;
     for (int q = 0; q < nseg; ++q) {
       const int a0 = seg_a[w][q], c0 = seg_c[w][q];
-      if (c0 <= kGroupHalf) continue;
+      if (c0 <= half) continue;
       any = true;
       float lo[3] = {INFINITY, INFINITY, INFINITY}, hi[3] = {-INFINITY, -INFINITY, -INFINITY};
       for (int i = a0 + lane; i < a0 + c0; i += 32) {
@@ -2866,7 +2867,7 @@ __global__ void __launch_bounds__(32 * kGWarps)
     for (int i = lane; i < c; i += 32) {
       const int q = segid[w][i];
       float k = 0.f;
-      if (seg_c[w][q] > kGroupHalf) {
+      if (seg_c[w][q] > half) {
         const float4 p = pos[val[w][cur][i]];
         const int ax = seg_ax[w][q];
         k = ax == 0 ? p.x : (ax == 1 ? p.y : p.z);
@@ -2878,7 +2879,7 @@ __global__ void __launch_bounds__(32 * kGWarps)
       const int q = segid[w][i];
       const int a0 = seg_a[w][q], c0 = seg_c[w][q];
       int np = i;
-      if (c0 > kGroupHalf) {
+      if (c0 > half) {
         const float ki = key[w][i];
         int r = 0;
         for (int j = a0; j < a0 + c0; ++j) {
@@ -2891,13 +2892,13 @@ __global__ void __launch_bounds__(32 * kGWarps)
     }
     __syncwarp();
     cur ^= 1;
-    // split every segment above kGroupHalf
+    // split every segment above `half`
     if (lane == 0) {
       int16_t na[kGW / 16 + 1], nc[kGW / 16 + 1];
       int n2 = 0;
       for (int q = 0; q < nseg; ++q) {
         const int a0 = seg_a[w][q], c0 = seg_c[w][q];
-        if (c0 <= kGroupHalf) {
+        if (c0 <= half) {
           na[n2] = int16_t(a0);
           nc[n2++] = int16_t(c0);
           continue;
@@ -3399,15 +3400,13 @@ inline unsigned grid_for(int64_t n, int threads, int64_t cap = 0) {
 
 DeviceTree::~DeviceTree() {
   void *ptrs[] = {epos_, tpos_, oid_, toid_, idx_, nodes_, ppm_, chunk_node_, chunk_base_,
-                  left_cnt_, left_base_, acc_, ticket_, ctl_, scan_tmp_, node_tmp_, fallback_, counters_, leaf_ids_,
-                  up_, processed_, roots_, leafdesc_, segs_, idx_list_, table_, items_, items_tmp_, gidx_,
+                  left_cnt_, left_base_, acc_, ticket_, scan_tmp_, node_tmp_, fallback_, counters_, leaf_ids_,
+                  up_, processed_, roots_, leafdesc_, segs_, idx_list_, items_, items_tmp_, gidx_,
                   tight_chunks_, tight_nodes_, segs_local_, ridx_, sub_nodes_, sub_first_,
-                  sub_hist_, sub_tot_, wpre_, chains_};
+                  sub_hist_, wpre_, chains_};
   for (void *p : ptrs)
     if (p) cudaFree(p);
   if (h_counters_) cudaFreeHost(h_counters_);
-  if (h_sub_) cudaFreeHost(h_sub_);
-  if (h_ctl_) cudaFreeHost(h_ctl_);
   if (aux_) {
     cudaStreamSynchronize(aux_);
     cudaStreamDestroy(aux_);
@@ -3456,31 +3455,33 @@ cudaError_t DeviceTree::build(const TreeConfig &cfg, int64_t n, const float4 *po
   DT_CHECK(grow(tight_chunks_, cap_tc_,
                 (size_t(n) / kTightChunk + kTightNodes + 1) * (sizeof(TightChunk) / sizeof(double)), s));
   DT_CHECK(grow(tight_nodes_, cap_tn_, size_t(kTightNodes) * (sizeof(TightNode) / sizeof(double)), s));
-  DT_CHECK(grow(epos_, cap_e_, nn, s));
+  // (room for the pseudo-particles of an even tree behind the particles: the
+  // table is epos_ with them appended)
+  DT_CHECK(grow(epos_, cap_e_, nn + size_t(cfg.tdpts) * (4 * nn / std::max(1, cfg.nd) + 64), s));
   DT_CHECK(grow(tpos_, cap_t_, nn, s));
   DT_CHECK(grow(oid_, cap_o_, nn, s));
   DT_CHECK(grow(toid_, cap_to_, nn, s));
   DT_CHECK(grow(idx_, cap_i_, nn, s));
   DT_CHECK(grow(ridx_, cap_ri_, nn, s));
+  // counters, subtree totals and level extents in one block (and a pinned
+  // copy), zeroed and read back together
+  constexpr size_t kTotOff = C_COUNT * sizeof(int64_t), kCtlOff = kTotOff + kSubDepth * sizeof(int64_t);
+  constexpr size_t kStateBytes = kCtlOff + sizeof(LevelCtl);
+  static_assert(kCtlOff % alignof(LevelCtl) == 0, "alignment");
   if (!counters_) {
-    DT_CHECK(cudaMalloc(&counters_, C_COUNT * sizeof(int64_t)));
-    DT_CHECK(cudaHostAlloc(&h_counters_, C_COUNT * sizeof(int64_t), cudaHostAllocDefault));
+    DT_CHECK(cudaHostAlloc(&h_counters_, kStateBytes, cudaHostAllocDefault));
+    DT_CHECK(cudaFuncSetAttribute(k_subtree, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                  kSubMax * kSubBytes));
+    DT_CHECK(cudaMalloc(&counters_, kStateBytes));
     // the kernels' error flag lives in a counter slot: read back with the counters
     walk_err_ = reinterpret_cast<int32_t *>(counters_ + C_ERR);
   }
-  auto *ctl = reinterpret_cast<LevelCtl *>(ctl_);
-  if (!ctl) {
-    DT_CHECK(cudaMalloc(&ctl_, sizeof(LevelCtl)));
-    DT_CHECK(cudaHostAlloc(&h_ctl_, sizeof(LevelCtl), cudaHostAllocDefault));
-    DT_CHECK(cudaHostAlloc(&h_sub_, kSubDepth * sizeof(int64_t), cudaHostAllocDefault));
-    DT_CHECK(cudaMalloc(&sub_tot_, kSubDepth * sizeof(int64_t)));
-    DT_CHECK(cudaFuncSetAttribute(k_subtree, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                  kSubMax * kSubBytes));
-    ctl = reinterpret_cast<LevelCtl *>(ctl_);
-  }
-  auto *hc = reinterpret_cast<LevelCtl *>(h_ctl_);
-  DT_CHECK(cudaMemsetAsync(counters_, 0, C_COUNT * sizeof(int64_t), s));
-  DT_CHECK(cudaMemsetAsync(ctl_, 0, sizeof(LevelCtl), s));
+  auto at = [](int64_t *p, size_t off) { return reinterpret_cast<char *>(p) + off; };
+  auto *ctl = reinterpret_cast<LevelCtl *>(at(counters_, kCtlOff));
+  auto *hc = reinterpret_cast<LevelCtl *>(at(h_counters_, kCtlOff));
+  auto *sub_tot = reinterpret_cast<int64_t *>(at(counters_, kTotOff));
+  const auto *h_sub = reinterpret_cast<const int64_t *>(at(h_counters_, kTotOff));
+  DT_CHECK(cudaMemsetAsync(counters_, 0, kStateBytes, s));
   const size_t want_nodes = size_t(std::max<int64_t>(64, 4 * n / std::max(1, cfg.nd) + 64));
   DT_CHECK(grow(nodes_, cap_nodes_, want_nodes, s));
   if (n > 0) {
@@ -3573,17 +3574,14 @@ cudaError_t DeviceTree::build(const TreeConfig &cfg, int64_t n, const float4 *po
                      nodes_, ctl, roots_, epos_, oid_, tpos_, toid_, sub_nodes_, sub_first_,
                      sub_hist_, cap, cfg.force_cm_fallback, cfg.nd, counters_);
       launch_chained(k_subtree_scan, kSubDepth, kScanThreads, 0, s, ctl, sub_hist_,
-                     int32_t(max_roots), sub_tot_);
+                     int32_t(max_roots), sub_tot);
       launch_chained(k_subtree_place, unsigned(max_roots), 256, 0, s, nodes_, ctl, roots_,
-                     sub_nodes_, sub_first_, sub_hist_, int32_t(max_roots), sub_tot_,
+                     sub_nodes_, sub_first_, sub_hist_, int32_t(max_roots), sub_tot,
                      int64_t(cap_nodes_));
       info_.launches += 3;
-      DT_CHECK(cudaMemcpyAsync(h_sub_, sub_tot_, kSubDepth * sizeof(int64_t), cudaMemcpyDeviceToHost, s));
     }
     DT_CHECK(cudaGetLastError());
-    DT_CHECK(cudaMemcpyAsync(hc, ctl_, sizeof(LevelCtl), cudaMemcpyDeviceToHost, s));
-    DT_CHECK(cudaMemcpyAsync(h_counters_, counters_, C_COUNT * sizeof(int64_t),
-                             cudaMemcpyDeviceToHost, s));
+    DT_CHECK(cudaMemcpyAsync(h_counters_, counters_, kStateBytes, cudaMemcpyDeviceToHost, s));
     DT_CHECK(cudaStreamSynchronize(s));
     const int32_t err = *reinterpret_cast<const int32_t *>(h_counters_ + C_ERR);
     if (err == 4) {
@@ -3628,23 +3626,23 @@ cudaError_t DeviceTree::build(const TreeConfig &cfg, int64_t n, const float4 *po
     if (hc->done) {
       if (!subtrees) break;
       int64_t total = level_ne;
-      for (int d = 0; d < kSubDepth; ++d) total += h_sub_[d];
+      for (int d = 0; d < kSubDepth; ++d) total += h_sub[d];
       if (total > INT32_MAX) return cudaErrorInvalidValue;
       if (size_t(total) > cap_nodes_) {
         DT_CHECK(grow(nodes_, cap_nodes_, size_t(total), s, true));
         launch_chained(k_subtree_place, unsigned(max_roots), 256, 0, s, nodes_, ctl, roots_,
-                       sub_nodes_, sub_first_, sub_hist_, int32_t(max_roots), sub_tot_,
+                       sub_nodes_, sub_first_, sub_hist_, int32_t(max_roots), sub_tot,
                        int64_t(cap_nodes_));
         ++info_.launches;
         DT_CHECK(cudaGetLastError());
       }
       // the ranges that hold every node after its parent: levels, then subtree
       // depths
-      int64_t at = level_ne;
-      level_begin.push_back(int32_t(at));
-      for (int d = 0; d < kSubDepth && h_sub_[d] > 0; ++d) {
-        at += h_sub_[d];
-        level_begin.push_back(int32_t(at));
+      int64_t end = level_ne;
+      level_begin.push_back(int32_t(end));
+      for (int d = 0; d < kSubDepth && h_sub[d] > 0; ++d) {
+        end += h_sub[d];
+        level_begin.push_back(int32_t(end));
       }
       level_ne = int32_t(total);
       break;
@@ -3665,19 +3663,18 @@ cudaError_t DeviceTree::build(const TreeConfig &cfg, int64_t n, const float4 *po
   // a binary tree's leaves: the processed ones are at most as many
   const int64_t max_leaves = (int64_t(nnodes) + 1) / 2;
   DT_CHECK(grow(ppm_, cap_ppm_, size_t(nnodes) * k + 1, s));
-  DT_CHECK(grow(table_, cap_tab_, size_t(std::max<int64_t>(ntab, 1)), s));
+  DT_CHECK(grow(epos_, cap_e_, size_t(std::max<int64_t>(ntab, 1)), s, true));
+  float4 *table = epos_;
   DT_CHECK(grow(up_, cap_up_, size_t(nnodes), s));
   DT_CHECK(grow(processed_, cap_pr_, size_t(nnodes), s));
   DT_CHECK(grow(leaf_ids_, cap_leaf_, size_t(max_leaves), s));
-  if (n > 0)
-    DT_CHECK(cudaMemcpyAsync(table_, epos_, size_t(n) * sizeof(float4), cudaMemcpyDeviceToDevice, s));
   const unsigned gN = unsigned((nnodes + 127) / 128), gP = unsigned((int64_t(nnodes) * 32 + 127) / 128);
   launch_chained(k_links, gN, 128, 0, s, nodes_, nnodes, up_);
   if (k == 12)
-    launch_chained(k_pseudo_up<12>, gP, 128, 0, s, nodes_, nnodes, up_, epos_, ppm_, table_, n, cfg,
+    launch_chained(k_pseudo_up<12>, gP, 128, 0, s, nodes_, nnodes, up_, epos_, ppm_, table, n, cfg,
                    processed_);
   else
-    launch_chained(k_pseudo_up<1>, gP, 128, 0, s, nodes_, nnodes, up_, epos_, ppm_, table_, n, cfg,
+    launch_chained(k_pseudo_up<1>, gP, 128, 0, s, nodes_, nnodes, up_, epos_, ppm_, table, n, cfg,
                    processed_);
   launch_chained(k_leaf_rank, gN, 128, 0, s, nodes_, nnodes, up_, processed_, leaf_ids_, counters_);
   info_.launches += 3;
@@ -3704,13 +3701,12 @@ cudaError_t DeviceTree::build(const TreeConfig &cfg, int64_t n, const float4 *po
   // then place them (a leaf with more than kLocalSegs segments sends the
   // build to a second, placing walk)
   DT_CHECK(grow(segs_local_, cap_segl_, nlw * kLocalSegs, s));
-  DT_CHECK(cudaMemsetAsync(counters_ + C_SEGOVF, 0, sizeof(int64_t), s));
   launch_chained(k_walk<2>, unsigned((max_leaves + kWalkWarps - 1) / kWalkWarps), 32 * kWalkWarps,
                  0, s, nodes_, nnodes, leaf_ids_, max_leaves, cfg, n, seg_cnt, list_len, nullptr,
                  nullptr, nullptr, segs_local_, walk_err_, counters_);
   ++info_.launches;
   // the groups after the walk's blocks, which then have their SMs first
-  DT_CHECK(launch_groups(max_leaves, group_, aux_));
+  DT_CHECK(launch_groups(max_leaves, group_, cfg.halves ? kGroupHalf : group_, aux_));
   DT_CHECK(cudaEventRecord(ev_groups_, aux_));
   groups_ready_ = group_;
   if (max_leaves <= kScanPairMax) {
@@ -3741,8 +3737,6 @@ cudaError_t DeviceTree::build(const TreeConfig &cfg, int64_t n, const float4 *po
   DT_CHECK(grow(segs_, cap_seg_, size_t(std::max<int64_t>(nseg, 1)), s));
   DT_CHECK(grow(idx_list_, cap_idx_, size_t(std::max<int64_t>(nent, 1)), s));
   DT_CHECK(grow(leafdesc_, cap_ld_, nlw, s));
-  DT_CHECK(cudaMemsetAsync(counters_ + C_BUCKET, 0, 32 * sizeof(int64_t), s));
-  DT_CHECK(cudaMemsetAsync(counters_ + C_TICKET, 0, sizeof(int64_t), s));
   if (nleaves > 0) {
     int64_t *kept = node_tmp_ + 4 * nlw;
     const unsigned blocks =
@@ -3754,10 +3748,10 @@ cudaError_t DeviceTree::build(const TreeConfig &cfg, int64_t n, const float4 *po
                      counters_);
       ++info_.launches;
       launch_chained(k_expand_pruned<false>, blocks, 256, 0, s, nullptr, segs_, seg_base, seg_cnt,
-                     list_base, nodes_, leaf_ids_, nleaves, table_, cfg.prune2, idx_list_, kept);
+                     list_base, nodes_, leaf_ids_, nleaves, table, cfg.prune2, idx_list_, kept);
     } else {
       launch_chained(k_expand_pruned<true>, blocks, 256, 0, s, segs_local_, segs_, seg_base,
-                     seg_cnt, list_base, nodes_, leaf_ids_, nleaves, table_, cfg.prune2, idx_list_,
+                     seg_cnt, list_base, nodes_, leaf_ids_, nleaves, table, cfg.prune2, idx_list_,
                      kept);
     }
     ++info_.launches;
@@ -3821,7 +3815,7 @@ cudaError_t DeviceTree::regroup(int group, int64_t jsplit, cudaStream_t s) {
   DT_CHECK(cudaMemsetAsync(counters_ + C_BUCKET, 0, 32 * sizeof(int64_t), s));
   DT_CHECK(cudaMemsetAsync(counters_ + C_TICKET, 0, sizeof(int64_t), s));
   if (nleaves > 0) {
-    DT_CHECK(launch_groups(nleaves, group, s));
+    DT_CHECK(launch_groups(nleaves, group, group, s));
     launch_chained(k_leaf_items<false>, unsigned((nleaves + 127) / 128), 128, 0, s, nullptr,
                    nullptr, nleaves, nullptr, nullptr, nullptr, leafdesc_, jsplit, group,
                    counters_);
@@ -3830,11 +3824,11 @@ cudaError_t DeviceTree::regroup(int group, int64_t jsplit, cudaStream_t s) {
   return fill_items(jsplit, s);
 }
 
-cudaError_t DeviceTree::launch_groups(int64_t max_leaves, int G, cudaStream_t s) {
+cudaError_t DeviceTree::launch_groups(int64_t max_leaves, int G, int half, cudaStream_t s) {
   k_groups_warp<<<unsigned((max_leaves + kGWarps - 1) / kGWarps), 32 * kGWarps, 0, s>>>(
-      nodes_, leaf_ids_, counters_ + C_NLEAF, epos_, gidx_, G);
+      nodes_, leaf_ids_, counters_ + C_NLEAF, epos_, gidx_, G, half);
   k_groups<<<unsigned((max_leaves + kGroupThreads - 1) / kGroupThreads), kGroupThreads, 0, s>>>(
-      nodes_, leaf_ids_, counters_ + C_NLEAF, epos_, gidx_, G);
+      nodes_, leaf_ids_, counters_ + C_NLEAF, epos_, gidx_, G, half);
   info_.launches += 2;
   return cudaGetLastError();
 }

@@ -49,6 +49,7 @@ struct TreeConfig {
   float prune2;               // > 0: the index lists keep only entries within
                               // sqrt(prune2) of their leaf's box (the kernels'
                               // cull radius); 0: every list entry
+  bool halves;            // order each group of 32 so that its first 16 and the rest are compact
 };
 
 // Result sizes of a device build.
@@ -72,9 +73,9 @@ class DeviceTree {
   // input index, `table()` holds the position table (particles in tree order,
   // then tdpts pseudo-particles per node), and the processed leaves' lists,
   // work items and group index are built.  `jsplit` bounds the list range of
-  // one work item.  Synchronizes `s` once per tree level down to the first
-  // level whose nodes all fit one block; that level's subtrees are built
-  // whole, one block each, with one synchronisation.
+  // one work item.  Synchronizes `s` after the tree (which is made without a
+  // look from the host, unless a level has centres of mass to certify), after
+  // the list counts and after the item counts.
   cudaError_t build(const TreeConfig &cfg, int64_t n, const float4 *pos_in, int64_t jsplit,
                     cudaStream_t s);
 
@@ -85,7 +86,7 @@ class DeviceTree {
 
   const DeviceTreeInfo &info() const { return info_; }
   const int32_t *perm() const { return oid_; }
-  const float4 *table() const { return table_; }
+  const float4 *table() const { return epos_; }
   const LeafDesc *leaves() const { return leafdesc_; }
   const SegDesc *segs() const { return segs_; }
   const int32_t *index() const { return idx_list_; }
@@ -122,8 +123,9 @@ class DeviceTree {
   cudaStream_t aux_ = nullptr;
   cudaEvent_t ev_fork_ = nullptr, ev_groups_ = nullptr;
   int groups_ready_ = 0;  // G of groups launched on aux_ and not yet joined
-  cudaError_t launch_groups(int64_t max_leaves, int G, cudaStream_t s);
-  // elements: current and scratch (x, y, z, m) + input index
+  cudaError_t launch_groups(int64_t max_leaves, int G, int half, cudaStream_t s);
+  // elements: current and scratch (x, y, z, m) + input index; epos_ ends as the
+  // position table, the pseudo-particles behind the particles
   float4 *epos_ = nullptr, *tpos_ = nullptr;
   int32_t *oid_ = nullptr, *toid_ = nullptr, *idx_ = nullptr;
   int32_t *ridx_ = nullptr;  // partition: positions of the right elements by their rank
@@ -138,7 +140,6 @@ class DeviceTree {
   unsigned char *acc_ = nullptr;  // per node: statistics in the making
   unsigned *ticket_ = nullptr;    // per node: its chunks done
   size_t cap_ac_ = 0;
-  unsigned char *ctl_ = nullptr, *h_ctl_ = nullptr;  // the levels' extents, and a pinned copy
   cudaError_t grow_chunks(size_t chunks, size_t nodes, cudaStream_t s);
   int32_t *left_cnt_ = nullptr, *left_base_ = nullptr;
   int32_t *wpre_ = nullptr;  // per chunk: each warp's left elements before its share
@@ -152,8 +153,9 @@ class DeviceTree {
   size_t cap_fb_ = 0;
   double *tight_chunks_ = nullptr, *tight_nodes_ = nullptr;  // tight c.m. certification
   size_t cap_tc_ = 0, cap_tn_ = 0;
-  int64_t *counters_ = nullptr;  // device scalars
-  int64_t *h_counters_ = nullptr;  // pinned mirror
+  // device scalars, per-depth subtree totals and the levels' extents, one
+  // block, and a pinned copy
+  int64_t *counters_ = nullptr, *h_counters_ = nullptr;
   // lists
   int32_t *leaf_ids_ = nullptr;
   size_t cap_leaf_ = 0;
@@ -168,23 +170,19 @@ class DeviceTree {
   size_t cap_segl_ = 0;
   int32_t *idx_list_ = nullptr;
   size_t cap_idx_ = 0;
-  float4 *table_ = nullptr;
-  size_t cap_tab_ = 0;
   PairItem *items_ = nullptr, *items_tmp_ = nullptr;
   size_t cap_items_ = 0, cap_items_tmp_ = 0;
   int32_t *gidx_ = nullptr;
   size_t cap_gidx_ = 0;
   int32_t *walk_err_ = nullptr;
   // whole subtrees in one block (k_subtree): node scratch, per-root depth
-  // bookkeeping, placement offsets, per-depth totals (and their pinned copy)
+  // bookkeeping, placement offsets
   DNode *sub_nodes_ = nullptr;
   int32_t *sub_first_ = nullptr;
   int2 *roots_ = nullptr;  // subtree roots: node, element buffer
   size_t cap_ro_ = 0;
   int32_t *sub_hist_ = nullptr;
-  int64_t *sub_tot_ = nullptr;
   size_t cap_sub_ = 0, cap_sf_ = 0, cap_sh_ = 0;
-  int64_t *h_sub_ = nullptr;
   bool sub_off_ = false;  // when set, every level runs in the level loop
 };
 
