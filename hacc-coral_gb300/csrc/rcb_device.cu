@@ -294,12 +294,13 @@ struct LevelCtl {
   int32_t next_level;  // the level made last
   int32_t begin[kCtlLevels];  // first node of a level, by level modulo kCtlLevels
 };
-// A chunk is PT elements a thread of its block: 16 (4096 elements) keep the
-// per-block work (reductions, tickets) small beside the elements where there
-// are enough of them to fill the GPU; sets of up to kSmallSet take 4, four
-// times as many blocks whose threads go through a quarter of the dependent
-// loads (a level of 68 thousand elements: 62 us with 16).
-constexpr int64_t kSmallSet = 1 << 20;
+// A chunk is PT elements a thread of its block: the fewest of 4, 8 and 16 that
+// leave at most kLevelBlocks chunks an SM, one wave of blocks.  More elements a
+// thread are more dependent loads (a level of 68 thousand elements: 62 us with
+// 16, 44 with 4); more blocks than a wave, and the per-block work (reductions,
+// tickets) counts twice (the levels of a 1.15 M set: 0.66 ms with 16 or 4, 0.60
+// with 8; of 2.6 M: 1.10 ms with 16, 1.31 with 4, 1.13 with 24).
+constexpr int64_t kLevelBlocks = 4;
 template <int PT>
 __host__ __device__ constexpr int32_t chunk_size() { return PT * kChunkThreads; }
 template <int PT>
@@ -3496,11 +3497,13 @@ cudaError_t DeviceTree::build(const TreeConfig &cfg, int64_t n, const float4 *po
   // bookkeeping, every level runs here.
   const bool subtrees = n == 0 || (!sub_off_ && cfg.force_cm_fallback != 2);
   const int32_t sub_max = subtrees ? kSubMax : -1;
-  const bool small = n <= kSmallSet;
-  const int64_t chunk = small ? chunk_size<4>() : chunk_size<16>();
+  const int64_t wave = kLevelBlocks * sm_count();
+  const int pt = n <= wave * chunk_size<4>() ? 4 : (n <= wave * chunk_size<8>() ? 8 : 16);
+  const int64_t chunk = int64_t(pt) * kChunkThreads;
 #define LEVEL_LAUNCH(kern, grid, ...)                                             \
   do {                                                                            \
-    if (small) launch_chained(kern<4>, grid, kChunkThreads, 0, s, __VA_ARGS__);   \
+    if (pt == 4) launch_chained(kern<4>, grid, kChunkThreads, 0, s, __VA_ARGS__); \
+    else if (pt == 8) launch_chained(kern<8>, grid, kChunkThreads, 0, s, __VA_ARGS__); \
     else launch_chained(kern<16>, grid, kChunkThreads, 0, s, __VA_ARGS__);        \
     ++info_.launches;                                                             \
   } while (0)
