@@ -2553,6 +2553,18 @@ __global__ void __launch_bounds__(32 * kWalkWarps)
   }
 }
 
+// Room in the buffers that the list kernels write, for launches made before the
+// host has seen the counts: they do nothing where a count is above it (or the
+// walk has failed or needs its second pass), and the host launches them again
+// once it has made room.  idx < 0: the host knows that there is room.
+struct ListRoom {
+  int64_t idx, segs, items;
+};
+__device__ __forceinline__ bool lists_fit(const int64_t *counters, const ListRoom &R) {
+  return R.idx < 0 || (counters[C_NENT] <= R.idx && counters[C_NSEG] <= R.segs &&
+                       counters[C_SEGOVF] == 0 && counters[C_ERR] == 0);
+}
+
 // Expands each leaf's segments into the index array at the leaf's list_base,
 // keeping only the entries within sqrt(cull2) of the leaf's box (cull2 <= 0:
 // every entry): the others are farther than the cutoff from every particle of
@@ -2569,10 +2581,12 @@ __global__ void __launch_bounds__(256)
     k_expand_pruned(const int2 *__restrict__ local, SegDesc *__restrict__ segs,
                     const int64_t *__restrict__ seg_base, const int64_t *__restrict__ seg_cnt,
                     const int64_t *__restrict__ list_base, const DNode *__restrict__ nodes,
-                    const int32_t *__restrict__ leaf_ids, int64_t nleaves,
-                    const float4 *__restrict__ table, float cull2, int32_t *__restrict__ idx,
-                    int64_t *__restrict__ kept) {
+                    const int32_t *__restrict__ leaf_ids, const int64_t *__restrict__ counters,
+                    ListRoom room, const float4 *__restrict__ table, float cull2,
+                    int32_t *__restrict__ idx, int64_t *__restrict__ kept) {
   chain_enter();
+  if (!lists_fit(counters, room)) return;
+  const int64_t nleaves = counters[C_NLEAF];
   constexpr int kU = 4;
   const unsigned full = 0xffffffffu;
   const int lane = threadIdx.x & 31;
@@ -2936,10 +2950,12 @@ __device__ __forceinline__ int len_bucket(int64_t len) {
 // list statistics.
 template <bool DESC>
 __global__ void __launch_bounds__(128)
-    k_leaf_items(const DNode *nodes, const int32_t *leaf_ids, int64_t nleaves,
-                 const int64_t *list_len, const int64_t *kept_len, const int64_t *list_base,
-                 LeafDesc *ld, int64_t jsplit, int G, int64_t *counters) {
+    k_leaf_items(const DNode *nodes, const int32_t *leaf_ids, const int64_t *list_len,
+                 const int64_t *kept_len, const int64_t *list_base, LeafDesc *ld, int64_t jsplit,
+                 int G, int64_t *counters, ListRoom room) {
   chain_enter();
+  if (!lists_fit(counters, room)) return;
+  const int64_t nleaves = counters[C_NLEAF];
   __shared__ unsigned long long hist[32];
   __shared__ bool last;
   if (threadIdx.x < 32) hist[threadIdx.x] = 0;
@@ -3000,9 +3016,11 @@ __global__ void __launch_bounds__(128)
 }
 
 __global__ void __launch_bounds__(128)
-    k_item_fill(const LeafDesc *ld, int64_t nleaves, int64_t jsplit, int G, int64_t *counters,
-                PairItem *items) {
+    k_item_fill(const LeafDesc *ld, int64_t jsplit, int G, int64_t *counters, PairItem *items,
+                ListRoom room) {
   chain_enter();
+  if (!lists_fit(counters, room) || (room.idx >= 0 && counters[C_NITEMS] > room.items)) return;
+  const int64_t nleaves = counters[C_NLEAF];
   // positions inside the block's share of each bucket, then one global
   // reservation a bucket
   __shared__ unsigned long long cnt[32], base[32];
@@ -3721,9 +3739,41 @@ cudaError_t DeviceTree::build(const TreeConfig &cfg, int64_t n, const float4 *po
     DT_CHECK(scan_counted(list_len, list_base, max_leaves, counters_ + C_NENT, scan_tmp_, s));
   }
   DT_CHECK(cudaGetLastError());
-  // leaves, segments, entries, the overflow flag and the error flag in one copy
-  DT_CHECK(cudaMemcpyAsync(h_counters_ + C_NLEAF, counters_ + C_NLEAF,
-                           (C_ERR + 1 - C_NLEAF) * sizeof(int64_t), cudaMemcpyDeviceToHost, s));
+  DT_CHECK(grow(leafdesc_, cap_ld_, nlw, s));
+  int64_t *kept = node_tmp_ + 4 * nlw;
+  constexpr ListRoom kRoom{-1, -1, -1};
+  // the index lists and the work items' counts, from the walk's regions or from
+  // a second walk's segments
+  auto expand = [&](bool local, int64_t leaves, const ListRoom &room) {
+    const unsigned blocks = unsigned(std::min<int64_t>((leaves + 7) / 8, int64_t(sm_count()) * 64));
+    if (local)
+      launch_chained(k_expand_pruned<true>, blocks, 256, 0, s, segs_local_, segs_, seg_base, seg_cnt,
+                     list_base, nodes_, leaf_ids_, counters_, room, table, cfg.prune2, idx_list_,
+                     kept);
+    else
+      launch_chained(k_expand_pruned<false>, blocks, 256, 0, s, nullptr, segs_, seg_base, seg_cnt,
+                     list_base, nodes_, leaf_ids_, counters_, room, table, cfg.prune2, idx_list_,
+                     kept);
+    launch_chained(k_leaf_items<true>, unsigned((leaves + 127) / 128), 128, 0, s, nodes_, leaf_ids_,
+                   list_len, kept, list_base, leafdesc_, jsplit, group_, counters_, room);
+    info_.launches += 2;
+  };
+  // With the buffers of an earlier build the lists and the items are launched
+  // before the host has seen their sizes; one look then tells whether all of it
+  // fitted.  (A look after the walk and another after the item counts cost a
+  // kick of 5 to 70 thousand particles 25 us.)
+  const ListRoom room{int64_t(cap_idx_), int64_t(cap_seg_), int64_t(cap_items_)};
+  const bool ahead = room.idx > 0 && room.segs > 0 && room.items > 0;
+  if (ahead) {
+    expand(true, max_leaves, room);
+    DT_CHECK(cudaStreamWaitEvent(s, ev_groups_, 0));
+    groups_ready_ = 0;
+    launch_chained(k_item_fill, unsigned((max_leaves + 127) / 128), 128, 0, s, leafdesc_, jsplit,
+                   group_, counters_, items_, room);
+    ++info_.launches;
+    DT_CHECK(cudaGetLastError());
+  }
+  DT_CHECK(cudaMemcpyAsync(h_counters_, counters_, C_COUNT * sizeof(int64_t), cudaMemcpyDeviceToHost, s));
   DT_CHECK(cudaStreamSynchronize(s));
   const int32_t h_err = *reinterpret_cast<const int32_t *>(h_counters_ + C_ERR);
   if (h_err) {
@@ -3737,36 +3787,25 @@ cudaError_t DeviceTree::build(const TreeConfig &cfg, int64_t n, const float4 *po
   const int64_t nent = h_counters_[C_NENT];
   info_.segments = nseg;
   info_.list_entries = nent;
-  DT_CHECK(grow(segs_, cap_seg_, size_t(std::max<int64_t>(nseg, 1)), s));
-  DT_CHECK(grow(idx_list_, cap_idx_, size_t(std::max<int64_t>(nent, 1)), s));
-  DT_CHECK(grow(leafdesc_, cap_ld_, nlw, s));
-  if (nleaves > 0) {
-    int64_t *kept = node_tmp_ + 4 * nlw;
-    const unsigned blocks =
-        unsigned(std::min<int64_t>((nleaves + 7) / 8, int64_t(sm_count()) * 64));
-    if (h_counters_[C_SEGOVF]) {
-      const unsigned gW = unsigned((nleaves + kWalkWarps - 1) / kWalkWarps);
-      launch_chained(k_walk<1>, gW, 32 * kWalkWarps, 0, s, nodes_, nnodes, leaf_ids_, nleaves, cfg,
-                     n, nullptr, nullptr, seg_base, list_base, segs_, nullptr, walk_err_,
-                     counters_);
-      ++info_.launches;
-      launch_chained(k_expand_pruned<false>, blocks, 256, 0, s, nullptr, segs_, seg_base, seg_cnt,
-                     list_base, nodes_, leaf_ids_, nleaves, table, cfg.prune2, idx_list_, kept);
-    } else {
-      launch_chained(k_expand_pruned<true>, blocks, 256, 0, s, segs_local_, segs_, seg_base,
-                     seg_cnt, list_base, nodes_, leaf_ids_, nleaves, table, cfg.prune2, idx_list_,
-                     kept);
+  const bool local = !h_counters_[C_SEGOVF];
+  if (!ahead || !local || nent > room.idx || nseg > room.segs) {
+    DT_CHECK(grow(segs_, cap_seg_, size_t(std::max<int64_t>(nseg, 1)), s));
+    DT_CHECK(grow(idx_list_, cap_idx_, size_t(std::max<int64_t>(nent, 1)), s));
+    if (nleaves > 0) {
+      if (!local) {
+        const unsigned gW = unsigned((nleaves + kWalkWarps - 1) / kWalkWarps);
+        launch_chained(k_walk<1>, gW, 32 * kWalkWarps, 0, s, nodes_, nnodes, leaf_ids_, nleaves, cfg,
+                       n, nullptr, nullptr, seg_base, list_base, segs_, nullptr, walk_err_,
+                       counters_);
+        ++info_.launches;
+      }
+      expand(local, nleaves, kRoom);
     }
-    ++info_.launches;
-    launch_chained(k_leaf_items<true>, unsigned((nleaves + 127) / 128), 128, 0, s, nodes_,
-                   leaf_ids_, nleaves, list_len, kept, list_base, leafdesc_, jsplit, group_,
-                   counters_);
-    ++info_.launches;
+    DT_CHECK(cudaGetLastError());
+    DT_CHECK(fill_items(jsplit, s));
+  } else {
+    DT_CHECK(place_items(jsplit, h_counters_[C_NITEMS] <= room.items, s));
   }
-  DT_CHECK(cudaGetLastError());
-
-  // ---- work items ----
-  DT_CHECK(fill_items(jsplit, s));
   lists_ms_ = std::chrono::duration<double, std::milli>(std::chrono::steady_clock::now() - t1).count();
   return cudaSuccess;
 }
@@ -3819,9 +3858,9 @@ cudaError_t DeviceTree::regroup(int group, int64_t jsplit, cudaStream_t s) {
   DT_CHECK(cudaMemsetAsync(counters_ + C_TICKET, 0, sizeof(int64_t), s));
   if (nleaves > 0) {
     DT_CHECK(launch_groups(nleaves, group, group, s));
-    launch_chained(k_leaf_items<false>, unsigned((nleaves + 127) / 128), 128, 0, s, nullptr,
-                   nullptr, nleaves, nullptr, nullptr, nullptr, leafdesc_, jsplit, group,
-                   counters_);
+    launch_chained(k_leaf_items<false>, unsigned((nleaves + 127) / 128), 128, 0, s, nullptr, nullptr,
+                   nullptr, nullptr, nullptr, leafdesc_, jsplit, group, counters_,
+                   ListRoom{-1, -1, -1});
     ++info_.launches;
   }
   return fill_items(jsplit, s);
@@ -3843,14 +3882,21 @@ cudaError_t DeviceTree::fill_items(int64_t jsplit, cudaStream_t s) {
   groups_ready_ = 0;
   DT_CHECK(cudaMemcpyAsync(h_counters_, counters_, C_COUNT * sizeof(int64_t), cudaMemcpyDeviceToHost, s));
   DT_CHECK(cudaStreamSynchronize(s));
+  return place_items(jsplit, false, s);
+}
+
+// The items' totals from the counters read back, and the items themselves
+// unless they are placed already.
+cudaError_t DeviceTree::place_items(int64_t jsplit, bool placed, cudaStream_t s) {
+  const int64_t nleaves = info_.processed_leaves;
   const int64_t nitems = nleaves > 0 ? h_counters_[C_NITEMS] : 0;
   info_.items = nitems;
   info_.pairs = h_counters_[C_PAIRS];
   padded_pairs_ = h_counters_[C_PADDED];
   DT_CHECK(grow(items_, cap_items_, size_t(std::max<int64_t>(nitems, 1)), s));
-  if (nitems > 0) {
-    launch_chained(k_item_fill, unsigned((nleaves + 127) / 128), 128, 0, s, leafdesc_, nleaves,
-                   jsplit, group_, counters_, items_);
+  if (nitems > 0 && !placed) {
+    launch_chained(k_item_fill, unsigned((nleaves + 127) / 128), 128, 0, s, leafdesc_, jsplit,
+                   group_, counters_, items_, ListRoom{-1, -1, -1});
     ++info_.launches;
   }
   return cudaGetLastError();

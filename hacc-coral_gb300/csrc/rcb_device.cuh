@@ -74,8 +74,8 @@ class DeviceTree {
   // then tdpts pseudo-particles per node), and the processed leaves' lists,
   // work items and group index are built.  `jsplit` bounds the list range of
   // one work item.  Synchronizes `s` after the tree (which is made without a
-  // look from the host, unless a level has centres of mass to certify), after
-  // the list counts and after the item counts.
+  // look from the host, unless a level has centres of mass to certify) and after
+  // the work items (and between, where the buffers have to grow).
   cudaError_t build(const TreeConfig &cfg, int64_t n, const float4 *pos_in, int64_t jsplit,
                     cudaStream_t s);
 
@@ -109,6 +109,7 @@ class DeviceTree {
   template <typename T>
   cudaError_t grow(T *&p, size_t &cap, size_t count, cudaStream_t s, bool keep = false);
   cudaError_t fill_items(int64_t jsplit, cudaStream_t s);
+  cudaError_t place_items(int64_t jsplit, bool placed, cudaStream_t s);
   // exclusive_scan_i64, adding its kernels to info_.launches
   cudaError_t scan_counted(const int64_t *in, int64_t *out, int64_t n, int64_t *total, int64_t *tmp,
                            cudaStream_t s);

@@ -37,3 +37,31 @@ def test_lists_in_the_host_builds_order(ctx, make, nd, tdpts, angle):
     # pseudo-particles (n and above) go by each build's own node numbers
     a, b = ctx.lists_index(), host.index()
     assert np.array_equal(np.minimum(a, p.n), np.minimum(b, p.n))
+
+
+def test_lists_launched_ahead_of_their_sizes(hsr_lib):
+    """One context over sets that do and do not fit the buffers of the call
+    before: more entries, fewer, the same entries in more work items, and lists
+    that need the second walk; each call's lists as the host builds them."""
+    ctx = hsr.Context()
+    try:
+        for n, side, nd, group in ((900, 9.0, 32, 32), (6000, 14.0, 16, 32), (900, 9.0, 32, 32),
+                                   (6000, 14.0, 64, 32), (6000, 14.0, 64, 16), (3000, 9.0, 2, 16),
+                                   (6000, 14.0, 16, 16), (1, 9.0, 32, 32), (6000, 14.0, 64, 16)):
+            ctx.set_tune("batched", 128, group)
+            p = synth.random_box(n, side, n + nd)
+            kp = synth.kick_params(p, nd=nd, fcoeff=1.0)
+            kp.min_force, kp.max_force = (0.2,) * 3, tuple(float(g) for g in p.nglt)
+            q, v = p.copy(), p.copy()
+            host = hsr.HostLists(q, kp)
+            ctx.rcb_kick(p, kp)
+            for a, b in zip(ctx.lists(), host.get()):
+                assert np.array_equal(a.view(np.uint8), b.view(np.uint8)), (n, nd, group)
+            fresh = hsr.Context()
+            fresh.set_tune("batched", 128, group)
+            fresh.rcb_kick(v, kp)
+            assert fresh.stats()["work_items"] == ctx.stats()["work_items"]
+            assert np.array_equal(p.vx, v.vx) and np.array_equal(p.id, v.id)
+            fresh.close()
+    finally:
+        ctx.close()
