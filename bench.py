@@ -606,8 +606,8 @@ def main():
         qb = [pinned_copy(b) for b in boxes]
         walls = []
         for r in range(3 + max(3, args.steps // 2)):
-            for q, b in zip(qb, boxes):
-                refill(q, b)
+            for qi, b in zip(qb, boxes):
+                refill(qi, b)
             t0 = time.perf_counter()
             stb = ctx.rcb_kick_batch(qb, kpb)
             if r >= 3:
