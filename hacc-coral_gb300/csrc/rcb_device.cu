@@ -2260,9 +2260,77 @@ __global__ void k_links(const DNode *nodes, int32_t nnodes, int2 *up) {
 // child's particles or points, left child first), so the points of a node run
 // in parallel and no level waits for a launch of its own.  A monopole leaf's
 // mass is the sequential float sum of its particles' masses, loaded 32 at a
-// time and added in order from shuffles.  (With one lane a node and a launch a
+// time and added in order from shuffles (monopole_climb).  (With one lane a node and a launch a
 // level, 12-point masses took 3.6 of the 9.8 ms of a clustered 48^3 forward and
 // adjoint, and a 32^3 kick's monopoles 52 us.)
+// A monopole's climb loads the parent's record and links, and the sibling's
+// count, while its own results become visible, and has its own mass in a
+// register, so a step waits for the fence, the arrival and the sibling's mass
+// only (a kick of 4780 particles: 365 to 348 us, of 67,836: 523 to 510).
+__device__ __forceinline__ void monopole_climb(DNode *nodes, int32_t nnodes, int2 *up,
+                                               const float4 *__restrict__ pos, float *ppm,
+                                               float4 *table, int64_t n, const TreeConfig &cfg,
+                                               int32_t *processed, int32_t t, int lane) {
+  const unsigned full = 0xffffffffu;
+  DNode T = nodes[t];
+  int2 U = up[t];
+  int32_t below = leaf_in_force_box(T, cfg) ? 1 : 0;
+  float m = 0.f;
+  // a leaf's mass in its particles' order; a leaf left by a failed split keeps
+  // zero (its children are empty)
+  if (T.count <= cfg.nd && T.count > 1) {
+    const float *w = reinterpret_cast<const float *>(pos + T.offset) + 3;
+    for (int32_t i0 = 0; i0 < T.count; i0 += 32) {
+      const float v = i0 + lane < T.count ? w[4 * (i0 + lane)] : 0.f;
+      const int nv = min(32, T.count - i0);
+      for (int i = 0; i < nv; ++i) m = fadd_(m, __shfl_sync(full, v, i));
+    }
+  }
+  for (int climbed = 0; climbed <= nnodes; ++climbed) {
+    const int32_t parent = U.x;
+    const bool left = U.y & kLeftChild;
+    const int32_t sib = left ? t + 1 : t - 1;
+    DNode TP{};
+    int2 UP = make_int2(-1, 0);
+    int32_t scount = 0, soff = 0;
+    if (t != 0) {
+      TP = nodes[parent];
+      UP = up[parent];
+      scount = nodes[sib].count;
+      soff = nodes[sib].offset;
+    }
+    if (lane == 0) {
+      const float tdr = fmul_(cfg.ppc, pptdr_(T));
+      float x, y, z;
+      pppt_<1>(0, tdr, T.xc, x, y, z);
+      ppm[t] = m;
+      table[n + t] = make_float4(x, y, z, m);
+      nodes[t].tdr = tdr;
+      processed[t] = below;
+    }
+    if (t == 0) return;
+    __threadfence();
+    __syncwarp();
+    int arrived = 0;
+    if (lane == 0) arrived = atomicAdd(&up[parent].y, 1) & 0xff;
+    if (__shfl_sync(full, arrived, 0) == 0) return;  // the sibling's warp goes on
+    __threadfence();
+    // the children's masses, left first; a child of one particle is that
+    // particle, one of none adds nothing
+    const float mine = T.count == 1 ? pos[T.offset].w : m;
+    const float other = scount > 1 ? __ldcg(ppm + sib) : (scount == 1 ? pos[soff].w : 0.f);
+    below += __ldcg(processed + sib);
+    const float l = left ? mine : other, r = left ? other : mine;
+    const int32_t lc = left ? T.count : scount, rc = left ? scount : T.count;
+    m = 0.f;
+    if (lc > 0) m = fadd_(m, l);
+    if (rc > 0) m = fadd_(m, r);
+    t = parent;
+    T = TP;
+    U = UP;
+  }
+}
+
 template <int K>
 __global__ void __launch_bounds__(128)
     k_pseudo_up(DNode *nodes, int32_t nnodes, int2 *up, const float4 *__restrict__ pos, float *ppm,
@@ -2273,6 +2341,10 @@ __global__ void __launch_bounds__(128)
   int32_t t = int32_t((int64_t(blockIdx.x) * blockDim.x + threadIdx.x) >> 5);
   if (t >= nnodes) return;  // whole warps
   if (nodes[t].cl != 0) return;
+  if (K == 1) {
+    monopole_climb(nodes, nnodes, up, pos, ppm, table, n, cfg, processed, t, lane);
+    return;
+  }
   for (int climbed = 0; climbed <= nnodes; ++climbed) {
     const DNode T = nodes[t];
     const float tdr = fmul_(cfg.ppc, pptdr_(T));
@@ -2286,20 +2358,10 @@ __global__ void __launch_bounds__(128)
       // failed split keeps zero masses (its children are empty)
       if (T.count <= cfg.nd && T.count > K) {
         const float4 *p = pos + T.offset;
-        if (K == 1) {
-          // every term's weight is 1/1 + 0 + 0 (PointMass with rj2 == 0)
-          const float *w = reinterpret_cast<const float *>(p) + 3;
-          for (int32_t i0 = 0; i0 < T.count; i0 += 32) {
-            const float v = i0 + lane < T.count ? w[4 * (i0 + lane)] : 0.f;
-            const int nv = min(32, T.count - i0);
-            for (int i = 0; i < nv; ++i) P.m = fadd_(P.m, fmul_(__shfl_sync(full, v, i), 1.0f));
-          }
-        } else {
 #pragma unroll 4
-          for (int32_t i = 0; i < T.count; ++i) {
-            const float4 q = p[i];
-            P.add(q.x, q.y, q.z, q.w, tdr, T.xc);
-          }
+        for (int32_t i = 0; i < T.count; ++i) {
+          const float4 q = p[i];
+          P.add(q.x, q.y, q.z, q.w, tdr, T.xc);
         }
       }
     } else {
