@@ -477,7 +477,12 @@ void quiet_tables(int ng, double *filter, double *denom, double *gradient) {
   for (int kk = 0; kk < ng; ++kk) denom[kk] = a0 + a1 * c1[kk] + a2 * c2[kk] + a3 * c3[kk];
 }
 
-Solver::~Solver() { release(); }
+Solver::~Solver() {
+  release();
+  if (aux_) cudaStreamDestroy(aux_);
+  if (ev_fork_) cudaEventDestroy(ev_fork_);
+  if (ev_join_) cudaEventDestroy(ev_join_);
+}
 
 void Solver::release() {
   if (have_fwd_) cufftDestroy(fwd_);
@@ -486,9 +491,10 @@ void Solver::release() {
   if (have_inv1_) cufftDestroy(inv1_);
   have_fwd_ = have_inv_ = have_fwd3_ = have_inv1_ = false;
   for (void *p : {(void *)rho_, real_, spec_, gspec_, greal_, green_, gtab_, (void *)grad_,
-                  (void *)adj_})
+                  (void *)adj_, aspec3_, aspec_, (void *)phibar_})
     if (p) cudaFree(p);
-  rho_ = adj_ = nullptr;
+  rho_ = adj_ = phibar_ = nullptr;
+  aspec3_ = aspec_ = nullptr;
   real_ = spec_ = gspec_ = greal_ = green_ = gtab_ = nullptr;
   grad_ = nullptr;
   ng_ = 0;
@@ -652,7 +658,18 @@ bool Solver::prepare_vjp(std::string *err) {
   const int64_t m = int64_t(ng) * ng * ng, mh = int64_t(ng) * ng * nh;
   if (!adj_ && !cu_ok(cudaMalloc(&adj_, 3 * m * sizeof(float)), "pm adjoint fields", err))
     return false;
-  if (prec_ == PREC_F64) return true;  // the forward solve's own plans
+  if (prec_ == PREC_F64) return true;  // the forward solve's own plans and grids
+  if (!aspec3_ && !cu_ok(cudaMalloc(&aspec3_, 3 * mh * sizeof(float2)), "pm adjoint spectra", err))
+    return false;
+  if (!aspec_ && !cu_ok(cudaMalloc(&aspec_, mh * sizeof(float2)), "pm adjoint spectrum", err))
+    return false;
+  if (!phibar_ && !cu_ok(cudaMalloc(&phibar_, m * sizeof(float)), "pm adjoint field", err))
+    return false;
+  if (!aux_ && !cu_ok(cudaStreamCreateWithFlags(&aux_, cudaStreamNonBlocking), "pm adjoint stream", err))
+    return false;
+  for (cudaEvent_t *e : {&ev_fork_, &ev_join_})
+    if (!*e && !cu_ok(cudaEventCreateWithFlags(e, cudaEventDisableTiming), "pm adjoint event", err))
+      return false;
   long long dims[3] = {ng, ng, ng};
   size_t ws = 0;
   if (!have_fwd3_) {
@@ -676,19 +693,23 @@ bool Solver::vjp(const Params &p, int64_t n, const float *x, const float *y, con
                  const float *vbx, const float *vby, const float *vbz, float *xbx, float *xby,
                  float *xbz, cudaStream_t s, std::string *err) {
   if (!prepare_vjp(err)) return false;
-  if (!deposit(p, n, x, y, z, s, err) || !solve(s, err)) return false;
-  if (n == 0) return true;
   const int ng = ng_, nh = ng / 2 + 1, nglt = ng + 2 * p.ngo + 1;
   const int64_t m = int64_t(ng) * ng * ng, mh = int64_t(ng) * ng * nh;
-  if (!cu_ok(cudaMemsetAsync(adj_, 0, 3 * m * sizeof(float), s), "pm adjoint clear", err))
-    return false;
-  k_adj_deposit<<<blocks_for(n), kThreads, 0, s>>>(n, x, y, z, vbx, vby, vbz, ng, p.ngo, nglt,
-                                                   adj_);
-  ++launches;
-  if (!cu_ok(cudaGetLastError(), "pm adjoint deposit", err)) return false;
   const float cm = p.gpscal * p.gpscal * p.gpscal;
   const float coef = p.fscal * p.tau;
+  // the deposit of the cotangents
+  auto adj_deposit = [&](cudaStream_t st) {
+    if (!cu_ok(cudaMemsetAsync(adj_, 0, 3 * m * sizeof(float), st), "pm adjoint clear", err))
+      return false;
+    k_adj_deposit<<<blocks_for(n), kThreads, 0, st>>>(n, x, y, z, vbx, vby, vbz, ng, p.ngo, nglt,
+                                                      adj_);
+    ++launches;
+    return cu_ok(cudaGetLastError(), "pm adjoint deposit", err);
+  };
   if (prec_ == PREC_F64) {
+    if (!deposit(p, n, x, y, z, s, err) || !solve(s, err)) return false;
+    if (n == 0) return true;
+    if (!adj_deposit(s)) return false;
     k_divergence<<<blocks_for(m), kThreads, 0, s>>>(ng, adj_, (double *)real_);
     if (!fft_ok(cufftExecD2Z(fwd_, (cufftDoubleReal *)real_, (cufftDoubleComplex *)spec_),
                 "pm adjoint forward transform", err))
@@ -700,24 +721,49 @@ bool Solver::vjp(const Params &p, int64_t n, const float *x, const float *y, con
     k_vjp_interp<double><<<blocks_for(n), kThreads, 0, s>>>(
         n, x, y, z, vbx, vby, vbz, ng, p.ngo, nglt, grad_, (const double *)real_, cm, coef, xbx,
         xby, xbz);
-  } else {
-    if (!fft_ok(cufftSetStream(fwd3_, s), "pm adjoint stream", err)) return false;
-    if (!fft_ok(cufftSetStream(inv1_, s), "pm adjoint stream", err)) return false;
-    if (!fft_ok(cufftExecR2C(fwd3_, (cufftReal *)adj_, (cufftComplex *)gspec_),
+    launches += 3;
+    fft_execs += 2;
+    return cu_ok(cudaGetLastError(), "pm adjoint kernels", err);
+  }
+  // Single precision: the density's solve and the cotangents' meet only at the
+  // particles, and their transforms are kernels of 5 to 10 us that leave most of
+  // the GPU idle, so the cotangents go on a second stream (double precision
+  // fills the FP64 pipe with either).  1.3 M particles on 100^3 cells: 246 us
+  // one after the other, 203 so.
+  struct Join {
+    cudaStream_t aux;
+    bool pending = false;
+    ~Join() {  // a return in between: nothing of the caller's may still be read
+      if (pending) cudaStreamSynchronize(aux);
+    }
+  } join{aux_};
+  if (n > 0) {
+    if (!cu_ok(cudaEventRecord(ev_fork_, s), "pm adjoint fork", err)) return false;
+    if (!cu_ok(cudaStreamWaitEvent(aux_, ev_fork_, 0), "pm adjoint fork", err)) return false;
+    join.pending = true;
+    if (!adj_deposit(aux_)) return false;
+    if (!fft_ok(cufftSetStream(fwd3_, aux_), "pm adjoint stream", err)) return false;
+    if (!fft_ok(cufftSetStream(inv1_, aux_), "pm adjoint stream", err)) return false;
+    if (!fft_ok(cufftExecR2C(fwd3_, (cufftReal *)adj_, (cufftComplex *)aspec3_),
                 "pm adjoint forward transform", err))
       return false;
-    k_adj_spectra<<<blocks_for(mh), kThreads, 0, s>>>(
-        ng, nh, (const float2 *)gspec_, (const float *)green_, (const float *)gtab_,
-        (float2 *)spec_);
-    // the density grid is free once the solve ran: the inverse lands there
-    if (!fft_ok(cufftExecC2R(inv1_, (cufftComplex *)spec_, (cufftReal *)rho_),
+    k_adj_spectra<<<blocks_for(mh), kThreads, 0, aux_>>>(
+        ng, nh, (const float2 *)aspec3_, (const float *)green_, (const float *)gtab_,
+        (float2 *)aspec_);
+    ++launches;
+    if (!cu_ok(cudaGetLastError(), "pm adjoint spectra", err)) return false;
+    if (!fft_ok(cufftExecC2R(inv1_, (cufftComplex *)aspec_, (cufftReal *)phibar_),
                 "pm adjoint inverse transform", err))
       return false;
-    k_vjp_interp<float><<<blocks_for(n), kThreads, 0, s>>>(n, x, y, z, vbx, vby, vbz, ng, p.ngo,
-                                                          nglt, grad_, rho_, cm, coef, xbx, xby,
-                                                          xbz);
+    if (!cu_ok(cudaEventRecord(ev_join_, aux_), "pm adjoint join", err)) return false;
   }
-  launches += prec_ == PREC_F64 ? 3 : 2;
+  if (!deposit(p, n, x, y, z, s, err) || !solve(s, err)) return false;
+  if (n == 0) return true;
+  if (!cu_ok(cudaStreamWaitEvent(s, ev_join_, 0), "pm adjoint join", err)) return false;
+  join.pending = false;
+  k_vjp_interp<float><<<blocks_for(n), kThreads, 0, s>>>(n, x, y, z, vbx, vby, vbz, ng, p.ngo, nglt,
+                                                        grad_, phibar_, cm, coef, xbx, xby, xbz);
+  ++launches;
   fft_execs += 2;
   return cu_ok(cudaGetLastError(), "pm adjoint kernels", err);
 }

@@ -67,7 +67,8 @@ struct Timing {
 };
 
 // Plans, Green's function and grids for one (ng, precision); rebuilt when
-// either changes.  Everything runs on the stream given to each call.
+// either changes.  Everything runs on the stream given to each call, or on one
+// that waits for it and that it waits for before the call returns.
 class Solver {
  public:
   ~Solver();
@@ -112,6 +113,13 @@ class Solver {
   cufftHandle fwd3_ = 0, inv1_ = 0;
   bool have_fwd3_ = false, have_inv1_ = false;
   float *adj_ = nullptr;     // 3 x ng^3: deposited cotangents (float atomics)
+  // single-precision adjoint: its transforms run on a stream of their own
+  // beside the forward solve's, with their own grids (spectra of the deposits,
+  // the combined spectrum, phibar)
+  cudaStream_t aux_ = nullptr;
+  cudaEvent_t ev_fork_ = nullptr, ev_join_ = nullptr;
+  void *aspec3_ = nullptr, *aspec_ = nullptr;
+  float *phibar_ = nullptr;
   bool prepare_vjp(std::string *err);
   float *rho_ = nullptr;     // ng^3
   void *real_ = nullptr;     // ng^3 double: transform input, potential (double only)

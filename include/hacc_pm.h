@@ -68,8 +68,9 @@ typedef struct hsr_pm_stats {
   double t_d2h_ms;          /* host arrays: velocities back (events)        */
   int64_t h2d_bytes, d2h_bytes;
   int64_t kernel_launches;  /* this library's kernels                       */
-  int64_t fft_execs;        /* cuFFT executions (one forward, one batched
-                               inverse of the three components)             */
+  int64_t fft_execs;        /* cuFFT executions (one forward, one inverse:
+                               the potential, or in single precision the
+                               three components in a batch)                 */
 } hsr_pm_stats;
 
 /* The PM kick: v_d += fscal * tau * (inverse CIC of the d-th gradient
