@@ -1459,22 +1459,47 @@ __global__ void __launch_bounds__(kTightThreads)
   __syncthreads();
   if (!last) return;
   __threadfence();
-  for (int f = threadIdx.x; f < nt; f += blockDim.x) {
-    double hi[4] = {0, 0, 0, 0}, lo[4] = {0, 0, 0, 0}, a[4] = {0, 0, 0, 0};
-    for (int32_t g = cbase[f]; g < cbase[f + 1]; ++g) {
-      TightChunk &c = chunks[g];
-      for (int q = 0; q < 4; ++q) {
-        c.pre[q] = hi[q] + lo[q];
-        dd_add(hi[q], lo[q], c.hi[q], c.lo[q]);
-        a[q] = __dadd_ru(a[q], c.a[q]);
-      }
+  // a node at a time, 64 threads a sum: each adds up a run of chunks, one a sum
+  // the 64 runs, and then each goes through its run again for the prefixes (a
+  // thread a node took 2.4 of the 2.6 ms of a node of 2.4 M elements)
+  constexpr int kRuns = kTightThreads / 4;
+  __shared__ double rh[4][kRuns], rl[4][kRuns], ra[4][kRuns];
+  const int q = threadIdx.x / kRuns, run = threadIdx.x % kRuns;
+  for (int f = 0; f < nt; ++f) {
+    const int32_t c0 = cbase[f], nc = cbase[f + 1] - c0;
+    const int32_t per = (nc + kRuns - 1) / kRuns;
+    const int32_t g0 = c0 + min(nc, run * per), g1 = c0 + min(nc, (run + 1) * per);
+    double hi = 0, lo = 0, a = 0;
+    for (int32_t g = g0; g < g1; ++g) {
+      dd_add(hi, lo, chunks[g].hi[q], chunks[g].lo[q]);
+      a = __dadd_ru(a, chunks[g].a[q]);
     }
-    for (int q = 0; q < 4; ++q) {
-      tn[f].hi[q] = hi[q];
-      tn[f].lo[q] = lo[q];
-      tn[f].a[q] = a[q];
+    rh[q][run] = hi;
+    rl[q][run] = lo;
+    ra[q][run] = a;
+    __syncthreads();
+    if (run == 0) {
+      hi = lo = a = 0;
+      for (int r = 0; r < kRuns && r * per < nc; ++r) {
+        const double h = rh[q][r], l = rl[q][r];
+        rh[q][r] = hi;  // before the run
+        rl[q][r] = lo;
+        dd_add(hi, lo, h, l);
+        a = __dadd_ru(a, ra[q][r]);
+      }
+      tn[f].hi[q] = hi;
+      tn[f].lo[q] = lo;
+      tn[f].a[q] = a;
       tn[f].b[q] = 0.0;
     }
+    __syncthreads();
+    hi = rh[q][run];
+    lo = rl[q][run];
+    for (int32_t g = g0; g < g1; ++g) {
+      chunks[g].pre[q] = hi + lo;
+      dd_add(hi, lo, chunks[g].hi[q], chunks[g].lo[q]);
+    }
+    __syncthreads();  // the next node's runs take these ones' place
   }
   if (threadIdx.x == 0) counters[C_TDONE1] = 0;
 }
