@@ -52,7 +52,7 @@ enum { C_NFALLBACK = 2, C_NLEAF = 3, C_NSEG = 4, C_NENT = 5,
        C_SUBFB = 80, C_CHAINS = 81, C_TICKET = 82, C_SEQ = 83, C_COUNT = 84 };
 
 // Segments a leaf's walk can leave in its own region of the one-pass walk (8
-// bytes each); a leaf with more sends the build to a second, placing walk.
+// bytes each); a leaf with more is walked a second time, its segments placed.
 constexpr int kLocalSegs = 256;
 
 __device__ __forceinline__ float warp_min(float v) {
@@ -2475,7 +2475,8 @@ constexpr int kWalkReserve = 256;  // fills, to one node at a time over the last
 
 // The leaves are the first counters[C_NLEAF] of leaf_ids (max_leaves bounds
 // them: the host need not wait for their number).
-// MODE 1: writes the segments at seg_base / list_base; 2: counts (segments and
+// MODE 1, leaves with more than kLocalSegs segments only: writes the segments at
+// seg_base / list_base; 2: counts (segments and
 // entries per leaf) and writes the first kLocalSegs segments (start, count) of
 // each leaf into its own region, flagging leaves with more in
 // counters[C_SEGOVF].
@@ -2499,6 +2500,7 @@ __global__ void __launch_bounds__(32 * kWalkWarps)
     if (MODE == 2 && lane == 0) seg_cnt[li] = list_len[li] = 0;
     return;
   }
+  if (MODE == 1 && seg_cnt[li] <= kLocalSegs) return;  // its region holds them
   int2 *const st = stack_[w];
   const int32_t tl = leaf_ids[li];
   const DNode T = nodes[tl];
@@ -2660,10 +2662,10 @@ __device__ __forceinline__ bool lists_fit(const int64_t *counters, const ListRoo
 // as in the batched kernel), then its segments 32 at a time as one run of
 // entries -- the segment of a lane's entry from the segment starts inside the
 // 32-entry window, so short segments leave no lane idle -- kU windows' loads
-// in flight, the kept entries compacted by ballot.  LOCAL: the segments come
-// from the one-pass walk's regions and are also packed leaf after leaf into
-// segs, with their place in the full lists.
-template <bool LOCAL>
+// in flight, the kept entries compacted by ballot.  The segments come from the
+// walk's regions and are also packed leaf after leaf into segs, with their place
+// in the full lists; a leaf with more segments than its region holds has them
+// there already, from the second walk.
 __global__ void __launch_bounds__(256)
     k_expand_pruned(const int2 *__restrict__ local, SegDesc *__restrict__ segs,
                     const int64_t *__restrict__ seg_base, const int64_t *__restrict__ seg_cnt,
@@ -2692,11 +2694,12 @@ __global__ void __launch_bounds__(256)
     int32_t *out = idx + lbase;
     int64_t nk = 0, done = 0;  // entries kept, entries before this batch of segments
     const int nsegs = int(seg_cnt[li]);
+    const bool local_segs = nsegs <= kLocalSegs;
     for (int q0 = 0; q0 < nsegs; q0 += 32) {
       const bool on = q0 + lane < nsegs;
       int start = 0, count = 0;
       if (on) {
-        if (LOCAL) {
+        if (local_segs) {
           const int2 S = local[li * kLocalSegs + q0 + lane];
           start = S.x;
           count = S.y;
@@ -2714,7 +2717,7 @@ __global__ void __launch_bounds__(256)
       }
       const int pre = incl - count;
       const int total = __shfl_sync(full, incl, 31);
-      if (LOCAL && on) segs[sbase + q0 + lane] = SegDesc{start, count, lbase + done + pre};
+      if (local_segs && on) segs[sbase + q0 + lane] = SegDesc{start, count, lbase + done + pre};
       const int shift = start - pre;  // table index of entry e of this segment: shift + e
       for (int b0 = 0; b0 < total; b0 += 32 * kU) {
         float4 J[kU];
@@ -3806,8 +3809,8 @@ cudaError_t DeviceTree::build(const TreeConfig &cfg, int64_t n, const float4 *po
           *list_base = node_tmp_ + 3 * nlw;
   DT_CHECK(grow(scan_tmp_, cap_scan_, size_t(scan_tmp_size(int64_t(nlw))), s));
   // one pass writing each leaf's segments into its own region; the scans
-  // then place them (a leaf with more than kLocalSegs segments sends the
-  // build to a second, placing walk)
+  // then place them (a leaf with more than kLocalSegs segments is walked a
+  // second time)
   DT_CHECK(grow(segs_local_, cap_segl_, nlw * kLocalSegs, s));
   launch_chained(k_walk<2>, unsigned((max_leaves + kWalkWarps - 1) / kWalkWarps), 32 * kWalkWarps,
                  0, s, nodes_, nnodes, leaf_ids_, max_leaves, cfg, n, seg_cnt, list_len, nullptr,
@@ -3829,18 +3832,12 @@ cudaError_t DeviceTree::build(const TreeConfig &cfg, int64_t n, const float4 *po
   DT_CHECK(grow(leafdesc_, cap_ld_, nlw, s));
   int64_t *kept = node_tmp_ + 4 * nlw;
   constexpr ListRoom kRoom{-1, -1, -1};
-  // the index lists and the work items' counts, from the walk's regions or from
-  // a second walk's segments
-  auto expand = [&](bool local, int64_t leaves, const ListRoom &room) {
+  // the index lists and the work items' counts
+  auto expand = [&](int64_t leaves, const ListRoom &room) {
     const unsigned blocks = unsigned(std::min<int64_t>((leaves + 7) / 8, int64_t(sm_count()) * 64));
-    if (local)
-      launch_chained(k_expand_pruned<true>, blocks, 256, 0, s, segs_local_, segs_, seg_base, seg_cnt,
-                     list_base, nodes_, leaf_ids_, counters_, room, table, cfg.prune2, idx_list_,
-                     kept);
-    else
-      launch_chained(k_expand_pruned<false>, blocks, 256, 0, s, nullptr, segs_, seg_base, seg_cnt,
-                     list_base, nodes_, leaf_ids_, counters_, room, table, cfg.prune2, idx_list_,
-                     kept);
+    launch_chained(k_expand_pruned, blocks, 256, 0, s, segs_local_, segs_, seg_base, seg_cnt,
+                   list_base, nodes_, leaf_ids_, counters_, room, table, cfg.prune2, idx_list_,
+                   kept);
     launch_chained(k_leaf_items<true>, unsigned((leaves + 127) / 128), 128, 0, s, nodes_, leaf_ids_,
                    list_len, kept, list_base, leafdesc_, jsplit, group_, counters_, room);
     info_.launches += 2;
@@ -3852,7 +3849,7 @@ cudaError_t DeviceTree::build(const TreeConfig &cfg, int64_t n, const float4 *po
   const ListRoom room{int64_t(cap_idx_), int64_t(cap_seg_), int64_t(cap_items_)};
   const bool ahead = room.idx > 0 && room.segs > 0 && room.items > 0;
   if (ahead) {
-    expand(true, max_leaves, room);
+    expand(max_leaves, room);
     DT_CHECK(cudaStreamWaitEvent(s, ev_groups_, 0));
     groups_ready_ = 0;
     launch_chained(k_item_fill, unsigned((max_leaves + 127) / 128), 128, 0, s, leafdesc_, jsplit,
@@ -3882,11 +3879,11 @@ cudaError_t DeviceTree::build(const TreeConfig &cfg, int64_t n, const float4 *po
       if (!local) {
         const unsigned gW = unsigned((nleaves + kWalkWarps - 1) / kWalkWarps);
         launch_chained(k_walk<1>, gW, 32 * kWalkWarps, 0, s, nodes_, nnodes, leaf_ids_, nleaves, cfg,
-                       n, nullptr, nullptr, seg_base, list_base, segs_, nullptr, walk_err_,
+                       n, seg_cnt, nullptr, seg_base, list_base, segs_, nullptr, walk_err_,
                        counters_);
         ++info_.launches;
       }
-      expand(local, nleaves, kRoom);
+      expand(nleaves, kRoom);
     }
     DT_CHECK(cudaGetLastError());
     DT_CHECK(fill_items(jsplit, s));
