@@ -543,8 +543,7 @@ void export_lists(const hsr::RcbHost &H, const float *tab, int64_t *leaf_offset,
 }
 
 // Splits each processed leaf into ceil(count/32) spatially compact groups
-// (recursive halving along the longest axis, left part a multiple of 32; a
-// group's first 16 particles are the lower half of its longest axis) and
+// (recursive halving along the longest axis, left part a multiple of 32) and
 // emits one batched-kernel item per group and list chunk of at most `jsplit`
 // entries, sorted by list length, longest first.  gidx has n entries: each
 // leaf's range holds a permutation of its particles, grouped.
@@ -563,24 +562,21 @@ void make_items(hsr::RcbHost &H, const std::vector<int64_t> &list_begin, int64_t
   items.resize(size_t(item_base[nl]));
   H.pool().parallel_for(nl, 16, [&](int64_t b, int64_t e) {
     std::vector<int32_t> tmp;
-    struct Seg {
-      int32_t a, c;
-      bool half;  // of a group already listed
-    };
-    std::vector<Seg> stack;
-    std::vector<std::pair<int32_t, int32_t>> out;
+    std::vector<std::pair<int32_t, int32_t>> stack, out;
     for (int64_t l = b; l < e; ++l) {
       const auto &L = leaves[l];
       if (L.count <= 0) continue;  // an empty root leaf has no groups and no items
       tmp.resize(size_t(L.count));
       for (int64_t i = 0; i < L.count; ++i) tmp[i] = int32_t(L.offset + i);
       out.clear();
-      stack.assign(1, {0, int32_t(L.count), false});
+      stack.assign(1, {0, int32_t(L.count)});
       while (!stack.empty()) {
-        const auto [a, c, half] = stack.back();
+        auto [a, c] = stack.back();
         stack.pop_back();
-        if (c <= G && c > 0 && !half) out.push_back({a, c});
-        if (c <= 16) continue;
+        if (c <= G) {
+          if (c > 0) out.push_back({a, c});
+          continue;
+        }
         float lo[3] = {1e30f, 1e30f, 1e30f}, hi[3] = {-1e30f, -1e30f, -1e30f};
         for (int32_t i = a; i < a + c; ++i) {
           const hsr::Elem &q = el[tmp[i]];
@@ -594,15 +590,15 @@ void make_items(hsr::RcbHost &H, const std::vector<int64_t> &list_begin, int64_t
         for (int k = 1; k < 3; ++k)
           if (hi[k] - lo[k] > hi[d] - lo[d]) d = k;
         const int32_t ng = (c + G - 1) / G;
-        const int32_t left = c > G ? G * ((ng + 1) / 2) : 16;
+        const int32_t left = G * ((ng + 1) / 2);
         auto key = [&](int32_t i) {
           const hsr::Elem &q = el[i];
           return d == 0 ? q.x : d == 1 ? q.y : q.z;
         };
         std::nth_element(tmp.begin() + a, tmp.begin() + a + left, tmp.begin() + a + c,
                          [&](int32_t u, int32_t v) { return key(u) < key(v); });
-        stack.push_back({a + left, c - left, c <= G});
-        stack.push_back({a, left, c <= G});
+        stack.push_back({a + left, c - left});
+        stack.push_back({a, left});
       }
       std::copy(tmp.begin(), tmp.end(), gidx.begin() + L.offset);
       const int64_t nch = std::max<int64_t>(1, (L.list_len + jsplit - 1) / jsplit);

@@ -151,35 +151,11 @@ __device__ __forceinline__ float rsqrt_ftz(float s) {
   return y;
 }
 
-// One pair in the s form (batched kernel): FMA chain from rsm^2 straight to
-// s, polynomial in s, weight zeroed outside the cutoff (and, for Step16, at
-// r2 == 0).
-template <bool DROP_SELF>
-__device__ __forceinline__ void pair_acc_s(float xi, float yi, float zi, const float4 pj,
-                                           const LawS &L, float &ax, float &ay, float &az) {
-  const float dx = pj.x - xi;
-  const float dy = pj.y - yi;
-  const float dz = pj.z - zi;
-  const float s = fmaf(dx, dx, fmaf(dy, dy, fmaf(dz, dz, L.rsm2)));
-  const float y = rsqrt_ftz(s);
-  float q = L.nb[6];
-  q = fmaf(q, s, L.nb[5]);
-  q = fmaf(q, s, L.nb[4]);
-  q = fmaf(q, s, L.nb[3]);
-  q = fmaf(q, s, L.nb[2]);
-  q = fmaf(q, s, L.nb[1]);
-  q = fmaf(q, s, L.nb[0]);
-  float w = pj.w * fmaf(y, y * y, q);
-  const bool in = DROP_SELF ? (s < L.scut && s > L.rsm2) : (s < L.scut);
-  w = in ? w : 0.f;
-  ax = fmaf(w, dx, ax);
-  ay = fmaf(w, dy, ay);
-  az = fmaf(w, dz, az);
-}
-
-// Two pairs at once in the s form, on the packed FP32 pipe operations of
-// sm_100+ (__ffma2_rn and friends: each component rounds as the scalar
-// operation does): particle i against list entries a and b, given as
+// Two pairs at once in the s form (batched kernel: a chain of multiply-adds from
+// rsm^2 straight to s, the polynomial in s, the weight zeroed outside the cutoff
+// and, for Step16, at r2 == 0), on the packed FP32 pipe operations of sm_100+
+// (__ffma2_rn and friends: each component rounds as the scalar operation does):
+// particle i against list entries a and b, given as
 // A = (x_a, x_b, y_a, y_b) and B = (z_a, z_b, m_a, m_b).  (nxi, nyi, nzi) hold
 // -x_i twice; x_j + (-x_i) is x_j - x_i exactly.  The accumulators keep the a
 // and b sums apart.
