@@ -2103,14 +2103,23 @@ __global__ void __launch_bounds__(kSubThreads, 1)
   }
 }
 
+// Whether every subtree root's records are there: a block of k_subtree that
+// gives up (C_ERR) leaves its row of sub_first and its column of hist as an
+// earlier build, of another shape, left them, and the host looks only after the
+// kernels below have run.
+__device__ __forceinline__ bool subtrees_made(const LevelCtl *ctl, const int64_t *counters) {
+  return ctl->done && !ctl->abort && counters[C_ERR] == 0;
+}
+
 // Per depth below the subtree roots (a block each): every root's first node
 // among that depth's (exclusive scan over the roots) and the depth's total.
 __global__ void __launch_bounds__(kScanThreads)
-    k_subtree_scan(const LevelCtl *ctl, int32_t *hist, int32_t max_roots, int64_t *tot) {
+    k_subtree_scan(const LevelCtl *ctl, const int64_t *counters, int32_t *hist, int32_t max_roots,
+                   int64_t *tot) {
   chain_enter();
   __shared__ int sh_warp[32];
   int32_t *row = hist + int64_t(blockIdx.x) * max_roots;
-  const int32_t nr = ctl->done && !ctl->abort ? ctl->nroots : 0;
+  const int32_t nr = subtrees_made(ctl, counters) ? ctl->nroots : 0;
   int run = 0;
   for (int32_t r0 = 0; r0 < nr; r0 += kScanThreads) {
     const int32_t r = r0 + int32_t(threadIdx.x);
@@ -2129,14 +2138,14 @@ __global__ void __launch_bounds__(kScanThreads)
 // Does nothing when the node array is too small (the host grows it and
 // launches this again).
 __global__ void __launch_bounds__(256)
-    k_subtree_place(DNode *nodes, const LevelCtl *ctl, const int2 *__restrict__ roots,
-                    const DNode *sub, const int32_t *sub_first,
+    k_subtree_place(DNode *nodes, const LevelCtl *ctl, const int64_t *counters,
+                    const int2 *__restrict__ roots, const DNode *sub, const int32_t *sub_first,
                     const int32_t *pos, int32_t max_roots, const int64_t *tot, int64_t node_cap) {
   chain_enter();
   __shared__ int fs[kSubDepth + 2];
   __shared__ int64_t base[kSubDepth + 1];
   const int32_t r = int32_t(blockIdx.x);
-  if (!ctl->done || ctl->abort || r >= ctl->nroots) return;
+  if (!subtrees_made(ctl, counters) || r >= ctl->nroots) return;
   const int32_t root = roots[r].x;
   for (int dd = threadIdx.x; dd <= kSubDepth + 1; dd += blockDim.x)
     fs[dd] = sub_first[int64_t(r) * (kSubDepth + 2) + dd];
@@ -3684,11 +3693,11 @@ cudaError_t DeviceTree::build(const TreeConfig &cfg, int64_t n, const float4 *po
       launch_chained(k_subtree, unsigned(max_roots), kSubThreads, size_t(cap) * kSubBytes, s,
                      nodes_, ctl, roots_, epos_, oid_, tpos_, toid_, sub_nodes_, sub_first_,
                      sub_hist_, cap, cfg.force_cm_fallback, cfg.nd, counters_);
-      launch_chained(k_subtree_scan, kSubDepth, kScanThreads, 0, s, ctl, sub_hist_,
+      launch_chained(k_subtree_scan, kSubDepth, kScanThreads, 0, s, ctl, counters_, sub_hist_,
                      int32_t(max_roots), sub_tot);
-      launch_chained(k_subtree_place, unsigned(max_roots), 256, 0, s, nodes_, ctl, roots_,
-                     sub_nodes_, sub_first_, sub_hist_, int32_t(max_roots), sub_tot,
-                     int64_t(cap_nodes_));
+      launch_chained(k_subtree_place, unsigned(max_roots), 256, 0, s, nodes_, ctl,
+                     counters_, roots_, sub_nodes_, sub_first_, sub_hist_, int32_t(max_roots),
+                     sub_tot, int64_t(cap_nodes_));
       info_.launches += 3;
     }
     DT_CHECK(cudaGetLastError());
@@ -3741,9 +3750,9 @@ cudaError_t DeviceTree::build(const TreeConfig &cfg, int64_t n, const float4 *po
       if (total > INT32_MAX) return cudaErrorInvalidValue;
       if (size_t(total) > cap_nodes_) {
         DT_CHECK(grow(nodes_, cap_nodes_, size_t(total), s, true));
-        launch_chained(k_subtree_place, unsigned(max_roots), 256, 0, s, nodes_, ctl, roots_,
-                       sub_nodes_, sub_first_, sub_hist_, int32_t(max_roots), sub_tot,
-                       int64_t(cap_nodes_));
+        launch_chained(k_subtree_place, unsigned(max_roots), 256, 0, s, nodes_, ctl,
+                       counters_, roots_, sub_nodes_, sub_first_, sub_hist_, int32_t(max_roots),
+                       sub_tot, int64_t(cap_nodes_));
         ++info_.launches;
         DT_CHECK(cudaGetLastError());
       }
