@@ -289,7 +289,8 @@ struct LevelCtl {
   int32_t done;        // no node is left for the level loop
   int32_t node_end;    // nodes of all levels
   unsigned mx_term, mx_mass;  // largest |w x|, |w y|, |w z| and |w|, as bits
-  unsigned mn_mass;    // smallest w by its bits, complemented
+  unsigned mn_bits;    // smallest w by its bits, sign and all, complemented
+  unsigned mx_bits;    // largest w by them
   unsigned ticket;     // chunks of the level counted
   int32_t next_level;  // the level made last
   int32_t begin[kCtlLevels];  // first node of a level, by level modulo kCtlLevels
@@ -424,12 +425,12 @@ struct SumScales {
   bool uniform, bad;
   unsigned h1, l1;  // iv and iv2 of the one mass
   unsigned wbits;
-  __device__ __forceinline__ SumScales(unsigned mx_term, unsigned mx_mass, unsigned mn_mass)
-      : c(mx_term), m(mx_mass) {
-    // (raw bits: equal only where sign and value are)
-    uniform = mx_mass == mn_mass;
-    bad = SumScale::bad(mx_term) || SumScale::bad(mx_mass);
-    wbits = mn_mass;
+  __device__ __forceinline__ explicit SumScales(const LevelCtl *ctl)
+      : c(ctl->mx_term), m(ctl->mx_mass) {
+    wbits = ctl->mx_bits;
+    // (the bits with the sign: as many +w as -w are no set of one mass)
+    uniform = wbits == ~ctl->mn_bits;
+    bad = SumScale::bad(ctl->mx_term) || SumScale::bad(ctl->mx_mass);
     const float v = __fadd_rn(__uint_as_float(wbits), m.m1);
     const float r = __fsub_rn(__uint_as_float(wbits), __fsub_rn(v, m.m1));
     h1 = __float_as_uint(v) - __float_as_uint(m.m1);
@@ -804,7 +805,7 @@ __global__ void __launch_bounds__(256)
     k_elements(const float4 *__restrict__ in, int64_t n, float4 *__restrict__ pos,
                int32_t *__restrict__ oid, LevelCtl *ctl) {
   chain_enter();
-  unsigned mt = 0, mm = 0, mn = 0xffffffffu;
+  unsigned mt = 0, mm = 0, mn = 0xffffffffu, mx = 0;
   for (int64_t i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x; i < n;
        i += int64_t(gridDim.x) * blockDim.x) {
     const float4 p = in[i];
@@ -815,23 +816,27 @@ __global__ void __launch_bounds__(256)
     mt = max(mt, __float_as_uint(fmul_(p.w, p.z)) & 0x7fffffffu);
     mm = max(mm, __float_as_uint(p.w) & 0x7fffffffu);
     mn = min(mn, __float_as_uint(p.w));
+    mx = max(mx, __float_as_uint(p.w));
   }
   mt = __reduce_max_sync(0xffffffffu, mt);
   mm = __reduce_max_sync(0xffffffffu, mm);
   mn = __reduce_min_sync(0xffffffffu, mn);
-  __shared__ unsigned sh[3];
-  if (threadIdx.x < 3) sh[threadIdx.x] = threadIdx.x < 2 ? 0u : 0xffffffffu;
+  mx = __reduce_max_sync(0xffffffffu, mx);
+  __shared__ unsigned sh[4];
+  if (threadIdx.x < 4) sh[threadIdx.x] = 0u;
   __syncthreads();
   if ((threadIdx.x & 31) == 0) {
     atomicMax(&sh[0], mt);
     atomicMax(&sh[1], mm);
-    atomicMin(&sh[2], mn);
+    atomicMax(&sh[2], ~mn);
+    atomicMax(&sh[3], mx);
   }
   __syncthreads();
   if (threadIdx.x == 0) {
     atomicMax(&ctl->mx_term, sh[0]);
     atomicMax(&ctl->mx_mass, sh[1]);
-    atomicMax(&ctl->mn_mass, ~sh[2]);  // the control block starts as zeros
+    atomicMax(&ctl->mn_bits, sh[2]);  // complemented: the control block starts as zeros
+    atomicMax(&ctl->mx_bits, sh[3]);
   }
 }
 
@@ -886,7 +891,7 @@ __global__ void __launch_bounds__(kChunkThreads)
   constexpr int kW = kChunkThreads / 32, kU = 4;
   __shared__ NodeAcc part[kW];
   const ChunkRange R = chunk_range<PT>(nodes, chunk_node, chunk_base, L.nb, int32_t(blockIdx.x));
-  const SumScales S(ctl->mx_term, ctl->mx_mass, ~ctl->mn_mass);
+  const SumScales S(ctl);
   LaneAcc a;
   a.zero();
   int cnt = 0;
@@ -1731,7 +1736,7 @@ __global__ void __launch_bounds__(kSubThreads, 1)
       hist[int64_t(dd) * gridDim.x + r] = 0;
     return;
   }
-  const SumScales S(ctl->mx_term, ctl->mx_mass, ~ctl->mn_mass);
+  const SumScales S(ctl);
   const int2 root = roots[r];
   const int rcnt = nodes[root.x].count;
   const int32_t roff = nodes[root.x].offset;

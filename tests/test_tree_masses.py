@@ -1,0 +1,39 @@
+"""The device tree's centre-of-mass sums over sets whose masses are not all the
+same, or not of ordinary size, against the host build: the same permutation of
+every array, bit for bit, and the same lists."""
+import numpy as np
+import pytest
+
+import hsr
+import synth
+
+pytestmark = pytest.mark.gpu
+
+
+def compare(ctx, x, mass, nd):
+    """The tree whole, the lists of the leaves in a corner; the kick's statistics."""
+    n = len(x)
+    zero = np.zeros((4, n), np.float32)
+    p = synth.Particles(*(np.ascontiguousarray(x[:, d], np.float32) for d in range(3)), *zero[:3],
+                        np.asarray(mass, np.float32), zero[3], np.arange(n, dtype=np.int64),
+                        np.zeros(n, np.uint16), nglt=(int(np.ceil(x.max())) + 1,) * 3)
+    kp = synth.kick_params(p, nd=nd, fcoeff=0.0)
+    corner = float(np.quantile(x, 0.3))
+    kp.min_force, kp.max_force = (-1.0,) * 3, (corner,) * 3
+    q = p.copy()
+    host = hsr.HostLists(q, kp)
+    stats = ctx.rcb_kick(p, kp)
+    for k in ("x", "y", "z", "mass", "id"):
+        assert np.array_equal(getattr(p, k).view(np.uint8), getattr(q, k).view(np.uint8)), k
+    assert stats["processed_leaves"] == host.nleaves
+    if host.nleaves:
+        for a, b in zip(ctx.lists(), host.get()):
+            assert np.array_equal(a.view(np.uint8), b.view(np.uint8))
+    return stats
+
+
+@pytest.mark.parametrize("n", [40, 3000, 8192, 9000, 70000])
+def test_one_magnitude_of_both_signs(ctx, n):
+    rng = np.random.default_rng(n)
+    x = (rng.random((n, 3)) * 20).astype(np.float32)
+    compare(ctx, x, np.where(rng.random(n) < 0.1, -1.0, 1.0), 8)
