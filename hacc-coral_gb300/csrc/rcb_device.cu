@@ -428,13 +428,15 @@ struct SumScales {
   __device__ __forceinline__ explicit SumScales(const LevelCtl *ctl)
       : c(ctl->mx_term), m(ctl->mx_mass) {
     wbits = ctl->mx_bits;
-    // (the bits with the sign: as many +w as -w are no set of one mass)
-    uniform = wbits == ~ctl->mn_bits;
     bad = SumScale::bad(ctl->mx_term) || SumScale::bad(ctl->mx_mass);
     const float v = __fadd_rn(__uint_as_float(wbits), m.m1);
     const float r = __fsub_rn(__uint_as_float(wbits), __fsub_rn(v, m.m1));
+    const float v2 = __fadd_rn(r, m.m2);
     h1 = __float_as_uint(v) - __float_as_uint(m.m1);
-    l1 = __float_as_uint(__fadd_rn(r, m.m2)) - __float_as_uint(m.m2);
+    l1 = __float_as_uint(v2) - __float_as_uint(m.m2);
+    // (the bits with the sign: as many +w as -w are no set of one mass; and one
+    // that the two integers do not hold goes the way that says so)
+    uniform = wbits == ~ctl->mn_bits && __fsub_rn(v2, m.m2) == r;
   }
   // The mass words of a node of `count` elements.
   __device__ __forceinline__ void masses(NodeAcc &a, int32_t count) const {

@@ -37,3 +37,12 @@ def test_one_magnitude_of_both_signs(ctx, n):
     rng = np.random.default_rng(n)
     x = (rng.random((n, 3)) * 20).astype(np.float32)
     compare(ctx, x, np.where(rng.random(n) < 0.1, -1.0, 1.0), 8)
+
+
+@pytest.mark.parametrize("n", [40, 3000, 9000])
+def test_one_mass_of_more_bits_than_the_sums_hold(ctx, n):
+    """A mass near the smallest normal numbers, whose last bits lie below the
+    sums' last place, on a lattice coarse enough that the terms' do not."""
+    rng = np.random.default_rng(n)
+    x = 256.0 * rng.integers(1, 17, (n, 3))
+    compare(ctx, x, np.full(n, (1 + 2.0**-20) * 2.0**-112), 8)
