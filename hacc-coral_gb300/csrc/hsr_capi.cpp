@@ -82,13 +82,16 @@ struct PinBuf {
 // Strict upper bound on r2 combining the pair kernel's `dist2 < fsrrmax2`
 // (RCBForceTree.cxx:612-613) with the law's own `r2 <= r2max`
 // (ForceLaw.cxx:140, 189), r2max = rmax^2 with FGrid's rmax (ForceLaw.cxx:32).
-float cut2(int law, float fsrrmax) {
+float law_cut2(int law, float fsrrmax) {
   const float fs2 = fsrrmax * fsrrmax;
   if (law == HSR_LAW_POLY5_STEP16) return fs2;
   const float rmax = 3.116326355f;
   const float r2max = rmax * rmax;
   return std::min(fs2, std::nextafter(r2max, std::numeric_limits<float>::infinity()));
 }
+
+// The same for the pair kernels, whose fill lies beyond kMaxCut2.
+float cut2(int law, float fsrrmax) { return std::min(law_cut2(law, fsrrmax), hsr::kMaxCut2); }
 
 // Squared distance bound of the batched kernel's box test: entries farther
 // than this from a group's bounding box are skipped.  It sits 1e-4 (relative)
@@ -2113,7 +2116,7 @@ hsr_status hsr_force_law(hsr_ctx *ctx, int32_t law, float rsm, float fsrrmax, in
   float *d = ctx->d_law.as<float>();
   cudaStream_t s = ctx->stream;
   CU(cudaMemcpyAsync(d, r2, size_t(n) * 4, cudaMemcpyHostToDevice, s), "H2D r2");
-  CU(hsr::launch_force_law(law, d, d + n, n, rsm * rsm, cut2(law, fsrrmax), s), "law kernel");
+  CU(hsr::launch_force_law(law, d, d + n, n, rsm * rsm, law_cut2(law, fsrrmax), s), "law kernel");
   CU(cudaMemcpyAsync(g, d + n, size_t(n) * 4, cudaMemcpyDeviceToHost, s), "D2H g");
   CU(cudaStreamSynchronize(s), "law kernel execution");
   return HSR_OK;

@@ -134,7 +134,7 @@ extern "C" hsr_status hsr_kick_lists_noalloc(const float *table, int64_t ntab, i
   const float fs2 = fsrrmax * fsrrmax;
   const float rmax = 3.116326355f, r2max = rmax * rmax;
   const float rc2 = law == HSR_LAW_POLY5_STEP16
-                        ? fs2
+                        ? (fs2 > hsr::kMaxCut2 ? hsr::kMaxCut2 : fs2)
                         : (fs2 < nextafterf(r2max, INFINITY) ? fs2 : nextafterf(r2max, INFINITY));
   const float rcull2 = rc2 * 1.0001f + 1e-6f;
   // persistent grid from the SM count and occupancy alone: the pair kernel

@@ -359,9 +359,9 @@ __global__ void __launch_bounds__(32 * kBatchedWarps, 4)
     if (lane < padded - nbuf) {
       const int e = nbuf + lane;
       const int o = 4 * (e >> 1) + (e & 1);
-      fa[o] = 1e18f;
-      fa[o + 2] = 1e18f;
-      fb[o] = 1e18f;
+      fa[o] = kFarAway;
+      fa[o + 2] = kFarAway;
+      fb[o] = kFarAway;
       fb[o + 2] = 0.f;
     }
     __syncwarp();
@@ -614,9 +614,9 @@ __global__ void __launch_bounds__(32 * kBatchedWarps, 2)
         const float wi = (LAW == LAW_POLY5_STEP16) ? fcoeff : fcoeff * P.w;
         VjpPair &G = grp[w][el >> 1];
         const int o = el & 1;
-        (&G.nxy.x)[o] = act ? -P.x : 1e18f;
-        (&G.nxy.z)[o] = act ? -P.y : 1e18f;
-        (&G.nz_u.x)[o] = act ? -P.z : 1e18f;
+        (&G.nxy.x)[o] = act ? -P.x : kFarAway;
+        (&G.nxy.z)[o] = act ? -P.y : kFarAway;
+        (&G.nz_u.x)[o] = act ? -P.z : kFarAway;
         (&G.nz_u.z)[o] = act ? wi * ux[pi] : 0.f;
         (&G.u.x)[o] = act ? wi * uy[pi] : 0.f;
         (&G.u.z)[o] = act ? wi * uz[pi] : 0.f;
@@ -703,8 +703,8 @@ __global__ void __launch_bounds__(32 * kBatchedWarps, 2)
       if (nbuf > 0) {
         // the remainder, filled up with far-away massless entries
         if (hw == 0 && el >= nbuf) {
-          ent[w][el][0] = make_float4(1e18f, 1e18f, 1e18f, 1e18f);
-          ent[w][el][1] = make_float4(1e18f, 1e18f, 0.f, 0.f);
+          ent[w][el][0] = make_float4(kFarAway, kFarAway, kFarAway, kFarAway);
+          ent[w][el][1] = make_float4(kFarAway, kFarAway, 0.f, 0.f);
           ent_idx[w][el] = -2;
         }
         __syncwarp();

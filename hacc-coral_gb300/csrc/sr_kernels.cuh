@@ -58,6 +58,13 @@ struct BuiltItems {
   unsigned int overflow;
 };
 
+// Coordinate of the entries and particles that fill up the pair kernels' lanes,
+// and the largest squared cutoff those kernels take: whatever the caller's
+// cutoff, the fill lies outside it (r2 of at least 3 kFarAway^2 from anything
+// real, where the law's polynomial overflows and a weight of zero is NaN).
+constexpr float kFarAway = 1e18f;
+constexpr float kMaxCut2 = 1e36f;
+
 // The law in terms of s = r2 + rsm^2, for the batched kernel: g = s^-3/2 +
 // q(s) with q(s) = -p(s - rsm^2) re-expanded in s (nb[k], computed in double
 // and rounded), and the cutoff as s < scut (scut = rcut2 + rsm^2 in float).
