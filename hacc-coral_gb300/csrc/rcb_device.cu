@@ -53,7 +53,15 @@ enum { C_NFALLBACK = 2, C_NLEAF = 3, C_NSEG = 4, C_NENT = 5,
 
 // Segments a leaf's walk can leave in its own region of the one-pass walk (8
 // bytes each); a leaf with more is walked a second time, its segments placed.
+// At most kLocalSegs, and fewer where the regions of every leaf that there can be
+// would take more than kWalkBytes (above 262,144 leaves): at a leaf size of 1 or
+// 2 the regions would be the largest buffer of all (2 KB a leaf, held as long as
+// the tree).
 constexpr int kLocalSegs = 256;
+constexpr int64_t kWalkBytes = int64_t(512) << 20;
+inline int local_segs(int64_t leaves) {
+  return int(std::min<int64_t>(kLocalSegs, kWalkBytes / (leaves * int64_t(sizeof(int2)))));
+}
 
 __device__ __forceinline__ float warp_min(float v) {
 #pragma unroll
@@ -2491,16 +2499,16 @@ constexpr int kWalkReserve = 256;  // fills, to one node at a time over the last
 
 // The leaves are the first counters[C_NLEAF] of leaf_ids (max_leaves bounds
 // them: the host need not wait for their number).
-// MODE 1, leaves with more than kLocalSegs segments only: writes the segments at
+// MODE 1, leaves with more than `room` segments only: writes the segments at
 // seg_base / list_base; 2: counts (segments and
-// entries per leaf) and writes the first kLocalSegs segments (start, count) of
+// entries per leaf) and writes the first `room` segments (start, count) of
 // each leaf into its own region, flagging leaves with more in
 // counters[C_SEGOVF].
 template <int MODE>
 __global__ void __launch_bounds__(32 * kWalkWarps)
     k_walk(const DNode *__restrict__ nodes, int32_t nnodes, const int32_t *leaf_ids,
            int64_t max_leaves, TreeConfig cfg, int64_t n, int64_t *seg_cnt, int64_t *list_len,
-           const int64_t *seg_base, const int64_t *list_base, SegDesc *segs, int2 *local,
+           const int64_t *seg_base, const int64_t *list_base, SegDesc *segs, int2 *local, int room,
            int32_t *err, int64_t *counters) {
   chain_enter();
   static_assert(MODE == 1 || MODE == 2, "walk mode");
@@ -2516,7 +2524,7 @@ __global__ void __launch_bounds__(32 * kWalkWarps)
     if (MODE == 2 && lane == 0) seg_cnt[li] = list_len[li] = 0;
     return;
   }
-  if (MODE == 1 && seg_cnt[li] <= kLocalSegs) return;  // its region holds them
+  if (MODE == 1 && seg_cnt[li] <= room) return;  // its region holds them
   int2 *const st = stack_[w];
   const int32_t tl = leaf_ids[li];
   const DNode T = nodes[tl];
@@ -2540,7 +2548,7 @@ __global__ void __launch_bounds__(32 * kWalkWarps)
       if (on) segs[sb + q] = SegDesc{start, count, lb + len + incl - count};
       len += __shfl_sync(full, incl, 31);
     } else {
-      if (on && q < kLocalSegs) local[li * kLocalSegs + q] = make_int2(start, count);
+      if (on && q < room) local[li * room + q] = make_int2(start, count);
       len += __reduce_add_sync(full, incl);
     }
     nseg += __popc(m);
@@ -2654,7 +2662,7 @@ __global__ void __launch_bounds__(32 * kWalkWarps)
   if (MODE == 2 && lane == 0) {
     seg_cnt[li] = nseg;
     list_len[li] = len;
-    if (nseg > kLocalSegs) atomicExch((unsigned long long *)&counters[C_SEGOVF], 1ull);
+    if (nseg > room) atomicExch((unsigned long long *)&counters[C_SEGOVF], 1ull);
   }
 }
 
@@ -2683,7 +2691,7 @@ __device__ __forceinline__ bool lists_fit(const int64_t *counters, const ListRoo
 // in the full lists; a leaf with more segments than its region holds has them
 // there already, from the second walk.
 __global__ void __launch_bounds__(256)
-    k_expand_pruned(const int2 *__restrict__ local, SegDesc *__restrict__ segs,
+    k_expand_pruned(const int2 *__restrict__ local, int local_room, SegDesc *__restrict__ segs,
                     const int64_t *__restrict__ seg_base, const int64_t *__restrict__ seg_cnt,
                     const int64_t *__restrict__ list_base, const DNode *__restrict__ nodes,
                     const int32_t *__restrict__ leaf_ids, const int64_t *__restrict__ counters,
@@ -2710,13 +2718,13 @@ __global__ void __launch_bounds__(256)
     int32_t *out = idx + lbase;
     int64_t nk = 0, done = 0;  // entries kept, entries before this batch of segments
     const int nsegs = int(seg_cnt[li]);
-    const bool local_segs = nsegs <= kLocalSegs;
+    const bool in_region = nsegs <= local_room;
     for (int q0 = 0; q0 < nsegs; q0 += 32) {
       const bool on = q0 + lane < nsegs;
       int start = 0, count = 0;
       if (on) {
-        if (local_segs) {
-          const int2 S = local[li * kLocalSegs + q0 + lane];
+        if (in_region) {
+          const int2 S = local[li * local_room + q0 + lane];
           start = S.x;
           count = S.y;
         } else {
@@ -2733,7 +2741,7 @@ __global__ void __launch_bounds__(256)
       }
       const int pre = incl - count;
       const int total = __shfl_sync(full, incl, 31);
-      if (local_segs && on) segs[sbase + q0 + lane] = SegDesc{start, count, lbase + done + pre};
+      if (in_region && on) segs[sbase + q0 + lane] = SegDesc{start, count, lbase + done + pre};
       const int shift = start - pre;  // table index of entry e of this segment: shift + e
       for (int b0 = 0; b0 < total; b0 += 32 * kU) {
         float4 J[kU];
@@ -3825,12 +3833,13 @@ cudaError_t DeviceTree::build(const TreeConfig &cfg, int64_t n, const float4 *po
           *list_base = node_tmp_ + 3 * nlw;
   DT_CHECK(grow(scan_tmp_, cap_scan_, size_t(scan_tmp_size(int64_t(nlw))), s));
   // one pass writing each leaf's segments into its own region; the scans
-  // then place them (a leaf with more than kLocalSegs segments is walked a
-  // second time)
-  DT_CHECK(grow(segs_local_, cap_segl_, nlw * kLocalSegs, s));
+  // then place them (a leaf with more segments than that is walked a second
+  // time)
+  const int room_segs = local_segs(max_leaves);
+  DT_CHECK(grow(segs_local_, cap_segl_, std::max<size_t>(nlw * size_t(room_segs), 1), s));
   launch_chained(k_walk<2>, unsigned((max_leaves + kWalkWarps - 1) / kWalkWarps), 32 * kWalkWarps,
                  0, s, nodes_, nnodes, leaf_ids_, max_leaves, cfg, n, seg_cnt, list_len, nullptr,
-                 nullptr, nullptr, segs_local_, walk_err_, counters_);
+                 nullptr, nullptr, segs_local_, room_segs, walk_err_, counters_);
   ++info_.launches;
   // the groups after the walk's blocks, which then have their SMs first
   DT_CHECK(launch_groups(max_leaves, group_, cfg.halves ? kGroupHalf : group_, aux_));
@@ -3851,9 +3860,9 @@ cudaError_t DeviceTree::build(const TreeConfig &cfg, int64_t n, const float4 *po
   // the index lists and the work items' counts
   auto expand = [&](int64_t leaves, const ListRoom &room) {
     const unsigned blocks = unsigned(std::min<int64_t>((leaves + 7) / 8, int64_t(sm_count()) * 64));
-    launch_chained(k_expand_pruned, blocks, 256, 0, s, segs_local_, segs_, seg_base, seg_cnt,
-                   list_base, nodes_, leaf_ids_, counters_, room, table, cfg.prune2, idx_list_,
-                   kept);
+    launch_chained(k_expand_pruned, blocks, 256, 0, s, segs_local_, room_segs, segs_, seg_base,
+                   seg_cnt, list_base, nodes_, leaf_ids_, counters_, room, table, cfg.prune2,
+                   idx_list_, kept);
     launch_chained(k_leaf_items<true>, unsigned((leaves + 127) / 128), 128, 0, s, nodes_, leaf_ids_,
                    list_len, kept, list_base, leafdesc_, jsplit, group_, counters_, room);
     info_.launches += 2;
@@ -3895,7 +3904,7 @@ cudaError_t DeviceTree::build(const TreeConfig &cfg, int64_t n, const float4 *po
       if (!local) {
         const unsigned gW = unsigned((nleaves + kWalkWarps - 1) / kWalkWarps);
         launch_chained(k_walk<1>, gW, 32 * kWalkWarps, 0, s, nodes_, nnodes, leaf_ids_, nleaves, cfg,
-                       n, seg_cnt, nullptr, seg_base, list_base, segs_, nullptr, walk_err_,
+                       n, seg_cnt, nullptr, seg_base, list_base, segs_, nullptr, room_segs, walk_err_,
                        counters_);
         ++info_.launches;
       }
