@@ -3000,6 +3000,8 @@ __global__ void __launch_bounds__(32 * kGWarps)
         const float4 p = pos[val[w][cur][i]];
         const int ax = seg_ax[w][q];
         k = ax == 0 ? p.x : (ax == 1 ? p.y : p.z);
+        // NaN last: ranks that leave no slot out
+        k = k == k ? k : INFINITY;
       }
       key[w][i] = k;
     }
