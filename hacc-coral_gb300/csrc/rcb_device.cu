@@ -2533,6 +2533,7 @@ __global__ void __launch_bounds__(32 * kWalkWarps)
   const float tan_oa = cfg.tan_oa;
   const int k = cfg.tdpts;
   int64_t nseg = 0, len = 0;
+  int2 *const region = local + li * room;
   const int64_t sb = MODE == 1 ? seg_base[li] : 0, lb = MODE == 1 ? list_base[li] : 0;
   // the lanes' segments (start, count), in lane order, where `on`
   auto emit = [&](bool on, int32_t start, int32_t count) {
@@ -2548,7 +2549,7 @@ __global__ void __launch_bounds__(32 * kWalkWarps)
       if (on) segs[sb + q] = SegDesc{start, count, lb + len + incl - count};
       len += __shfl_sync(full, incl, 31);
     } else {
-      if (on && q < room) local[li * room + q] = make_int2(start, count);
+      if (on && q < room) region[q] = make_int2(start, count);
       len += __reduce_add_sync(full, incl);
     }
     nseg += __popc(m);
@@ -2719,12 +2720,13 @@ __global__ void __launch_bounds__(256)
     int64_t nk = 0, done = 0;  // entries kept, entries before this batch of segments
     const int nsegs = int(seg_cnt[li]);
     const bool in_region = nsegs <= local_room;
+    const int2 *const region = local + li * local_room;
     for (int q0 = 0; q0 < nsegs; q0 += 32) {
       const bool on = q0 + lane < nsegs;
       int start = 0, count = 0;
       if (on) {
         if (in_region) {
-          const int2 S = local[li * local_room + q0 + lane];
+          const int2 S = region[q0 + lane];
           start = S.x;
           count = S.y;
         } else {

@@ -46,3 +46,38 @@ def test_one_mass_of_more_bits_than_the_sums_hold(ctx, n):
     rng = np.random.default_rng(n)
     x = 256.0 * rng.integers(1, 17, (n, 3))
     compare(ctx, x, np.full(n, (1 + 2.0**-20) * 2.0**-112), 8)
+
+
+def _heavy(rng, n, factor):  # one particle that outweighs the rest
+    m = np.ones(n, np.float32)
+    m[n // 3] = factor
+    return m
+
+
+def _spread(rng, n, factor):
+    return (factor ** rng.random(n)).astype(np.float32)
+
+
+def _species(rng, n, factor):
+    return np.where(rng.random(n) < 0.5, np.float32(1), np.float32(factor))
+
+
+# ranges on both sides of the one from which the sums take the third integer,
+# and beyond what that holds; with a far particle, masses of one value too
+@pytest.mark.parametrize("make,factor,far", [
+    (_heavy, 2.0**11, None), (_heavy, 2.0**12, None), (_heavy, 1e6, None), (_heavy, 1e-6, None),
+    (_heavy, 1e9, None), (_heavy, 1e15, None), (_spread, 1e4, None), (_spread, 1e8, None),
+    (_species, 1e6, None), (_heavy, 1.0, 1e4), (_heavy, 1.0, 1e9), (_heavy, 1.0, -1e9),
+    (_heavy, 1e6, 1e6), (_heavy, 0.0, None)])
+@pytest.mark.parametrize("n,nd", [(3000, 4), (30000, 16), (300000, 64)])
+def test_sets_of_wide_range(ctx, n, nd, make, factor, far):
+    rng = np.random.default_rng(n)
+    x = (rng.random((n, 3)) * 30).astype(np.float32)
+    if far is not None:
+        x[n // 2, 1] = far
+    st = compare(ctx, x, make(rng, n, factor), nd)
+    # what the third integer holds is decided without the sequential sums: by 40
+    # in a thousand nodes' three quotients at most, 2^-31 of a term's range a term
+    # against the 2^-25 that a quotient is rounded by
+    if make is _heavy and 1e6 <= max(factor, abs(far or 0)) <= 1e9:
+        assert st["cm_fallbacks"] <= 0.04 * st["nodes"]
