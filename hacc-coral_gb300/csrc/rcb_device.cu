@@ -299,6 +299,8 @@ struct LevelCtl {
   unsigned mx_term, mx_mass;  // largest |w x|, |w y|, |w z| and |w|, as bits
   unsigned mn_bits;    // smallest w by its bits, sign and all, complemented
   unsigned mx_bits;    // largest w by them
+  unsigned mn_term;    // smallest over the elements of the largest of |w x|, |w y| and |w z|,
+  unsigned mn_mass;    // and smallest |w|, zeros aside, as bits, complemented
   unsigned ticket;     // chunks of the level counted
   int32_t next_level;  // the level made last
   int32_t begin[kCtlLevels];  // first node of a level, by level modulo kCtlLevels
@@ -387,6 +389,11 @@ __device__ __forceinline__ float o2f(uint32_t o) {
 // conversion to or from a 64-bit type, runs at a small fraction of that rate on
 // this part.  One scale for the three coordinates' terms and one for the masses,
 // from the largest of the whole set.
+//
+// In a set of wide range (one particle a million times heavier than the rest,
+// or that much farther away) two integers hold too few bits of the small terms,
+// and nearly every centre of mass would be left to the sequential sums.  There a
+// third integer, on multiples of 2^(k-67), takes what the second leaves.
 // ---------------------------------------------------------------------------
 struct SumScale {
   int k;        // the scale's exponent
@@ -394,20 +401,26 @@ struct SumScale {
   __device__ __forceinline__ explicit SumScale(unsigned mx) {
     const int e = int(mx >> 23) - 127;  // mx < 2^(e+1); subnormal or zero: -127
     k = max(e + 3, -80);
-    m1 = __uint_as_float((unsigned(k + 127) << 23) | 0x400000u);
-    m2 = __uint_as_float((unsigned(k - 22 + 127) << 23) | 0x400000u);
+    m1 = binade(k);
+    m2 = binade(k - 22);
   }
+  __device__ static __forceinline__ float binade(int e) {  // 1.5 2^e
+    return __uint_as_float((unsigned(e + 127) << 23) | 0x400000u);
+  }
+  __device__ __forceinline__ float m3() const { return binade(k - 44); }
   // terms too large for the scale's arithmetic, infinities and NaN
   __device__ static __forceinline__ bool bad(unsigned mx) { return mx >= (247u << 23); }
 };
 
 // Reduced statistics of a set of elements (a node, a warp's share).
 struct alignas(16) NodeAcc {
-  long long h[4], l[4];     // sums of iv and iv2 (x, y, z, m)
-  unsigned o[4];            // ors of iv2's bits: the terms' least significant one
+  // sums (x, y, z, m) of iv and iv2; wide: of iv and of iv2 2^22 + iv3
+  long long h[4], l[4];
+  // the terms' least significant bit: ors of iv2's bits; wide: of low_mark's
+  unsigned o[4];
   unsigned lo[3], hi[3];    // bounding box (f2o)
   unsigned wmin;            // smallest mass (f2o)
-  unsigned trunc;           // some term had bits below 2^(k-45)
+  unsigned trunc;           // some term had bits below the last integer's
 };
 constexpr int kAccWords16 = int(sizeof(NodeAcc) / 16);
 static_assert(sizeof(NodeAcc) == 112, "NodeAcc is seven 16-byte words");
@@ -425,33 +438,82 @@ __device__ __forceinline__ void acc_zero(NodeAcc &a) {
   a.trunc = 0u;
 }
 
+// The lowest set bit (0 to 43, by the low 22 bits of iv2 and iv3) of a wide
+// term as one of 31 marks, and the lowest position that a mark can stand for.
+__device__ __forceinline__ unsigned low_mark(unsigned iv2, unsigned iv3) {
+  const unsigned lo = iv3 & 0x3fffffu, hi = iv2 & 0x3fffffu;
+  if (!(lo | hi)) return 0u;
+  const int at = lo ? __ffs(int(lo)) - 1 : 21 + __ffs(int(hi));
+  return 1u << (at * 5 / 7);
+}
+__device__ __forceinline__ int low_of_mark(int mark) { return (7 * mark + 4) / 5; }
+
+// Whether a set's range calls for the third integer: its largest mass 2^12 times
+// its smallest, or its largest term 2^20 times the largest of the element that
+// has the smallest one (2^10 times is what a box of millions has beside its
+// origin); zeros aside.  Two integers lose whole sets a little above (a kick of
+// 2.6 M particles in 137 cells, one of them 10^5 times as heavy or at 10^7 cells:
+// 24 and 27 ms, with three 3.0 and 2.9), and below the third only costs (the same
+// without that one: 2.90 and 3.01 ms; masses spread over a factor of 10^4: 3.44
+// and 3.04).
+constexpr int kWideTerm = 20, kWideMass = 12;
+__host__ __device__ __forceinline__ bool wide_range(const LevelCtl &ctl) {
+  // (bits of positive floats: 2^23 a power of two; nothing but zeros: ~0)
+  const unsigned t = ~ctl.mn_term, m = ~ctl.mn_mass;
+  return (ctl.mx_term > t && ctl.mx_term - t >= unsigned(kWideTerm) << 23) ||
+         (ctl.mx_mass > m && ctl.mx_mass - m >= unsigned(kWideMass) << 23);
+}
+
 // The scales of a set's terms, and its mass where all are the same (the
 // simulation's own kicks set them all to 1): the mass sums then follow from the
 // counts and cost nothing.
 struct SumScales {
   SumScale c, m;
-  bool uniform, bad;
-  unsigned h1, l1;  // iv and iv2 of the one mass
+  bool uniform, bad, wide;
   unsigned wbits;
-  __device__ __forceinline__ explicit SumScales(const LevelCtl *ctl)
-      : c(ctl->mx_term), m(ctl->mx_mass) {
+  __device__ __forceinline__ SumScales(const LevelCtl *ctl, bool wide_sums)
+      : c(ctl->mx_term), m(ctl->mx_mass), wide(wide_sums) {
     wbits = ctl->mx_bits;
     bad = SumScale::bad(ctl->mx_term) || SumScale::bad(ctl->mx_mass);
-    const float v = __fadd_rn(__uint_as_float(wbits), m.m1);
-    const float r = __fsub_rn(__uint_as_float(wbits), __fsub_rn(v, m.m1));
-    const float v2 = __fadd_rn(r, m.m2);
-    h1 = __float_as_uint(v) - __float_as_uint(m.m1);
-    l1 = __float_as_uint(v2) - __float_as_uint(m.m2);
     // (the bits with the sign: as many +w as -w are no set of one mass; and one
-    // that the two integers do not hold goes the way that says so)
-    uniform = wbits == ~ctl->mn_bits && __fsub_rn(v2, m.m2) == r;
+    // that the integers do not hold goes the way that says so)
+    int h;
+    long long l;
+    unsigned o;
+    uniform = wbits == ~ctl->mn_bits && mass_digits(h, l, o);
+  }
+  // The integers of the one mass, as NodeAcc sums them; whether they hold it.
+  __device__ __forceinline__ bool mass_digits(int &h, long long &l, unsigned &o) const {
+    const float w = __uint_as_float(wbits);
+    const float v = __fadd_rn(w, m.m1);
+    const float r = __fsub_rn(w, __fsub_rn(v, m.m1));
+    const float v2 = __fadd_rn(r, m.m2);
+    const float r2 = __fsub_rn(r, __fsub_rn(v2, m.m2));
+    const unsigned iv2 = __float_as_uint(v2) - __float_as_uint(m.m2);
+    h = int(__float_as_uint(v) - __float_as_uint(m.m1));
+    l = int(iv2);
+    o = iv2;
+    if (!wide) return r2 == 0.f;
+    const float m3 = m.m3(), v3 = __fadd_rn(r2, m3);
+    const unsigned iv3 = __float_as_uint(v3) - __float_as_uint(m3);
+    l = (l << 22) + int(iv3);
+    o = low_mark(iv2, iv3);
+    return __fsub_rn(v3, m3) == r2;
   }
   // The mass words of a node of `count` elements.
   __device__ __forceinline__ void masses(NodeAcc &a, int32_t count) const {
     if (!uniform) return;
-    a.h[3] = (long long)int(h1) * count;
-    a.l[3] = (long long)int(l1) * count;
-    a.o[3] = l1;
+    int h;
+    long long l;
+    mass_digits(h, l, a.o[3]);
+    a.h[3] = (long long)h * count;
+    if (!wide) {
+      a.l[3] = l * count;
+    } else {  // |l| <= 2^43: what passes 2^44 goes to h
+      const __int128 p = __int128(l) * count;
+      a.h[3] += (long long)(p >> 44);
+      a.l[3] = (long long)p & ((1ll << 44) - 1);
+    }
     a.wmin = f2o(__uint_as_float(wbits));
   }
 };
@@ -484,12 +546,17 @@ __device__ __forceinline__ T reduce8(T v0, T v1, T v2, T v3, T v4, T v5, T v6, T
 }
 
 // One lane's share.
+template <bool WIDE>
 struct LaneAcc {
   unsigned h[4], l[4], o[4];  // sums of the bits of v and v2 (modulo 2^32), ors of v2's
+  unsigned t[WIDE ? 4 : 1], ot[WIDE ? 4 : 1];  // the same of the third integer
   float lo[3], hi[3], wmin, left;
   __device__ __forceinline__ void zero() {
 #pragma unroll
-    for (int q = 0; q < 4; ++q) h[q] = l[q] = o[q] = 0u;
+    for (int q = 0; q < 4; ++q) {
+      h[q] = l[q] = o[q] = 0u;
+      if (WIDE) t[q] = ot[q] = 0u;
+    }
 #pragma unroll
     for (int d = 0; d < 3; ++d) {
       lo[d] = INFINITY;
@@ -498,11 +565,19 @@ struct LaneAcc {
     wmin = INFINITY;
     left = 0.f;
   }
-  __device__ __forceinline__ void term(int q, float t, const SumScale &s) {
-    const float v = __fadd_rn(t, s.m1);
-    const float r = __fsub_rn(t, __fsub_rn(v, s.m1));
+  __device__ __forceinline__ void term(int q, float x, const SumScale &s) {
+    const float v = __fadd_rn(x, s.m1);
+    const float r = __fsub_rn(x, __fsub_rn(v, s.m1));
     const float v2 = __fadd_rn(r, s.m2);
-    left = fmaxf(left, fabsf(__fsub_rn(__fsub_rn(v2, s.m2), r)));
+    if (WIDE) {
+      const float r2 = __fsub_rn(r, __fsub_rn(v2, s.m2));
+      const float m3 = s.m3(), v3 = __fadd_rn(r2, m3);
+      left = fmaxf(left, fabsf(__fsub_rn(__fsub_rn(v3, m3), r2)));
+      t[q] += __float_as_uint(v3);
+      ot[q] |= __float_as_uint(v3);
+    } else {
+      left = fmaxf(left, fabsf(__fsub_rn(__fsub_rn(v2, s.m2), r)));
+    }
     h[q] += __float_as_uint(v);
     l[q] += __float_as_uint(v2);
     o[q] |= __float_as_uint(v2);
@@ -521,7 +596,7 @@ struct LaneAcc {
   }
   // The sums of a warp (W = 32; of each eight lanes, W = 8) into *out, word by
   // word from different lanes; cnt: this lane's elements (at most 512), few: the
-  // warp's are at most 1023 (an int holds their sums).
+  // warp's are at most 1023 (an int holds the sums of one integer).
   template <int W>
   __device__ __forceinline__ void reduce(NodeAcc *out, bool write, int cnt, bool few,
                                          const SumScales &S) const {
@@ -533,16 +608,30 @@ struct LaneAcc {
     }
     hv[3] = S.uniform ? 0 : int(h[3] - unsigned(cnt) * __float_as_uint(S.m.m1));
     lv[3] = S.uniform ? 0 : int(l[3] - unsigned(cnt) * __float_as_uint(S.m.m2));
-    long long sum;
-    if (few) {
+    using LL = long long;
+    LL sum;
+    unsigned ov[4];
+#pragma unroll
+    for (int q = 0; q < 4; ++q) ov[q] = o[q];
+    if (WIDE) {
+      LL w[4];
+#pragma unroll
+      for (int q = 0; q < 4; ++q) {
+        const bool on = q < 3 || !S.uniform;
+        const SumScale &sc = q < 3 ? S.c : S.m;
+        w[q] = on ? LL(lv[q]) * (1 << 22) + int(t[q] - unsigned(cnt) * __float_as_uint(sc.m3())) : 0;
+        ov[q] = low_mark(o[q], ot[q]);
+      }
+      sum = reduce8<W>(LL(hv[0]), LL(hv[1]), LL(hv[2]), LL(hv[3]), w[0], w[1], w[2], w[3],
+                       [](LL a, LL b) { return a + b; });
+    } else if (few) {
       sum = reduce8<W>(hv[0], hv[1], hv[2], hv[3], lv[0], lv[1], lv[2], lv[3],
                        [](int a, int b) { return a + b; });
     } else {
-      using LL = long long;
       sum = reduce8<W>(LL(hv[0]), LL(hv[1]), LL(hv[2]), LL(hv[3]), LL(lv[0]), LL(lv[1]), LL(lv[2]),
                        LL(lv[3]), [](LL a, LL b) { return a + b; });
     }
-    const unsigned bits = reduce4<W>(o[0], o[1], o[2], o[3], [](unsigned a, unsigned b) { return a | b; });
+    const unsigned bits = reduce4<W>(ov[0], ov[1], ov[2], ov[3], [](unsigned a, unsigned b) { return a | b; });
     // minima; the upper bounds complemented, and 0 where a term was truncated
     const unsigned mn = reduce8<W>(f2o(lo[0]), f2o(lo[1]), f2o(lo[2]), ~f2o(hi[0]), ~f2o(hi[1]),
                                    ~f2o(hi[2]), f2o(wmin), left != 0.f ? 0u : 1u,
@@ -585,10 +674,11 @@ __device__ __forceinline__ double pow2(int e) {  // normal range
 }
 __device__ __forceinline__ float pow2f(int e) { return __uint_as_float(unsigned(e + 127) << 23); }
 
-// Correctly rounded double of h 2^22 + l (units of 2^(k-45)).
-__device__ double units_to_double(long long h, long long l) {
-  if (h < (1ll << 40) && h > -(1ll << 40)) return __ll2double_rn((h << 22) + l);
-  const __int128 v = (__int128(h) << 22) + l;
+// Correctly rounded double of h 2^22 + l (units of 2^(k-45)); wide: of h 2^44 + l
+// (units of 2^(k-67)).
+__device__ double units_to_double(long long h, long long l, bool wide = false) {
+  if (!wide && h < (1ll << 40) && h > -(1ll << 40)) return __ll2double_rn((h << 22) + l);
+  const __int128 v = (__int128(h) << (wide ? 44 : 22)) + l;
   const bool neg = v < 0;
   const unsigned __int128 u = neg ? (unsigned __int128)(-v) : (unsigned __int128)v;
   const unsigned long long hi = (unsigned long long)(u >> 64), lo = (unsigned long long)u;
@@ -620,7 +710,7 @@ __device__ bool certify(double sx, double bx, double sm, double bm, float *out) 
 }
 
 // The sums of a node's terms and what bounds their distance from the
-// reference's sequential ones, in units of 2^(k-45).
+// reference's sequential ones, in units of 2^(k-45) (wide: 2^(k-67)).
 struct NodeSums {
   double x[4];   // the exact sums, rounded to double
   float abs[4];  // at least sum |terms|
@@ -628,7 +718,7 @@ struct NodeSums {
   bool exact[4];  // the reference's sum is exactly x
 };
 
-__device__ __forceinline__ NodeSums node_sums(const NodeAcc &A, int32_t count) {
+__device__ __forceinline__ NodeSums node_sums(const NodeAcc &A, int32_t count, bool wide) {
   NodeSums S;
   // The reference's sequential sum lies within (n - 1) u sum|terms| of the
   // exact sum, to first order; (n + 64) u (1 + 2^-20) covers the rest.  The sums
@@ -640,17 +730,19 @@ __device__ __forceinline__ NodeSums node_sums(const NodeAcc &A, int32_t count) {
   const bool wpos = o2f(A.wmin) >= 0.f;
 #pragma unroll
   for (int q = 0; q < 4; ++q) {
-    S.x[q] = units_to_double(A.h[q], A.l[q]);
+    S.x[q] = units_to_double(A.h[q], A.l[q], wide);
     const float xa = __double2float_ru(fabs(S.x[q]));
     // sum of |terms|: the sum itself where none is negative, else n times the
     // scale's largest term (2^(k-2))
     const bool pos = wpos && (q == 3 || o2f(A.lo[q]) >= 0.f);
-    S.abs[q] = pos ? __fadd_ru(xa, slack) : __fmul_ru(n, 0x1p43f);
+    S.abs[q] = pos ? __fadd_ru(xa, slack) : __fmul_ru(n, wide ? 0x1p65f : 0x1p43f);
     // Exact: every term a multiple of 2^emin (none truncated) and the
     // magnitudes summing below 2^(53 + emin) -- then the reference's
     // sequential sum and this one are the same exact value, a double.
-    const unsigned b = A.o[q] & 0x3fffffu;
-    const int emin = b ? __ffs(int(b)) - 1 : 22;  // no iv2: whole multiples of 2^22 units
+    const unsigned b = wide ? A.o[q] : A.o[q] & 0x3fffffu;
+    const int at = b ? __ffs(int(b)) - 1 : 31;
+    // no iv2 (and iv3): whole multiples of 2^22 (2^44) units
+    const int emin = wide ? low_of_mark(at) : min(at, 22);
     S.exact[q] = !A.trunc && S.abs[q] < pow2f(53 + emin);
     S.err[q] = S.exact[q] ? 0.f : __fadd_ru(__fmaf_ru(g, S.abs[q], slack), __fmul_ru(xa, 0x1p-52f));
   }
@@ -785,8 +877,8 @@ __device__ bool decide_node(DNode &N, const NodeAcc &A, const SumScales &S, int3
     N.split_dim = (l0 > l1 && l0 > l2) ? 0 : (l1 > l2 ? 1 : 2);
   }
   if (force_fallback != 0 || S.bad) return false;
-  return quotients_f32(A, N.count, S.c.k, S.m.k, N.xc) ||
-         quotients(node_sums(A, N.count), S.c.k, S.m.k, N.xc);
+  return (!S.wide && quotients_f32(A, N.count, S.c.k, S.m.k, N.xc)) ||
+         quotients(node_sums(A, N.count, S.wide), S.c.k, S.m.k, N.xc);
 }
 
 // A tighter bound for sums that node_sums leaves open: an addition rounds only
@@ -815,16 +907,20 @@ __global__ void __launch_bounds__(256)
     k_elements(const float4 *__restrict__ in, int64_t n, float4 *__restrict__ pos,
                int32_t *__restrict__ oid, LevelCtl *ctl) {
   chain_enter();
-  unsigned mt = 0, mm = 0, mn = 0xffffffffu, mx = 0;
+  unsigned mt = 0, mm = 0, mn = 0xffffffffu, mx = 0, nt = 0xffffffffu, nm = 0xffffffffu;
   for (int64_t i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x; i < n;
        i += int64_t(gridDim.x) * blockDim.x) {
     const float4 p = in[i];
     pos[i] = p;
     oid[i] = int32_t(i);
-    mt = max(mt, __float_as_uint(fmul_(p.w, p.x)) & 0x7fffffffu);
-    mt = max(mt, __float_as_uint(fmul_(p.w, p.y)) & 0x7fffffffu);
-    mt = max(mt, __float_as_uint(fmul_(p.w, p.z)) & 0x7fffffffu);
-    mm = max(mm, __float_as_uint(p.w) & 0x7fffffffu);
+    const unsigned t = max(max(__float_as_uint(fmul_(p.w, p.x)) & 0x7fffffffu,
+                               __float_as_uint(fmul_(p.w, p.y)) & 0x7fffffffu),
+                           __float_as_uint(fmul_(p.w, p.z)) & 0x7fffffffu);
+    const unsigned w = __float_as_uint(p.w) & 0x7fffffffu;
+    mt = max(mt, t);
+    mm = max(mm, w);
+    nt = min(nt, t - 1u);  // (zero as the largest: it is left aside)
+    nm = min(nm, w - 1u);
     mn = min(mn, __float_as_uint(p.w));
     mx = max(mx, __float_as_uint(p.w));
   }
@@ -832,14 +928,18 @@ __global__ void __launch_bounds__(256)
   mm = __reduce_max_sync(0xffffffffu, mm);
   mn = __reduce_min_sync(0xffffffffu, mn);
   mx = __reduce_max_sync(0xffffffffu, mx);
-  __shared__ unsigned sh[4];
-  if (threadIdx.x < 4) sh[threadIdx.x] = 0u;
+  nt = __reduce_min_sync(0xffffffffu, nt);
+  nm = __reduce_min_sync(0xffffffffu, nm);
+  __shared__ unsigned sh[6];
+  if (threadIdx.x < 6) sh[threadIdx.x] = 0u;
   __syncthreads();
   if ((threadIdx.x & 31) == 0) {
     atomicMax(&sh[0], mt);
     atomicMax(&sh[1], mm);
     atomicMax(&sh[2], ~mn);
     atomicMax(&sh[3], mx);
+    atomicMax(&sh[4], ~nt);
+    atomicMax(&sh[5], ~nm);
   }
   __syncthreads();
   if (threadIdx.x == 0) {
@@ -847,6 +947,8 @@ __global__ void __launch_bounds__(256)
     atomicMax(&ctl->mx_mass, sh[1]);
     atomicMax(&ctl->mn_bits, sh[2]);  // complemented: the control block starts as zeros
     atomicMax(&ctl->mx_bits, sh[3]);
+    atomicMax(&ctl->mn_term, sh[4]);
+    atomicMax(&ctl->mn_mass, sh[5]);
   }
 }
 
@@ -887,10 +989,37 @@ __global__ void __launch_bounds__(256)
   ctl->node_end = 1;
 }
 
+// A chunk's `len` elements into its warps' records.
+template <int PT, bool WIDE>
+__device__ __forceinline__ void chunk_sums(const float4 *__restrict__ pos, int32_t len,
+                                           const SumScales &S, NodeAcc *part) {
+  constexpr int kU = 4;
+  LaneAcc<WIDE> a;
+  a.zero();
+  int cnt = 0;
+  for (int j0 = 0; j0 < PT && j0 * kChunkThreads < len; j0 += kU) {
+    float4 p[kU];
+#pragma unroll
+    for (int u = 0; u < kU; ++u) {
+      const int e = (j0 + u) * kChunkThreads + threadIdx.x;
+      if (e < len) p[u] = pos[e];
+    }
+#pragma unroll
+    for (int u = 0; u < kU; ++u) {
+      const int e = (j0 + u) * kChunkThreads + threadIdx.x;
+      if (e < len) {
+        a.add(p[u], S);
+        ++cnt;
+      }
+    }
+  }
+  a.template reduce<32>(&part[threadIdx.x >> 5], true, cnt, true, S);  // a warp has at most 512 elements
+}
+
 // Statistics of every node of the level, and its split decision by the block
 // that adds a node's last chunk.
 template <int PT>
-__global__ void __launch_bounds__(kChunkThreads)
+__global__ void __launch_bounds__(kChunkThreads, kLevelBlocks)
     k_level_stats(const float4 *__restrict__ pos, DNode *nodes, LevelCtl *ctl, int32_t level,
                   const int32_t *__restrict__ chunk_node, const int32_t *__restrict__ chunk_base,
                   NodeAcc *acc, unsigned *ticket, int32_t *fallback, int64_t *counters,
@@ -898,39 +1027,29 @@ __global__ void __launch_bounds__(kChunkThreads)
   chain_enter();
   LevelSpan L;
   if (!level_runs(ctl, level, L, true) || int32_t(blockIdx.x) >= L.nchunk) return;
-  constexpr int kW = kChunkThreads / 32, kU = 4;
+  constexpr int kW = kChunkThreads / 32;
   __shared__ NodeAcc part[kW];
   const ChunkRange R = chunk_range<PT>(nodes, chunk_node, chunk_base, L.nb, int32_t(blockIdx.x));
-  const SumScales S(ctl);
-  LaneAcc a;
-  a.zero();
-  int cnt = 0;
-  for (int j0 = 0; j0 < PT && j0 * kChunkThreads < R.len; j0 += kU) {
-    float4 p[kU];
-#pragma unroll
-    for (int u = 0; u < kU; ++u) {
-      const int e = (j0 + u) * kChunkThreads + threadIdx.x;
-      if (e < R.len) p[u] = pos[R.begin + e];
-    }
-#pragma unroll
-    for (int u = 0; u < kU; ++u) {
-      const int e = (j0 + u) * kChunkThreads + threadIdx.x;
-      if (e < R.len) {
-        a.add(p[u], S);
-        ++cnt;
-      }
-    }
-  }
-  a.reduce<32>(&part[threadIdx.x >> 5], true, cnt, true, S);  // a warp has at most 512 elements
+  const SumScales S(ctl, wide_range(*ctl));
+  if (S.wide) chunk_sums<PT, true>(pos + R.begin, R.len, S, part);
+  else chunk_sums<PT, false>(pos + R.begin, R.len, S, part);
   __syncthreads();
   if (threadIdx.x >= 32) return;
   // a thread per word: the warps' records into the node's, one atomic each
   NodeAcc &T = acc[R.node - L.nb];
   const int f = threadIdx.x;
+  long long sum = 0;
+  unsigned bits = 0;
+  if (f < kAccWords) merge_word(part, kW, f, &sum, &bits);
+  if (S.wide) {
+    // what passes 2^44 of the lower integers' sums goes to the upper ones', so
+    // that the chunks of any node fit 64 bits
+    const long long up = f >= 4 && f < 8 ? (sum + (1ll << 43)) >> 44 : 0;
+    sum -= up * (1ll << 44);
+    const long long add = __shfl_down_sync(0xffffffffu, up, 4);
+    if (f < 4) sum += add;
+  }
   if (f < kAccWords) {
-    long long sum;
-    unsigned bits;
-    merge_word(part, kW, f, &sum, &bits);
     unsigned *word = reinterpret_cast<unsigned *>(&T) + 8 + f;
     if (f < 8) atomicAdd(reinterpret_cast<unsigned long long *>(&T) + f, (unsigned long long)sum);
     else if (acc_or(f)) atomicOr(word, bits);
@@ -1700,6 +1819,7 @@ constexpr int kSubBatch = 256;       // nodes of a level taken at a time
 constexpr int kSubLevel = 512;       // level whose nodes stay in shared memory
 constexpr int kSubDepth = 48;        // deepest level below a root; deeper: the level loop
 constexpr int kSubBytes = 16 + 3 * 2;  // shared memory an element
+constexpr int kErrRange = 6;         // C_ERR: launched for a set of the other range
 
 // Barrier over the warps of a team: named barrier 1 + team for teams of
 // several warps (at most 8 teams), __syncwarp for one warp.
@@ -1719,6 +1839,7 @@ struct SubNode {
   float xc[3];
 };
 
+template <bool WIDE>
 __global__ void __launch_bounds__(kSubThreads, 1)
     k_subtree(const DNode *__restrict__ nodes, const LevelCtl *ctl, const int2 *__restrict__ roots,
               float4 *pos_a, int32_t *oid_a, const float4 *pos_b, const int32_t *oid_b, DNode *sub,
@@ -1741,12 +1862,17 @@ __global__ void __launch_bounds__(kSubThreads, 1)
   __shared__ int nopen, largest;
   if (!ctl->done || ctl->abort) return;
   const int32_t r = int32_t(blockIdx.x);
+  if (wide_range(*ctl) != WIDE) {  // the host launches the other one
+    if (r < ctl->nroots && threadIdx.x == 0)
+      atomicCAS(reinterpret_cast<int32_t *>(counters + C_ERR), 0, kErrRange);
+    return;
+  }
   if (r >= ctl->nroots) {  // the host launched for the most there can be
     for (int dd = int(threadIdx.x); dd < kSubDepth; dd += kSubThreads)
       hist[int64_t(dd) * gridDim.x + r] = 0;
     return;
   }
-  const SumScales S(ctl);
+  const SumScales S(ctl, WIDE);
   const int2 root = roots[r];
   const int rcnt = nodes[root.x].count;
   const int32_t roff = nodes[root.x].offset;
@@ -1828,17 +1954,18 @@ __global__ void __launch_bounds__(kSubThreads, 1)
         // few enough warps that a lane has about 8 elements: what a warp's
         // reduction costs is some 4 elements a lane
         const int uw = nw == 1 ? 1 : min(nw, max(1, c / 256));
-        LaneAcc a;
+        LaneAcc<WIDE> a;
         a.zero();
         int cnt = 0;
         if (oct) {
           for (int e = sl; e < c; e += 8, ++cnt) a.add(P[cur[lo + e]], S);
           __syncwarp();
-          a.reduce<8>(&st[min(f, kSubBatch - 1)], f < F, cnt, true, S);
+          a.template reduce<8>(&st[min(f, kSubBatch - 1)], f < F, cnt, true, S);
         } else if (wi < uw) {
           for (int e = tl; e < c; e += uw * 32, ++cnt) a.add(P[cur[lo + e]], S);
           __syncwarp();
-          a.reduce<32>(uw == 1 ? &st[f] : &wst[warp], true, cnt, 32 * ((c + uw * 32 - 1) / (uw * 32)) <= 1023, S);
+          a.template reduce<32>(uw == 1 ? &st[f] : &wst[warp], true, cnt,
+                                32 * ((c + uw * 32 - 1) / (uw * 32)) <= 1023, S);
         }
         if (nw > 1) {
           team_sync(team, nw);
@@ -1876,9 +2003,9 @@ __global__ void __launch_bounds__(kSubThreads, 1)
           float xc[3];
           bool ok = false;
           if (force_fallback == 0 && !S.bad) {
-            NodeSums Q = node_sums(st[f], c);
+            NodeSums Q = node_sums(st[f], c, S.wide);
             int low[4] = {0, 0, 0, 0};
-            const int ux = S.c.k - 45, um = S.m.k - 45;
+            const int low_e = S.wide ? 67 : 45, ux = S.c.k - low_e, um = S.m.k - low_e;
             for (int e = lane; e < c; e += 32) {
               const float4 p = P[cur[lo + e]];
               low[0] += lsb_exp(fmul_(p.w, p.x)) < last_place(Q.abs[0]) + ux;
@@ -3607,8 +3734,9 @@ cudaError_t DeviceTree::build(const TreeConfig &cfg, int64_t n, const float4 *po
   static_assert(kCtlOff % alignof(LevelCtl) == 0, "alignment");
   if (!counters_) {
     DT_CHECK(cudaHostAlloc(&h_counters_, kStateBytes, cudaHostAllocDefault));
-    DT_CHECK(cudaFuncSetAttribute(k_subtree, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                  kSubMax * kSubBytes));
+    for (auto *k : {k_subtree<false>, k_subtree<true>})
+      DT_CHECK(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                    kSubMax * kSubBytes));
     DT_CHECK(cudaMalloc(&counters_, kStateBytes));
     // the kernels' error flag lives in a counter slot: read back with the counters
     walk_err_ = reinterpret_cast<int32_t *>(counters_ + C_ERR);
@@ -3709,8 +3837,8 @@ cudaError_t DeviceTree::build(const TreeConfig &cfg, int64_t n, const float4 *po
       DT_CHECK(grow(sub_first_, cap_sf_, size_t(max_roots) * (kSubDepth + 2), s));
       DT_CHECK(grow(sub_hist_, cap_sh_, size_t(max_roots) * kSubDepth, s));
       const int32_t cap = int32_t((std::min<int64_t>(n, sub_max) + 7) & ~int64_t(7));
-      launch_chained(k_subtree, unsigned(max_roots), kSubThreads, size_t(cap) * kSubBytes, s,
-                     nodes_, ctl, roots_, epos_, oid_, tpos_, toid_, sub_nodes_, sub_first_,
+      launch_chained(wide_ ? k_subtree<true> : k_subtree<false>, unsigned(max_roots), kSubThreads,
+                     size_t(cap) * kSubBytes, s, nodes_, ctl, roots_, epos_, oid_, tpos_, toid_, sub_nodes_, sub_first_,
                      sub_hist_, cap, cfg.force_cm_fallback, cfg.nd, counters_);
       launch_chained(k_subtree_scan, kSubDepth, kScanThreads, 0, s, ctl, counters_, sub_hist_,
                      int32_t(max_roots), sub_tot);
@@ -3730,7 +3858,11 @@ cudaError_t DeviceTree::build(const TreeConfig &cfg, int64_t n, const float4 *po
       sub_off_ = false;
       return e;
     }
-    if (err) {
+    if (err == kErrRange) {
+      // the levels are there; the subtrees again, by the other kernel
+      wide_ = !wide_;
+      DT_CHECK(cudaMemsetAsync(walk_err_, 0, sizeof(int32_t), s));
+    } else if (err) {
       err_ = err == 3 ? "subtree: a node outgrew the block's shared memory"
                       : "partition chain check failed";
       return cudaErrorUnknown;
@@ -3744,6 +3876,7 @@ cudaError_t DeviceTree::build(const TreeConfig &cfg, int64_t n, const float4 *po
     nroots = hc->nroots;
     level_ne = hc->node_end;
     level_max = X.maxcnt;
+    if (err == kErrRange) continue;
     if (hc->abort) {
       // undecided centres of mass in this level: certify them, or sum as the
       // reference does, then go on from its left counts
