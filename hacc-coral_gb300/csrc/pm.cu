@@ -153,10 +153,11 @@ __global__ void __launch_bounds__(kThreads)
 // -D_a potential need one inverse transform, not three.  The double-precision
 // transforms are bound by the FP64 pipe (0.93 of the 1.07 ms of a 128^3 kick
 // were one forward and three inverse transforms; 0.68 ms now); the differences
-// read the potential from L2.  The potential's rounding, about 1e-16 of it, is some
-// ng / 2 pi times larger beside the gradient's than before: below 1e-13 at the
-// largest grid, with the fields rounded to float (6e-8).  Single precision has
-// no such room and keeps the three spectra.
+// read the potential from L2.  The potential's rounding, about 1e-16 of it, weighs
+// up to ng / 2 pi times more beside the gradient: 1e-13 of the fields' rms at
+// 256^3 (2e-14 for white noise) and some 2e-12 at the largest grid, with the
+// fields rounded to float (6e-8).  Single precision has no such room and keeps
+// the three spectra.
 // A thread per (y, z) column marches `span` cells along x with its five x values
 // in registers; the y and z neighbours come through L1.  Up to 16 cells, fewer
 // where that would leave SMs without a block: a march is a chain of L2 loads
