@@ -47,7 +47,7 @@ constexpr int kChainSteps = 32;     // chain steps before a subtree block jumps 
 constexpr int kPlainSteps = 4;      // single chain steps before the chunk partition jumps runs
 
 enum { C_NFALLBACK = 2, C_NLEAF = 3, C_NSEG = 4, C_NENT = 5,
-       C_PAIRS = 6, C_PADDED = 7, C_NITEMS = 8, C_MAXLEN = 9, C_TDONE1 = 10, C_TDONE2 = 11,
+       C_PAIRS = 6, C_PADDED = 7, C_NITEMS = 8, C_TDONE1 = 10, C_TDONE2 = 11,
        C_NTIGHT = 12, C_SEGOVF = 13, C_ERR = 15, C_BUCKET = 16, C_FILL = 48,
        C_SUBFB = 80, C_CHAINS = 81, C_TICKET = 82, C_SEQ = 83, C_COUNT = 84 };
 
@@ -1458,7 +1458,7 @@ __global__ void __launch_bounds__(256)
 
 // ---------------------------------------------------------------------------
 // Tight certification of the centre of mass for the nodes the loose bound
-// could not decide (k_stats_final's fallback list, at most kTightNodes of
+// could not decide (the list that k_level_stats leaves, at most kTightNodes of
 // them per level).  The reference's sequential sum s_k = fl(s_{k-1} + t_k)
 // differs from the exact sum by sum_k d_k, where the rounding error d_k is
 // zero when s_{k-1} and t_k are both multiples of ulp(s_k) (then the exact
@@ -3206,7 +3206,7 @@ __global__ void __launch_bounds__(128)
   if (threadIdx.x < 32) hist[threadIdx.x] = 0;
   __syncthreads();
   const int64_t li = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
-  long long pairs = 0, padded = 0, mx = 0;
+  long long pairs = 0, padded = 0;
   if (li < nleaves) {
     LeafDesc d{};
     if (DESC) {
@@ -3219,7 +3219,6 @@ __global__ void __launch_bounds__(128)
       ld[li] = d;
       pairs = (long long)T.count * list_len[li];
       padded = (long long)((T.count + 31) / 32) * 32 * d.kept_len;
-      mx = d.kept_len;
     } else {
       d = ld[li];
     }
@@ -3231,12 +3230,10 @@ __global__ void __launch_bounds__(128)
     for (int o = 16; o > 0; o >>= 1) {
       pairs += __shfl_xor_sync(0xffffffffu, pairs, o);
       padded += __shfl_xor_sync(0xffffffffu, padded, o);
-      mx = max(mx, __shfl_xor_sync(0xffffffffu, mx, o));
     }
     if ((threadIdx.x & 31) == 0) {
       atomicAdd((unsigned long long *)&counters[C_PAIRS], (unsigned long long)pairs);
       atomicAdd((unsigned long long *)&counters[C_PADDED], (unsigned long long)padded);
-      atomicMax((long long *)&counters[C_MAXLEN], mx);
     }
   }
   __syncthreads();
@@ -3350,8 +3347,8 @@ __global__ void k_outputs(KickArrays in, const float4 *__restrict__ table,
 }
 
 // A kick's results into the caller's device arrays, all ten in one launch
-// (thirteen copies before: 3 us each at a few thousand particles, where they
-// were a tenth of the call).
+// (thirteen copies are 3 us each at a few thousand particles, a tenth of the
+// call).
 __global__ void k_finish(const float4 *__restrict__ table, const float *__restrict__ vel,
                          KickArrays st, KickArrays out, int64_t n) {
   chain_enter();
@@ -3406,7 +3403,6 @@ __global__ void k_scatter3_f32(const float *__restrict__ in, int64_t stride,
   }
 }
 
-// acc holds, per node, sum over it and its ancestors of xbar_P / M_P.
 // Monopole pseudo-particle gradients passed to the particles: a warp per
 // leaf sums xbar / m of the nodes on its root-to-leaf path (root first, the
 // same float additions as a level-by-level top-down pass) and adds m_k times
@@ -3665,7 +3661,7 @@ inline unsigned grid_for(int64_t n, int threads, int64_t cap = 0) {
 DeviceTree::~DeviceTree() {
   void *ptrs[] = {epos_, tpos_, oid_, toid_, idx_, nodes_, ppm_, chunk_node_, chunk_base_,
                   left_cnt_, left_base_, acc_, ticket_, scan_tmp_, node_tmp_, fallback_, counters_, leaf_ids_,
-                  up_, processed_, roots_, leafdesc_, segs_, idx_list_, items_, items_tmp_, gidx_,
+                  up_, processed_, roots_, leafdesc_, segs_, idx_list_, items_, gidx_,
                   tight_chunks_, tight_nodes_, segs_local_, ridx_, sub_nodes_, sub_first_,
                   sub_hist_, wpre_, chains_};
   for (void *p : ptrs)
@@ -4123,7 +4119,6 @@ cudaError_t DeviceTree::launch_groups(int64_t max_leaves, int G, int half, cudaS
 
 // The items of the leaves whose buckets k_leaf_items placed; joins the groups.
 cudaError_t DeviceTree::fill_items(int64_t jsplit, cudaStream_t s) {
-  const int64_t nleaves = info_.processed_leaves;
   if (groups_ready_) DT_CHECK(cudaStreamWaitEvent(s, ev_groups_, 0));  // launched by build()
   groups_ready_ = 0;
   DT_CHECK(cudaMemcpyAsync(h_counters_, counters_, C_COUNT * sizeof(int64_t), cudaMemcpyDeviceToHost, s));

@@ -171,8 +171,8 @@ class DeviceTree {
   size_t cap_segl_ = 0;
   int32_t *idx_list_ = nullptr;
   size_t cap_idx_ = 0;
-  PairItem *items_ = nullptr, *items_tmp_ = nullptr;
-  size_t cap_items_ = 0, cap_items_tmp_ = 0;
+  PairItem *items_ = nullptr;
+  size_t cap_items_ = 0;
   int32_t *gidx_ = nullptr;
   size_t cap_gidx_ = 0;
   int32_t *walk_err_ = nullptr;

@@ -505,10 +505,10 @@ cudaError_t launch_tag_items(const PairItem *in, PairItem *out, int64_t n, int b
 // pairs, lanes 16-31 the second.  The entry's sums over the particles stay in
 // the lane (one exchange between the half-warps per 16 entries, then the
 // atomics), the particles' sums over the entries stay in registers until the
-// list ends.  With a lane per particle, as before, every entry's sum had to
-// cross the warp through shared memory: a quarter of the kernel's
-// instructions (64^3 Zel'dovich set: 456 us before, 320 us now; eight 96^3
-// boxes: 9.0 ms, 7.1 ms).  What bounds it: dispatch.  A packed operation takes two
+// list ends.  (A lane per particle makes every entry's sum cross the warp through
+// shared memory, a quarter of that kernel's instructions.  64^3 Zel'dovich set:
+// 456 us with a lane per particle, 320 with one per entry; eight 96^3 boxes: 9.0
+// and 7.1 ms.)  What bounds it: dispatch.  A packed operation takes two
 // dispatch slots, 82 of the 98 that a pair of particles against an entry
 // needs here.
 // ---------------------------------------------------------------------------

@@ -134,16 +134,21 @@ __global__ void __launch_bounds__(kRadixThreads)
 }
 
 // ---- counting sort by cell --------------------------------------------------
-// Three radix passes and ten permutations with their copies back were 45
-// launches and 210 us at 88,000 particles, most of it launch gaps and 22
-// blocks on 152 SMs.  Here a particle's place is its cell's offset plus its
-// rank among the cell's particles: six launches.  A cell's particles arrive in
+// A particle's place is its cell's offset plus its rank among the cell's
+// particles: six launches, where three radix passes with their scans take 15
+// and leave most SMs without a block below a few hundred thousand particles.  A cell's particles arrive in
 // any order, so each counts the ones of its cell with a smaller index, which
 // makes the sort stable.  Particles outside the box get a pseudo-cell for
 // every 32 indices behind the grid's cells, which keeps their order with the
 // same rule and no long cell.
 constexpr uint32_t kOutRun = 32;       // indices per pseudo-cell
-constexpr int kMaxOcc = 1024;          // longest cell whose ranks are counted
+// Longest cell whose ranks are counted: a set with a longer one has paid for both
+// sorts.  A whole sub-cycle call less its kick, 2.6 M particles: 1.88 ms counted
+// with a cell of 900, 2.04 by both with one of 1100 (1.95 by radix alone); but
+// with half of them in cells of 1000 or 1100 2.19 counted and 1.92 by radix, and
+// with five cells of 20,000 3.01 and 1.96.  70 thousand, a cell of 1100: 0.39
+// counted, 0.45 by radix, 0.50 by both.
+constexpr int kMaxOcc = 1024;
 constexpr int kCellThreads = 256;
 constexpr int kCellPer = 16;
 constexpr int kCellTile = kCellThreads * kCellPer;  // cells per block of the scan
@@ -362,8 +367,11 @@ struct ResortLayout {
   }
   // The counting sort goes through every cell twice and a radix pass through
   // every particle three times, so a grid of many more cells than particles
-  // takes the radix sort; so does one of more than 16 M cells, whose tiles
-  // are too many to be added up by each block.
+  // takes the radix sort (a sub-cycle call less its kick: 0.37 ms counted and
+  // 0.45 by radix for 70 thousand particles in 80^3 cells, 0.53 and 0.62 for 300
+  // thousand in 128^3, seven cells a particle each; at 27 a particle 0.56 and
+  // 0.62: the line is on the safe side); so does one of more than 16 M cells,
+  // whose tiles are too many to be added up by each block.
   static bool counted(int64_t n, const int32_t ng[3]) {
     return grid_cells(ng) <= 8 * n && cells(n, ng) <= kMaxTiles * kCellTile;
   }

@@ -29,8 +29,8 @@ def _set(n, line, first):
                            np.zeros(n, np.uint16), nglt=(30, 30, 30))
 
 
-def _compare(ctx, p):
-    kp = synth.kick_params(p, nd=1, fcoeff=0.0)
+def _compare(ctx, p, nd=1):
+    kp = synth.kick_params(p, nd=nd, fcoeff=0.0)
     # the leaves of a corner: the tree is compared whole
     kp.min_force, kp.max_force = (0.5,) * 3, (5.0,) * 3
     q = p.copy()
@@ -44,8 +44,8 @@ def _compare(ctx, p):
 
 
 # 48 particles of a line reach level 47, the deepest a block holds; 70 reach 69
-@pytest.mark.parametrize("n,line,first", [(0, 48, 1.0), (0, 49, 1.0), (0, 70, 1.0), (100, 70, 1e-35),
-                                          (20000, 70, 1e-35)])
+@pytest.mark.parametrize("n,line,first", [(0, 48, 1.0), (0, 49, 1.0), (0, 70, 1.0),
+                                          (100, 70, 1e-35), (20000, 70, 1e-35)])
 def test_deep_tree_after_another(hsr_lib, n, line, first):
     ctx = hsr.Context()
     try:
@@ -55,3 +55,16 @@ def test_deep_tree_after_another(hsr_lib, n, line, first):
         _compare(ctx, _set(9000, 1, 1.0))
     finally:
         ctx.close()
+
+
+def test_more_than_64_levels_of_large_nodes(ctx):
+    """Masses growing by exp(70) along a line of 200,000: 68 levels of nodes too
+    large for a subtree block, each with centres of mass to certify, 77 in all."""
+    n = 200_000
+    x = np.full((n, 3), 3.0, np.float32)
+    x[:, 0] = 1 + 0.125 * np.arange(n)
+    z = np.zeros((4, n), np.float32)
+    p = synth.Particles(*(np.ascontiguousarray(x[:, d]) for d in range(3)), *z[:3],
+                        np.exp(70.0 * np.arange(n) / n).astype(np.float32), z[3],
+                        np.arange(n, dtype=np.int64), np.zeros(n, np.uint16), nglt=(25001, 4, 4))
+    _compare(ctx, p, nd=64)

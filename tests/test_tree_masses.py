@@ -1,6 +1,6 @@
 """The device tree's centre-of-mass sums over sets whose masses are not all the
-same, or not of ordinary size, against the host build: the same permutation of
-every array, bit for bit, and the same lists."""
+same, or not of ordinary size, and nodes that are not split, against the host
+build: the same permutation of every array, bit for bit, and the same lists."""
 import numpy as np
 import pytest
 
@@ -81,3 +81,15 @@ def test_sets_of_wide_range(ctx, n, nd, make, factor, far):
     # against the 2^-25 that a quotient is rounded by
     if make is _heavy and 1e6 <= max(factor, abs(far or 0)) <= 1e9:
         assert st["cm_fallbacks"] <= 0.04 * st["nodes"]
+
+
+@pytest.mark.parametrize("n,nd", [(30000, 9000), (30000, 40000), (70000, 20000)])
+def test_leaves_larger_than_a_subtree_block(ctx, n, nd):
+    rng = np.random.default_rng(n + nd)
+    compare(ctx, (rng.random((n, 3)) * 20).astype(np.float32), np.ones(n), nd)
+
+
+@pytest.mark.parametrize("n", [300, 9000])
+def test_one_place(ctx, n):
+    """Every split leaves a part empty: the root is the only leaf, above its size."""
+    compare(ctx, np.full((n, 3), 0.1, np.float32), np.ones(n), 16)
