@@ -47,7 +47,7 @@ constexpr int kChainSteps = 32;     // chain steps before a subtree block jumps 
 constexpr int kPlainSteps = 4;      // single chain steps before the chunk partition jumps runs
 
 enum { C_NFALLBACK = 2, C_NLEAF = 3, C_NSEG = 4, C_NENT = 5,
-       C_PAIRS = 6, C_PADDED = 7, C_NITEMS = 8, C_TDONE1 = 10, C_TDONE2 = 11,
+       C_PAIRS = 6, C_PADDED = 7, C_NITEMS = 8, C_BIG = 9, C_TDONE1 = 10, C_TDONE2 = 11,
        C_NTIGHT = 12, C_SEGOVF = 13, C_ERR = 15, C_BUCKET = 16, C_FILL = 48,
        C_SUBFB = 80, C_CHAINS = 81, C_TICKET = 82, C_SEQ = 83, C_COUNT = 84 };
 
@@ -2916,6 +2916,7 @@ constexpr int kGroupHalf = 16;  // particles of a group with a box of their own 
 constexpr int kGW = 256;     // leaves up to this size are grouped by one warp
 constexpr int kGWarps = 4;   // warps (leaves) per block of k_groups_warp
 constexpr int kGroupThreads = 256;
+constexpr int kGroupBlocks = 8;  // blocks of k_groups an SM holds (2048 threads)
 
 // Where a segment of c > kGroupHalf particles is split: between groups, and a
 // group between its first 16 particles and the rest.
@@ -3043,36 +3044,29 @@ __device__ void group_large_leaf(const DNode &T, const float4 *__restrict__ pos,
   for (int i = threadIdx.x; i < c; i += blockDim.x) gidx[T.offset + i] = val[i];
 }
 
-// The leaves too large for k_groups_warp, block by block: each block looks
-// kGroupThreads leaves over and groups the large ones among them (a block a
-// leaf, most of them returning at once, took 31 us of a 128^3 kick).
+// The leaves that k_groups_warp found too large, a block each at a time: as many
+// blocks as the SMs hold share them out.  (A block a leaf of the whole set, most
+// of them returning at once, takes 31 us of a 128^3 kick; a block per 256 leaves,
+// one after the other, 11 ms of a 32^3 kick with leaves of 512.)
 __global__ void __launch_bounds__(kGroupThreads)
-    k_groups(const DNode *nodes, const int32_t *leaf_ids, const int64_t *nleaves,
+    k_groups(const DNode *nodes, const int32_t *big, const int64_t *nbig,
              const float4 *__restrict__ pos, int32_t *gidx, int G, int half) {
-  __shared__ int32_t big[kGroupThreads];
-  __shared__ int nbig;
-  if (threadIdx.x == 0) nbig = 0;
-  __syncthreads();
-  const int64_t li = int64_t(blockIdx.x) * kGroupThreads + threadIdx.x;
-  if (li < *nleaves) {
-    const int32_t t = leaf_ids[li];
-    if (nodes[t].count > kGW) big[atomicAdd(&nbig, 1)] = t;
-  }
-  __syncthreads();
-  for (int b = 0; b < nbig; ++b) {
+  const int64_t n = *nbig;
+  for (int64_t b = blockIdx.x; b < n; b += gridDim.x) {
     group_large_leaf(nodes[big[b]], pos, gidx, G, half);
     __syncthreads();  // the next leaf reuses the shared arrays
   }
 }
 
 // Warp-per-leaf grouping for leaves of at most kGW particles (the usual
-// case; larger leaves take k_groups).  Same median splits as k_groups: per
+// case; larger leaves are left to k_groups, in big).  Same median splits as k_groups: per
 // level, every segment above `half` particles is sorted along its longest
 // axis by ranking (each element counts the keys below its own, ties by
 // position) and split at group_split().
 __global__ void __launch_bounds__(32 * kGWarps)
     k_groups_warp(const DNode *nodes, const int32_t *leaf_ids, const int64_t *nleaves,
-                  const float4 *__restrict__ pos, int32_t *gidx, int G, int half) {
+                  const float4 *__restrict__ pos, int32_t *gidx, int G, int half, int32_t *big,
+                  int64_t *nbig) {
   __shared__ float key[kGWarps][kGW];
   __shared__ int32_t val[kGWarps][2][kGW];
   __shared__ uint8_t segid[kGWarps][kGW];
@@ -3083,6 +3077,8 @@ __global__ void __launch_bounds__(32 * kGWarps)
   if (li >= *nleaves) return;
   const DNode &T = nodes[leaf_ids[li]];
   const int c = T.count;
+  if (c > kGW && lane == 0)
+    big[atomicAdd(reinterpret_cast<unsigned long long *>(nbig), 1ull)] = leaf_ids[li];
   if (c <= 0 || c > kGW) return;
   if (c <= half) {
     for (int i = lane; i < c; i += 32) gidx[T.offset + i] = T.offset + i;
@@ -3659,7 +3655,7 @@ inline unsigned grid_for(int64_t n, int threads, int64_t cap = 0) {
 // ---------------------------------------------------------------------------
 
 DeviceTree::~DeviceTree() {
-  void *ptrs[] = {epos_, tpos_, oid_, toid_, idx_, nodes_, ppm_, chunk_node_, chunk_base_,
+  void *ptrs[] = {epos_, tpos_, oid_, toid_, idx_, nodes_, ppm_, chunk_node_, chunk_base_, big_leaves_,
                   left_cnt_, left_base_, acc_, ticket_, scan_tmp_, node_tmp_, fallback_, counters_, leaf_ids_,
                   up_, processed_, roots_, leafdesc_, segs_, idx_list_, items_, gidx_,
                   tight_chunks_, tight_nodes_, segs_local_, ridx_, sub_nodes_, sub_first_,
@@ -3936,6 +3932,7 @@ cudaError_t DeviceTree::build(const TreeConfig &cfg, int64_t n, const float4 *po
   DT_CHECK(grow(up_, cap_up_, size_t(nnodes), s));
   DT_CHECK(grow(processed_, cap_pr_, size_t(nnodes), s));
   DT_CHECK(grow(leaf_ids_, cap_leaf_, size_t(max_leaves), s));
+  DT_CHECK(grow(big_leaves_, cap_big_, size_t(max_leaves), s));
   const unsigned gN = unsigned((nnodes + 127) / 128), gP = unsigned((int64_t(nnodes) * 32 + 127) / 128);
   launch_chained(k_links, gN, 128, 0, s, nodes_, nnodes, up_);
   if (k == 12)
@@ -4098,6 +4095,7 @@ cudaError_t DeviceTree::regroup(int group, int64_t jsplit, cudaStream_t s) {
   const int64_t nleaves = info_.processed_leaves;
   DT_CHECK(cudaMemsetAsync(counters_ + C_BUCKET, 0, 32 * sizeof(int64_t), s));
   DT_CHECK(cudaMemsetAsync(counters_ + C_TICKET, 0, sizeof(int64_t), s));
+  DT_CHECK(cudaMemsetAsync(counters_ + C_BIG, 0, sizeof(int64_t), s));
   if (nleaves > 0) {
     DT_CHECK(launch_groups(nleaves, group, group, s));
     launch_chained(k_leaf_items<false>, unsigned((nleaves + 127) / 128), 128, 0, s, nullptr, nullptr,
@@ -4110,9 +4108,9 @@ cudaError_t DeviceTree::regroup(int group, int64_t jsplit, cudaStream_t s) {
 
 cudaError_t DeviceTree::launch_groups(int64_t max_leaves, int G, int half, cudaStream_t s) {
   k_groups_warp<<<unsigned((max_leaves + kGWarps - 1) / kGWarps), 32 * kGWarps, 0, s>>>(
-      nodes_, leaf_ids_, counters_ + C_NLEAF, epos_, gidx_, G, half);
-  k_groups<<<unsigned((max_leaves + kGroupThreads - 1) / kGroupThreads), kGroupThreads, 0, s>>>(
-      nodes_, leaf_ids_, counters_ + C_NLEAF, epos_, gidx_, G, half);
+      nodes_, leaf_ids_, counters_ + C_NLEAF, epos_, gidx_, G, half, big_leaves_, counters_ + C_BIG);
+  k_groups<<<unsigned(std::min<int64_t>(max_leaves, int64_t(sm_count()) * kGroupBlocks)),
+             kGroupThreads, 0, s>>>(nodes_, big_leaves_, counters_ + C_BIG, epos_, gidx_, G, half);
   info_.launches += 2;
   return cudaGetLastError();
 }

@@ -158,8 +158,8 @@ class DeviceTree {
   // block, and a pinned copy
   int64_t *counters_ = nullptr, *h_counters_ = nullptr;
   // lists
-  int32_t *leaf_ids_ = nullptr;
-  size_t cap_leaf_ = 0;
+  int32_t *leaf_ids_ = nullptr, *big_leaves_ = nullptr;  // big: too large for a warp to group
+  size_t cap_leaf_ = 0, cap_big_ = 0;
   int2 *up_ = nullptr;             // per node: parent, arrivals from below
   int32_t *processed_ = nullptr;   // per node: processed leaves below it
   size_t cap_up_ = 0, cap_pr_ = 0;
