@@ -2751,7 +2751,7 @@ __global__ void __launch_bounds__(32 * kWalkWarps)
               ++nout;
             }
             expand = nout > 0;
-          } else if (big || dist2 <= fsr2) {
+          } else if (big || !(dist2 > fsr2)) {  // (a node without mass: NaN)
             nout = 1;
             o0 = big || Q.count <= k ? make_int2(Q.offset, Q.count)
                                      : make_int2(int32_t(n + int64_t(t) * k), k);

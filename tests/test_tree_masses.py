@@ -10,14 +10,22 @@ import synth
 pytestmark = pytest.mark.gpu
 
 
-def compare(ctx, x, mass, nd):
+def same_bits(a, b):
+    return np.array_equal(a.view(np.uint8), b.view(np.uint8))
+
+
+def same_or_nan(a, b):  # (NaN has other bits on each machine)
+    return np.array_equal(a, b, equal_nan=a.dtype == np.float32)
+
+
+def compare(ctx, x, mass, nd, lists=4, same=same_bits, **opening):
     """The tree whole, the lists of the leaves in a corner; the kick's statistics."""
     n = len(x)
     zero = np.zeros((4, n), np.float32)
     p = synth.Particles(*(np.ascontiguousarray(x[:, d], np.float32) for d in range(3)), *zero[:3],
                         np.asarray(mass, np.float32), zero[3], np.arange(n, dtype=np.int64),
                         np.zeros(n, np.uint16), nglt=(int(np.ceil(x.max())) + 1,) * 3)
-    kp = synth.kick_params(p, nd=nd, fcoeff=0.0)
+    kp = synth.kick_params(p, nd=nd, fcoeff=0.0, **opening)
     corner = float(np.quantile(x, 0.3))
     kp.min_force, kp.max_force = (-1.0,) * 3, (corner,) * 3
     q = p.copy()
@@ -27,8 +35,8 @@ def compare(ctx, x, mass, nd):
         assert np.array_equal(getattr(p, k).view(np.uint8), getattr(q, k).view(np.uint8)), k
     assert stats["processed_leaves"] == host.nleaves
     if host.nleaves:
-        for a, b in zip(ctx.lists(), host.get()):
-            assert np.array_equal(a.view(np.uint8), b.view(np.uint8))
+        for a, b in zip(ctx.lists()[:lists], host.get()):
+            assert same(a, b)
     return stats
 
 
@@ -93,3 +101,20 @@ def test_leaves_larger_than_a_subtree_block(ctx, n, nd):
 def test_one_place(ctx, n):
     """Every split leaves a part empty: the root is the only leaf, above its size."""
     compare(ctx, np.full((n, 3), 0.1, np.float32), np.ones(n), 16)
+
+
+def _massless(nd, share):
+    rng = np.random.default_rng(nd)
+    x = (rng.random((3001, 3)) * 20).astype(np.float32)
+    return x, np.where(rng.random(3001) < share, 0.0, 1.0), nd
+
+
+MASSLESS = [(1, 1, 0.1), (2, 1, 0.5), (8, 1, 0.1), (8, 1, 1.2), (2, 12, 0.5)]
+
+
+@pytest.mark.parametrize("share", [0.2, 0.7])
+@pytest.mark.parametrize("nd,tdpts,angle", MASSLESS)
+def test_lists_with_massless_nodes(ctx, nd, tdpts, angle, share):
+    """Nodes whose particles have no mass have no centre of mass (NaN): no test
+    of a distance from it holds, the one that drops far nodes neither."""
+    compare(ctx, *_massless(nd, share), lists=3, tdpts=tdpts, open_angle=angle)
