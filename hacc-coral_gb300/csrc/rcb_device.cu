@@ -2454,8 +2454,7 @@ __device__ __forceinline__ void monopole_climb(DNode *nodes, int32_t nnodes, int
   float m = 0.f;
   // a leaf's mass in its particles' order; a leaf left by a failed split keeps
   // zero (its children are empty)
-  bool sources = T.count <= cfg.nd && T.count > 1;
-  if (sources) {
+  if (T.count <= cfg.nd && T.count > 1) {
     const float *w = reinterpret_cast<const float *>(pos + T.offset) + 3;
     for (int32_t i0 = 0; i0 < T.count; i0 += 32) {
       const float v = i0 + lane < T.count ? w[4 * (i0 + lane)] : 0.f;
@@ -2476,14 +2475,10 @@ __device__ __forceinline__ void monopole_climb(DNode *nodes, int32_t nnodes, int
       scount = nodes[sib].count;
       soff = nodes[sib].offset;
     }
-    const float tdr = fmul_(cfg.ppc, pptdr_(T));
-    float x, y, z;
-    pppt_<1>(0, tdr, T.xc, x, y, z);
-    // the point's offset from the centre is 0, or NaN where the centre is (a node
-    // without mass) or the box is not finite: then so is each source's share
-    const float off = norm2_(fsub_(x, T.xc[0]), fsub_(y, T.xc[1]), fsub_(z, T.xc[2]));
-    if (sources && off != 0.f) m = off;
     if (lane == 0) {
+      const float tdr = fmul_(cfg.ppc, pptdr_(T));
+      float x, y, z;
+      pppt_<1>(0, tdr, T.xc, x, y, z);
       ppm[t] = m;
       table[n + t] = make_float4(x, y, z, m);
       nodes[t].tdr = tdr;
@@ -2506,7 +2501,6 @@ __device__ __forceinline__ void monopole_climb(DNode *nodes, int32_t nnodes, int
     m = 0.f;
     if (lc > 0) m = fadd_(m, l);
     if (rc > 0) m = fadd_(m, r);
-    sources = lc > 0 || rc > 0;
     t = parent;
     T = TP;
     U = UP;

@@ -118,11 +118,3 @@ def test_lists_with_massless_nodes(ctx, nd, tdpts, angle, share):
     """Nodes whose particles have no mass have no centre of mass (NaN): no test
     of a distance from it holds, the one that drops far nodes neither."""
     compare(ctx, *_massless(nd, share), lists=3, tdpts=tdpts, open_angle=angle)
-
-
-@pytest.mark.parametrize("share", [0.2, 0.7])
-@pytest.mark.parametrize("nd,tdpts,angle", MASSLESS)
-def test_pseudo_particles_of_massless_nodes(ctx, nd, tdpts, angle, share):
-    """A node without a centre of mass has a pseudo-particle of mass NaN, and so
-    have the nodes above it."""
-    compare(ctx, *_massless(nd, share), same=same_or_nan, tdpts=tdpts, open_angle=angle)
