@@ -457,7 +457,7 @@ __device__ __forceinline__ int low_of_mark(int mark) { return (7 * mark + 4) / 5
 // without that one: 2.90 and 3.01 ms; masses spread over a factor of 10^4: 3.44
 // and 3.04).
 constexpr int kWideTerm = 20, kWideMass = 12;
-__host__ __device__ __forceinline__ bool wide_range(const LevelCtl &ctl) {
+__device__ __forceinline__ bool wide_range(const LevelCtl &ctl) {
   // (bits of positive floats: 2^23 a power of two; nothing but zeros: ~0)
   const unsigned t = ~ctl.mn_term, m = ~ctl.mn_mass;
   return (ctl.mx_term > t && ctl.mx_term - t >= unsigned(kWideTerm) << 23) ||
@@ -952,12 +952,17 @@ __global__ void __launch_bounds__(256)
   }
 }
 
-// The root, its chunks and the first level.
+// The root, its chunks and the first level.  The launches that follow were made
+// for a set of either range (`wide`): where it is the other one, there is no level
+// and nothing is done, and the host launches all of it again for this one.
+constexpr int kErrRange = 6;  // C_ERR: the other range
 template <int PT>
 __global__ void __launch_bounds__(256)
     k_root(DNode *nodes, int64_t n, TreeConfig cfg, LevelCtl *ctl, int32_t *chunk_node,
-           int32_t *chunk_base, NodeAcc *acc, unsigned *ticket, int2 *roots, int32_t sub_max) {
+           int32_t *chunk_base, NodeAcc *acc, unsigned *ticket, int2 *roots, int32_t sub_max,
+           bool wide, int32_t *err) {
   chain_enter();
+  const bool other = wide_range(*ctl) != wide;
   const int32_t nc = chunks_of<PT>(int32_t(n));
   const bool sub = n <= sub_max;
   if (!sub)
@@ -980,13 +985,14 @@ __global__ void __launch_bounds__(256)
     acc_zero(acc[0]);
     ticket[0] = 0u;
   }
-  ctl->lev[0] = LevelSpan{0, sub ? 0 : 1, 0, 1, nc, 1, int32_t(n), 0};
+  ctl->lev[0] = LevelSpan{0, sub || other ? 0 : 1, 0, 1, nc, 1, int32_t(n), 0};
   ctl->lev[1] = LevelSpan{-1, 0, 0, 0, 0, 0, 0, 0};
   ctl->begin[0] = 0;
   if (sub) roots[0] = make_int2(0, 0);
   ctl->nroots = sub ? 1 : 0;
-  ctl->done = sub;
+  ctl->done = sub && !other;
   ctl->node_end = 1;
+  if (other) *err = kErrRange;
 }
 
 // A chunk's `len` elements into its warps' records.
@@ -1018,7 +1024,7 @@ __device__ __forceinline__ void chunk_sums(const float4 *__restrict__ pos, int32
 
 // Statistics of every node of the level, and its split decision by the block
 // that adds a node's last chunk.
-template <int PT>
+template <int PT, bool WIDE = false>
 __global__ void __launch_bounds__(kChunkThreads, kLevelBlocks)
     k_level_stats(const float4 *__restrict__ pos, DNode *nodes, LevelCtl *ctl, int32_t level,
                   const int32_t *__restrict__ chunk_node, const int32_t *__restrict__ chunk_base,
@@ -1030,9 +1036,8 @@ __global__ void __launch_bounds__(kChunkThreads, kLevelBlocks)
   constexpr int kW = kChunkThreads / 32;
   __shared__ NodeAcc part[kW];
   const ChunkRange R = chunk_range<PT>(nodes, chunk_node, chunk_base, L.nb, int32_t(blockIdx.x));
-  const SumScales S(ctl, wide_range(*ctl));
-  if (S.wide) chunk_sums<PT, true>(pos + R.begin, R.len, S, part);
-  else chunk_sums<PT, false>(pos + R.begin, R.len, S, part);
+  const SumScales S(ctl, WIDE);
+  chunk_sums<PT, WIDE>(pos + R.begin, R.len, S, part);
   __syncthreads();
   if (threadIdx.x >= 32) return;
   // a thread per word: the warps' records into the node's, one atomic each
@@ -1041,7 +1046,7 @@ __global__ void __launch_bounds__(kChunkThreads, kLevelBlocks)
   long long sum = 0;
   unsigned bits = 0;
   if (f < kAccWords) merge_word(part, kW, f, &sum, &bits);
-  if (S.wide) {
+  if (WIDE) {
     // what passes 2^44 of the lower integers' sums goes to the upper ones', so
     // that the chunks of any node fit 64 bits
     const long long up = f >= 4 && f < 8 ? (sum + (1ll << 43)) >> 44 : 0;
@@ -1075,6 +1080,9 @@ __global__ void __launch_bounds__(kChunkThreads, kLevelBlocks)
   }
   nodes[R.node] = N;
 }
+
+template <int PT>
+constexpr auto k_level_stats_wide = k_level_stats<PT, true>;
 
 // Left counts of the level's chunks and each warp's left elements before its
 // share of the chunk (the shares of k_part_left); only the split coordinate is
@@ -1819,7 +1827,6 @@ constexpr int kSubBatch = 256;       // nodes of a level taken at a time
 constexpr int kSubLevel = 512;       // level whose nodes stay in shared memory
 constexpr int kSubDepth = 48;        // deepest level below a root; deeper: the level loop
 constexpr int kSubBytes = 16 + 3 * 2;  // shared memory an element
-constexpr int kErrRange = 6;         // C_ERR: launched for a set of the other range
 
 // Barrier over the warps of a team: named barrier 1 + team for teams of
 // several warps (at most 8 teams), __syncwarp for one warp.
@@ -1862,11 +1869,6 @@ __global__ void __launch_bounds__(kSubThreads, 1)
   __shared__ int nopen, largest;
   if (!ctl->done || ctl->abort) return;
   const int32_t r = int32_t(blockIdx.x);
-  if (wide_range(*ctl) != WIDE) {  // the host launches the other one
-    if (r < ctl->nroots && threadIdx.x == 0)
-      atomicCAS(reinterpret_cast<int32_t *>(counters + C_ERR), 0, kErrRange);
-    return;
-  }
   if (r >= ctl->nroots) {  // the host launched for the most there can be
     for (int dd = int(threadIdx.x); dd < kSubDepth; dd += kSubThreads)
       hist[int64_t(dd) * gridDim.x + r] = 0;
@@ -3799,7 +3801,8 @@ cudaError_t DeviceTree::build(const TreeConfig &cfg, int64_t n, const float4 *po
     if (batch > 0) DT_CHECK(grow(chains_, cap_ch_, size_t(std::max<int64_t>(n, 1)), s));
     auto *acc = reinterpret_cast<NodeAcc *>(acc_);
     if (!started) {
-      LEVEL_LAUNCH(k_root, 1, nodes_, n, cfg, ctl, cn[0], cb[0], acc, ticket_, roots_, sub_max);
+      LEVEL_LAUNCH(k_root, 1, nodes_, n, cfg, ctl, cn[0], cb[0], acc, ticket_, roots_, sub_max,
+                   wide_, walk_err_);
       started = true;
     }
     float4 *pb[2] = {epos_, tpos_};
@@ -3808,7 +3811,10 @@ cudaError_t DeviceTree::build(const TreeConfig &cfg, int64_t n, const float4 *po
       const int32_t l = level + i;
       const int from = l & 1, to = from ^ 1;
       const unsigned grid = unsigned(n / chunk + wide(i) + 1);
-      if (counted)
+      if (counted && wide_)
+        LEVEL_LAUNCH(k_level_stats_wide, grid, pb[from], nodes_, ctl, l, cn[from], cb[from], acc, ticket_,
+                     fallback_, counters_, cfg.force_cm_fallback, cfg.nd);
+      else if (counted)
         LEVEL_LAUNCH(k_level_stats, grid, pb[from], nodes_, ctl, l, cn[from], cb[from], acc, ticket_,
                      fallback_, counters_, cfg.force_cm_fallback, cfg.nd);
       counted = true;
@@ -3850,11 +3856,13 @@ cudaError_t DeviceTree::build(const TreeConfig &cfg, int64_t n, const float4 *po
       sub_off_ = false;
       return e;
     }
-    if (err == kErrRange) {
-      // the levels are there; the subtrees again, by the other kernel
+    if (err == kErrRange) {  // (in the first pass only)
       wide_ = !wide_;
+      started = false;
       DT_CHECK(cudaMemsetAsync(walk_err_, 0, sizeof(int32_t), s));
-    } else if (err) {
+      continue;
+    }
+    if (err) {
       err_ = err == 3 ? "subtree: a node outgrew the block's shared memory"
                       : "partition chain check failed";
       return cudaErrorUnknown;
@@ -3868,7 +3876,6 @@ cudaError_t DeviceTree::build(const TreeConfig &cfg, int64_t n, const float4 *po
     nroots = hc->nroots;
     level_ne = hc->node_end;
     level_max = X.maxcnt;
-    if (err == kErrRange) continue;
     if (hc->abort) {
       // undecided centres of mass in this level: certify them, or sum as the
       // reference does, then go on from its left counts

@@ -185,7 +185,7 @@ class DeviceTree {
   int32_t *sub_hist_ = nullptr;
   size_t cap_sub_ = 0, cap_sf_ = 0, cap_sh_ = 0;
   bool sub_off_ = false;  // when set, every level runs in the level loop
-  bool wide_ = false;     // the last set's range: the subtrees' kernel to launch first
+  bool wide_ = false;     // the last set's range: its kernels are launched first
 };
 
 // The ten arrays of a kick: x, y, z, vx, vy, vz, mass, phi; ids; masks.
