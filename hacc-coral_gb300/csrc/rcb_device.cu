@@ -296,11 +296,11 @@ struct LevelCtl {
   int32_t nroots;      // subtree roots so far
   int32_t done;        // no node is left for the level loop
   int32_t node_end;    // nodes of all levels
-  unsigned mx_term, mx_mass;  // largest |w x|, |w y|, |w z| and |w|, as bits
-  unsigned mn_bits;    // smallest w by its bits, sign and all, complemented
-  unsigned mx_bits;    // largest w by them
-  unsigned mn_term;    // smallest over the elements of the largest of |w x|, |w y| and |w z|,
-  unsigned mn_mass;    // and smallest |w|, zeros aside, as bits, complemented
+  // the set's range, as bits of floats: largest |w x|, |w y|, |w z|, |w|; smallest and
+  // largest w by its bits, sign and all; smallest over the elements of the largest
+  // of |w x|, |w y| and |w z|, and smallest |w|, zeros aside.  (Maxima only, of
+  // the minima's complements: the block starts as zeros.)
+  unsigned range[8];
   unsigned ticket;     // chunks of the level counted
   int32_t next_level;  // the level made last
   int32_t begin[kCtlLevels];  // first node of a level, by level modulo kCtlLevels
@@ -449,19 +449,28 @@ __device__ __forceinline__ unsigned low_mark(unsigned iv2, unsigned iv3) {
 __device__ __forceinline__ int low_of_mark(int mark) { return (7 * mark + 4) / 5; }
 
 // Whether a set's range calls for the third integer: its largest mass 2^12 times
-// its smallest, or its largest term 2^20 times the largest of the element that
-// has the smallest one (2^10 times is what a box of millions has beside its
-// origin); zeros aside.  Two integers lose whole sets a little above (a kick of
-// 2.6 M particles in 137 cells, one of them 10^5 times as heavy or at 10^7 cells:
-// 24 and 27 ms, with three 3.0 and 2.9), and below the third only costs (the same
-// without that one: 2.90 and 3.01 ms; masses spread over a factor of 10^4: 3.44
-// and 3.04).
-constexpr int kWideTerm = 20, kWideMass = 12;
-__device__ __forceinline__ bool wide_range(const LevelCtl &ctl) {
+// its smallest; its largest term 2^20 times the largest of the element that has the
+// smallest one (2^10 times is what a box of millions has beside its origin); or the
+// largest term of one axis 2^5 times that of another (a sheet, a column); zeros
+// aside.  Two integers lose whole sets a little above (a kick of 2.6 M particles in
+// 137 cells, one of them 10^5 times as heavy or at 10^7 cells: 24 and 27 ms, with
+// three 3.0 and 2.9; the tree of a sheet of 2 M, 2^-8 as thick as wide: 3.5 and 0.93
+// ms), and below the third only costs (the kick without the heavy one: 2.90 and
+// 3.01 ms; masses spread over a factor of 10^4: 3.44 and 3.04; sheets of 70 thousand
+// and 2 M, 2^-5: trees of 0.245 and 1.09 ms, with three 0.255 and 0.94).
+constexpr int kWideTerm = 20, kWideMass = 12, kWideAxis = 5;
+__device__ __forceinline__ unsigned largest_term(const LevelCtl *ctl) {
+  return max(max(ctl->range[0], ctl->range[1]), ctl->range[2]);
+}
+__device__ __forceinline__ bool wide_range(const LevelCtl *ctl) {
   // (bits of positive floats: 2^23 a power of two; nothing but zeros: ~0)
-  const unsigned t = ~ctl.mn_term, m = ~ctl.mn_mass;
-  return (ctl.mx_term > t && ctl.mx_term - t >= unsigned(kWideTerm) << 23) ||
-         (ctl.mx_mass > m && ctl.mx_mass - m >= unsigned(kWideMass) << 23);
+  const unsigned mx = largest_term(ctl), m = ctl->range[3], lt = ~ctl->range[6], lm = ~ctl->range[7];
+  bool wide = (mx > lt && mx - lt >= unsigned(kWideTerm) << 23) ||
+              (m > lm && m - lm >= unsigned(kWideMass) << 23);
+#pragma unroll
+  for (int d = 0; d < 3; ++d)
+    wide |= ctl->range[d] != 0u && mx - ctl->range[d] >= unsigned(kWideAxis) << 23;
+  return wide;
 }
 
 // The scales of a set's terms, and its mass where all are the same (the
@@ -472,15 +481,15 @@ struct SumScales {
   bool uniform, bad, wide;
   unsigned wbits;
   __device__ __forceinline__ SumScales(const LevelCtl *ctl, bool wide_sums)
-      : c(ctl->mx_term), m(ctl->mx_mass), wide(wide_sums) {
-    wbits = ctl->mx_bits;
-    bad = SumScale::bad(ctl->mx_term) || SumScale::bad(ctl->mx_mass);
+      : c(largest_term(ctl)), m(ctl->range[3]), wide(wide_sums) {
+    wbits = ctl->range[5];
+    bad = SumScale::bad(largest_term(ctl)) || SumScale::bad(ctl->range[3]);
     // (the bits with the sign: as many +w as -w are no set of one mass; and one
     // that the integers do not hold goes the way that says so)
     int h;
     long long l;
     unsigned o;
-    uniform = wbits == ~ctl->mn_bits && mass_digits(h, l, o);
+    uniform = wbits == ~ctl->range[4] && mass_digits(h, l, o);
   }
   // The integers of the one mass, as NodeAcc sums them; whether they hold it.
   __device__ __forceinline__ bool mass_digits(int &h, long long &l, unsigned &o) const {
@@ -907,49 +916,41 @@ __global__ void __launch_bounds__(256)
     k_elements(const float4 *__restrict__ in, int64_t n, float4 *__restrict__ pos,
                int32_t *__restrict__ oid, LevelCtl *ctl) {
   chain_enter();
-  unsigned mt = 0, mm = 0, mn = 0xffffffffu, mx = 0, nt = 0xffffffffu, nm = 0xffffffffu;
+  unsigned mt[3] = {0, 0, 0}, mm = 0, mn = 0xffffffffu, mx = 0, nt = 0xffffffffu, nm = 0xffffffffu;
   for (int64_t i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x; i < n;
        i += int64_t(gridDim.x) * blockDim.x) {
     const float4 p = in[i];
     pos[i] = p;
     oid[i] = int32_t(i);
-    const unsigned t = max(max(__float_as_uint(fmul_(p.w, p.x)) & 0x7fffffffu,
-                               __float_as_uint(fmul_(p.w, p.y)) & 0x7fffffffu),
-                           __float_as_uint(fmul_(p.w, p.z)) & 0x7fffffffu);
+    const unsigned t[3] = {__float_as_uint(fmul_(p.w, p.x)) & 0x7fffffffu,
+                           __float_as_uint(fmul_(p.w, p.y)) & 0x7fffffffu,
+                           __float_as_uint(fmul_(p.w, p.z)) & 0x7fffffffu};
     const unsigned w = __float_as_uint(p.w) & 0x7fffffffu;
-    mt = max(mt, t);
+#pragma unroll
+    for (int d = 0; d < 3; ++d) mt[d] = max(mt[d], t[d]);
     mm = max(mm, w);
-    nt = min(nt, t - 1u);  // (zero as the largest: it is left aside)
+    nt = min(nt, max(max(t[0], t[1]), t[2]) - 1u);  // (zero as the largest: it is left aside)
     nm = min(nm, w - 1u);
     mn = min(mn, __float_as_uint(p.w));
     mx = max(mx, __float_as_uint(p.w));
   }
-  mt = __reduce_max_sync(0xffffffffu, mt);
+#pragma unroll
+  for (int d = 0; d < 3; ++d) mt[d] = __reduce_max_sync(0xffffffffu, mt[d]);
   mm = __reduce_max_sync(0xffffffffu, mm);
   mn = __reduce_min_sync(0xffffffffu, mn);
   mx = __reduce_max_sync(0xffffffffu, mx);
   nt = __reduce_min_sync(0xffffffffu, nt);
   nm = __reduce_min_sync(0xffffffffu, nm);
-  __shared__ unsigned sh[6];
-  if (threadIdx.x < 6) sh[threadIdx.x] = 0u;
+  const unsigned v[8] = {mt[0], mt[1], mt[2], mm, ~mn, mx, ~nt, ~nm};  // as LevelCtl::range
+  __shared__ unsigned sh[8];
+  if (threadIdx.x < 8) sh[threadIdx.x] = 0u;
   __syncthreads();
   if ((threadIdx.x & 31) == 0) {
-    atomicMax(&sh[0], mt);
-    atomicMax(&sh[1], mm);
-    atomicMax(&sh[2], ~mn);
-    atomicMax(&sh[3], mx);
-    atomicMax(&sh[4], ~nt);
-    atomicMax(&sh[5], ~nm);
+#pragma unroll
+    for (int i = 0; i < 8; ++i) atomicMax(&sh[i], v[i]);
   }
   __syncthreads();
-  if (threadIdx.x == 0) {
-    atomicMax(&ctl->mx_term, sh[0]);
-    atomicMax(&ctl->mx_mass, sh[1]);
-    atomicMax(&ctl->mn_bits, sh[2]);  // complemented: the control block starts as zeros
-    atomicMax(&ctl->mx_bits, sh[3]);
-    atomicMax(&ctl->mn_term, sh[4]);
-    atomicMax(&ctl->mn_mass, sh[5]);
-  }
+  if (threadIdx.x < 8) atomicMax(&ctl->range[threadIdx.x], sh[threadIdx.x]);
 }
 
 // The root, its chunks and the first level.  The launches that follow were made
@@ -962,7 +963,7 @@ __global__ void __launch_bounds__(256)
            int32_t *chunk_base, NodeAcc *acc, unsigned *ticket, int2 *roots, int32_t sub_max,
            bool wide, int32_t *err) {
   chain_enter();
-  const bool other = wide_range(*ctl) != wide;
+  const bool other = wide_range(ctl) != wide;
   const int32_t nc = chunks_of<PT>(int32_t(n));
   const bool sub = n <= sub_max;
   if (!sub)

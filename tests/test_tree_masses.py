@@ -118,3 +118,15 @@ def test_lists_with_massless_nodes(ctx, nd, tdpts, angle, share):
     """Nodes whose particles have no mass have no centre of mass (NaN): no test
     of a distance from it holds, the one that drops far nodes neither."""
     compare(ctx, *_massless(nd, share), lists=3, tdpts=tdpts, open_angle=angle)
+
+
+@pytest.mark.parametrize("axes", [(2,), (1, 2), (0,)])
+def test_flat_sets(ctx, axes):
+    """Axes a thousandth as long as the others: their terms, too, keep the bits
+    that decide the centres of mass (one in a few hundred nodes went to the
+    sequential sums)."""
+    n = 500_000
+    x = np.random.default_rng(4).random((n, 3)) * 100
+    x[:, axes] *= 1e-3
+    st = compare(ctx, x.astype(np.float32), np.ones(n), 64)
+    assert st["cm_fallbacks"] <= 5e-4 * st["nodes"]
