@@ -654,17 +654,27 @@ bool Solver::export_fields(float *rho, float *grad, bool to_host, cudaStream_t s
   return cu_ok(cudaStreamSynchronize(s), "pm export", err);
 }
 
+// Single precision: the largest grid whose adjoint solve runs beside the density's.
+// On small grids its transforms are kernels of 5 to 10 us that leave most of the
+// GPU idle (double precision fills the FP64 pipe with either): 1.3 M particles on
+// 100^3 cells 246 us one after the other, 203 side by side; 192^3 0.95 and 0.89 ms,
+// 384^3 7.60 and 7.48.  On larger ones the second set of grids, 20 bytes a cell and
+// a fifth of all, would buy a hundredth of the time.
+constexpr int kBesideGrid = 512;
+
 bool Solver::prepare_vjp(std::string *err) {
   const int ng = ng_, nh = ng / 2 + 1;
   const int64_t m = int64_t(ng) * ng * ng, mh = int64_t(ng) * ng * nh;
   if (!adj_ && !cu_ok(cudaMalloc(&adj_, 3 * m * sizeof(float)), "pm adjoint fields", err))
     return false;
   if (prec_ == PREC_F64) return true;  // the forward solve's own plans and grids
-  if (!aspec3_ && !cu_ok(cudaMalloc(&aspec3_, 3 * mh * sizeof(float2)), "pm adjoint spectra", err))
+  const bool beside = ng <= kBesideGrid;
+  if (beside && !aspec3_ &&
+      !cu_ok(cudaMalloc(&aspec3_, 3 * mh * sizeof(float2)), "pm adjoint spectra", err))
     return false;
-  if (!aspec_ && !cu_ok(cudaMalloc(&aspec_, mh * sizeof(float2)), "pm adjoint spectrum", err))
+  if (beside && !aspec_ && !cu_ok(cudaMalloc(&aspec_, mh * sizeof(float2)), "pm adjoint spectrum", err))
     return false;
-  if (!phibar_ && !cu_ok(cudaMalloc(&phibar_, m * sizeof(float)), "pm adjoint field", err))
+  if (beside && !phibar_ && !cu_ok(cudaMalloc(&phibar_, m * sizeof(float)), "pm adjoint field", err))
     return false;
   if (!aux_ && !cu_ok(cudaStreamCreateWithFlags(&aux_, cudaStreamNonBlocking), "pm adjoint stream", err))
     return false;
@@ -727,10 +737,26 @@ bool Solver::vjp(const Params &p, int64_t n, const float *x, const float *y, con
     return cu_ok(cudaGetLastError(), "pm adjoint kernels", err);
   }
   // Single precision: the density's solve and the cotangents' meet only at the
-  // particles, and their transforms are kernels of 5 to 10 us that leave most of
-  // the GPU idle, so the cotangents go on a second stream (double precision
-  // fills the FP64 pipe with either).  1.3 M particles on 100^3 cells: 246 us
-  // one after the other, 203 so.
+  // particles, and on grids up to kBesideGrid the cotangents go on a second stream
+  // with grids of their own; on larger ones they follow in the solve's grids.
+  const bool beside = ng <= kBesideGrid;
+  void *const spec3 = beside ? aspec3_ : gspec_, *const spec1 = beside ? aspec_ : spec_;
+  float *const phibar = beside ? phibar_ : rho_;
+  auto adjoint = [&](cudaStream_t st) {
+    if (!adj_deposit(st)) return false;
+    if (!fft_ok(cufftSetStream(fwd3_, st), "pm adjoint stream", err)) return false;
+    if (!fft_ok(cufftSetStream(inv1_, st), "pm adjoint stream", err)) return false;
+    if (!fft_ok(cufftExecR2C(fwd3_, (cufftReal *)adj_, (cufftComplex *)spec3),
+                "pm adjoint forward transform", err))
+      return false;
+    k_adj_spectra<<<blocks_for(mh), kThreads, 0, st>>>(ng, nh, (const float2 *)spec3,
+                                                       (const float *)green_, (const float *)gtab_,
+                                                       (float2 *)spec1);
+    ++launches;
+    if (!cu_ok(cudaGetLastError(), "pm adjoint spectra", err)) return false;
+    return fft_ok(cufftExecC2R(inv1_, (cufftComplex *)spec1, (cufftReal *)phibar),
+                  "pm adjoint inverse transform", err);
+  };
   struct Join {
     cudaStream_t aux;
     bool pending = false;
@@ -738,32 +764,23 @@ bool Solver::vjp(const Params &p, int64_t n, const float *x, const float *y, con
       if (pending) cudaStreamSynchronize(aux);
     }
   } join{aux_};
-  if (n > 0) {
+  if (n > 0 && beside) {
     if (!cu_ok(cudaEventRecord(ev_fork_, s), "pm adjoint fork", err)) return false;
     if (!cu_ok(cudaStreamWaitEvent(aux_, ev_fork_, 0), "pm adjoint fork", err)) return false;
     join.pending = true;
-    if (!adj_deposit(aux_)) return false;
-    if (!fft_ok(cufftSetStream(fwd3_, aux_), "pm adjoint stream", err)) return false;
-    if (!fft_ok(cufftSetStream(inv1_, aux_), "pm adjoint stream", err)) return false;
-    if (!fft_ok(cufftExecR2C(fwd3_, (cufftReal *)adj_, (cufftComplex *)aspec3_),
-                "pm adjoint forward transform", err))
-      return false;
-    k_adj_spectra<<<blocks_for(mh), kThreads, 0, aux_>>>(
-        ng, nh, (const float2 *)aspec3_, (const float *)green_, (const float *)gtab_,
-        (float2 *)aspec_);
-    ++launches;
-    if (!cu_ok(cudaGetLastError(), "pm adjoint spectra", err)) return false;
-    if (!fft_ok(cufftExecC2R(inv1_, (cufftComplex *)aspec_, (cufftReal *)phibar_),
-                "pm adjoint inverse transform", err))
-      return false;
+    if (!adjoint(aux_)) return false;
     if (!cu_ok(cudaEventRecord(ev_join_, aux_), "pm adjoint join", err)) return false;
   }
   if (!deposit(p, n, x, y, z, s, err) || !solve(s, err)) return false;
   if (n == 0) return true;
-  if (!cu_ok(cudaStreamWaitEvent(s, ev_join_, 0), "pm adjoint join", err)) return false;
-  join.pending = false;
+  if (beside) {
+    if (!cu_ok(cudaStreamWaitEvent(s, ev_join_, 0), "pm adjoint join", err)) return false;
+    join.pending = false;
+  } else if (!adjoint(s)) {
+    return false;
+  }
   k_vjp_interp<float><<<blocks_for(n), kThreads, 0, s>>>(n, x, y, z, vbx, vby, vbz, ng, p.ngo, nglt,
-                                                        grad_, phibar_, cm, coef, xbx, xby, xbz);
+                                                        grad_, phibar, cm, coef, xbx, xby, xbz);
   ++launches;
   fft_execs += 2;
   return cu_ok(cudaGetLastError(), "pm adjoint kernels", err);

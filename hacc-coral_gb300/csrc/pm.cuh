@@ -113,9 +113,9 @@ class Solver {
   cufftHandle fwd3_ = 0, inv1_ = 0;
   bool have_fwd3_ = false, have_inv1_ = false;
   float *adj_ = nullptr;     // 3 x ng^3: deposited cotangents (float atomics)
-  // single-precision adjoint: its transforms run on a stream of their own
-  // beside the forward solve's, with their own grids (spectra of the deposits,
-  // the combined spectrum, phibar)
+  // single-precision adjoint on grids that leave room on the GPU: its transforms
+  // run on a stream of their own beside the forward solve's, with their own grids
+  // (spectra of the deposits, the combined spectrum, phibar)
   cudaStream_t aux_ = nullptr;
   cudaEvent_t ev_fork_ = nullptr, ev_join_ = nullptr;
   void *aspec3_ = nullptr, *aspec_ = nullptr;
